@@ -162,6 +162,20 @@ static void host_twiddle(long m, long n, int sign, double* re, double* im) {
   *im = sign * si;
 }
 
+// exp(-2 pi i m / n) as two floats
+static void pair_twiddle(long m, long n, float* w) {
+  double re, im;
+  host_twiddle(m, n, -1, &re, &im);
+  w[0] = (float)re;
+  w[1] = (float)im;
+}
+
+static int ilog2(long n) {
+  int m = 0;
+  while ((1L << m) < n) ++m;
+  return m;
+}
+
 static int upload_real(pa_ctx* c, void* dst, const std::vector<double>& v) {
   if (c->fp64) {
     CK(cudaMemcpy(dst, v.data(), v.size() * 8, cudaMemcpyHostToDevice), "upload");
@@ -263,6 +277,7 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
   pa::Buffers& b = c->b;
   memset(&b, 0, sizeof(b));
   b.N = N;
+  b.NP = pa::pair_pad(N, s.nfftf);
   b.nfft = s.nfft;
   b.Ninterp = s.Ninterp;
   b.nfftf = s.nfftf;
@@ -309,7 +324,9 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
   ALLOC(b.shftf, sizeof(double) * nifo * (size_t)N);
   for (int k = 0; k < 2; k++) {
     if (c->fp64) ALLOC(b.ph0[k], 8 * nifo * (size_t)N);  // tmp1 (FP32 forms keep it in xm)
-    ALLOC(b.xm[k], 32 * nifo * (size_t)N);  // FP32: one 32-byte record; FP64: two double2
+    // FP32: data and phase terms, 16 bytes each; FP64: two double2
+    ALLOC(b.xm[k], 32 * nifo * (size_t)(c->fp64 ? N : b.NP));
+    CK(cudaMemset(b.xm[k], 0, 32 * nifo * (size_t)(c->fp64 ? N : b.NP)), "cudaMemset");
     ALLOC(b.sums[k], sizeof(double) * 8);
     ALLOC(b.sums_r[k], sizeof(double) * 4);
   }
@@ -344,26 +361,36 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
   }
   CK(cudaMemcpy((void*)b.spline_invp, invp, sizeof(invp), cudaMemcpyHostToDevice), "upload spline");
   CK(cudaMemcpy((void*)b.spline_p, p, sizeof(p), cudaMemcpyHostToDevice), "upload spline");
-  if ((rc = make_twiddles(c, s.nfft, -1, &c->tw_fwd))) return rc;
   if ((rc = make_twiddles(c, s.Ninterp, +1, &c->tw_inv))) return rc;
-  if ((rc = make_twiddles(c, s.nfft, +1, &c->tw_invh))) return rc;
-  if ((rc = make_twiddles(c, s.nfftf, -1, &c->tw_main))) return rc;
-  if (!c->fp64) {  // inter-pass twiddle tables of the spindown transform, per split
-    const long L = s.nfftf;
-    int lg = 0;
-    while ((1L << lg) < L) ++lg;
-    for (int sp = 0; sp < 2; sp++) {
-      if (sp == 1 && !(lg & 1)) {
-        b.tw_pass[1] = b.tw_pass[0];
+  if (c->fp64) {
+    if ((rc = make_twiddles(c, s.nfft, -1, &c->tw_fwd))) return rc;
+    if ((rc = make_twiddles(c, s.nfft, +1, &c->tw_invh))) return rc;
+    if ((rc = make_twiddles(c, s.nfftf, -1, &c->tw_main))) return rc;
+  } else {
+    const int lens[2] = {s.nfft, s.nfftf};
+    std::vector<float> v(512);
+    auto up = [&](const void** dst) -> int {
+      void* p = nullptr;
+      if (int r = dalloc(c, &p, v.size() * sizeof(float))) return r;
+      CK(cudaMemcpy(p, v.data(), v.size() * sizeof(float), cudaMemcpyHostToDevice), "upload");
+      *dst = p;
+      return PA_OK;
+    };
+    for (int m = 0; m < 256; m++) pair_twiddle(m, 256, &v[2 * m]);
+    if ((rc = up(&b.pair_tw1))) return rc;
+    for (int t = 0; t < 2; t++) {
+      if (t == 1 && s.nfftf == s.nfft) {
+        b.pair_row[1] = b.pair_row[0];
+        b.pair_pass[1] = b.pair_pass[0];
         break;
       }
-      const int l1 = pa::pass_logl1(lg, sp);
-      std::vector<double> v(2 * (size_t)L);
-      for (long j = 0; j < L; j++) host_twiddle(pa::tw_pass_exp(j, L, l1), L, -1, &v[2 * j], &v[2 * j + 1]);
-      void* p = nullptr;
-      if ((rc = dalloc(c, &p, v.size() * c->rsz))) return rc;
-      if ((rc = upload_real(c, p, v))) return rc;
-      b.tw_pass[sp] = p;
+      const int lg = ilog2(lens[t]);
+      v.resize(2 * (size_t)pa::pair_row_table(lg));
+      for (int j = 0; j < pa::pair_row_table(lg); j++) pair_twiddle(pa::pair_row_exp(j, lg), lens[t] / 256, &v[2 * j]);
+      if ((rc = up(&b.pair_row[t]))) return rc;
+      v.resize(2 * (size_t)lens[t]);
+      for (long j = 0; j < lens[t]; j++) pair_twiddle(pa::pair_pass_exp(j, lg), lens[t], &v[2 * j]);
+      if ((rc = up(&b.pair_pass[t]))) return rc;
     }
   }
   for (int k = 0; k < 4; k++) {
@@ -376,9 +403,6 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
   c->eng = c->fp64 ? pa::make_engine_f64(b) : pa::make_engine_f32(b, c->cfg.phase_mode);
   if (!c->eng) return fail(c, PA_ERR_NOMEM, "engine allocation failed");
   c->eng->prof = &c->prof;
-  // default factor split: for two detectors in the FP32 forms, the one with
-  // 256-point columns (the radix-16 spindown pass A): swapped for nfftf = 2^17
-  if (!c->fp64 && nifo == 2 && s.nfftf == (1 << 17)) c->eng->set_split(1);
   CK(cudaEventCreate(&c->ev0), "cudaEventCreate");
   CK(cudaEventCreate(&c->ev1), "cudaEventCreate");
   CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming), "cudaEventCreate");
@@ -1033,8 +1057,8 @@ int pa_autotune(pa_ctx* c, const pa_sky* tasks, int ntasks, const pa_opts* o, co
   // buffers, two lanes with a quarter or half each
   const int m = c->sb_max;
   const int cands[6][2] = {{1, m / 4}, {1, m / 2}, {1, 3 * m / 4}, {1, m}, {2, m / 4}, {2, m / 2}};
-  // the factor split is a choice only for odd log2(nfftf)
-  const int nsplit = (c->sett.nfftf & 0xAAAAAAAA) ? 2 : 1;
+  // the factor split is a choice only in the FP64 form and for odd log2(nfftf)
+  const int nsplit = c->fp64 && (c->sett.nfftf & 0xAAAAAAAA) ? 2 : 1;
   double best = 1e300;
   int bsb = sb0, bsp = sp0, bln = ln0;
   std::vector<pa::DevCand> out;
@@ -1087,18 +1111,16 @@ int pa_debug_prelude(pa_ctx* c, int pm, int mm, int nn, double* xa, double* xb, 
   CK(cudaStreamSynchronize(c->stream), "sync");
   cudaError_t e = c->eng->prelude(sky_args(c, h, 0), 0, c->stream_pre);
   if (e != cudaSuccess) return cuda_fail(c, e, "prelude");
-  const size_t n = (size_t)c->nifo * 2 * c->sett.N;
-  std::vector<char> buf(n * 2 * 8);  // FP64 pairs or 32-byte FP32 records
+  const size_t n = (size_t)c->nifo * (c->fp64 ? c->sett.N : c->b.NP);
+  std::vector<char> buf(n * 4 * c->rsz);
   double sums[4];
   CK(cudaMemcpyAsync(buf.data(), c->b.xm[0], buf.size(), cudaMemcpyDeviceToHost, c->stream_pre), "copy");
   CK(cudaMemcpyAsync(sums, c->b.sums[0], sizeof(sums), cudaMemcpyDeviceToHost, c->stream_pre), "copy");
   CK(cudaStreamSynchronize(c->stream_pre), "prelude");
   const int N = c->sett.N;
-  const int sw = c->eng->swapped_det();
   for (int d = 0; d < c->nifo; d++)
     for (int arr = 0; arr < 2; arr++) {
       double* dst = arr == 0 ? xa : xb;
-      const int half = d == sw ? 1 - arr : arr;  // {xb, xa} records
       if (!dst) continue;
       for (int i = 0; i < N; i++) {
         double re, im;
@@ -1107,10 +1129,10 @@ int pa_debug_prelude(pa_ctx* c, int pm, int mm, int nn, double* xa, double* xb, 
           re = ((double*)buf.data())[2 * src];
           im = ((double*)buf.data())[2 * src + 1];
         } else {
-          // 32-byte records {xa.re, xa.im, xb.re, xb.im | phase terms}
-          const size_t src = 8 * ((size_t)d * N + i) + 2 * half;
+          // {a.re, b.re, a.im, b.im}
+          const size_t src = 4 * ((size_t)d * c->b.NP + i) + arr;
           re = ((float*)buf.data())[src];
-          im = ((float*)buf.data())[src + 1];
+          im = ((float*)buf.data())[src + 2];
         }
         dst[2 * ((size_t)d * N + i)] = re;
         dst[2 * ((size_t)d * N + i) + 1] = im;
@@ -1236,13 +1258,10 @@ struct NoAllocExit {
   }
 };
 alignas(64) unsigned char g_noalloc_engine_mem[4096];
-// host staging: the largest twiddle set (tw1 + tw2 + 1024 + L/1024 complex
-// doubles for L <= 2^16) and one real array of N floats
-double g_noalloc_tw[2 * (256 + 256 + 1024 + 64)];
-float g_noalloc_tw_f[2 * (256 + 256 + 1024 + 64)];
+// host staging: the largest twiddle table, one real array of N floats
+float g_noalloc_tw[2 * kNoAllocMaxNfftf];
 float g_noalloc_real[kNoAllocMaxN];
 float g_noalloc_F[kNoAllocMaxNfftf];
-float g_noalloc_tw_pass[2 * kNoAllocMaxNfftf];  // host staging of Buffers::tw_pass
 
 // 256-byte aligned bump layout inside the scratch array
 struct Bump {
@@ -1268,7 +1287,7 @@ int noalloc_fail(int code, const char* fmt, ...) {
 
 // Lays the buffers of one search out in the scratch (or only sizes them
 // when base == nullptr); returns the bytes used.
-size_t noalloc_layout(char* base, const pa_settings& s, int nifo, pa::Buffers* b, void* tw[4][4], void** Fn) {
+size_t noalloc_layout(char* base, const pa_settings& s, int nifo, pa::Buffers* b, void** Fn) {
   Bump m{base};
   const size_t N = s.N, cs = 8;
   const int bins = s.nmax - s.nmin;
@@ -1286,7 +1305,8 @@ size_t noalloc_layout(char* base, const pa_settings& s, int nifo, pa::Buffers* b
   b->u = (double*)m.take(16 * nifo * 2 * 2 * N);
   b->y2 = m.take(cs * nifo * 2 * 2 * N);
   b->shftf = (double*)m.take(8 * nifo * N);
-  b->xm[0] = b->xm[1] = m.take(32 * nifo * N);  // 32-byte records
+  b->NP = pa::pair_pad(s.N, s.nfftf);
+  b->xm[0] = b->xm[1] = m.take(32 * nifo * (size_t)b->NP);
   b->sums[0] = b->sums[1] = (double*)m.take(8 * 8);
   b->sums_r[0] = b->sums_r[1] = m.take(8 * 4);
   b->part = (double*)m.take(8 * 2 * nifo * ((N + 255) / 256));
@@ -1298,15 +1318,13 @@ size_t noalloc_layout(char* base, const pa_settings& s, int nifo, pa::Buffers* b
   *Fn = m.take(4 * (size_t)bins);  // normalised F (the output)
   b->cand = (pa::DevCand*)m.take(sizeof(pa::DevCand) * kNoAllocCandCap);
   b->ncand = (int*)m.take(16);
-  b->tw_pass[0] = m.take(cs * (size_t)s.nfftf);
-  b->tw_pass[1] = m.take(cs * (size_t)s.nfftf);
-  const int lens[4] = {s.nfft, s.Ninterp, s.nfftf, s.nfft};
-  for (int t = 0; t < 4; t++) {
-    int lg = 0;
-    while ((1 << lg) < lens[t]) ++lg;
-    const int n4[4] = {1 << ((lg + 1) / 2), 1 << (lg / 2), 1024, lens[t] / 1024};
-    for (int k = 0; k < 4; k++) tw[t][k] = m.take(cs * (size_t)n4[k]);
+  b->pair_tw1 = m.take(cs * 256);
+  for (int t = 0; t < 2; t++) {
+    const int L = t ? s.nfftf : s.nfft;
+    b->pair_row[t] = m.take(cs * (size_t)pa::pair_row_table(ilog2(L)));
+    b->pair_pass[t] = m.take(cs * (size_t)L);
   }
+  for (int k = 2; k < 4; k++) b->tw_inv[k] = m.take(cs * (size_t)(k == 2 ? 1024 : s.Ninterp / 1024));
   b->N = s.N;
   b->nfft = s.nfft;
   b->Ninterp = s.Ninterp;
@@ -1320,39 +1338,20 @@ size_t noalloc_layout(char* base, const pa_settings& s, int nifo, pa::Buffers* b
   b->sbatch = 1;
   b->lane_sb = 1;
   b->cand_cap = kNoAllocCandCap;
-  for (int k = 0; k < 4; k++) {
-    b->tw_fwd[k] = tw[0][k];
-    b->tw_inv[k] = tw[1][k];
-    b->tw_main[k] = tw[2][k];
-    b->tw_invh[k] = tw[3][k];
-  }
   return m.off;
 }
 
-// Twiddle tables of length L and sign into the device pointers t[0..3],
-// through the static host staging arrays.
-cudaError_t noalloc_twiddles(int L, int sign, void* const* t, cudaStream_t st) {
-  int lg = 0;
-  while ((1 << lg) < L) ++lg;
-  const int L1 = 1 << ((lg + 1) / 2), L2 = 1 << (lg / 2);
-  const int lens[4] = {L1, L2, 1024, L / 1024};
-  for (int k = 0; k < 4; k++) {
-    for (int j = 0; j < lens[k]; j++) {
-      long num, den;
-      if (k == 0) { num = j; den = L1; }
-      else if (k == 1) { num = j; den = L2; }
-      else if (k == 2) { num = j; den = L; }
-      else { num = (long)j * 1024; den = L; }
-      host_twiddle(num, den, sign, &g_noalloc_tw[2 * j], &g_noalloc_tw[2 * j + 1]);
-      g_noalloc_tw_f[2 * j] = (float)g_noalloc_tw[2 * j];
-      g_noalloc_tw_f[2 * j + 1] = (float)g_noalloc_tw[2 * j + 1];
-    }
-    cudaError_t e = cudaMemcpyAsync(t[k], g_noalloc_tw_f, sizeof(float) * 2 * lens[k], cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(st);  // the staging array is reused
-    if (e != cudaSuccess) return e;
+// n twiddles exp(-2 pi i m(j) / den) (conjugated for sign > 0) to device
+// memory, through the static host staging array.
+template <class Exp>
+cudaError_t noalloc_twiddles(const void* dst, long n, long den, int sign, cudaStream_t st, Exp m) {
+  for (long j = 0; j < n; j++) {
+    pair_twiddle(m(j), den, &g_noalloc_tw[2 * j]);
+    if (sign > 0) g_noalloc_tw[2 * j + 1] = -g_noalloc_tw[2 * j + 1];
   }
-  return cudaSuccess;
+  cudaError_t e = cudaMemcpyAsync((void*)dst, g_noalloc_tw, sizeof(float) * 2 * n, cudaMemcpyHostToDevice, st);
+  if (e != cudaSuccess) return e;
+  return cudaStreamSynchronize(st);  // the staging array is reused
 }
 
 }  // namespace
@@ -1380,9 +1379,8 @@ extern "C" int pa_fstat_noalloc(const pa_settings* sett, const pa_detector* det,
   if (device < 0 || device >= kNoAllocMaxDevices || device >= pa_device_count())
     return noalloc_fail(PA_ERR_NODEV, "pa_fstat_noalloc: no CUDA device %d", device);
   pa::Buffers b;
-  void* tw[4][4];
   void* Fn = nullptr;
-  const size_t need = noalloc_layout(nullptr, *sett, nifo, &b, tw, &Fn);
+  const size_t need = noalloc_layout(nullptr, *sett, nifo, &b, &Fn);
   if (need > kNoAllocBytes)
     return noalloc_fail(PA_ERR_ARG, "pa_fstat_noalloc: needs %zu bytes of scratch, the array holds %zu", need,
                         kNoAllocBytes);
@@ -1406,7 +1404,7 @@ extern "C" int pa_fstat_noalloc(const pa_settings* sett, const pa_detector* det,
     g_noalloc_dev_ptr[device] = ptr;
     g_noalloc_ctx_id[device] = ctx_id;
   }
-  noalloc_layout((char*)g_noalloc_dev_ptr[device], *sett, nifo, &b, tw, &Fn);
+  noalloc_layout((char*)g_noalloc_dev_ptr[device], *sett, nifo, &b, &Fn);
 
   // host-side scalars of the sky point, as job_core computes them
   pa_ctx c;
@@ -1451,28 +1449,20 @@ extern "C" int pa_fstat_noalloc(const pa_settings* sett, const pa_detector* det,
   }
   NCK(cudaMemcpyAsync((void*)b.spline_invp, invp, sizeof(invp), cudaMemcpyHostToDevice, st), "upload");
   NCK(cudaMemcpyAsync((void*)b.spline_p, p, sizeof(p), cudaMemcpyHostToDevice, st), "upload");
-  NCK(noalloc_twiddles(sett->nfft, -1, tw[0], st), "twiddles");
-  NCK(noalloc_twiddles(sett->Ninterp, +1, tw[1], st), "twiddles");
-  NCK(noalloc_twiddles(sett->nfftf, -1, tw[2], st), "twiddles");
-  NCK(noalloc_twiddles(sett->nfft, +1, tw[3], st), "twiddles");
-  for (int sp = 0; sp < 2; sp++) {
-    const long L = sett->nfftf;
-    int lg = 0;
-    while ((1L << lg) < L) ++lg;
-    const int l1 = pa::pass_logl1(lg, sp);
-    for (long j = 0; j < L; j++) {
-      double re, im;
-      host_twiddle(pa::tw_pass_exp(j, L, l1), L, -1, &re, &im);
-      g_noalloc_tw_pass[2 * j] = (float)re;
-      g_noalloc_tw_pass[2 * j + 1] = (float)im;
-    }
-    NCK(cudaMemcpyAsync((void*)b.tw_pass[sp], g_noalloc_tw_pass, sizeof(float) * 2 * L, cudaMemcpyHostToDevice,
-                        st), "twiddles");
-    NCK(cudaStreamSynchronize(st), "twiddles");  // the staging array is reused
+  NCK(noalloc_twiddles(b.pair_tw1, 256, 256, -1, st, [](long j) { return j; }), "twiddles");
+  NCK(noalloc_twiddles(b.tw_inv[2], 1024, sett->Ninterp, +1, st, [](long j) { return j; }), "twiddles");
+  NCK(noalloc_twiddles(b.tw_inv[3], sett->Ninterp / 1024, sett->Ninterp, +1, st, [](long j) { return 1024 * j; }),
+      "twiddles");
+  for (int t = 0; t < 2; t++) {
+    const int L = t ? sett->nfftf : sett->nfft, lg = ilog2(L);
+    NCK(noalloc_twiddles(b.pair_row[t], pa::pair_row_table(lg), L / 256, -1, st,
+                         [&](long j) { return pa::pair_row_exp((int)j, lg); }), "twiddles");
+    NCK(noalloc_twiddles(b.pair_pass[t], L, L, -1, st, [&](long j) { return pa::pair_pass_exp(j, lg); }), "twiddles");
   }
   // what must start at zero
   NCK(cudaMemsetAsync(b.counter, 0, 16, st), "memset");
   NCK(cudaMemsetAsync(b.ncand, 0, 16, st), "memset");
+  NCK(cudaMemsetAsync(b.xm[0], 0, 32 * nifo * (size_t)b.NP, st), "memset");
 
   pa::Engine* eng = pa::make_engine_f32_fixed_at(g_noalloc_engine_mem, sizeof(g_noalloc_engine_mem), b);
   if (!eng) return noalloc_fail(PA_ERR_NOMEM, "pa_fstat_noalloc: engine storage too small");

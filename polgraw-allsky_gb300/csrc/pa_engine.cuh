@@ -25,6 +25,7 @@
 
 #include "pa_engine.h"
 #include "pa_fft.cuh"
+#include "pa_pair.cuh"
 
 namespace pa {
 
@@ -90,7 +91,7 @@ template <typename R, int PM>
 __global__ void __launch_bounds__(256)
     k_prelude_mod(const double* __restrict__ xDat, const double* __restrict__ DetSSB,
                   const R* __restrict__ cosmodf, const R* __restrict__ sinmodf,
-                  const DetConst* __restrict__ dc, const SkyArgs sky, int N,
+                  const DetConst* __restrict__ dc, const SkyArgs sky, int N, int NP,
                   typename CT<R>::T* __restrict__ xin, double* __restrict__ shftf, void* ph0,
                   double* __restrict__ part, double* __restrict__ sums, R* __restrict__ sums_r,
                   unsigned int* __restrict__ counter) {
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(256)
     b2r = bb * bb;
     // shft, shftf, _tmp1 (jobcore.c:285-295)
     const double* D = DetSSB + 3 * ((size_t)d * N + i);
-    const size_t o = (size_t)d * N + i;
+    const size_t o = (size_t)d * N + i, op = (size_t)d * NP + i;
     const double di = (double)i;
     R sp, cp;
     if (sizeof(R) == 8) {
@@ -164,27 +165,22 @@ __global__ void __launch_bounds__(256)
       // 2 i shft, the non-integer part of _tmp1 = i^2 + 2 i shft
       const double p2 = __dmul_rn(di + di, shft);
       const uint64_t ii2 = (uint64_t)i * (uint64_t)i;
-      // the phase coefficients fill the upper half of the sample's 32-byte
-      // record (the resampled data fill the lower half)
-      uint4 hi16;
       if (PM == PM_FIXED) {
         // spindown phase s1(ss) tmp1 = s1(ss_base) tmp1 + (ss - ss_base) (M5 tmp1)
         // as 64-bit fixed-point turns: the i^2 part exactly in integers from
         // the fixed-point coefficients, the 2 i shft part from its FP64 value
         const uint64_t A = sky.s1f * ii2 + turns_fixed(sky.s1_0 * p2);
         const uint64_t B = sky.m5f * ii2 + turns_fixed(sky.M5 * p2);
-        hi16 = make_uint4((unsigned)A, (unsigned)(A >> 32), (unsigned)B, (unsigned)(B >> 32));
+        reinterpret_cast<uint4*>(ph0)[op] = make_uint4((unsigned)A, (unsigned)(A >> 32), (unsigned)B, (unsigned)(B >> 32));
       } else {
         const double tmp1 = (double)ii2 + p2;
         if (PM == PM_FF) {
           const float hi = (float)tmp1;
-          hi16 = make_uint4(__float_as_uint(hi), __float_as_uint((float)(tmp1 - (double)hi)), 0u, 0u);
+          reinterpret_cast<float2*>(ph0)[op] = make_float2(hi, (float)(tmp1 - (double)hi));
         } else {
-          const unsigned long long tb = (unsigned long long)__double_as_longlong(tmp1);
-          hi16 = make_uint4((unsigned)tb, (unsigned)(tb >> 32), 0u, 0u);
+          reinterpret_cast<double*>(ph0)[op] = tmp1;
         }
       }
-      reinterpret_cast<uint4*>(ph0)[2 * o + 1] = hi16;
       // prelude phase het0 i + oms shft (jobcore.c:299) in fixed-point
       // turns: het0/2pi exactly in integers, oms shft/2pi from its FP64 value
       const uint64_t t = sky.h0f * (uint64_t)i + turns_fixed(sky.oms_t * shft);
@@ -257,15 +253,13 @@ __global__ void __launch_bounds__(256)
 // ------------------------------------------------------------------
 // FFT loaders / storers
 
+// The zero-padded input of a transform.
 template <typename R> struct PlainLoader {
   typedef typename CT<R>::T T;
   static constexpr int kTraceKind = KK_FFT_FWD_A;
-  static constexpr bool kEarlyLoads = true;  // no prologue: loads before any barrier
-  static constexpr bool kTwiddleTable = false;
   const T* in;   // [batch][2][ld]
   int len, ld;
-  __device__ __forceinline__ void prologue(int, char*) const {}
-  __device__ __forceinline__ void load2(int batch, int n, T& a, T& b, const char*) const {
+  __device__ __forceinline__ void load2(int batch, int n, T& a, T& b) const {
     if (n < len) {
       a = in[((size_t)batch * 2 + 0) * ld + n];
       b = in[((size_t)batch * 2 + 1) * ld + n];
@@ -273,6 +267,32 @@ template <typename R> struct PlainLoader {
       a = b = mk((R)0, (R)0);
     }
   }
+  // the FP32 passes' interface (pa_pair.cuh)
+  template <int NIN, int NCHK> struct Ahead {
+    static constexpr int v = 4;
+  };
+  struct Ctx {
+    const float2 *a, *b;
+    int left;
+  };
+  struct Raw {
+    float2 a, b;
+  };
+  __device__ __forceinline__ int count() const { return len; }
+  __device__ __forceinline__ Ctx begin(int batch, int n0, int) const {
+    const float2* p = in + (size_t)batch * 2 * ld + n0;
+    return Ctx{p, p + ld, len - n0};
+  }
+  __device__ __forceinline__ void next(Ctx&) const {}
+  __device__ __forceinline__ Raw fetch(const Ctx& k, int off) const {
+    Raw r = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    if (off < k.left) {
+      r.a = k.a[off];
+      r.b = k.b[off];
+    }
+    return r;
+  }
+  __device__ __forceinline__ P2 value(const Ctx&, const Raw& r, int) const { return P2{pk(r.a.x, r.b.x), pk(r.a.y, r.b.y)}; }
 };
 
 // The interpolating inverse transform of jobcore.c:338-362 at half length.
@@ -288,26 +308,40 @@ template <typename R> struct PlainLoader {
 template <typename R> struct HalfShiftLoader {
   typedef typename CT<R>::T T;
   static constexpr int kTraceKind = KK_FFT_INV_A;
-  static constexpr bool kEarlyLoads = true;  // no prologue: loads before any barrier
-  static constexpr bool kTwiddleTable = false;
   const T* spec;    // [batch][2][nfft]
   const T* twlo;    // e^{+2 pi i m/Ninterp}, m < 1024
   const T* twhi;    // e^{+2 pi i 1024 m/Ninterp}
   int nfft, nyqst;
-  __device__ __forceinline__ void prologue(int, char*) const {}
-  __device__ __forceinline__ void load2(int batch, int j, T& a, T& b, const char*) const {
-    const T w0 = cmul(__ldg(&twlo[j & 1023]), __ldg(&twhi[j >> 10]));
-    const T w = j < nyqst ? w0 : mk(-w0.x, -w0.y);
+  __device__ __forceinline__ T phase(int j) const {
+    const T w = cmul(__ldg(&twlo[j & 1023]), __ldg(&twhi[j >> 10]));
+    return j < nyqst ? w : mk(-w.x, -w.y);
+  }
+  __device__ __forceinline__ void load2(int batch, int j, T& a, T& b) const {
+    const T w = phase(j);
     a = cmul(spec[((size_t)batch * 2 + 0) * nfft + j], w);
     b = cmul(spec[((size_t)batch * 2 + 1) * nfft + j], w);
   }
-};
-
-struct SpinCta {
-  double het1, s1;
-  uint64_t H;
-  unsigned ssr;  // ss - ss_base (>= 0), fixed-point form
-  float s1h, s1l, h1h, h1l;
+  // the FP32 passes' interface (pa_pair.cuh)
+  template <int NIN, int NCHK> struct Ahead {
+    static constexpr int v = 4;
+  };
+  struct Ctx {
+    const float2 *a, *b;
+    int n0;
+  };
+  struct Raw {
+    float2 a, b, w;
+  };
+  __device__ __forceinline__ int count() const { return nfft; }
+  __device__ __forceinline__ Ctx begin(int batch, int n0, int) const {
+    const float2* p = spec + (size_t)batch * 2 * nfft + n0;
+    return Ctx{p, p + nfft, n0};
+  }
+  __device__ __forceinline__ void next(Ctx&) const {}
+  __device__ __forceinline__ Raw fetch(const Ctx& k, int off) const { return Raw{k.a[off], k.b[off], phase(k.n0 + off)}; }
+  __device__ __forceinline__ P2 value(const Ctx&, const Raw& r, int) const {
+    return pmul(P2{pk(r.a.x, r.b.x), pk(r.a.y, r.b.y)}, r.w);
+  }
 };
 
 // Most spindowns in one launch of the spindown passes (the buffers are sized
@@ -334,17 +368,37 @@ inline uint64_t het1_turns_fixed(int ss, double M4, double M0) {
   return r;
 }
 
-// Per-launch spindown constants passed by value with the loader.  The
-// fixed-point form takes the het1 term of each batch item from the host
-// (H[batch]), so that no CTA of pass A waits on a chain of FP64 operations
-// before its first phase; the other forms form theirs per CTA (prologue).
-template <typename R, int PM> struct SpinHet {
-  static constexpr bool kHost = false;
+// Per-launch spindown constants of each batch item, formed on the host and
+// passed by value with the loader, so that no CTA of pass A waits on a chain
+// of FP64 operations before its first phase.  het1 = fmod(ss M4, M0) wrapped
+// (jobcore.c:466-467), s1 = ss M5 + s1_0 (one rounding).
+template <int PM> struct SpinHet {  // FP64 phase: the FP64 form and PM_F64
+  double het1[kSpinBatchMax], s1[kSpinBatchMax];
 };
-template <> struct SpinHet<float, PM_FIXED> {
-  static constexpr bool kHost = true;
-  unsigned long long H[kSpinBatchMax];
+template <> struct SpinHet<PM_FIXED> {
+  unsigned long long H[kSpinBatchMax];  // het1 as 64-bit fixed-point turns
 };
+template <> struct SpinHet<PM_FF> {
+  float4 c[kSpinBatchMax];  // s1 and het1 as two floats each
+};
+
+inline void spin_het_fill(SpinHet<PM_FIXED>& h, int k, int ss, const SkyArgs& sky, int) {
+  h.H[k] = het1_turns_fixed(ss, sky.M4, sky.M0);
+}
+inline void spin_het1_s1(int ss, const SkyArgs& sky, int s0_flag, double* het1, double* s1) {
+  *het1 = fmod(ss * sky.M4, sky.M0);
+  if (*het1 < 0) *het1 += sky.M0;
+  *s1 = s0_flag ? 0. : fma((double)ss, sky.M5, sky.s1_0);
+}
+inline void spin_het_fill(SpinHet<PM_F64>& h, int k, int ss, const SkyArgs& sky, int s0_flag) {
+  spin_het1_s1(ss, sky, s0_flag, &h.het1[k], &h.s1[k]);
+}
+inline void spin_het_fill(SpinHet<PM_FF>& h, int k, int ss, const SkyArgs& sky, int s0_flag) {
+  double het1, s1;
+  spin_het1_s1(ss, sky, s0_flag, &het1, &s1);
+  const float s1h = (float)s1, h1h = (float)het1;
+  h.c[k] = make_float4(s1h, (float)(s1 - (double)s1h), h1h, (float)(het1 - (double)h1h));
+}
 
 // (a * b) mod 2^64 for a 64-bit a and a 32-bit b
 __device__ __forceinline__ uint64_t mul64x32(uint64_t a, unsigned b) {
@@ -353,198 +407,142 @@ __device__ __forceinline__ uint64_t mul64x32(uint64_t a, unsigned b) {
 
 // Phase-modulated detector sum of the spindown loop (jobcore.c:455-623):
 //   x_{a,b}[n] = sum_d xm_{a,b,d}[n] exp(-i (het1 n + s1 tmp1_d[n]))  (n < N)
-template <typename R, int PM> struct SpinLoader {
-  typedef typename CT<R>::T T;
+// FP64 form:
+struct SpinLoader64 {
   static constexpr int kTraceKind = KK_SPIN_A;
-  // the fixed-point form needs no shared-memory constants (no barrier after
-  // the prologue)
-  static constexpr bool kPrologue = !SpinHet<R, PM>::kHost;
-  // generic pass A: first loads before any barrier (no prologue to wait for)
-  static constexpr bool kEarlyLoads = !kPrologue;
-  // generic pass A: inter-pass twiddles from Buffers::tw_pass (FP32 forms)
-  static constexpr bool kTwiddleTable = sizeof(R) == 4;
-  const T* xm;       // [nifo][2][N]
-  const void* ph0;   // FP64 form: tmp1 [nifo][N]; FP32 forms: unused
-  int N, nifo, ss0, ss_base, s0_flag;
-  double M0, M4, M5, s1_0;
-  SpinHet<R, PM> het;
+  const double2* xm;   // [nifo][2][N]
+  const double* tmp1;  // [nifo][N]
+  int N, nifo;
+  SpinHet<PM_F64> het;
 
-  // Spindown constants of batch item `batch`: the fixed-point form's from
-  // the launch parameters (registers), the other forms' from the prologue's
-  // shared-memory copy.
-  __device__ __forceinline__ SpinCta consts(int batch, const char* sm) const {
-    SpinCta k;
-    if constexpr (SpinHet<R, PM>::kHost) {
-      k.H = het.H[batch];
-      k.ssr = s0_flag ? 0u : (unsigned)(ss0 + batch - ss_base);
+  __device__ __forceinline__ void load2(int batch, int n, double2& va, double2& vb) const {
+    va = vb = mk(0., 0.);
+    if (n >= N) return;
+    const double het1 = het.het1[batch], s1 = het.s1[batch];
+    for (int d = 0; d < nifo; ++d) {
+      const double2 xa = xm[((size_t)d * 2 + 0) * N + n], xb = xm[((size_t)d * 2 + 1) * N + n];
+      // het1*i + s1*_tmp1 with the reference's rounding (jobcore.c:606)
+      const double ph = __dadd_rn(__dmul_rn(het1, (double)n), __dmul_rn(s1, tmp1[(size_t)d * N + n]));
+      double sn, cs;
+      sincos(ph, &sn, &cs);
+      // x * (cos - i sin)
+      va.x += xa.x * cs + xa.y * sn;
+      va.y += xa.y * cs - xa.x * sn;
+      vb.x += xb.x * cs + xb.y * sn;
+      vb.y += xb.y * cs - xb.x * sn;
+    }
+  }
+};
+
+// FP32 forms (pa_pair.cuh).  The data xm and the phase terms lie in two
+// arrays of 16 (or 8) bytes per detector and sample, so that each load of a
+// warp reads whole 128-byte lines; a thread takes all detectors of its
+// position, one sine and cosine each for both arrays.  The arrays have zeros
+// behind the N samples (stride NP), so that the lanes of a warp that reaches
+// the last row need no condition of their own.  NIFO: the number of
+// detectors (0: any, without loads ahead).
+template <int PM> struct SpinTerm {
+  typedef uint2 T;  // FP64 phase: tmp1; two-float phase: float2
+};
+template <> struct SpinTerm<PM_FIXED> {
+  typedef uint4 T;  // A, B
+};
+template <int PM, int NIFO> struct SpinLoader {
+  static constexpr int kTraceKind = KK_SPIN_A;
+  typedef typename SpinTerm<PM>::T Term;
+  static constexpr int ND = NIFO ? NIFO : 1;
+  static constexpr bool kQuarters = NIFO > 0;
+  // positions loaded ahead: as many as the 128 registers of a thread hold
+  // beside the NIN values
+  template <int NIN, int NCHK> struct Ahead {
+    static constexpr int v =
+        NIFO == 0 ? 0 : (NIFO == 1 ? 4 : (NIFO == 2 ? (NIN < 16 ? 3 : 1) : (NIN < 16 || NCHK > 0 ? 1 : 0)));
+  };
+  const float4* xm;  // [nifo][NP] {a.re, b.re, a.im, b.im}
+  const Term* ph;    // [nifo][NP]
+  int N, NP, nifo, ss_rel, s0_flag;  // ss_rel: first spindown of the launch less ss_base
+  SpinHet<PM> het;
+
+  struct Ctx {
+    const float4* x[ND];
+    const Term* p[ND];
+    unsigned long long hn, hstep;  // fixed point: H n, and H times the step of n
+    unsigned ssr;                  // spindown less ss_base
+    int n0;
+    double het1, s1;
+    float4 c;
+  };
+  struct Raw {
+    float4 x[ND];
+    Term p[ND];
+  };
+
+  __device__ __forceinline__ int count() const { return N; }
+  __device__ __forceinline__ Ctx begin(int batch, int n0, int step) const {
+    Ctx k;
+    k.n0 = n0;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      k.x[d] = xm + (size_t)d * NP + n0;
+      k.p[d] = ph + (size_t)d * NP + n0;
+    }
+    if constexpr (PM == PM_FIXED) {
+      const unsigned long long H = het.H[batch];
+      k.hn = mul64x32(H, (unsigned)n0);
+      k.hstep = mul64x32(H, (unsigned)step);
+      k.ssr = s0_flag ? 0u : (unsigned)(ss_rel + batch);
+    } else if constexpr (PM == PM_F64) {
+      k.het1 = het.het1[batch];
+      k.s1 = het.s1[batch];
     } else {
-      k = *reinterpret_cast<const SpinCta*>(sm);
+      k.c = het.c[batch];
     }
     return k;
   }
-
-  __device__ __forceinline__ void prologue(int batch, char* sm) const {
-    if (kPrologue && threadIdx.x == 0) {
-      SpinCta* p = reinterpret_cast<SpinCta*>(sm);
-      const int ss = ss0 + batch;
-      double het1 = fmod(ss * M4, M0);
-      if (het1 < 0) het1 += M0;
-      const double s1 = s0_flag ? 0. : ss * M5 + s1_0;
-      p->het1 = het1;
-      p->s1 = s1;
-      p->H = (uint64_t)__double2ull_rn(het1 * kTurnsPerRad64);
-      p->ssr = s0_flag ? 0u : (unsigned)(ss - ss_base);
-      p->s1h = (float)s1;
-      p->s1l = (float)(s1 - (double)p->s1h);
-      p->h1h = (float)het1;
-      p->h1l = (float)(het1 - (double)p->h1h);
-    }
+  __device__ __forceinline__ void next(Ctx& k) const {
+    if constexpr (PM == PM_FIXED) k.hn += k.hstep;
   }
-
-  __device__ __forceinline__ void load2(int batch, int n, T& va, T& vb, const char* sm) const {
-    va = vb = mk((R)0, (R)0);
-    if (n >= N) return;
-    const SpinCta pk = consts(batch, sm);
-    const SpinCta* p = &pk;
-    R accx = 0, accy = 0, bccx = 0, bccy = 0;
-    double base = 0.;
-    // fixed-point form: the high word of H n (the phase is formed from the
-    // high words of its terms, as in mod1h)
-    unsigned hn_hi = 0;
-    if (PM == PM_FIXED) hn_hi = __umulhi((unsigned)p->H, (unsigned)n) + (unsigned)(p->H >> 32) * (unsigned)n;
-    else if (PM == PM_F64) base = p->het1 * (double)n;
-    for (int d = 0; d < nifo; ++d) {
-      const size_t o = (size_t)d * N + n;
-      R sn, cs;
-      T xa, xb;
-      uint4 hi16 = make_uint4(0u, 0u, 0u, 0u);
-      if (sizeof(R) == 8) {
-        xa = xm[((size_t)d * 2 + 0) * N + n];
-        xb = xm[((size_t)d * 2 + 1) * N + n];
-      } else {
-        // one 32-byte record per detector and sample: xa, xb | phase terms
-        const float4 lo16 = __ldg(reinterpret_cast<const float4*>(xm) + 2 * o);
-        hi16 = __ldg(reinterpret_cast<const uint4*>(xm) + 2 * o + 1);
-        xa = mk((R)lo16.x, (R)lo16.y);
-        xb = mk((R)lo16.z, (R)lo16.w);
+  __device__ __forceinline__ Raw fetch(const Ctx& k, int off) const {
+    Raw r{};
+    if constexpr (NIFO > 0) {
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {
+        r.x[d] = __ldg(k.x[d] + off);
+        r.p[d] = __ldg(k.p[d] + off);
       }
-      if (sizeof(R) == 8) {
-        const double t1 = reinterpret_cast<const double*>(ph0)[o];
-        // het1*i + s1*_tmp1 with the reference's rounding (jobcore.c:606)
-        const double ph = __dadd_rn(__dmul_rn(p->het1, (double)n), __dmul_rn(p->s1, t1));
-        double sd, cd;
-        sincos(ph, &sd, &cd);
-        sn = (R)sd;
-        cs = (R)cd;
-      } else if (PM == PM_F64) {
-        const double t1 = __longlong_as_double((long long)(((unsigned long long)hi16.y << 32) | hi16.x));
-        const double ph = fma(p->s1, t1, base);
-        const double kk = rint(ph * kInvTwoPi);
-        double r = fma(-kk, kTwoPiHi, ph);
-        r = fma(-kk, kTwoPiLo, r);
-        float sf, cf;
-        sincosf((float)r, &sf, &cf);
-        sn = (R)sf;
-        cs = (R)cf;
-      } else if (PM == PM_FIXED) {
-        // top 32 bits of A + B ssr + H n (high words only, as mod1h) as a
-        // signed fraction of half a turn: angle = pi * x, x in [-1, 1); the
-        // hardware sine and cosine (absolute error <= 3.6e-7 there)
-        const unsigned th = hi16.y + (__umulhi(hi16.z, p->ssr) + hi16.w * p->ssr) + hn_hi;
-        float sf, cf;
-        __sincosf((float)(int)th * 1.4629180792671596e-9f, &sf, &cf);  // pi 2^-31
-        sn = (R)sf;
-        cs = (R)cf;
-      } else {
-        // compensated float-float phase
-        const float2 tt = make_float2(__uint_as_float(hi16.x), __uint_as_float(hi16.y));
-        float p1 = p->s1h * tt.x;
-        float e1 = fmaf(p->s1h, tt.x, -p1);
-        e1 = fmaf(p->s1h, tt.y, e1);
-        e1 = fmaf(p->s1l, tt.x, e1);
-        const float nf = (float)n;
-        float p2 = p->h1h * nf;
-        float e2 = fmaf(p->h1h, nf, -p2);
-        e2 = fmaf(p->h1l, nf, e2);
-        const float s = p1 + p2;
-        const float bb = s - p1;
-        const float err = (p1 - (s - bb)) + (p2 - bb);
-        const float e = err + e1 + e2;
-        const float kk = rintf(s * kInvTwoPiF);
-        float r = fmaf(-kk, kTwoPiF_A, s);
-        r = fmaf(-kk, kTwoPiF_B, r);
-        r = fmaf(-kk, kTwoPiF_C, r);
-        r += e;
-        float sf, cf;
-        sincosf(r, &sf, &cf);
-        sn = (R)sf;
-        cs = (R)cf;
-      }
-      // x * (cos - i sin)
-      accx += xa.x * cs + xa.y * sn;
-      accy += xa.y * cs - xa.x * sn;
-      bccx += xb.x * cs + xb.y * sn;
-      bccy += xb.y * cs - xb.x * sn;
     }
-    va = mk(accx, accy);
-    vb = mk(bccx, bccy);
+    return r;
   }
-
-  // The fixed-point form's term (FP32, n < N) with the high word of H n
-  // given by the caller (hn_hi, carried from position to position): the
-  // phase's high word is the sum of its three terms' high words.  The carries
-  // of the low words that this drops lower it by at most 2 units of 2^-32
-  // turns (3e-9 rad), far below the FP32 rounding of the angle that follows
-  // (up to 2^-25 of a half turn, 9e-8 rad).  The angle, in [-pi, pi), goes
-  // to the hardware sine and cosine (__sincosf: absolute error at most
-  // 2^-21.41 = 3.6e-7 in that range), which the radix-16 pass A needs once
-  // per detector and sample.  pa, pb as in mod1.
-  __device__ __forceinline__ void mod1h(int d, int n, unsigned hn_hi, unsigned ssr, T& pa, T& pb) const {
-    static_assert(sizeof(R) == 4 && PM == PM_FIXED, "fixed-point FP32 form only");
-    const size_t o = (size_t)d * N + n;
-    const float4 lo16 = __ldg(reinterpret_cast<const float4*>(xm) + 2 * o);
-    const uint4 hi16 = __ldg(reinterpret_cast<const uint4*>(xm) + 2 * o + 1);
-    const unsigned th = hi16.y + (__umulhi(hi16.z, ssr) + hi16.w * ssr) + hn_hi;
-    float sn, cs;
-    __sincosf((float)(int)th * 1.4629180792671596e-9f, &sn, &cs);  // pi 2^-31
-    pa = mk(lo16.x * cs + lo16.y * sn, lo16.y * cs - lo16.x * sn);
-    pb = mk(lo16.z * cs + lo16.w * sn, lo16.w * cs - lo16.z * sn);
-  }
-
-  // One detector's term of load2 (FP32 forms, n < N): xm_{a,b,d}[n] times
-  // exp(-i phase_d(n)), with the phase evaluated as load2 does; pa and pb
-  // follow the record's order (b first for the detector whose record
-  // halves the prelude swapped, Engine::swapped_det).
-  __device__ __forceinline__ void mod1(int d, int n, T& pa, T& pb, const SpinCta& pk) const {
-    static_assert(sizeof(R) == 4, "FP32 forms only");
-    const SpinCta* p = &pk;
-    const size_t o = (size_t)d * N + n;
-    const float4 lo16 = __ldg(reinterpret_cast<const float4*>(xm) + 2 * o);
-    const uint4 hi16 = __ldg(reinterpret_cast<const uint4*>(xm) + 2 * o + 1);
-    float sn, cs;
-    if (PM == PM_FIXED) {
-      const uint64_t A = ((uint64_t)hi16.y << 32) | hi16.x;
-      const uint64_t B = ((uint64_t)hi16.w << 32) | hi16.z;
-      const uint64_t t = A + mul64x32(B, p->ssr) + mul64x32(p->H, (unsigned)n);
-      const float x = (float)(int)(t >> 32) * 4.656612873077393e-10f;  // 2^-31
-      sincospif(x, &sn, &cs);
-    } else if (PM == PM_F64) {
-      const double t1 = __longlong_as_double((long long)(((unsigned long long)hi16.y << 32) | hi16.x));
-      const double ph = fma(p->s1, t1, p->het1 * (double)n);
-      const double kk = rint(ph * kInvTwoPi);
-      double r = fma(-kk, kTwoPiHi, ph);
+  // sine and cosine of the phase of one detector
+  __device__ __forceinline__ void phasor(const Ctx& k, const Term& p, int n, float* sn, float* cs) const {
+    if constexpr (PM == PM_FIXED) {
+      // The phase in turns, A + B ssr + H n, is formed from the high words of
+      // its three terms (H n is carried from position to position).  The
+      // carries of the low words that this drops lower it by at most 2 units
+      // of 2^-32 turns (3e-9 rad), far below the FP32 rounding of the angle
+      // that follows (up to 2^-25 of a half turn, 9e-8 rad).  The angle, in
+      // [-pi, pi), goes to the hardware sine and cosine (__sincosf: absolute
+      // error at most 2^-21.41 = 3.6e-7 in that range).
+      const unsigned th = p.y + (__umulhi(p.z, k.ssr) + p.w * k.ssr) + (unsigned)(k.hn >> 32);
+      __sincosf((float)(int)th * 1.4629180792671596e-9f, sn, cs);  // pi 2^-31
+    } else if constexpr (PM == PM_F64) {
+      const double t1 = __hiloint2double((int)p.y, (int)p.x);
+      const double ph_ = fma(k.s1, t1, k.het1 * (double)n);
+      const double kk = rint(ph_ * kInvTwoPi);
+      double r = fma(-kk, kTwoPiHi, ph_);
       r = fma(-kk, kTwoPiLo, r);
-      sincosf((float)r, &sn, &cs);
+      sincosf((float)r, sn, cs);
     } else {
-      const float2 tt = make_float2(__uint_as_float(hi16.x), __uint_as_float(hi16.y));
-      float p1 = p->s1h * tt.x;
-      float e1 = fmaf(p->s1h, tt.x, -p1);
-      e1 = fmaf(p->s1h, tt.y, e1);
-      e1 = fmaf(p->s1l, tt.x, e1);
+      // compensated float-float phase
+      const float2 tt = make_float2(__uint_as_float(p.x), __uint_as_float(p.y));
+      float p1 = k.c.x * tt.x;
+      float e1 = fmaf(k.c.x, tt.x, -p1);
+      e1 = fmaf(k.c.x, tt.y, e1);
+      e1 = fmaf(k.c.y, tt.x, e1);
       const float nf = (float)n;
-      float p2 = p->h1h * nf;
-      float e2 = fmaf(p->h1h, nf, -p2);
-      e2 = fmaf(p->h1l, nf, e2);
+      float p2 = k.c.z * nf;
+      float e2 = fmaf(k.c.z, nf, -p2);
+      e2 = fmaf(k.c.w, nf, e2);
       const float s = p1 + p2;
       const float bb = s - p1;
       const float err = (p1 - (s - bb)) + (p2 - bb);
@@ -554,112 +552,36 @@ template <typename R, int PM> struct SpinLoader {
       r = fmaf(-kk, kTwoPiF_B, r);
       r = fmaf(-kk, kTwoPiF_C, r);
       r += e;
-      sincosf(r, &sn, &cs);
+      sincosf(r, sn, cs);
     }
-    pa = mk(lo16.x * cs + lo16.y * sn, lo16.y * cs - lo16.x * sn);
-    pb = mk(lo16.z * cs + lo16.w * sn, lo16.w * cs - lo16.z * sn);
   }
-};
-
-// Spindown pass A for two detectors and L1 = 256 = 16 x 16 (the FP32 forms):
-// the column FFTs of k_pass_a as two radix-16 stages with one barrier
-// between them, each thread holding 16 values of one array.
-//   stage 1: warp w = b (n1 mod 16), lane = 2 col + arr.  At the 16 positions
-//     n1 = 16 a + b of column col the thread evaluates detector arr's term
-//     (mod1h in the fixed-point form, mod1 in the others) and swaps with its
-//     partner lane (lane ^ 1) the term of the array the partner keeps, so
-//     that it holds x_arr = term_0 + term_1: one sincos per detector and
-//     position, as the paired loader.  Detector 1's records hold {xb, xa}
-//     (k_splint swap_det), so the first term is always the one kept.
-//     16-point DFT over a, store Z[c][b].
-//   stage 2: warp = column, lane = 2 c + arr.  Twiddle W_256^{b c} (shared
-//     table at c * 17 + b, stored after stage 1), 16-point DFT over b gives
-//     Y[k1 = c + 16 d]; inter-pass twiddle W_L^{n2 k1} from a table of all
-//     of them (Buffers::tw_pass, L entries); stored like k_pass_a
-//     (the a|b values of one (n2, k1) adjacent, 256 contiguous bytes per warp).
-// Shared tile: Z[c][b][lane] at c * 514 + b * 32 + lane (float2); the pad of
-// 2 per c makes the stage-2 reads conflict-free (half-warp slots 2c + arr).
-template <int SIGN, int LOGL, int PM>
-__global__ void __launch_bounds__(512, 2)
-    k_pass_a16(const __grid_constant__ SpinLoader<float, PM> ld, const float2* __restrict__ tw1,
-               const float2* __restrict__ tw16, float2* __restrict__ ybuf) {
-  constexpr int LOGL1 = 8, LOGL2 = LOGL - LOGL1, ZC = 16 * 32 + 2;
-  CtaTrace trace_(KK_SPIN_A);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* z = reinterpret_cast<float2*>(smem_raw);
-  // twiddles of the stage-1 outputs, applied in stage 2: W_256^{b c} at
-  // c * 17 + b (the pitch of 17 makes the stage-2 reads conflict-free)
-  float2* tws = z + 16 * ZC;
-  char* lsm = reinterpret_cast<char*>(tws + 272);
-  const int batch = blockIdx.y;
-  const int c0 = blockIdx.x << 4;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  // loaded now, stored after stage 1: no barrier before the first record
-  // loads (except for the forms whose prologue fills shared memory)
-  float2 twv = make_float2(0.f, 0.f);
-  if (threadIdx.x < 272) {
-    const int tc = threadIdx.x / 17, tb = threadIdx.x - 17 * tc;
-    twv = tw1[tb * tc];
-  }
-  if constexpr (SpinLoader<float, PM>::kPrologue) {
-    ld.prologue(batch, lsm);
-    __syncthreads();
-  }
-  const SpinCta pk = ld.consts(batch, lsm);
-  float2 v[16];
-  {
-    const int arr = lane & 1;
-    const int n2 = c0 + (lane >> 1);
-    // fixed-point form: H n carried from position to position (exact, mod 2^64)
-    uint64_t hn = mul64x32(pk.H, (unsigned)((w << LOGL2) + n2));
-    const uint64_t hstep = pk.H << (4 + LOGL2);
+  __device__ __forceinline__ P2 value(const Ctx& k, const Raw& r, int off) const {
+    P2 v;
+    const int n = k.n0 + off;
+    if constexpr (NIFO > 0) {
 #pragma unroll
-    for (int a = 0; a < 16; ++a) {
-      const int n = ((16 * a + w) << LOGL2) + n2;
-      // detector 1's record holds {xb, xa} (k_splint swap_det): the first
-      // term is the array this lane keeps, the second its partner's
-      float2 mine = make_float2(0.f, 0.f), send = mine;
-      if constexpr (PM == PM_FIXED) {
-        if (n < ld.N) ld.mod1h(arr, n, (unsigned)(hn >> 32), pk.ssr, mine, send);
-        hn += hstep;
-      } else {
-        if (n < ld.N) ld.mod1(arr, n, mine, send, pk);
-      }
-      const float rx = __shfl_xor_sync(0xffffffffu, send.x, 1);
-      const float ry = __shfl_xor_sync(0xffffffffu, send.y, 1);
-      v[a] = make_float2(mine.x + rx, mine.y + ry);
+      for (int d = 0; d < ND; ++d) add_det(k, r.x[d], r.p[d], n, d == 0, v);
+    } else {
+      v = pzero();
+      for (int d = 0; d < nifo; ++d)
+        add_det(k, __ldg(&xm[(size_t)d * NP + n]), __ldg(&ph[(size_t)d * NP + n]), n, false, v);
     }
-    dft16<SIGN>(v);
-#pragma unroll
-    for (int c = 0; c < 16; ++c) z[c * ZC + w * 32 + lane] = v[c];
+    return v;
   }
-  if (threadIdx.x < 272) tws[threadIdx.x] = twv;
-  __syncthreads();
-  {
-    const int arr = lane & 1, c = lane >> 1;
-    const int n2 = c0 + w;
-    const float2* t2 = tws + c * 17;
-    v[0] = z[c * ZC + 2 * w + arr];
-#pragma unroll
-    for (int b = 1; b < 16; ++b) v[b] = cmul(z[c * ZC + b * 32 + 2 * w + arr], t2[b]);
-    dft16<SIGN>(v);
-    float2* yb = ybuf + ((size_t)batch << (LOGL + 1)) + ((size_t)n2 << (LOGL1 + 1)) + arr;
-    // inter-pass twiddle W_L^{n2 k1}, k1 = c + 16 d, from the table at
-    // [n2][k1] (one load per output instead of two table loads, their
-    // product and the exponent arithmetic)
-    const float2* tw = tw16 + ((size_t)n2 << 8) + c;
-#pragma unroll
-    for (int d = 0; d < 16; ++d) yb[2 * (c + 16 * d)] = cmul(v[d], __ldg(&tw[16 * d]));
+  // v (+)= x (cos - i sin)
+  __device__ __forceinline__ void add_det(const Ctx& k, const float4& x, const Term& p, int n, bool first, P2& v) const {
+    float sn, cs;
+    phasor(k, p, n, &sn, &cs);
+    const f2 re = pk(x.x, x.y), im = pk(x.z, x.w);
+    const f2 c2 = dup(cs), s2 = dup(sn), m2 = dup(-sn);
+    if (first) {
+      v.re = fma2(im, s2, mul2(re, c2));
+      v.im = fma2(re, m2, mul2(im, c2));
+    } else {
+      v.re = fma2(im, s2, fma2(re, c2, v.re));
+      v.im = fma2(re, m2, fma2(im, c2, v.im));
+    }
   }
-}
-
-template <class L> struct IsSpinF32 {
-  static constexpr bool value = false;
-  static constexpr int pm = 0;
-};
-template <int PM> struct IsSpinF32<SpinLoader<float, PM>> {
-  static constexpr bool value = true;
-  static constexpr int pm = PM;
 };
 
 // Complex output with a scale factor (resampling FFTs).
@@ -675,6 +597,12 @@ template <typename R> struct CStore {
     const size_t k = (size_t)k1 + ((size_t)k2 << logL1);
     out[((size_t)batch * 2 + 0) * ldo + k] = mk(a.x * scale, a.y * scale);
     out[((size_t)batch * 2 + 1) * ldo + k] = mk(b.x * scale, b.y * scale);
+  }
+  __device__ __forceinline__ void put(const Ctx& c, int batch, int k1, int k2, P2 v) const {
+    T a, b;
+    upk(v.re, a.x, b.x);
+    upk(v.im, a.y, b.y);
+    put(c, batch, k1, k2, a, b, 8);
   }
 };
 
@@ -695,6 +623,12 @@ template <typename R> struct FstatStore {
     const int k = k1 + (k2 << logL1);
     if (k >= nmin && k < nmax)
       F[(size_t)batch * bins + (k - nmin)] = (a.x * a.x + a.y * a.y) * c.ia + (b.x * b.x + b.y * b.y) * c.ib;
+  }
+  __device__ __forceinline__ void put(const Ctx& c, int batch, int k1, int k2, P2 v) const {
+    const int k = k1 + (k2 << 8);
+    float a, b;
+    upk(fma2(v.im, v.im, mul2(v.re, v.re)), a, b);
+    if (k >= nmin && k < nmax) F[(size_t)batch * bins + (k - nmin)] = fmaf(a, (float)c.ia, b * (float)c.ib);
   }
 };
 
@@ -717,6 +651,19 @@ template <typename R> struct InterpStore {
     const T xb = m < N ? xin[qb * N + m] : mk((R)0, (R)0);
     Pair<T>::st(yint + qa * Ninterp + 2 * (size_t)m, xa, mk(a.x * scale, a.y * scale));
     Pair<T>::st(yint + qb * Ninterp + 2 * (size_t)m, xb, mk(b.x * scale, b.y * scale));
+  }
+  __device__ __forceinline__ void put(const Ctx&, int batch, int k1, int k2, P2 v) const {
+    const int m = k1 + (k2 << 8);
+    const size_t qa = (size_t)batch * 2, qb = qa + 1;
+    float2 xa = make_float2(0.f, 0.f), xb = xa, a, b;
+    if (m < N) {
+      xa = xin[qa * N + m];
+      xb = xin[qb * N + m];
+    }
+    upk(mul2(v.re, dup(scale)), a.x, b.x);
+    upk(mul2(v.im, dup(scale)), a.y, b.y);
+    reinterpret_cast<float4*>(yint + qa * Ninterp)[m] = make_float4(xa.x, xa.y, a.x, a.y);
+    reinterpret_cast<float4*>(yint + qb * Ninterp)[m] = make_float4(xb.x, xb.y, b.x, b.y);
   }
 };
 
@@ -969,8 +916,8 @@ __global__ void __launch_bounds__(kSplineThreads)
 template <typename R>
 __global__ void __launch_bounds__(256)
     k_splint(const typename CT<R>::T* __restrict__ y, int ldy, const typename CT<R>::T* __restrict__ y2,
-             const double* __restrict__ shftf, const DetConst* __restrict__ dc, int N,
-             typename CT<R>::T* __restrict__ xm, int swap_det) {
+             const double* __restrict__ shftf, const DetConst* __restrict__ dc, int N, int NP,
+             typename CT<R>::T* __restrict__ xm) {
   typedef typename CT<R>::T T;
   CtaTrace trace_(KK_SPLINT);
   const int d = blockIdx.y;
@@ -1000,12 +947,8 @@ __global__ void __launch_bounds__(256)
     xm[((size_t)d * 2 + 0) * N + i] = out[0];
     xm[((size_t)d * 2 + 1) * N + i] = out[1];
   } else {
-    // lower half of the sample's 32-byte record: {xa, xb}, or {xb, xa} for
-    // detector swap_det (the radix-16 spindown pass A then needs no
-    // lane-dependent selects, SpinLoader::mod1r)
-    const int f = d == swap_det ? 1 : 0;
-    reinterpret_cast<float4*>(xm)[2 * ((size_t)d * N + i)] =
-        make_float4((float)out[f].x, (float)out[f].y, (float)out[1 - f].x, (float)out[1 - f].y);
+    reinterpret_cast<float4*>(xm)[(size_t)d * NP + i] =
+        make_float4((float)out[0].x, (float)out[1].x, (float)out[0].y, (float)out[1].y);
   }
 }
 
@@ -1218,23 +1161,12 @@ __global__ void __launch_bounds__(256)
 // ------------------------------------------------------------------
 // engine
 
-inline Geom make_geom(int L, int E) {
+inline Geom make_geom(int L) {
   Geom g;
   int m = 0;
   while ((1 << m) < L) ++m;
   g.L = L;
   g.logL = m;
-  g.logL1 = (m + 1) / 2;
-  g.logL2 = m / 2;
-  g.L1 = 1 << g.logL1;
-  g.L2 = 1 << g.logL2;
-  int logE = 0;
-  while ((1 << logE) < E) ++logE;
-  g.logC = logE - 1 - g.logL1;
-  g.C = 1 << g.logC;
-  g.logRr = logE - 1 - g.logL2;
-  g.Rr = 1 << g.logRr;
-  g.twlo_log = 10;
   return g;
 }
 
@@ -1245,20 +1177,6 @@ template <typename R, int PM> class EngineT : public Engine {
   long long launches_ = 0;
   int split_ = 0;
   int dev_ = 0;  // device the engine was made on (current at construction)
-  // spindown pass A of two detectors with L1 = 256: the radix-16 kernel
-  // (default) or the generic radix-4/8 one (environment PA_SPIN_PASS_A=radix8)
-  bool a16_ = true;
-
-  // The spindown pass A is the radix-16 kernel: FP32, two detectors, L1 =
-  // 256 with the current split (the template condition of fft_l).
-  bool use_a16() const {
-    if (sizeof(R) != 4 || b_.nifo != 2 || !a16_ || !b_.tw_pass[split_]) return false;
-    const int m = gm_.logL;
-    return (split_ ? m / 2 : (m + 1) / 2) == 8;
-  }
-  // Detector whose record halves the prelude stores as {xb, xa}: detector 1
-  // when the radix-16 pass A reads the records, else none (-1).
-  int swapped_det() const override { return use_a16() ? 1 : -1; }
 
   // CUDA events around a launch when profiling is on
   void pre(int kind, int items, cudaStream_t st) {
@@ -1287,9 +1205,9 @@ template <typename R, int PM> class EngineT : public Engine {
     }
   }
 
-  // tw: W_L1 and W_L2 tables of the default split (L1 = 2^ceil(m/2)), then
-  // the two halves of the inter-pass twiddle; SPLIT 1 swaps the factors and
-  // so the first two tables.
+  // FP64 form: tw: W_L1 and W_L2 tables of the default split (L1 =
+  // 2^ceil(m/2)), then the two halves of the inter-pass twiddle; SPLIT 1 swaps
+  // the factors and so the first two tables.
   template <int SIGN, int LOGL, int SPLIT, class Loader, class Storer>
   cudaError_t fft_l(const void* const* tw, const Loader& ld, const Storer& st, int batch, cudaStream_t stream,
                     int kind_a, int kind_b, void* ybuf) {
@@ -1297,8 +1215,6 @@ template <typename R, int PM> class EngineT : public Engine {
     constexpr int NT = TileCfg<R>::NT;
     const T* t1 = (const T*)tw[SPLIT ? 1 : 0];
     const T* t2 = (const T*)tw[SPLIT ? 0 : 1];
-    const T* tlo = (const T*)tw[2];
-    const T* thi = (const T*)tw[3];
     T* yb = (T*)ybuf;
     auto ka = k_pass_a<R, SIGN, LOGL, Loader, SPLIT>;
     auto kb = k_pass_b<R, SIGN, LOGL, Storer, SPLIT>;
@@ -1307,24 +1223,7 @@ template <typename R, int PM> class EngineT : public Engine {
     smem_attr(kb, G::smem_b, doneB);
     dim3 ga(G::L2 >> G::LOGC, batch), gb(G::L1 >> G::LOGRR, batch);
     pre(kind_a, batch, stream);
-    bool done = false;
-    if constexpr (IsSpinF32<Loader>::value && G::LOGL1 == 8 && G::C == 16 && NT == 512) {
-      // two detectors, L1 = 256: the two-stage radix-16 pass A
-      if (use_a16()) {
-        auto k16 = k_pass_a16<SIGN, LOGL, IsSpinF32<Loader>::pm>;
-        constexpr int smem16 = (16 * (16 * 32 + 2) + 272) * (int)sizeof(float2) + 128;
-        static std::atomic<unsigned long long> done16{0};
-        smem_attr(k16, smem16, done16);
-        k16<<<ga, 512, smem16, stream>>>(ld, t1, (const float2*)b_.tw_pass[SPLIT], yb);
-        done = true;
-      }
-    }
-    const T* twp = nullptr;
-    if constexpr (Loader::kTwiddleTable) {
-      twp = (const T*)b_.tw_pass[SPLIT];
-      if (!twp) return cudaErrorInvalidValue;
-    }
-    if (!done) ka<<<ga, NT, G::smem_a, stream>>>(ld, t1, tlo, thi, twp, yb);
+    ka<<<ga, NT, G::smem_a, stream>>>(ld, t1, (const T*)tw[2], (const T*)tw[3], yb);
     post(stream);
     pre(kind_b, batch, stream);
     kb<<<gb, NT, G::smem_b, stream>>>(st, t2, yb);
@@ -1333,9 +1232,33 @@ template <typename R, int PM> class EngineT : public Engine {
     return cudaGetLastError();
   }
 
+  // FP32 forms: which = 0: length nfft, 1: nfftf; HALF: only the outputs below
+  // half the length are wanted; NIN, NCHK: k_pair_a.
+  template <int SIGN, int LOGL, int LTA, int LOGS, int LTB, bool HALF, int NIN, int NCHK, class Loader, class Storer>
+  cudaError_t pair_l(int which, const Loader& ld, const Storer& st, int batch, cudaStream_t stream, int kind_a,
+                     int kind_b, void* ybuf) {
+    typedef PairShape<LOGL, LTA, LOGS> A;
+    typedef PairShape<LOGL, LTB> B;
+    auto ka = k_pair_a<SIGN, LOGL, LTA, LOGS, NIN, NCHK, Loader>;
+    auto kb = k_pair_b<SIGN, LOGL, LTB, Storer, HALF>;
+    static std::atomic<unsigned long long> doneA{0}, doneB{0};
+    smem_attr(ka, A::smem_a, doneA);
+    smem_attr(kb, B::smem_b, doneB);
+    dim3 ga(A::L2 >> A::LOGC, (batch + (1 << LOGS) - 1) >> LOGS), gb(256 >> B::LOGRR, batch);
+    pre(kind_a, batch, stream);
+    ka<<<ga, A::NT, A::smem_a, stream>>>(ld, (const float2*)b_.pair_tw1, (const float2*)b_.pair_pass[which],
+                                         (float4*)ybuf, batch);
+    post(stream);
+    pre(kind_b, batch, stream);
+    kb<<<gb, B::NT, B::smem_b, stream>>>(st, (const float2*)b_.pair_row[which], (const float4*)ybuf);
+    post(stream);
+    launches_ += 2;
+    return cudaGetLastError();
+  }
+
   // Dispatch on the transform length (2^12 .. 2^20) to the compile-time
-  // geometry of the passes; with SPLITS, odd lengths may take the swapped
-  // split (split = 1).
+  // geometry of the passes; FP64 form: with SPLITS, odd lengths may take the
+  // swapped split (split = 1).
   template <int SIGN, bool SPLITS = false, class Loader, class Storer>
   cudaError_t fft(const Geom& g, const void* const* tw, const Loader& ld, const Storer& st, int batch,
                   cudaStream_t stream, int kind_a, int kind_b, void* ybuf, int split = 0) {
@@ -1352,13 +1275,71 @@ template <typename R, int PM> class EngineT : public Engine {
     }
   }
 
+  // The resampling transforms (length nfft, at most 2^19) take half-size
+  // tiles: one or a few detectors give few CTAs, and they are waited for.
+  template <int SIGN, int NCHK, class Loader, class Storer>
+  cudaError_t pair_pre(const Loader& ld, const Storer& st, int batch, cudaStream_t stream, int kind_a, int kind_b) {
+    switch (gf_.logL) {
+#define PA_FFT_CASE(M) \
+  case M: return pair_l<SIGN, M, 11, 0, 11, false, 16, NCHK>(0, ld, st, batch, stream, kind_a, kind_b, b_.ybuf_pre);
+      PA_FFT_CASE(12) PA_FFT_CASE(13) PA_FFT_CASE(14) PA_FFT_CASE(15) PA_FFT_CASE(16)
+      PA_FFT_CASE(17) PA_FFT_CASE(18) PA_FFT_CASE(19)
+#undef PA_FFT_CASE
+      default: return cudaErrorInvalidValue;
+    }
+  }
+
+  // The spindown transform.  F is wanted on [nmin, nmax): below half the
+  // length in every search set up as the reference's (settings.c:50-55).
+  // The data fill more than half of the transform with fftpad = 1, and a
+  // quarter to a half of it with 2: pass A takes the 16 rows (of 16 x 16) in
+  // quarters, the last one of them with a condition, the empty ones left out.
+  // That is compiled for the fixed-point form of one to three detectors from
+  // 2^16 on; the others test every row.
+  template <int M, class Loader>
+  cudaError_t pair_main_l(const Loader& ld, const FstatStore<R>& st, int batch, cudaStream_t stream, void* yb) {
+    constexpr int A = KK_SPIN_A, B = KK_SPIN_B;
+    constexpr int LTA = 11, kLogS = 1, LTB = M >= 18 ? 12 : 11;
+    if (b_.nmax > b_.nfftf / 2) return pair_l<-1, M, LTA, kLogS, LTB, false, 16, 0>(1, ld, st, batch, stream, A, B, yb);
+    if constexpr (PM == PM_FIXED && M >= 16 && Loader::kQuarters) {
+      const int q = b_.nfftf / 4;
+      if (b_.N > 3 * q) return pair_l<-1, M, LTA, kLogS, LTB, true, 16, 12>(1, ld, st, batch, stream, A, B, yb);
+      if (b_.N > 2 * q) return pair_l<-1, M, LTA, kLogS, LTB, true, 12, 8>(1, ld, st, batch, stream, A, B, yb);
+      if (b_.N > q) return pair_l<-1, M, LTA, kLogS, LTB, true, 8, 4>(1, ld, st, batch, stream, A, B, yb);
+    }
+    return pair_l<-1, M, LTA, kLogS, LTB, true, 16, 0>(1, ld, st, batch, stream, A, B, yb);
+  }
+  template <class Loader>
+  cudaError_t pair_main(const Loader& ld, const FstatStore<R>& st, int batch, cudaStream_t stream, void* ybuf) {
+    switch (gm_.logL) {
+#define PA_FFT_CASE(M) \
+  case M: return pair_main_l<M>(ld, st, batch, stream, ybuf);
+      PA_FFT_CASE(12) PA_FFT_CASE(13) PA_FFT_CASE(14) PA_FFT_CASE(15) PA_FFT_CASE(16)
+      PA_FFT_CASE(17) PA_FFT_CASE(18) PA_FFT_CASE(19) PA_FFT_CASE(20)
+#undef PA_FFT_CASE
+      default: return cudaErrorInvalidValue;
+    }
+  }
+  template <int NIFO>
+  cudaError_t spin_main(const SkyArgs& sky, int slot, int ss0, int nb, int s0_flag, const FstatStore<R>& fs,
+                        cudaStream_t st, void* yb) {
+    SpinLoader<PM, NIFO> sl;
+    sl.xm = (const float4*)b_.xm[slot];
+    sl.ph = (const typename SpinTerm<PM>::T*)((const float4*)b_.xm[slot] + (size_t)b_.nifo * b_.NP);
+    sl.N = b_.N;
+    sl.NP = b_.NP;
+    sl.nifo = b_.nifo;
+    sl.ss_rel = ss0 - sky.ss_base;
+    sl.s0_flag = s0_flag;
+    for (int k = 0; k < nb; ++k) spin_het_fill(sl.het, k, ss0 + k, sky, s0_flag);
+    return pair_main(sl, fs, nb, st, yb);
+  }
+
  public:
   explicit EngineT(const Buffers& b) : b_(b) {
     cudaGetDevice(&dev_);
-    const char* pa = getenv("PA_SPIN_PASS_A");
-    a16_ = !(pa && strcmp(pa, "radix8") == 0);
-    gf_ = make_geom(b.nfft, TileCfg<R>::E);
-    gm_ = make_geom(b.nfftf, TileCfg<R>::E);
+    gf_ = make_geom(b.nfft);
+    gm_ = make_geom(b.nfftf);
   }
 
   long long launches() const override { return launches_; }
@@ -1385,22 +1366,25 @@ template <typename R, int PM> class EngineT : public Engine {
     const int nbx = (N + 255) / 256;
     pre(KK_PRELUDE_MOD, nifo, st);
     k_prelude_mod<R, PM><<<dim3(nbx, nifo), 256, 0, st>>>(
-        b_.xDat, b_.DetSSB, (const R*)b_.cosmodf, (const R*)b_.sinmodf, b_.dc, sky, N, (T*)b_.xin,
-        b_.shftf, sizeof(R) == 8 ? b_.ph0[slot] : b_.xm[slot], b_.part, b_.sums[slot],
+        b_.xDat, b_.DetSSB, (const R*)b_.cosmodf, (const R*)b_.sinmodf, b_.dc, sky, N, b_.NP, (T*)b_.xin,
+        b_.shftf, sizeof(R) == 8 ? b_.ph0[slot] : (void*)((float4*)b_.xm[slot] + (size_t)nifo * b_.NP), b_.part, b_.sums[slot],
         (R*)b_.sums_r[slot], b_.counter);
     post(st);
     launches_ += 1;
     // forward FFT of the zero-padded series (length nfft)
     PlainLoader<R> pl{(const T*)b_.xin, N, N};
     CStore<R> cs1{(T*)b_.spec, b_.nfft, (R)1};
-    cudaError_t e = fft<-1>(gf_, b_.tw_fwd, pl, cs1, nifo, st, KK_FFT_FWD_A, KK_FFT_FWD_B, b_.ybuf_pre);
+    cudaError_t e;
+    if constexpr (sizeof(R) == 4) e = pair_pre<-1, 0>(pl, cs1, nifo, st, KK_FFT_FWD_A, KK_FFT_FWD_B);
+    else e = fft<-1>(gf_, b_.tw_fwd, pl, cs1, nifo, st, KK_FFT_FWD_A, KK_FFT_FWD_B, b_.ybuf_pre);
     if (e != cudaSuccess) return e;
     // spectrum remap + backward FFT of length Ninterp, scale interpftpad/Ninterp
     // (jobcore.c:338-362), as a half-length transform (HalfShiftLoader)
     HalfShiftLoader<R> hl{(const T*)b_.spec, (const T*)b_.tw_inv[2], (const T*)b_.tw_inv[3], b_.nfft,
                           b_.nfft / 2 + 1};
     InterpStore<R> is{(T*)b_.yint, (const T*)b_.xin, N, b_.Ninterp, (R)(1.0 / b_.nfft)};
-    e = fft<+1>(gf_, b_.tw_invh, hl, is, nifo, st, KK_FFT_INV_A, KK_FFT_INV_B, b_.ybuf_pre);
+    if constexpr (sizeof(R) == 4) e = pair_pre<+1, 16>(hl, is, nifo, st, KK_FFT_INV_A, KK_FFT_INV_B);
+    else e = fft<+1>(gf_, b_.tw_invh, hl, is, nifo, st, KK_FFT_INV_A, KK_FFT_INV_B, b_.ybuf_pre);
     if (e != cudaSuccess) return e;
     // spline through the first 2N points of each resampled array
     const int n = 2 * N;
@@ -1421,7 +1405,7 @@ template <typename R, int PM> class EngineT : public Engine {
     post(st);
     pre(KK_SPLINT, nifo, st);
     k_splint<R><<<dim3(nbx, nifo), 256, 0, st>>>((const T*)b_.yint, b_.Ninterp, (const T*)b_.y2,
-                                                 b_.shftf, b_.dc, N, (T*)b_.xm[slot], swapped_det());
+                                                 b_.shftf, b_.dc, N, b_.NP, (T*)b_.xm[slot]);
     post(st);
     launches_ += 3;
     return cudaGetLastError();
@@ -1432,24 +1416,25 @@ template <typename R, int PM> class EngineT : public Engine {
     const size_t lo = (size_t)lane * b_.lane_sb;  // first spindown of the lane in ybuf and F
     T* const yb = (T*)b_.ybuf + lo * 2 * b_.nfftf;
     R* const Fl = (R*)b_.F + lo * b_.bins;
-    SpinLoader<R, PM> sl;
-    sl.xm = (const T*)b_.xm[slot];
-    sl.ph0 = b_.ph0[slot];
-    sl.ss_base = sky.ss_base;
-    sl.N = b_.N;
-    sl.nifo = b_.nifo;
-    sl.ss0 = ss0;
-    sl.s0_flag = s0_flag;
-    sl.M0 = sky.M0;
-    sl.M4 = sky.M4;
-    sl.M5 = sky.M5;
-    sl.s1_0 = sky.s1_0;
     if (nb > kSpinBatchMax) return cudaErrorInvalidValue;
-    if constexpr (SpinHet<R, PM>::kHost) {
-      for (int k = 0; k < nb; ++k) sl.het.H[k] = het1_turns_fixed(ss0 + k, sky.M4, sky.M0);
-    }
     FstatStore<R> fs{Fl, (const R*)b_.sums_r[slot], b_.nmin, b_.nmax, b_.bins};
-    cudaError_t e = fft<-1, true>(gm_, b_.tw_main, sl, fs, nb, st, KK_SPIN_A, KK_SPIN_B, yb, split_);
+    cudaError_t e;
+    if constexpr (sizeof(R) == 4) {
+      switch (b_.nifo) {
+        case 1: e = spin_main<1>(sky, slot, ss0, nb, s0_flag, fs, st, yb); break;
+        case 2: e = spin_main<2>(sky, slot, ss0, nb, s0_flag, fs, st, yb); break;
+        case 3: e = spin_main<3>(sky, slot, ss0, nb, s0_flag, fs, st, yb); break;
+        default: e = spin_main<0>(sky, slot, ss0, nb, s0_flag, fs, st, yb);
+      }
+    } else {
+      SpinLoader64 sl;
+      sl.xm = (const double2*)b_.xm[slot];
+      sl.tmp1 = (const double*)b_.ph0[slot];
+      sl.N = b_.N;
+      sl.nifo = b_.nifo;
+      for (int k = 0; k < nb; ++k) spin_het_fill(sl.het, k, ss0 + k, sky, s0_flag);
+      e = fft<-1, true>(gm_, b_.tw_main, sl, fs, nb, st, KK_SPIN_A, KK_SPIN_B, yb, split_);
+    }
     if (e != cudaSuccess) return e;
     const int nchunk = (b_.bins + 4095) / 4096;
     pre(KK_THRESHOLD, nb, st);

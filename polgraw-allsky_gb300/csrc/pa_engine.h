@@ -6,13 +6,39 @@
 
 namespace pa {
 
-// log2 of the pass-A column length L1 of a length 2^logL transform with
-// factor split `split` (0: L1 = 2^ceil(logL/2); 1, odd logL only: 2^floor)
-inline int pass_logl1(int logL, int split) { return (split && (logL & 1)) ? logL / 2 : (logL + 1) / 2; }
-// exponent m of W_L^m at entry j of Buffers::tw_pass[split]: the inter-pass
-// twiddle W_L^{n2 k1} at (n2 << logL1) + k1
-inline long tw_pass_exp(long j, long L, int logL1) {
-  return ((j >> logL1) * (j & ((1L << logL1) - 1))) % L;
+// The FFT passes of the FP32 forms (pa_pair.cuh): L = 256 L2.
+// log2 of the rows of a block of the intermediate
+constexpr int pair_row_block(int logL) { return logL >= 19 ? 0 : (logL <= 16 ? 3 : 19 - logL); }
+// radix of stage `stage` (0, 1, 2) of the row transforms; 1: no such stage
+constexpr int pair_radix(int logL, int stage) {
+  constexpr int r[9][3] = {{16, 1, 1}, {8, 1, 4}, {8, 1, 8}, {16, 1, 8}, {16, 1, 16},
+                           {8, 8, 8}, {16, 8, 8}, {16, 16, 8}, {16, 16, 16}};
+  return r[logL - 12][stage];
+}
+// entries of the row twiddle table: W_{Ns R}^{k r} at r Ns + k for the middle
+// stage (if any), then for the last one
+constexpr int pair_row_table(int logL) {
+  return (pair_radix(logL, 1) > 1 ? pair_radix(logL, 0) * pair_radix(logL, 1) : 0) + (1 << (logL - 8));
+}
+// samples of room for N of data in a transform of length L: a warp of pass A
+// reads four rows wherever the first of them has data
+constexpr int pair_pad(int N, int L) { return (N + 4 * (L / 256) + 16 + 7) / 8 * 8; }
+// exponent m of W_L^m at entry j of the inter-pass twiddle table: n2 k1 at the
+// place of (k1, n2) in the intermediate
+inline long pair_pass_exp(long j, int logL) {
+  const int lr = pair_row_block(logL);
+  const long k1 = (j & ((1L << lr) - 1)) + ((j >> (lr + logL - 8)) << lr);
+  const long n2 = (j >> lr) & ((1L << (logL - 8)) - 1);
+  return (n2 * k1) & ((1L << logL) - 1);
+}
+// exponent m of W_{L2}^m at entry j of the row twiddle table
+inline long pair_row_exp(int j, int logL) {
+  const long L2 = 1L << (logL - 8);
+  const int mid = pair_row_table(logL) - (int)L2;
+  const long n = j < mid ? mid : L2;                                       // Ns R
+  const long Ns = j < mid ? pair_radix(logL, 0) : L2 / (pair_radix(logL, 2) > 1 ? pair_radix(logL, 2) : L2);
+  const long q = j < mid ? j : j - mid;
+  return (q / Ns) * (q % Ns) * (L2 / n) % L2;
 }
 
 constexpr int kMaxDet = 8;
@@ -59,6 +85,7 @@ struct DevCand {
 // Device buffers owned by the context and shared with the engine.
 struct Buffers {
   int N, nfft, Ninterp, nfftf, nmin, nmax, bins, nblk, nifo, fftpad;
+  int NP;                           // FP32 forms: stride of xm's arrays (pair_pad)
   int sbatch;                       // spindowns per fused launch
   const double* xDat;               // [nifo][N]
   const double* DetSSB;             // [nifo][3N]
@@ -77,8 +104,10 @@ struct Buffers {
   // of one sky point runs while the spindowns of the previous one read the
   // other slot
   void* ph0[2];                     // FP64 form: tmp1 [nifo][N]
-  void* xm[2];                      // FP32 forms: [nifo][N] 32-byte records
-                                    // {xa, xb | phase terms}; FP64 form:
+  void* xm[2];                      // FP32 forms: [nifo][NP] float4 {a.re, b.re,
+                                    // a.im, b.im}, then [nifo][NP] phase terms
+                                    // (16 bytes in the fixed-point form, else
+                                    // 8), zeros from N on; FP64 form:
                                     // [nifo][2][N] double complex
   double* sums[2];                  // aa, bb, 1/aa, 1/bb
   void* sums_r[2];                  // 1/aa, 1/bb in the working precision
@@ -93,15 +122,17 @@ struct Buffers {
   DevCand* cand;
   int* ncand;
   int cand_cap;
-  // twiddle tables (Real complex) per transform
+  // twiddle tables (Real complex) per transform, FP64 form (FP32 forms: only
+  // tw_inv[2] and [3])
   const void* tw_fwd[4];            // nfft forward: tw1, tw2, twlo, twhi
   const void* tw_inv[4];            // Ninterp backward (its twlo/twhi give e^{+i pi j/nfft})
   const void* tw_invh[4];           // nfft backward (the half-length resampling transform)
   const void* tw_main[4];           // nfftf forward
-  // FP32 forms: the inter-pass twiddles W_L^{n2 k1} of the spindown
-  // transform (L = nfftf) at (n2 << logL1) + k1 for each factor split
-  // (pass_logl1), nfftf entries each; both pointers equal for even log2 L
-  const void* tw_pass[2];
+  // FP32 forms (all exp(-2 pi i ...)): W_256^m; the row twiddles and the
+  // inter-pass twiddles of the transforms of length nfft (0) and nfftf (1)
+  const void* pair_tw1;
+  const void* pair_row[2];
+  const void* pair_pass[2];
 };
 
 // Kernel kinds for the optional per-launch CUDA-event profile.
@@ -141,13 +172,11 @@ class Engine {
                                 int s0_flag, cudaStream_t st, void* Fdbg) = 0;
   virtual long long launches() const = 0;
   virtual size_t real_size() const = 0;
-  // Factor split of the spindown FFT (0: L1 = 2^ceil(m/2); 1: swapped, for
-  // odd m only; ignored for even m).
+  // Factor split of the FP64 form's spindown FFT (0: L1 = 2^ceil(m/2); 1:
+  // swapped, for odd m only; ignored for even m).  The FP32 forms have one
+  // factorisation and only keep the value.
   virtual void set_split(int split) = 0;
   virtual int split() const = 0;
-  // Detector whose 32-byte records (FP32 forms) hold {xb, xa} instead of
-  // {xa, xb}, as the prelude writes them for the current split; -1: none.
-  virtual int swapped_det() const = 0;
   // Per-CTA trace of this engine's kernels into buf (cap records of 48
   // bytes: start/end %globaltimer, start/end clock64, kernel kind, SM id);
   // buf == nullptr switches it off.  trace_count: records written so far

@@ -1,4 +1,5 @@
-// pa_fft.cuh -- shared-memory Stockham FFT building blocks for sm_103a.
+// pa_fft.cuh -- shared-memory Stockham FFT building blocks of the FP64 form,
+// for sm_103a (the FP32 forms: pa_pair.cuh).
 //
 // A length-L (L = L1*L2 = 2^m, 4096 <= L <= 2^20) complex FFT runs as two
 // fused passes of the four-step scheme:
@@ -44,14 +45,9 @@ template <int SIGN, class T> __device__ __forceinline__ T mulj(T a) {
   return SIGN > 0 ? mk(-a.y, a.x) : mk(a.y, -a.x);
 }
 
-// Tile geometry of one FFT length (host fills, kernels read by value).
+// Length of one transform.
 struct Geom {
-  int L, logL;       // transform length
-  int L1, logL1;     // pass-A (column) FFT length
-  int L2, logL2;     // pass-B (row) FFT length
-  int C, logC;       // columns per pass-A tile
-  int Rr, logRr;     // rows per pass-B tile
-  int twlo_log;      // log2 of the low twiddle table length (10)
+  int L, logL;
 };
 
 template <int SIGN, class T> __device__ __forceinline__ void dft2(T* v) {
@@ -92,50 +88,6 @@ template <int SIGN, class T> __device__ __forceinline__ void dft8(T* v) {
   v[7] = csub(e3, t3);
 }
 
-// x * exp(SIGN 2 pi i e / 16) for a compile-time e in 1 .. 9
-template <int SIGN, int e, class T> __device__ __forceinline__ T w16(T x) {
-  typedef decltype(x.x) R;
-  if (e == 4) return mulj<SIGN>(x);
-  // cos and sin of 2 pi e / 16 for e = 0 .. 9
-  constexpr double kc[10] = {1., 0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173, 0.,
-                             -0.38268343236508977173, -0.70710678118654752440, -0.92387953251128675613, -1.,
-                             -0.92387953251128675613};
-  constexpr double ks[10] = {0., 0.38268343236508977173, 0.70710678118654752440, 0.92387953251128675613, 1.,
-                             0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173, 0.,
-                             -0.38268343236508977173};
-  const R c = (R)kc[e], s = (R)(SIGN * ks[e]);
-  return mk(x.x * c - x.y * s, x.x * s + x.y * c);
-}
-
-// 16-point DFT in natural order, as 4 x 4: X[k1 + 4 k2] =
-// sum_n2 W4^{n2 k2} W16^{n2 k1} sum_n1 x[4 n1 + n2] W4^{n1 k1}
-template <int SIGN, class T> __device__ __forceinline__ void dft16(T* v) {
-#pragma unroll
-  for (int n2 = 0; n2 < 4; ++n2) dft4<SIGN>(v[n2], v[4 + n2], v[8 + n2], v[12 + n2]);
-  // v[n2 + 4 k1] now holds the inner transform (n2, k1)
-  v[5] = w16<SIGN, 1>(v[5]);
-  v[6] = w16<SIGN, 2>(v[6]);
-  v[7] = w16<SIGN, 3>(v[7]);
-  v[9] = w16<SIGN, 2>(v[9]);
-  v[10] = w16<SIGN, 4>(v[10]);
-  v[11] = w16<SIGN, 6>(v[11]);
-  v[13] = w16<SIGN, 3>(v[13]);
-  v[14] = w16<SIGN, 6>(v[14]);
-  v[15] = w16<SIGN, 9>(v[15]);
-  T o[16];
-#pragma unroll
-  for (int k1 = 0; k1 < 4; ++k1) {
-    T a = v[4 * k1], b = v[4 * k1 + 1], c = v[4 * k1 + 2], d = v[4 * k1 + 3];
-    dft4<SIGN>(a, b, c, d);
-    o[k1] = a;
-    o[k1 + 4] = b;
-    o[k1 + 8] = c;
-    o[k1 + 12] = d;
-  }
-#pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = o[k];
-}
-
 template <int SIGN, int RAD, class T> __device__ __forceinline__ void dftr(T* v) {
   if (RAD == 2) dft2<SIGN>(v);
   else if (RAD == 4) dft4v<SIGN>(v);
@@ -149,28 +101,6 @@ template <int SIGN, int RAD, class T> __device__ __forceinline__ void dftr(T* v)
 // lane mappings conflict-free: consecutive c (rows of 2*Cs elements) and
 // consecutive e (stride P*sizeof(T) = 16 bytes mod 128).
 template <class T> struct Pair;
-template <> struct Pair<float2> {
-  static constexpr int PADE = 2;
-  __device__ __forceinline__ static void ld(const float2* p, float2& a, float2& b) {
-    const float4 v = *reinterpret_cast<const float4*>(p);
-    a = make_float2(v.x, v.y);
-    b = make_float2(v.z, v.w);
-  }
-  __device__ __forceinline__ static void ldg(const float2* p, float2& a, float2& b) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(p));
-    a = make_float2(v.x, v.y);
-    b = make_float2(v.z, v.w);
-  }
-  // last read of the data: evict-first
-  __device__ __forceinline__ static void ldlast(const float2* p, float2& a, float2& b) {
-    const float4 v = __ldcs(reinterpret_cast<const float4*>(p));
-    a = make_float2(v.x, v.y);
-    b = make_float2(v.z, v.w);
-  }
-  __device__ __forceinline__ static void st(float2* p, float2 a, float2 b) {
-    *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
-  }
-};
 template <> struct Pair<double2> {
   static constexpr int PADE = 1;
   __device__ __forceinline__ static void ld(const double2* p, double2& a, double2& b) {
@@ -302,13 +232,6 @@ __device__ __forceinline__ void fft_front(T* s, const T* tw, const Src& src, con
 
 // Per-precision tile configuration.
 template <typename R> struct TileCfg;
-// (4096-element FP32 tiles with 256 threads and 4 CTAs per SM were measured
-// 1% slower on the spindown passes)
-template <> struct TileCfg<float> {
-  static constexpr int E = 8192;   // complex elements per tile (64 KB)
-  static constexpr int NT = 512;   // threads per CTA
-  static constexpr int MINB = 2;   // resident CTAs per SM the registers are sized for
-};
 template <> struct TileCfg<double> {
   static constexpr int E = 4096;   // 64 KB
   static constexpr int NT = 256;
@@ -331,7 +254,7 @@ template <typename R, int LOGL, int SPLIT = 0> struct FftShape {
   static constexpr int LOGC = logE - 1 - LOGL1, C = 1 << LOGC;      // pass-A columns per tile
   static constexpr int LOGRR = logE - 1 - LOGL2, RR = 1 << LOGRR;   // pass-B rows per tile
   static constexpr int PA = tile_pitch<R>(C), PB = tile_pitch<R>(RR);
-  static constexpr int smem_a = (L1 * PA + L1) * (int)sizeof(typename CT<R>::T) + 128;
+  static constexpr int smem_a = (L1 * PA + L1) * (int)sizeof(typename CT<R>::T);
   static constexpr int smem_b = (L2 * PB + L2) * (int)sizeof(typename CT<R>::T);
   static_assert(C <= L2 && RR <= L1, "transform too short for the tile");
 };
@@ -399,16 +322,13 @@ struct CtaTrace {
 // item (blockIdx.y).  The first radix stage takes its inputs from the
 // loader in registers; the last stage (lanes along k1) applies the
 // inter-pass twiddle W_L^{n2 k1} and writes Y[n2][k1][a|b] straight to
-// global memory, 16 contiguous bytes per lane.  The twiddle comes from the
-// table twp of all of them at (n2 << LOGL1) + k1 when the loader's
-// kTwiddleTable is set (the spindown transform of the FP32 forms), else as
-// the product of the two tables twlo, twhi.
-// Loader: prologue(batch, smem scratch) and load2(batch, n, a, b, scratch).
+// global memory.  The twiddle is the product of the two tables twlo, twhi.
+// Loader: load2(batch, n, a, b).
 template <typename R, int SIGN, int LOGL, class Loader, int SPLIT = 0>
 __global__ void __launch_bounds__(TileCfg<R>::NT, TileCfg<R>::MINB)
     k_pass_a(const __grid_constant__ Loader ld, const typename CT<R>::T* __restrict__ tw1,
              const typename CT<R>::T* __restrict__ twlo, const typename CT<R>::T* __restrict__ twhi,
-             const typename CT<R>::T* __restrict__ twp, typename CT<R>::T* __restrict__ ybuf) {
+             typename CT<R>::T* __restrict__ ybuf) {
   typedef typename CT<R>::T T;
   typedef FftShape<R, LOGL, SPLIT> G;
   constexpr int E = G::E, NT = G::NT, P = G::PA;
@@ -416,14 +336,12 @@ __global__ void __launch_bounds__(TileCfg<R>::NT, TileCfg<R>::MINB)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* s = reinterpret_cast<T*>(smem_raw);
   T* tws = s + G::L1 * P;
-  char* lsm = reinterpret_cast<char*>(tws + G::L1);   // loader scratch
   const int batch = blockIdx.y;
   const int c0 = blockIdx.x << G::LOGC;
-  auto src = [&](int n1, int c, T& a, T& b) { ld.load2(batch, (n1 << G::LOGL2) + c0 + c, a, b, lsm); };
-  if constexpr (Loader::kEarlyLoads && G::L1 <= NT) {
-    // no loader constants in shared memory: the column twiddles are stored
-    // at the end of the first stage (as in pass B), no barrier before the
-    // first loads
+  auto src = [&](int n1, int c, T& a, T& b) { ld.load2(batch, (n1 << G::LOGL2) + c0 + c, a, b); };
+  if constexpr (G::L1 <= NT) {
+    // the column twiddles are stored at the end of the first stage (as in
+    // pass B), no barrier before the first loads
     const T twv = threadIdx.x < G::L1 ? tw1[threadIdx.x] : T();
     auto fill = [&]() {
       if (threadIdx.x < G::L1) tws[threadIdx.x] = twv;
@@ -431,7 +349,6 @@ __global__ void __launch_bounds__(TileCfg<R>::NT, TileCfg<R>::MINB)
     fft_front<SIGN, E, NT, G::LOGL1, G::LOGC, P>(s, tws, src, fill);
   } else {
     for (int m = threadIdx.x; m < G::L1; m += NT) tws[m] = tw1[m];
-    ld.prologue(batch, lsm);
     __syncthreads();
     fft_front<SIGN, E, NT, G::LOGL1, G::LOGC, P>(s, tws, src);
   }
@@ -449,13 +366,8 @@ __global__ void __launch_bounds__(TileCfg<R>::NT, TileCfg<R>::MINB)
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       const int k1 = j + r * Ns;
-      T W;
-      if constexpr (Loader::kTwiddleTable) {
-        W = __ldg(&twp[((size_t)n2 << G::LOGL1) + k1]);
-      } else {
-        const int m = (n2 * k1) & Lmask;
-        W = cmul(__ldg(&twlo[m & 1023]), __ldg(&twhi[m >> 10]));
-      }
+      const int m = (n2 * k1) & Lmask;
+      const T W = cmul(__ldg(&twlo[m & 1023]), __ldg(&twhi[m >> 10]));
       Pair<T>::st(yb + (((size_t)n2 << G::LOGL1) + k1) * 2, cmul(va[r], W), cmul(vb[r], W));
     }
   }
