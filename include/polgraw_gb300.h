@@ -343,8 +343,9 @@ typedef struct pa_ascent_opts {
 /* Device copies of the data the followup program reads (xDat, DetSSB,
  * sig2, phir, c1..c9 per detector; followup init.c:326-460) and the
  * cos/sin(omr i) tables of its init_arrays() (followup init.c:464-475).
- * Uses sett->N, oms, omr; cfg->precision selects FP32 data with FP64 phase
- * (PA_PREC_MIXED) or every stage in FP64 (PA_PREC_FP64); cfg->device. */
+ * Uses sett->N, oms, omr; cfg->precision selects FP32 sums with the phase in
+ * 64-bit fixed point (PA_PREC_MIXED, whatever cfg->phase_mode is) or every
+ * stage in FP64 (PA_PREC_FP64); cfg->device. */
 pa_followup *pa_followup_create(const pa_settings *sett, const pa_detector *det, int nifo,
                                 const pa_config *cfg, int *status);
 void pa_followup_destroy(pa_followup *fu);

@@ -5,23 +5,21 @@
 // gradient ascent, and the reference simplex amoeba (:971-1174) with its
 // evaluations batched on the device.
 //
-// Device layout (per context):
-//   xd  [nifo][N]      Real   xDat
-//   pos [nifo][N][3]   double DetSSB (x y z interleaved, as the input file)
-//   cm, sm [N]         Real   cos/sin(omr i), FP64-computed (init.c:464-475)
+// The mixed form (FP32 sums, the phase in 64-bit fixed point) is in
+// pa_followup_f32.cuh; the FP64 form is here:
+//   xd  [nifo][N]      xDat
+//   pos [nifo][N][3]   DetSSB (x y z interleaved, as the input file)
+//   cm, sm [N]         cos/sin(omr i) (init.c:464-475)
 // Per evaluated point k:
 //   cand[k]            scalars of the point (phase terms, seeds)
 //   coef[k][d][20]     modvir factors of detector d and their sky derivatives
-//   part[k][p][6|4]    FP64 partial sums of chunk p (fixed order)
+//   part[k][p][6|4]    partial sums of chunk p (fixed order)
 //
 // Work split: chunk p covers kChunk samples of one detector; a CTA stages
 // its chunk in shared memory and each warp runs kCandPerWarp points over it
 // (lanes stride the samples), then reduces across lanes and writes one
-// FP64 partial per point and chunk.  A second kernel sums the partials of a
+// partial per point and chunk.  A second kernel sums the partials of a
 // point in a fixed order, so results do not depend on the batch.
-//
-// Phase: FP64 (the reference's expression, in turns for the mixed form so
-// that the reduction mod 1 is exact), sin/cos in the working precision.
 // Nothing here waits on another CTA or kernel.
 #include <math.h>
 #include <stdarg.h>
@@ -33,6 +31,7 @@
 #include <vector>
 
 #include "../../include/polgraw_gb300.h"
+#include "pa_f32x2.cuh"
 #include "pa_trace.h"
 
 namespace {
@@ -63,27 +62,6 @@ __device__ __forceinline__ unsigned long long fu_turns_fixed(double x) {
 
 thread_local std::string g_fu_create_error;
 
-// Per-point scalars.  Phase terms in FP64; everything else in the working
-// precision R.
-template <typename R>
-struct FuCand {
-  double f, s;          // sgnlo[0], sgnlo[1] (radians)
-  // mixed form, phase in turns: f i/2pi + s i^2/2pi as 64-bit fixed point
-  // (exact integer products), (f + oms + 2 s i) shft/2pi from FP64
-  unsigned long long ffx, sfx;  // f/2pi, s/2pi in fixed-point turns
-  double fo_t, st2;     // (f + oms)/2pi, 2s/2pi
-  double nS[3];         // source unit vector
-  float nSf[3];         // FP32 copy (derivative factors); hi parts of nS
-  float nSl[3];         // lo parts of nS (two-float phase)
-  float foh, fol, s2h, s2l;  // (f + oms)/2pi and 2s/2pi as two floats
-  R nD[3], nA[3];       // d nS / d delta, d nS / d alpha
-  R om0, s2;            // f + oms, 2 s (d phase / d shft = om0 + s2 i)
-  // adjoint seeds: conj(X) parts and the factors of dF/dX, dF/dA
-  R xar, xai, xbr, xbi, ka, kb, qa, qb;
-  int active;
-  int pad;
-};
-
 // Per-detector inputs of the modvir() formula (settings.c:281-325).
 struct FuDet {
   double amod[9];
@@ -92,6 +70,20 @@ struct FuDet {
 
 struct FuDets {
   FuDet d[PA_MAX_DETECTORS];
+};
+
+#include "pa_followup_f32.cuh"
+
+// Per-point scalars of the FP64 form.
+struct FuCand {
+  double f, s;          // sgnlo[0], sgnlo[1] (radians)
+  double nS[3];         // source unit vector
+  double nD[3], nA[3];  // d nS / d delta, d nS / d alpha
+  double om0, s2;       // f + oms, 2 s (d phase / d shft = om0 + s2 i)
+  // adjoint seeds: conj(X) parts and the factors of dF/dX, dF/dA
+  double xar, xai, xbr, xbi, ka, kb, qa, qb;
+  int active;
+  int pad;
 };
 
 // ---------------------------------------------------------------------
@@ -103,13 +95,11 @@ struct FuDets {
 // with c, s the rotated sidereal cos/sin of the sample; d/dalpha acts on
 // (c, s) only: dc/dalpha = -s, ds/dalpha = c.
 // ---------------------------------------------------------------------
-template <typename R>
 __global__ void k_fu_prep(const double* __restrict__ pts, int n, const unsigned char* __restrict__ mask,
-                          FuCand<R>* __restrict__ cand, R* __restrict__ coef, FuDets dets, int nifo,
-                          double oms) {
+                          FuCand* __restrict__ cand, double* __restrict__ coef, FuDets dets, int nifo, double oms) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
-  FuCand<R> c;
+  FuCand c;
   c.active = mask ? (int)mask[k] : 1;
   const double f = pts[4 * k + 0], s = pts[4 * k + 1], de = pts[4 * k + 2], al = pts[4 * k + 3];
   double sa, ca, sd, cd;
@@ -117,30 +107,18 @@ __global__ void k_fu_prep(const double* __restrict__ pts, int n, const unsigned 
   sincos(de, &sd, &cd);
   c.f = f;
   c.s = s;
-  c.ffx = fu_turns_fixed(f * kInv2Pi);
-  c.sfx = fu_turns_fixed(s * kInv2Pi);
-  c.fo_t = (f + oms) * kInv2Pi;
-  c.st2 = 2. * s * kInv2Pi;
   c.nS[0] = ca * cd;
   c.nS[1] = sa * cd;
   c.nS[2] = sd;
-  for (int j = 0; j < 3; j++) {
-    c.nSf[j] = (float)c.nS[j];
-    c.nSl[j] = (float)(c.nS[j] - (double)c.nSf[j]);
-  }
-  c.foh = (float)c.fo_t;
-  c.fol = (float)(c.fo_t - (double)c.foh);
-  c.s2h = (float)c.st2;
-  c.s2l = (float)(c.st2 - (double)c.s2h);
-  c.nD[0] = (R)(-ca * sd);
-  c.nD[1] = (R)(-sa * sd);
-  c.nD[2] = (R)cd;
-  c.nA[0] = (R)(-sa * cd);
-  c.nA[1] = (R)(ca * cd);
-  c.nA[2] = (R)0;
-  c.om0 = (R)(f + oms);
-  c.s2 = (R)(2. * s);
-  c.xar = c.xai = c.xbr = c.xbi = c.ka = c.kb = c.qa = c.qb = (R)0;
+  c.nD[0] = -ca * sd;
+  c.nD[1] = -sa * sd;
+  c.nD[2] = cd;
+  c.nA[0] = -sa * cd;
+  c.nA[1] = ca * cd;
+  c.nA[2] = 0.;
+  c.om0 = f + oms;
+  c.s2 = 2. * s;
+  c.xar = c.xai = c.xbr = c.xbi = c.ka = c.kb = c.qa = c.qb = 0.;
   c.pad = 0;
   cand[k] = c;
   const double c2d = cd * cd, c2sd = sd * cd;
@@ -149,131 +127,57 @@ __global__ void k_fu_prep(const double* __restrict__ pts, int n, const unsigned 
     const double* K = dets.d[d].amod;
     const double cosalfr = ca * dets.d[d].cphir + sa * dets.d[d].sphir;
     const double sinalfr = sa * dets.d[d].cphir - ca * dets.d[d].sphir;
-    R* q = coef + ((size_t)k * nifo + d) * kCoef;
-    q[0] = (R)cosalfr;
-    q[1] = (R)sinalfr;
+    double* q = coef + ((size_t)k * nifo + d) * kCoef;
+    q[0] = cosalfr;
+    q[1] = sinalfr;
     // a
-    q[2] = (R)(K[0] * (2. - c2d));               // A1
-    q[3] = (R)(2. * K[1] * (2. - c2d));          // A2
-    q[4] = (R)(K[2] * c2sd);                     // A3
-    q[5] = (R)(K[3] * c2sd);                     // A4
-    q[6] = (R)(-K[0] * (2. - c2d) + K[4] * c2d); // A0
+    q[2] = K[0] * (2. - c2d);                // A1
+    q[3] = 2. * K[1] * (2. - c2d);           // A2
+    q[4] = K[2] * c2sd;                      // A3
+    q[5] = K[3] * c2sd;                      // A4
+    q[6] = -K[0] * (2. - c2d) + K[4] * c2d;  // A0
     // b
-    q[7] = (R)(K[5] * sd);                       // B1
-    q[8] = (R)(2. * K[6] * sd);                  // B2
-    q[9] = (R)(K[7] * cd);                       // B3
-    q[10] = (R)(K[8] * cd);                      // B4
-    q[11] = (R)(-K[5] * sd);                     // B0
+    q[7] = K[5] * sd;                        // B1
+    q[8] = 2. * K[6] * sd;                   // B2
+    q[9] = K[7] * cd;                        // B3
+    q[10] = K[8] * cd;                       // B4
+    q[11] = -K[5] * sd;                      // B0
     // da/ddelta
-    q[12] = (R)(-2. * K[0] * dc2d);              // D1 (c^2)
-    q[13] = (R)(-2. * K[1] * dc2d);              // D2 (c s)
-    q[14] = (R)(K[2] * dc2sd);                   // D3 (c)
-    q[15] = (R)(K[3] * dc2sd);                   // D4 (s)
-    q[16] = (R)((K[0] + K[4]) * dc2d);           // D0
+    q[12] = -2. * K[0] * dc2d;               // D1 (c^2)
+    q[13] = -2. * K[1] * dc2d;               // D2 (c s)
+    q[14] = K[2] * dc2sd;                    // D3 (c)
+    q[15] = K[3] * dc2sd;                    // D4 (s)
+    q[16] = (K[0] + K[4]) * dc2d;            // D0
     // db/ddelta = E1 c^2 + E2 c s + E3 c + E4 s + E0
     // (E3 = -K7 sd and E4 = -K8 sd are formed in the adjoint kernel)
-    q[17] = (R)(2. * K[5] * cd);                 // E1
-    q[18] = (R)(2. * K[6] * cd);                 // E2
-    q[19] = (R)(-K[5] * cd);                     // E0
+    q[17] = 2. * K[5] * cd;                  // E1
+    q[18] = 2. * K[6] * cd;                  // E2
+    q[19] = -K[5] * cd;                      // E0
   }
 }
 
 // Makes the adjoint pass run for the points selected by need[] with the
 // constants and seeds their last forward pass left in cand[].
-template <typename R>
-__global__ void k_fu_select(FuCand<R>* __restrict__ cand, int n, const unsigned char* __restrict__ need) {
+__global__ void k_fu_select(FuCand* __restrict__ cand, int n, const unsigned char* __restrict__ need) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) cand[k].active = (int)need[k];
 }
 
-template <typename R>
 struct Sample {
-  R x, cm, sm;
-  float r0f, r1f, r2f;   // FP32 copy of the position (derivative factors); hi parts
-  float r0l, r1l, r2l;   // lo parts (two-float phase)
+  double x, cm, sm;
   double r0, r1, r2;
   double di;             // the sample index as FP64
 };
 
-// The phase of sample i for point c, returned as sin and cos in R.
-//   FP64 form: phi = f (i + shft) + (s i) i + (oms + 2 s i) shft
-//              (followup.c:460-462 order, no contraction)
-//   mixed:     phi/2pi = [f i + s i^2]/2pi + (f + oms + 2 s i) shft/2pi with
-//              the bracket in exact 64-bit fixed-point turns and the rest in
-//              FP64 reduced to fixed point; sin/cos of the top 32 bits in
-//              FP32 (sincospif).  Three FP64 operations besides shft.
-template <typename R>
-__device__ __forceinline__ void fu_phase(const FuCand<R>& c, double oms, int i, double di, double shft, R* sn,
-                                         R* cs) {
-  if (sizeof(R) == 8) {
-    const double phi = __dadd_rn(__dadd_rn(__dmul_rn(c.f, __dadd_rn(di, shft)), __dmul_rn(__dmul_rn(c.s, di), di)),
-                                 __dmul_rn(__dadd_rn(oms, __dmul_rn(__dmul_rn(2., c.s), di)), shft));
-    double s_, c_;
-    sincos(phi, &s_, &c_);
-    *sn = (R)s_;
-    *cs = (R)c_;
-  } else {
-    const unsigned long long ui = (unsigned long long)i;
-    const unsigned long long t =
-        c.ffx * ui + c.sfx * (ui * ui) + fu_turns_fixed(fma(c.st2, di, c.fo_t) * shft);
-    float s_, c_;
-    // (the hardware __sincosf measured no faster here, where the FP64 pipe
-    // bounds the kernel, and doubles the error against the FP64 form)
-    sincospif((float)(int)(t >> 32) * 4.656612873077393e-10f, &s_, &c_);
-    *sn = (R)s_;
-    *cs = (R)c_;
-  }
+// The phase of sample i for point c (followup.c:460-462 order, no
+// contraction): phi = f (i + shft) + (s i) i + (oms + 2 s i) shft
+__device__ __forceinline__ void fu_phase(const FuCand& c, double oms, double di, double shft, double* sn, double* cs) {
+  const double phi = __dadd_rn(__dadd_rn(__dmul_rn(c.f, __dadd_rn(di, shft)), __dmul_rn(__dmul_rn(c.s, di), di)),
+                               __dmul_rn(__dadd_rn(oms, __dmul_rn(__dmul_rn(2., c.s), di)), shft));
+  sincos(phi, sn, cs);
 }
 
-// Two-float (compensated) form of the mixed phase: shft = nS.R, the factor
-// (f + oms + 2 s i)/2pi and their product with float pairs (about 44
-// significant bits; error-free products by fma, sums by TwoSum), the product
-// reduced mod 1 exactly (Sterbenz) and added, as fixed point, to the exact
-// integer part [f i + s i^2]/2pi.  No FP64 operation per (point, sample).
-struct F2 {
-  float h, l;
-};
-__device__ __forceinline__ F2 f2_mul(float ah, float al, float bh, float bl) {
-  const float p = __fmul_rn(ah, bh);
-  float e = __fmaf_rn(ah, bh, -p);
-  e = __fmaf_rn(ah, bl, e);
-  e = __fmaf_rn(al, bh, e);
-  return F2{p, e};
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  const float s = __fadd_rn(a.h, b.h);
-  const float bb = __fsub_rn(s, a.h);
-  const float r = __fadd_rn(__fadd_rn(__fsub_rn(a.h, __fsub_rn(s, bb)), __fsub_rn(b.h, bb)), __fadd_rn(a.l, b.l));
-  const float h = __fadd_rn(s, r);
-  return F2{h, __fsub_rn(r, __fsub_rn(h, s))};
-}
-template <typename R>
-__device__ __forceinline__ void fu_phase_ff(const FuCand<R>& c, int i, const Sample<R>& v, R* sn, R* cs) {
-  // shft = sum_k nS_k R_k
-  F2 sh = f2_mul(c.nSf[0], c.nSl[0], v.r0f, v.r0l);
-  sh = f2_add(sh, f2_mul(c.nSf[1], c.nSl[1], v.r1f, v.r1l));
-  sh = f2_add(sh, f2_mul(c.nSf[2], c.nSl[2], v.r2f, v.r2l));
-  // w = (f + oms)/2pi + (2s/2pi) i  (i < 2^24 is exact in FP32)
-  const float fi = (float)i;
-  const F2 w = f2_add(F2{c.foh, c.fol}, f2_mul(c.s2h, c.s2l, fi, 0.f));
-  const F2 t = f2_mul(w.h, w.l, sh.h, sh.l);
-  // t mod 1: h - rint(h) is exact
-  const float fr = __fadd_rn(__fsub_rn(t.h, rintf(t.h)), t.l);
-  const unsigned long long ui = (unsigned long long)i;
-  const unsigned long long tt =
-      c.ffx * ui + c.sfx * (ui * ui) + ((unsigned long long)(long long)__float2ll_rn(fr * 4294967296.f) << 32);
-  // the top 32 bits as an angle in [-pi, pi); hardware sine and cosine
-  // (absolute error <= 2^-21.41 = 3.6e-7 there): this form has no FP64
-  // operation per (point, sample), and the accurate sincospif is its largest
-  // instruction block
-  float s_, c_;
-  __sincosf((float)(int)(tt >> 32) * 1.4629180792671596e-9f, &s_, &c_);  // pi 2^-31
-  *sn = (R)s_;
-  *cs = (R)c_;
-}
-
-template <typename R>
-__device__ __forceinline__ R warp_sum(R v) {
+__device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -287,14 +191,14 @@ __device__ __forceinline__ R warp_sum(R v) {
 //                   + da/dtheta (x ka Re(conj(Xa)E) + 2 qa a) + (b terms) ]
 //   (x 1/sig2), with E = e^{-i phi}, ka = 2 seed/A, qa = -seed |Xa|^2/A^2.
 // ---------------------------------------------------------------------
-template <typename R, bool ADJ, bool FF = false>
-__global__ void __launch_bounds__(kThreads) k_fu_sums(const R* __restrict__ xd, const double* __restrict__ pos,
-                                                      const R* __restrict__ cmf, const R* __restrict__ smf,
-                                                      const FuCand<R>* __restrict__ cand, const R* __restrict__ coef,
+template <bool ADJ>
+__global__ void __launch_bounds__(kThreads) k_fu_sums(const double* __restrict__ xd, const double* __restrict__ pos,
+                                                      const double* __restrict__ cmf, const double* __restrict__ smf,
+                                                      const FuCand* __restrict__ cand, const double* __restrict__ coef,
                                                       FuDets dets, int n, int N, int nifo, int nch, double oms,
                                                       double* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char fu_smem[];
-  Sample<R>* sh = reinterpret_cast<Sample<R>*>(fu_smem);
+  Sample* sh = reinterpret_cast<Sample*>(fu_smem);
   const int P = nifo * nch;
   const int p = blockIdx.x;
   const int d = p / nch;
@@ -302,7 +206,7 @@ __global__ void __launch_bounds__(kThreads) k_fu_sums(const R* __restrict__ xd, 
   const int cnt = min(kChunk, N - base);
   for (int j = threadIdx.x; j < cnt; j += kThreads) {
     const int i = base + j;
-    Sample<R> v;
+    Sample v;
     v.x = xd[(size_t)d * N + i];
     v.cm = cmf[i];
     v.sm = smf[i];
@@ -310,49 +214,37 @@ __global__ void __launch_bounds__(kThreads) k_fu_sums(const R* __restrict__ xd, 
     v.r0 = r[0];
     v.r1 = r[1];
     v.r2 = r[2];
-    v.r0f = (float)v.r0;
-    v.r1f = (float)v.r1;
-    v.r2f = (float)v.r2;
-    v.r0l = (float)(v.r0 - (double)v.r0f);
-    v.r1l = (float)(v.r1 - (double)v.r1f);
-    v.r2l = (float)(v.r2 - (double)v.r2f);
     v.di = (double)i;
     sh[j] = v;
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double is2 = dets.d[d].inv_sig2;
-  const R k7 = (R)dets.d[d].amod[7], k8 = (R)dets.d[d].amod[8];
+  const double k7 = dets.d[d].amod[7], k8 = dets.d[d].amod[8];
   for (int q = 0; q < kCandPerWarp; q++) {
     const int k = blockIdx.y * kCandPerCta + warp * kCandPerWarp + q;
     if (k >= n) break;
-    const FuCand<R> c = cand[k];
+    const FuCand c = cand[k];
     if (!c.active) continue;
-    const R* cf = coef + ((size_t)k * nifo + d) * kCoef;
-    R Q[kCoef];
+    const double* cf = coef + ((size_t)k * nifo + d) * kCoef;
+    double Q[kCoef];
 #pragma unroll
     for (int t = 0; t < kCoef; t++) Q[t] = cf[t];
-    const R cosalfr = Q[0], sinalfr = Q[1];
-    R acc[6] = {(R)0, (R)0, (R)0, (R)0, (R)0, (R)0};
-    const R sd_ = (R)c.nS[2];  // sin(delta), for E3 = -K7 sd, E4 = -K8 sd
+    const double cosalfr = Q[0], sinalfr = Q[1];
+    double acc[6] = {0., 0., 0., 0., 0., 0.};
+    const double sd_ = c.nS[2];  // sin(delta), for E3 = -K7 sd, E4 = -K8 sd
     for (int j = lane; j < cnt; j += 32) {
-      const Sample<R> v = sh[j];
-      const int i = base + j;
-      const R cc = cosalfr * v.cm + sinalfr * v.sm;
-      const R ss = sinalfr * v.cm - cosalfr * v.sm;
-      const R c2 = cc * cc, cs = cc * ss;
-      const R a = (R)2 * Q[2] * c2 + Q[3] * cs + Q[4] * cc + Q[5] * ss + Q[6];
-      const R b = (R)2 * Q[7] * c2 + Q[8] * cs + Q[9] * cc + Q[10] * ss + Q[11];
-      R sn, co;
-      double shft = 0.;
-      if (FF) {
-        fu_phase_ff<R>(c, i, v, &sn, &co);
-      } else {
-        shft = c.nS[0] * v.r0 + c.nS[1] * v.r1 + c.nS[2] * v.r2;
-        fu_phase<R>(c, oms, i, v.di, shft, &sn, &co);
-      }
+      const Sample v = sh[j];
+      const double cc = cosalfr * v.cm + sinalfr * v.sm;
+      const double ss = sinalfr * v.cm - cosalfr * v.sm;
+      const double c2 = cc * cc, cs = cc * ss;
+      const double a = 2. * Q[2] * c2 + Q[3] * cs + Q[4] * cc + Q[5] * ss + Q[6];
+      const double b = 2. * Q[7] * c2 + Q[8] * cs + Q[9] * cc + Q[10] * ss + Q[11];
+      double sn, co;
+      const double shft = c.nS[0] * v.r0 + c.nS[1] * v.r1 + c.nS[2] * v.r2;
+      fu_phase(c, oms, v.di, shft, &sn, &co);
       if (!ADJ) {
-        const R xa = v.x * a, xb = v.x * b;
+        const double xa = v.x * a, xb = v.x * b;
         acc[0] += xa * co;
         acc[1] -= xa * sn;
         acc[2] += xb * co;
@@ -361,29 +253,23 @@ __global__ void __launch_bounds__(kThreads) k_fu_sums(const R* __restrict__ xd, 
         acc[5] += b * b;
       } else {
         // conj(X) E with E = co - i sn
-        const R rea = c.xar * co - c.xai * sn, ima = -(c.xar * sn + c.xai * co);
-        const R reb = c.xbr * co - c.xbi * sn, imb = -(c.xbr * sn + c.xbi * co);
-        const R gph = v.x * (c.ka * a * ima + c.kb * b * imb);
-        const R ga = v.x * c.ka * rea + (R)2 * c.qa * a;
-        const R gb = v.x * c.kb * reb + (R)2 * c.qb * b;
-        const R fi = (R)i;
-        // derivative factors in the working precision (FP32 copies of the
-        // position in the mixed form: no per-sample conversions)
-        const R r0 = sizeof(R) == 4 ? (R)v.r0f : (R)v.r0, r1 = sizeof(R) == 4 ? (R)v.r1f : (R)v.r1,
-                r2 = sizeof(R) == 4 ? (R)v.r2f : (R)v.r2;
-        const R sh_ = (sizeof(R) == 4 || FF) ? (R)(c.nSf[0] * v.r0f + c.nSf[1] * v.r1f + c.nSf[2] * v.r2f)
-                                             : (R)shft;
-        const R sh_de = c.nD[0] * r0 + c.nD[1] * r1 + c.nD[2] * r2;
-        const R sh_al = c.nA[0] * r0 + c.nA[1] * r1;
-        const R om = c.om0 + c.s2 * fi;
+        const double rea = c.xar * co - c.xai * sn, ima = -(c.xar * sn + c.xai * co);
+        const double reb = c.xbr * co - c.xbi * sn, imb = -(c.xbr * sn + c.xbi * co);
+        const double gph = v.x * (c.ka * a * ima + c.kb * b * imb);
+        const double ga = v.x * c.ka * rea + 2. * c.qa * a;
+        const double gb = v.x * c.kb * reb + 2. * c.qb * b;
+        const double fi = v.di;
+        const double sh_de = c.nD[0] * v.r0 + c.nD[1] * v.r1 + c.nD[2] * v.r2;
+        const double sh_al = c.nA[0] * v.r0 + c.nA[1] * v.r1;
+        const double om = c.om0 + c.s2 * fi;
         // d a / d alpha, d b / d alpha
-        const R a_al = -ss * ((R)4 * Q[2] * cc + Q[3] * ss + Q[4]) + cc * (Q[3] * cc + Q[5]);
-        const R b_al = -ss * ((R)4 * Q[7] * cc + Q[8] * ss + Q[9]) + cc * (Q[8] * cc + Q[10]);
+        const double a_al = -ss * (4. * Q[2] * cc + Q[3] * ss + Q[4]) + cc * (Q[3] * cc + Q[5]);
+        const double b_al = -ss * (4. * Q[7] * cc + Q[8] * ss + Q[9]) + cc * (Q[8] * cc + Q[10]);
         // d a / d delta, d b / d delta
-        const R a_de = Q[12] * c2 + Q[13] * cs + Q[14] * cc + Q[15] * ss + Q[16];
-        const R b_de = Q[17] * c2 + Q[18] * cs - k7 * sd_ * cc - k8 * sd_ * ss + Q[19];
-        acc[0] += gph * (fi + sh_);
-        acc[1] += gph * (fi * fi + (R)2 * fi * sh_);
+        const double a_de = Q[12] * c2 + Q[13] * cs + Q[14] * cc + Q[15] * ss + Q[16];
+        const double b_de = Q[17] * c2 + Q[18] * cs - k7 * sd_ * cc - k8 * sd_ * ss + Q[19];
+        acc[0] += gph * (fi + shft);
+        acc[1] += gph * (fi * fi + 2. * fi * shft);
         acc[2] += gph * om * sh_de + ga * a_de + gb * b_de;
         acc[3] += gph * om * sh_al + ga * a_al + gb * b_al;
       }
@@ -392,8 +278,8 @@ __global__ void __launch_bounds__(kThreads) k_fu_sums(const R* __restrict__ xd, 
     double* out = part + ((size_t)k * P + p) * NA;
 #pragma unroll
     for (int t = 0; t < NA; t++) {
-      const R v = warp_sum<R>(acc[t]);
-      if (lane == 0) out[t] = (double)v * is2;
+      const double v = warp_sum(acc[t]);
+      if (lane == 0) out[t] = v * is2;
     }
   }
 }
@@ -410,9 +296,8 @@ __device__ __forceinline__ double fixed_sum(const double* __restrict__ p, int P,
 
 // F and fstat_out (followup.c:508-529) per point; res[k] = {Xa, Xb, A, B}
 // kept for the adjoint.  One warp per point.
-template <typename R>
 __global__ void k_fu_final(const double* __restrict__ part, const double* __restrict__ pts,
-                           FuCand<R>* __restrict__ cand, int n, int P, double* __restrict__ res,
+                           FuCand* __restrict__ cand, int n, int P, double* __restrict__ res,
                            double* __restrict__ Fo, double* __restrict__ out, const double* __restrict__ seed) {
   const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -439,19 +324,18 @@ __global__ void k_fu_final(const double* __restrict__ part, const double* __rest
   }
   // seeds of the adjoint pass
   const double sd = seed ? seed[k] : 1.0;
-  FuCand<R>& c = cand[k];
-  c.xar = (R)xr;
-  c.xai = (R)xi;
-  c.xbr = (R)yr;
-  c.xbi = (R)yi;
-  c.ka = (R)(2. * sd / A);
-  c.kb = (R)(2. * sd / B);
-  c.qa = (R)(-sd * (xr * xr + xi * xi) / (A * A));
-  c.qb = (R)(-sd * (yr * yr + yi * yi) / (B * B));
+  FuCand& c = cand[k];
+  c.xar = xr;
+  c.xai = xi;
+  c.xbr = yr;
+  c.xbi = yi;
+  c.ka = (2. * sd / A);
+  c.kb = (2. * sd / B);
+  c.qa = (-sd * (xr * xr + xi * xi) / (A * A));
+  c.qb = (-sd * (yr * yr + yi * yi) / (B * B));
 }
 
-template <typename R>
-__global__ void k_fu_final_adj(const double* __restrict__ part, const FuCand<R>* __restrict__ cand, int n, int P,
+__global__ void k_fu_final_adj(const double* __restrict__ part, const FuCand* __restrict__ cand, int n, int P,
                                double* __restrict__ grad) {
   const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -606,22 +490,34 @@ __global__ void k_asc_export(const AscentState* __restrict__ st, int n, double* 
 struct pa_followup {
   int dev = 0;
   bool fp64 = false;
-  bool ffphase = false;  // mixed form with the two-float phase
   int N = 0, nifo = 0, nch = 0;
   double oms = 0.;
   FuDets dets;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  void* xd = nullptr;
   double* pos = nullptr;
-  void* cm = nullptr;
-  void* sm = nullptr;
+  // FP64 form
+  double* xd = nullptr;
+  double* cm = nullptr;
+  double* sm = nullptr;
+  // mixed form: samples [nifo][nch][2][1024] float4 {x u_0 .. x u_3},
+  // {x u_4, r}, the chunks' motion, and bounds of r and of the curvature
+  float4* samp = nullptr;
+  fu32::Chunk* chunk = nullptr;
+  fu32::Gram gram;
+  double restmax = 0., curvmax = 0.;
+  int adj_fast = 1;
   // per-batch buffers (grown on demand)
   int cap = 0;
   double* pts = nullptr;
-  void* cand = nullptr;
-  void* coef = nullptr;
-  double* part = nullptr;
+  FuCand* cand = nullptr;        // FP64 form
+  fu32::Point* point = nullptr;  // mixed form
+  double* coef = nullptr;
+  void* part = nullptr;
+  double* totals = nullptr;      // mixed form: U, W per point and detector
+  float* seeds = nullptr;        // mixed form: adjoint factors per point and detector
+  int* list = nullptr;           // mixed form: active points
+  int* nlist = nullptr;
   double* res = nullptr;
   double* F = nullptr;
   double* out = nullptr;
@@ -655,17 +551,18 @@ static int fu_fail(pa_followup* f, int code, const char* fmt, ...) {
     if (e_ != cudaSuccess) return fu_fail(f, PA_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e_)); \
   } while (0)
 
-static size_t fu_rsz(const pa_followup* f) { return f->fp64 ? 8 : 4; }
-
 static void fu_free_batch(pa_followup* f) {
-  void* ps[] = {f->pts, f->cand, f->coef, f->part, f->res, f->F, f->out, f->grad, f->seed,
-                f->mask, f->need, f->asc, f->iters, f->counter, f->trial};
+  void* ps[] = {f->pts, f->cand, f->point, f->coef, f->part, f->totals, f->seeds, f->list, f->nlist, f->res, f->F,
+                f->out, f->grad, f->seed, f->mask, f->need, f->asc, f->iters, f->counter, f->trial};
   for (void* p : ps)
     if (p) cudaFree(p);
   f->pts = nullptr;
   f->cand = nullptr;
-  f->coef = nullptr;
+  f->point = nullptr;
+  f->coef = f->totals = nullptr;
   f->part = nullptr;
+  f->seeds = nullptr;
+  f->list = f->nlist = nullptr;
   f->res = f->F = f->out = f->grad = f->seed = f->trial = nullptr;
   f->mask = f->need = nullptr;
   f->asc = nullptr;
@@ -678,13 +575,21 @@ static int fu_reserve(pa_followup* f, int n) {
   fu_free_batch(f);
   const int c = std::max(n, 64);
   const size_t P = (size_t)f->nifo * f->nch;
-  const size_t candsz = f->fp64 ? sizeof(FuCand<double>) : sizeof(FuCand<float>);
 #define FALLOC(ptr, bytes) FCK(cudaMalloc((void**)&(ptr), (bytes)), "cudaMalloc")
   FALLOC(f->pts, sizeof(double) * 4 * c);
-  FALLOC(f->cand, candsz * c);
-  FALLOC(f->coef, fu_rsz(f) * kCoef * f->nifo * (size_t)c);
-  FALLOC(f->part, sizeof(double) * 6 * P * c);
-  FALLOC(f->res, sizeof(double) * 6 * c);
+  FALLOC(f->coef, sizeof(double) * kCoef * f->nifo * (size_t)c);
+  if (f->fp64) {
+    FALLOC(f->cand, sizeof(FuCand) * c);
+    FALLOC(f->part, sizeof(double) * 6 * P * c);
+    FALLOC(f->res, sizeof(double) * 6 * c);
+  } else {
+    FALLOC(f->point, sizeof(fu32::Point) * c);
+    FALLOC(f->part, sizeof(float) * fu32::kPartF * P * c);
+    FALLOC(f->totals, sizeof(double) * 2 * fu32::kU * f->nifo * (size_t)c);
+    FALLOC(f->seeds, sizeof(float) * 2 * fu32::kU * f->nifo * (size_t)c);
+    FALLOC(f->list, sizeof(int) * c);
+    FALLOC(f->nlist, sizeof(int));
+  }
   FALLOC(f->F, sizeof(double) * c);
   FALLOC(f->out, sizeof(double) * 11 * c);
   FALLOC(f->grad, sizeof(double) * 4 * c);
@@ -700,66 +605,81 @@ static int fu_reserve(pa_followup* f, int n) {
   return PA_OK;
 }
 
-template <typename R>
-static size_t fu_smem() {
-  return sizeof(Sample<R>) * kChunk;
+constexpr size_t kFuSmem = sizeof(Sample) * kChunk;
+
+// One launch of the FP64 form's sums.
+template <bool ADJ>
+static void fu_sums(pa_followup* f, int n, dim3 grid) {
+  k_fu_sums<ADJ><<<grid, kThreads, kFuSmem, f->stream>>>(f->xd, f->pos, f->cm, f->sm, f->cand, f->coef, f->dets, n, f->N,
+                                                         f->nifo, f->nch, f->oms, (double*)f->part);
 }
 
-// One launch of the sums kernel in the context's phase form.
-template <typename R, bool ADJ>
-static void fu_sums(pa_followup* f, int n, dim3 grid) {
-  FuCand<R>* cand = (FuCand<R>*)f->cand;
-  if (sizeof(R) == 4 && f->ffphase)
-    k_fu_sums<R, ADJ, true><<<grid, kThreads, fu_smem<R>(), f->stream>>>(
-        (const R*)f->xd, f->pos, (const R*)f->cm, (const R*)f->sm, cand, (const R*)f->coef, f->dets, n, f->N,
-        f->nifo, f->nch, f->oms, f->part);
-  else
-    k_fu_sums<R, ADJ, false><<<grid, kThreads, fu_smem<R>(), f->stream>>>(
-        (const R*)f->xd, f->pos, (const R*)f->cm, (const R*)f->sm, cand, (const R*)f->coef, f->dets, n, f->N,
-        f->nifo, f->nch, f->oms, f->part);
+// The mixed form's adjoint pass for n points, or those of the list.
+static void fu32_adjoint(pa_followup* f, int n, const int* list) {
+  const int P = f->nifo * f->nch;
+  fu32::k_sums<true><<<fu32::sum_grid(true, n, P), fu32::kThreads, 0, f->stream>>>(
+      f->samp, f->chunk, f->pos, f->point, f->seeds, list, f->nlist, n, f->N, f->nifo, f->nch, f->adj_fast,
+      (float*)f->part);
+  fu32::k_final_adj<<<(n + 7) / 8, 256, 0, f->stream>>>((const float*)f->part, f->point, f->coef, f->chunk, f->dets, list,
+                                                        f->nlist, n, f->nifo, f->nch, f->adj_fast, f->oms, f->totals,
+                                                        f->grad);
+  f->launches += 2;
 }
 
 // Forward (and optionally adjoint) evaluation of n points already in
-// f->pts; mask (device, may be null) selects the active points.
-template <typename R>
-static int fu_eval_t(pa_followup* f, int n, const unsigned char* mask, bool want_out, bool adjoint,
-                     const double* seed_dev) {
+// f->pts; mask (device, may be null) selects the active points; grad: an
+// adjoint pass follows, here or later.
+static int fu_eval(pa_followup* f, int n, const unsigned char* mask, bool want_out, bool adjoint,
+                   const double* seed_dev, bool grad) {
   const int P = f->nifo * f->nch;
-  FuCand<R>* cand = (FuCand<R>*)f->cand;
-  k_fu_prep<R><<<(n + 127) / 128, 128, 0, f->stream>>>(f->pts, n, mask, cand, (R*)f->coef, f->dets, f->nifo,
-                                                          f->oms);
-  dim3 grid(P, (n + kCandPerCta - 1) / kCandPerCta);
-  fu_sums<R, false>(f, n, grid);
-  k_fu_final<R><<<(n + 7) / 8, 256, 0, f->stream>>>(f->part, f->pts, cand, n, P, f->res, f->F,
-                                                     want_out ? f->out : nullptr, seed_dev);
-  f->launches += 3;
-  if (adjoint) {
-    fu_sums<R, true>(f, n, grid);
-    k_fu_final_adj<R><<<(n + 7) / 8, 256, 0, f->stream>>>(f->part, cand, n, P, f->grad);
-    f->launches += 2;
+  if (f->fp64) {
+    double* part = (double*)f->part;
+    k_fu_prep<<<(n + 127) / 128, 128, 0, f->stream>>>(f->pts, n, mask, f->cand, f->coef, f->dets, f->nifo, f->oms);
+    dim3 grid(P, (n + kCandPerCta - 1) / kCandPerCta);
+    fu_sums<false>(f, n, grid);
+    k_fu_final<<<(n + 7) / 8, 256, 0, f->stream>>>(part, f->pts, f->cand, n, P, f->res, f->F, want_out ? f->out : nullptr,
+                                                   seed_dev);
+    f->launches += 3;
+    if (adjoint) {
+      fu_sums<true>(f, n, grid);
+      k_fu_final_adj<<<(n + 7) / 8, 256, 0, f->stream>>>(part, f->cand, n, P, f->grad);
+      f->launches += 2;
+    }
+  } else {
+    int* list = mask ? f->list : nullptr;
+    if (list) FCK(cudaMemsetAsync(f->nlist, 0, sizeof(int), f->stream), "memset");
+    auto prep = grad ? fu32::k_prep<true> : fu32::k_prep<false>;
+    prep<<<(n + 7) / 8, 64, 0, f->stream>>>(f->pts, n, mask, f->point, f->coef, f->dets, f->gram, f->nifo, f->oms,
+                                            f->restmax, f->curvmax, f->N, list, f->nlist);
+    fu32::k_sums<false><<<fu32::sum_grid(false, n, P), fu32::kThreads, 0, f->stream>>>(
+        f->samp, f->chunk, f->pos, f->point, nullptr, list, f->nlist, n, f->N, f->nifo, f->nch, 1, (float*)f->part);
+    fu32::k_final<<<(n + 7) / 8, 256, 0, f->stream>>>((const float*)f->part, f->pts, f->point, f->coef, f->dets, list,
+                                                      f->nlist, n, f->nifo, f->nch, f->totals, f->F,
+                                                      want_out ? f->out : nullptr, seed_dev, f->seeds);
+    f->launches += 3;
+    if (adjoint) fu32_adjoint(f, n, list);
   }
   FCK(cudaGetLastError(), "followup launch");
   return PA_OK;
 }
 
-// Adjoint pass only, for the points selected by need[] (device).
-template <typename R>
-static int fu_adjoint_t(pa_followup* f, int n, const unsigned char* need) {
+// Adjoint pass only, for the points selected by need[] (device), with the
+// constants and seeds of their last forward pass.
+static int fu_adjoint(pa_followup* f, int n, const unsigned char* need) {
   const int P = f->nifo * f->nch;
-  FuCand<R>* cand = (FuCand<R>*)f->cand;
-  k_fu_select<R><<<(n + 255) / 256, 256, 0, f->stream>>>(cand, n, need);
-  dim3 grid(P, (n + kCandPerCta - 1) / kCandPerCta);
-  fu_sums<R, true>(f, n, grid);
-  k_fu_final_adj<R><<<(n + 7) / 8, 256, 0, f->stream>>>(f->part, cand, n, P, f->grad);
-  f->launches += 3;
+  if (f->fp64) {
+    k_fu_select<<<(n + 255) / 256, 256, 0, f->stream>>>(f->cand, n, need);
+    fu_sums<true>(f, n, dim3(P, (n + kCandPerCta - 1) / kCandPerCta));
+    k_fu_final_adj<<<(n + 7) / 8, 256, 0, f->stream>>>((const double*)f->part, f->cand, n, P, f->grad);
+    f->launches += 3;
+  } else {
+    FCK(cudaMemsetAsync(f->nlist, 0, sizeof(int), f->stream), "memset");
+    fu32::k_list<<<(n + 255) / 256, 256, 0, f->stream>>>(need, n, f->list, f->nlist);
+    f->launches++;
+    fu32_adjoint(f, n, f->list);
+  }
   FCK(cudaGetLastError(), "followup adjoint launch");
   return PA_OK;
-}
-
-static int fu_eval(pa_followup* f, int n, const unsigned char* mask, bool want_out, bool adjoint,
-                   const double* seed_dev) {
-  return f->fp64 ? fu_eval_t<double>(f, n, mask, want_out, adjoint, seed_dev)
-                 : fu_eval_t<float>(f, n, mask, want_out, adjoint, seed_dev);
 }
 
 static int fu_begin(pa_followup* f, int n) {
@@ -777,6 +697,67 @@ static int fu_end(pa_followup* f) {
   FCK(cudaEventElapsedTime(&ms, f->ev0, f->ev1), "event time");
   f->last_ms += ms;
   return PA_OK;
+}
+
+// The mixed form's inputs: per chunk the parabola through the first, middle and
+// last position, and per sample x u_k and the rest of the position; the matrix
+// of the u_k; the bounds that the fast phase is chosen by.
+static void fu32_samples(pa_followup* f, const pa_detector* det, const std::vector<double>& cw,
+                         const std::vector<double>& sw, std::vector<float4>* samp, std::vector<fu32::Chunk>* chunk) {
+  const int N = f->N, L = fu32::kChunk;
+  samp->assign((size_t)f->nifo * f->nch * 2 * L, make_float4(0.f, 0.f, 0.f, 0.f));
+  chunk->resize((size_t)f->nifo * f->nch);
+  memset(&f->gram, 0, sizeof(f->gram));
+  for (int i = 0; i < N; i++) {
+    const double c = cw[i], s = sw[i], u[fu32::kU] = {1., c, s, c * c - s * s, 2. * s * c};
+    for (int k = 0; k < fu32::kU; k++)
+      for (int l = 0; l <= k; l++) f->gram.g[k][l] += u[k] * u[l];
+  }
+  for (int k = 0; k < fu32::kU; k++)
+    for (int l = 0; l < k; l++) f->gram.g[l][k] = f->gram.g[k][l];
+  f->restmax = f->curvmax = 0.;
+  for (int p = 0; p < f->nifo * f->nch; p++) {
+    const int d = p / f->nch, base = (p - d * f->nch) * L, cnt = std::min(L, N - base);
+    fu32::Chunk& h = (*chunk)[p];
+    const double* R = det[d].DetSSB + 3 * (size_t)base;
+    const int e = cnt - 1, m = e / 2;
+    double curv = 0.;
+    for (int t = 0; t < 3; t++) {
+      // Newton's divided differences on samples 0, m, e
+      const double y0 = R[t], ym = R[3 * (size_t)m + t], ye = R[3 * (size_t)e + t];
+      double V = 0., A = 0.;
+      if (m > 0) {
+        const double d1 = (ym - y0) / m;
+        A = ((ye - ym) / (e - m) - d1) / e;
+        V = d1 - A * m;
+      } else if (e > 0) {
+        V = (ye - y0) / e;
+      }
+      h.R0[t] = y0;
+      h.V[t] = V;
+      h.A[t] = A;
+      curv += A * A;
+    }
+    // (not std::max: a NaN has to stay)
+    const double cv = sqrt(curv);
+    if (!(cv <= f->curvmax)) f->curvmax = cv;
+    float4* s0 = &(*samp)[(size_t)p * 2 * L];
+    for (int j = 0; j < cnt; j++) {
+      const int i = base + j;
+      const double x = det[d].xDat[i], c = cw[i], s = sw[i];
+      double r[3], rr = 0.;
+      for (int t = 0; t < 3; t++) {
+        r[t] = R[3 * (size_t)j + t] - ((h.A[t] * j + h.V[t]) * j + h.R0[t]);
+        rr += r[t] * r[t];
+      }
+      const double rv = sqrt(rr);
+      if (!(rv <= f->restmax)) f->restmax = rv;
+      s0[j] = make_float4((float)x, (float)(x * c), (float)(x * s), (float)(x * (c * c - s * s)));
+      s0[L + j] = make_float4((float)(x * (2. * s * c)), (float)r[0], (float)r[1], (float)r[2]);
+    }
+  }
+  // sum g j r is left out of sum g i R: 2 x 1024 restmax against i^2 ~ N^2 / 12
+  f->adj_fast = 2. * L * f->restmax <= (double)N * N / 12. * 5.96e-8;
 }
 
 extern "C" {
@@ -801,7 +782,6 @@ pa_followup* pa_followup_create(const pa_settings* sett, const pa_detector* det,
   f = new pa_followup();
   f->dev = c.device;
   f->fp64 = c.precision == PA_PREC_FP64;
-  f->ffphase = !f->fp64 && c.phase_mode == PA_PHASE_FF;
   f->N = sett->N;
   f->nifo = nifo;
   f->nch = (sett->N + kChunk - 1) / kChunk;
@@ -825,43 +805,44 @@ pa_followup* pa_followup_create(const pa_settings* sett, const pa_detector* det,
   if ((e = cudaEventCreate(&f->ev0)) != cudaSuccess) return bail("event", e);
   if ((e = cudaEventCreate(&f->ev1)) != cudaSuccess) return bail("event", e);
   const int N = sett->N;
-  const size_t rs = f->fp64 ? 8 : 4;
-  if ((e = cudaMalloc(&f->xd, rs * nifo * (size_t)N)) != cudaSuccess) return bail("cudaMalloc", e);
   if ((e = cudaMalloc((void**)&f->pos, sizeof(double) * 3 * nifo * (size_t)N)) != cudaSuccess)
     return bail("cudaMalloc", e);
-  if ((e = cudaMalloc(&f->cm, rs * N)) != cudaSuccess) return bail("cudaMalloc", e);
-  if ((e = cudaMalloc(&f->sm, rs * N)) != cudaSuccess) return bail("cudaMalloc", e);
-  // host staging: xDat and cos/sin(omr i) (followup init.c:470-475) in the
-  // working precision, DetSSB as is
-  std::vector<double> xd64((size_t)nifo * N), c64(N), s64(N);
-  for (int d = 0; d < nifo; d++) memcpy(&xd64[(size_t)d * N], det[d].xDat, sizeof(double) * N);
+  for (int d = 0; d < nifo; d++)
+    if ((e = cudaMemcpy(f->pos + (size_t)d * 3 * N, det[d].DetSSB, sizeof(double) * 3 * N,
+                        cudaMemcpyHostToDevice)) != cudaSuccess)
+      return bail("upload", e);
+  // cos/sin(omr i) (followup init.c:470-475)
+  std::vector<double> c64(N), s64(N);
   for (int i = 0; i < N; i++) {
     const double omrt = sett->omr * i;
     c64[i] = cos(omrt);
     s64[i] = sin(omrt);
   }
-  auto up = [&](void* dst, const std::vector<double>& src) -> cudaError_t {
-    if (f->fp64) return cudaMemcpy(dst, src.data(), sizeof(double) * src.size(), cudaMemcpyHostToDevice);
-    std::vector<float> t(src.size());
-    for (size_t j = 0; j < src.size(); j++) t[j] = (float)src[j];
-    return cudaMemcpy(dst, t.data(), sizeof(float) * t.size(), cudaMemcpyHostToDevice);
-  };
-  if ((e = up(f->xd, xd64)) != cudaSuccess) return bail("upload", e);
-  if ((e = up(f->cm, c64)) != cudaSuccess) return bail("upload", e);
-  if ((e = up(f->sm, s64)) != cudaSuccess) return bail("upload", e);
-  for (int d = 0; d < nifo; d++)
-    if ((e = cudaMemcpy(f->pos + (size_t)d * 3 * N, det[d].DetSSB, sizeof(double) * 3 * N,
-                        cudaMemcpyHostToDevice)) != cudaSuccess)
-      return bail("upload", e);
-  const size_t smem = f->fp64 ? fu_smem<double>() : fu_smem<float>();
   if (f->fp64) {
-    cudaFuncSetAttribute(k_fu_sums<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_fu_sums<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if ((e = cudaMalloc((void**)&f->xd, sizeof(double) * nifo * (size_t)N)) != cudaSuccess) return bail("cudaMalloc", e);
+    if ((e = cudaMalloc((void**)&f->cm, sizeof(double) * N)) != cudaSuccess) return bail("cudaMalloc", e);
+    if ((e = cudaMalloc((void**)&f->sm, sizeof(double) * N)) != cudaSuccess) return bail("cudaMalloc", e);
+    for (int d = 0; d < nifo; d++)
+      if ((e = cudaMemcpy(f->xd + (size_t)d * N, det[d].xDat, sizeof(double) * N, cudaMemcpyHostToDevice)) != cudaSuccess)
+        return bail("upload", e);
+    if ((e = cudaMemcpy(f->cm, c64.data(), sizeof(double) * N, cudaMemcpyHostToDevice)) != cudaSuccess)
+      return bail("upload", e);
+    if ((e = cudaMemcpy(f->sm, s64.data(), sizeof(double) * N, cudaMemcpyHostToDevice)) != cudaSuccess)
+      return bail("upload", e);
+    cudaFuncSetAttribute(k_fu_sums<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFuSmem);
+    cudaFuncSetAttribute(k_fu_sums<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFuSmem);
   } else {
-    cudaFuncSetAttribute(k_fu_sums<float, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_fu_sums<float, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_fu_sums<float, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_fu_sums<float, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    std::vector<float4> samp;
+    std::vector<fu32::Chunk> chunk;
+    fu32_samples(f, det, c64, s64, &samp, &chunk);
+    if ((e = cudaMalloc((void**)&f->samp, sizeof(float4) * samp.size())) != cudaSuccess) return bail("cudaMalloc", e);
+    if ((e = cudaMalloc((void**)&f->chunk, sizeof(fu32::Chunk) * chunk.size())) != cudaSuccess)
+      return bail("cudaMalloc", e);
+    if ((e = cudaMemcpy(f->samp, samp.data(), sizeof(float4) * samp.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+      return bail("upload", e);
+    if ((e = cudaMemcpy(f->chunk, chunk.data(), sizeof(fu32::Chunk) * chunk.size(), cudaMemcpyHostToDevice)) !=
+        cudaSuccess)
+      return bail("upload", e);
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return bail("set-up", e);
   if (status) *status = PA_OK;
@@ -873,7 +854,7 @@ void pa_followup_destroy(pa_followup* f) {
   cudaSetDevice(f->dev);
   if (f->stream) cudaStreamSynchronize(f->stream);
   fu_free_batch(f);
-  void* ps[] = {f->xd, f->pos, f->cm, f->sm};
+  void* ps[] = {f->xd, f->pos, f->cm, f->sm, f->samp, f->chunk};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (f->ev0) cudaEventDestroy(f->ev0);
@@ -897,7 +878,7 @@ int pa_fstatnet(pa_followup* f, const double* sgnlo, int n, double* out) {
   int rc = fu_begin(f, n);
   if (rc) return rc;
   FCK(cudaMemcpyAsync(f->pts, sgnlo, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, f->stream), "copy");
-  if ((rc = fu_eval(f, n, nullptr, true, false, nullptr))) return rc;
+  if ((rc = fu_eval(f, n, nullptr, true, false, nullptr, false))) return rc;
   FCK(cudaMemcpyAsync(out, f->out, sizeof(double) * 11 * n, cudaMemcpyDeviceToHost, f->stream), "copy");
   return fu_end(f);
 }
@@ -912,7 +893,7 @@ int pa_fstatnet_grad(pa_followup* f, const double* sgnlo, int n, const double* s
   FCK(cudaMemcpyAsync(f->pts, sgnlo, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, f->stream), "copy");
   if (seed)
     FCK(cudaMemcpyAsync(f->seed, seed, sizeof(double) * n, cudaMemcpyHostToDevice, f->stream), "copy");
-  if ((rc = fu_eval(f, n, nullptr, false, true, seed ? f->seed : nullptr))) return rc;
+  if ((rc = fu_eval(f, n, nullptr, false, true, seed ? f->seed : nullptr, true))) return rc;
   FCK(cudaMemcpyAsync(F, f->F, sizeof(double) * n, cudaMemcpyDeviceToHost, f->stream), "copy");
   FCK(cudaMemcpyAsync(grad, f->grad, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, f->stream), "copy");
   return fu_end(f);
@@ -932,7 +913,7 @@ int pa_followup_ascent(pa_followup* f, double* sgnlo, int n, const pa_ascent_opt
   if (rc) return rc;
   const int nb = (n + 255) / 256;
   FCK(cudaMemcpyAsync(f->pts, sgnlo, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, f->stream), "copy");
-  if ((rc = fu_eval(f, n, nullptr, false, true, nullptr))) return rc;
+  if ((rc = fu_eval(f, n, nullptr, false, true, nullptr, true))) return rc;
   const double* sc = opts->scale;
   k_asc_init<<<nb, 256, 0, f->stream>>>(f->asc, n, f->pts, f->F, f->grad, sc[0], sc[1], sc[2], sc[3], step0);
   f->launches++;
@@ -942,13 +923,13 @@ int pa_followup_ascent(pa_followup* f, double* sgnlo, int n, const pa_ascent_opt
     // trial points -> f->pts (the evaluation reads them from there)
     k_asc_propose<<<nb, 256, 0, f->stream>>>(f->asc, n, sc[0], sc[1], sc[2], sc[3], min_step, f->pts, f->mask);
     f->launches++;
-    if ((rc = fu_eval(f, n, f->mask, false, false, nullptr))) break;
+    if ((rc = fu_eval(f, n, f->mask, false, false, nullptr, true))) break;
     cudaMemsetAsync(f->counter, 0, sizeof(int), f->stream);
     k_asc_decide<<<nb, 256, 0, f->stream>>>(f->asc, n, sc[0], sc[1], sc[2], sc[3], f->F, f->need, f->counter);
     f->launches++;
     // gradient at the accepted points: the trial evaluation left their
     // constants and adjoint seeds in cand[]; only the adjoint pass runs
-    if ((rc = f->fp64 ? fu_adjoint_t<double>(f, n, f->need) : fu_adjoint_t<float>(f, n, f->need))) break;
+    if ((rc = fu_adjoint(f, n, f->need))) break;
     k_asc_take_grad<<<nb, 256, 0, f->stream>>>(f->asc, n, sc[0], sc[1], sc[2], sc[3], f->need, f->grad);
     f->launches++;
     if (cudaGetLastError() != cudaSuccess) {
@@ -967,7 +948,7 @@ int pa_followup_ascent(pa_followup* f, double* sgnlo, int n, const pa_ascent_opt
   // final points and their fstat_out
   k_asc_export<<<nb, 256, 0, f->stream>>>(f->asc, n, f->pts, f->iters);
   f->launches++;
-  if ((rc = fu_eval(f, n, nullptr, true, false, nullptr))) return rc;
+  if ((rc = fu_eval(f, n, nullptr, true, false, nullptr, false))) return rc;
   FCK(cudaMemcpyAsync(sgnlo, f->pts, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, f->stream), "copy");
   FCK(cudaMemcpyAsync(out, f->out, sizeof(double) * 11 * n, cudaMemcpyDeviceToHost, f->stream), "copy");
   if (iters) FCK(cudaMemcpyAsync(iters, f->iters, sizeof(int) * n, cudaMemcpyDeviceToHost, f->stream), "copy");

@@ -551,8 +551,8 @@ class Followup:
 
     def __init__(self, settings: Settings, dets, nifo: int, precision: int = PA_PREC_MIXED, device: int = 0,
                  phase_mode: int = PA_PHASE_F64):
-        """phase_mode: PA_PHASE_F64 (FP64 phase, the default) or PA_PHASE_FF
-        (compensated two-float phase) in the mixed precision."""
+        """phase_mode: any of the search's; the mixed form's phase is the same
+        (fixed point, from FP64 values per 1024 samples) in all of them."""
         self.lib = load()
         cfg = Config(precision, phase_mode, 0, device)
         st = C.c_int(0)
