@@ -77,10 +77,14 @@ struct pa_ctx {
 static int active_lanes(const pa_ctx* c) { return c->prof.on ? 1 : c->lanes; }
 static cudaStream_t prelude_stream(const pa_ctx* c) { return c->prof.on ? c->stream : c->stream_pre; }
 
-// sky points per captured part of a batch (launch_tasks): the first part
-// kGraphFirst, each next one twice the previous, up to kGraphPart
-constexpr size_t kGraphFirst = 16;
+// With graphs on, a batch is launched in parts (part_bounds): the first sky
+// point directly, so that the device starts at once, then captured parts of
+// kGraphFirst sky points and twice the previous one each, up to kGraphPart.
+constexpr size_t kGraphFirst = 2;
 constexpr size_t kGraphPart = 256;
+
+// candidates copied back together with their count
+constexpr int kCandFirst = 1024;
 
 static void drop_graphs(pa_ctx* c) {
   for (auto& g : c->gexec_parts)
@@ -696,48 +700,49 @@ pa::SkyArgs sky_args(const pa_ctx* c, const SkyHost& h, int task) {
   return a;
 }
 
-// Enqueues one sky point: its prelude on the prelude stream into slot
-// task % 2 (after the spindowns that last read that slot), and its spindown
-// batches after the prelude, on the main stream or, with two lanes,
-// alternately on the main stream and stream2 (*lane: the lane of the next
-// batch, carried over from sky point to sky point).
-int enqueue_sky(pa_ctx* c, const SkyHost& h, const pa_opts* o, int task, void* Fdbg, int Fss,
-                bool wait_slot = true, int* lane = nullptr) {
-  const pa::SkyArgs a = sky_args(c, h, task);
+// Enqueues the prelude of a sky point on `sp` into slot task % 2; wait_slot:
+// after the spindowns that last read that slot (on lane 1 too with wait_lane1).
+int enqueue_prelude(pa_ctx* c, const SkyHost& h, int task, cudaStream_t sp, bool wait_slot, bool wait_lane1) {
   const int slot = task & 1;
-  const int lanes = Fdbg ? 1 : active_lanes(c);
-  cudaStream_t sp = prelude_stream(c);
   if (wait_slot) {
     CK(cudaStreamWaitEvent(sp, c->ev_spin[slot], 0), "cudaStreamWaitEvent");
-    // (the debug path is never captured: it may wait on lane 1's reads of an
-    // earlier call too)
-    if (lanes == 2 || Fdbg) CK(cudaStreamWaitEvent(sp, c->ev_spin2[slot], 0), "cudaStreamWaitEvent");
+    if (wait_lane1) CK(cudaStreamWaitEvent(sp, c->ev_spin2[slot], 0), "cudaStreamWaitEvent");
   }
-  cudaError_t e = c->eng->prelude(a, slot, sp);
+  cudaError_t e = c->eng->prelude(sky_args(c, h, task), slot, sp);
   if (e != cudaSuccess) return cuda_fail(c, e, "prelude launch");
-  CK(cudaEventRecord(c->ev_pre[slot], sp), "cudaEventRecord");
-  CK(cudaStreamWaitEvent(c->stream, c->ev_pre[slot], 0), "cudaStreamWaitEvent");
-  if (lanes == 2) CK(cudaStreamWaitEvent(c->stream2, c->ev_pre[slot], 0), "cudaStreamWaitEvent");
-  if (Fdbg) {
-    e = c->eng->spindowns(a, slot, 0, Fss, 1, o->trl, o->white_flag, o->s0_flag, c->stream, Fdbg);
+  return PA_OK;
+}
+
+// Enqueues the spindown batches of a sky point, on the main stream or, with
+// two lanes, alternately on the main stream and stream2 (*lane: the lane of the
+// next batch, carried over from sky point to sky point); with `sp`, after the
+// prelude that was enqueued last on that stream.  *lane1_reads: stream2 reads
+// the slot (ev_spin2 is recorded).
+int enqueue_spins(pa_ctx* c, const SkyHost& h, const pa_opts* o, int task, int lanes, int* lane, cudaStream_t sp,
+                  bool* lane1_reads) {
+  const pa::SkyArgs a = sky_args(c, h, task);
+  const int slot = task & 1;
+  // (a single batch has no use for the other lane)
+  const bool both = lanes == 2 && (h.nss > c->b.sbatch || *lane != 0);
+  if (sp && (sp != c->stream || both)) {
+    CK(cudaEventRecord(c->ev_pre[slot], sp), "cudaEventRecord");
+    if (sp != c->stream) CK(cudaStreamWaitEvent(c->stream, c->ev_pre[slot], 0), "cudaStreamWaitEvent");
+    if (both) CK(cudaStreamWaitEvent(c->stream2, c->ev_pre[slot], 0), "cudaStreamWaitEvent");
+  }
+  // full launches and one remainder: splitting into equal launches (200 as
+  // 4 x 50 instead of 3 x 64 + 8) was measured 1.5% slower, as each
+  // launch's last partial wave of CTAs costs a whole wave
+  for (int ss = h.smin; ss <= h.smax; ss += c->b.sbatch) {
+    const int nb = std::min(c->b.sbatch, h.smax - ss + 1);
+    const int l = lanes == 2 ? *lane : 0;
+    cudaError_t e = c->eng->spindowns(a, slot, l, ss, nb, o->trl, o->white_flag, o->s0_flag, l ? c->stream2 : c->stream,
+                                      nullptr);
     if (e != cudaSuccess) return cuda_fail(c, e, "spindown launch");
-  } else {
-    // full launches and one remainder: splitting into equal launches (200 as
-    // 4 x 50 instead of 3 x 64 + 8) was measured 1.5% slower, as each
-    // launch's last partial wave of CTAs costs a whole wave
-    int l0 = 0;
-    int* ln = lane ? lane : &l0;
-    for (int ss = h.smin; ss <= h.smax; ss += c->b.sbatch) {
-      const int nb = std::min(c->b.sbatch, h.smax - ss + 1);
-      const int l = lanes == 2 ? *ln : 0;
-      e = c->eng->spindowns(a, slot, l, ss, nb, o->trl, o->white_flag, o->s0_flag, l ? c->stream2 : c->stream,
-                            nullptr);
-      if (e != cudaSuccess) return cuda_fail(c, e, "spindown launch");
-      if (lanes == 2) *ln ^= 1;
-    }
+    if (lanes == 2) *lane ^= 1;
   }
   CK(cudaEventRecord(c->ev_spin[slot], c->stream), "cudaEventRecord");
-  if (lanes == 2) CK(cudaEventRecord(c->ev_spin2[slot], c->stream2), "cudaEventRecord");
+  if (both) CK(cudaEventRecord(c->ev_spin2[slot], c->stream2), "cudaEventRecord");
+  *lane1_reads = both;
   return PA_OK;
 }
 
@@ -747,41 +752,78 @@ bool cand_less(const pa::DevCand& x, const pa::DevCand& y) {
   return x.ii < y.ii;
 }
 
+// What one part of a batch leaves to the next.
+struct Carry {
+  int lane = 0;            // lane of the next spindown batch
+  size_t ready = ~(size_t)0;  // sky point whose prelude the part before enqueued
+};
+
+bool has_work(const SkyHost& h) { return h.inside && h.nss > 0; }
+
 // Enqueues sky points [t0, t1) of a batch on the context's streams: the
 // candidate counter reset (for the batch's first part), then every sky point
 // (prelude on the prelude stream forked from the main stream, spindowns on
-// the main stream), and the join of the prelude stream back into the main
-// stream.  Slots are reused across sky points through their events; the
-// first use of each slot in a part needs no wait (the work before it on the
-// main stream -- the previous part or call -- has finished when the part
-// starts).  Works unchanged under stream capture.
-int enqueue_tasks(pa_ctx* c, const std::vector<SkyHost>& hs, const pa_opts* o, size_t t0, size_t t1,
-                  bool reset) {
+// the main stream or the lanes), the prelude of the next part's first sky
+// point (so that the next part begins with spindowns), and the join of the
+// streams back into the main stream.  Slots are reused across sky points
+// through their events; the first use of each slot in a part needs no wait
+// (the work before it on the main stream -- the previous part or call -- has
+// finished when the part starts).  A single sky point runs on the main stream
+// alone, and on stream2 only if it has several batches: nothing overlaps its
+// prelude.  Works unchanged under stream capture.
+int enqueue_tasks(pa_ctx* c, const std::vector<SkyHost>& hs, const pa_opts* o, size_t t0, size_t t1, bool reset,
+                  Carry* carry) {
   const int lanes = active_lanes(c);
+  const bool solo = hs.size() == 1;
+  cudaStream_t sp = solo ? c->stream : prelude_stream(c);
   if (reset) CK(cudaMemsetAsync(c->b.ncand, 0, sizeof(int), c->stream), "memset");
-  CK(cudaEventRecord(c->ev_fork, c->stream), "cudaEventRecord");
-  CK(cudaStreamWaitEvent(c->stream_pre, c->ev_fork, 0), "cudaStreamWaitEvent");
-  if (lanes == 2) CK(cudaStreamWaitEvent(c->stream2, c->ev_fork, 0), "cudaStreamWaitEvent");
-  bool used[2] = {false, false};
-  int lane = 0;
-  for (size_t t = t0; t < t1; t++) {
-    if (!hs[t].inside || hs[t].nss == 0) continue;
-    const int slot = (int)t & 1;
-    int rc = enqueue_sky(c, hs[t], o, (int)t, nullptr, 0, used[slot], &lane);
-    if (rc) return rc;
-    used[slot] = true;
+  bool lane1 = lanes == 2 && !solo;  // stream2 takes part
+  if (solo && has_work(hs[0])) lane1 = lanes == 2 && hs[0].nss > c->b.sbatch;
+  if (sp != c->stream || lane1) {
+    CK(cudaEventRecord(c->ev_fork, c->stream), "cudaEventRecord");
+    if (sp != c->stream) CK(cudaStreamWaitEvent(sp, c->ev_fork, 0), "cudaStreamWaitEvent");
+    if (lane1) CK(cudaStreamWaitEvent(c->stream2, c->ev_fork, 0), "cudaStreamWaitEvent");
   }
-  CK(cudaEventRecord(c->ev_join, c->stream_pre), "cudaEventRecord");
-  CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "cudaStreamWaitEvent");
-  if (lanes == 2) {
+  bool used[2] = {false, false}, used1[2] = {false, false};
+  auto prelude = [&](size_t t) { return enqueue_prelude(c, hs[t], (int)t, sp, used[t & 1], used1[t & 1]); };
+  for (size_t t = t0; t < t1; t++) {
+    if (!has_work(hs[t])) continue;
+    int rc = PA_OK;
+    const bool ready = carry->ready == t;
+    if (!ready && (rc = prelude(t))) return rc;
+    if ((rc = enqueue_spins(c, hs[t], o, (int)t, lane1 ? 2 : 1, &carry->lane, ready ? nullptr : sp,
+                            &used1[t & 1])))
+      return rc;
+    used[t & 1] = true;
+  }
+  for (size_t t = t1; t < hs.size(); t++)
+    if (has_work(hs[t])) {
+      int rc = prelude(t);
+      if (rc) return rc;
+      carry->ready = t;
+      break;
+    }
+  if (sp != c->stream) {
+    CK(cudaEventRecord(c->ev_join, sp), "cudaEventRecord");
+    CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0), "cudaStreamWaitEvent");
+  }
+  if (lane1) {
     CK(cudaEventRecord(c->ev_join2, c->stream2), "cudaEventRecord");
     CK(cudaStreamWaitEvent(c->stream, c->ev_join2, 0), "cudaStreamWaitEvent");
   }
   return PA_OK;
 }
 
-int enqueue_tasks(pa_ctx* c, const std::vector<SkyHost>& hs, const pa_opts* o) {
-  return enqueue_tasks(c, hs, o, 0, hs.size(), true);
+// First sky point of every part of a batch of n, and n: one sky point, then
+// captured parts.  The host captures part k + 1 while the device runs part k;
+// only the direct launch of the first sky point precedes device work, and
+// capturing a sky point takes the host far less time than the device takes to
+// search it.
+std::vector<size_t> part_bounds(size_t n) {
+  std::vector<size_t> bound{0, std::min<size_t>(1, n)};
+  for (size_t step = kGraphFirst; bound.back() < n; step = std::min(kGraphPart, 2 * step))
+    bound.push_back(std::min(n, bound.back() + step));
+  return bound;
 }
 
 // Replaces *exec by an executable graph of g: updated in place when the
@@ -803,34 +845,27 @@ int graph_exec_from(cudaGraph_t g, cudaGraphExec_t* exec, std::string* err) {
   return PA_OK;
 }
 
-// Enqueues the batch directly, or captures it into the context's graph and
-// launches that.  The timing event ev0 goes on the stream right before the
-// work (after the capture and graph update, which are host work).
+// Enqueues the batch directly, or in parts as CUDA graphs.  The timing event
+// ev0 goes on the stream right before the work.
 int launch_tasks(pa_ctx* c, const std::vector<SkyHost>& hs, const pa_opts* o) {
   pa::TraceRange trace_("launch (capture, graph launch)");
   const bool graph = c->graphs && !c->prof.on;
-  if (!graph) {
-    CK(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
-    return enqueue_tasks(c, hs, o);
-  }
-  // The batch is captured in parts, each into its own executable graph
-  // (updated in place when the part's launch structure repeats), and each
-  // part is launched as soon as it is captured: the host captures part k + 1
-  // while the device runs part k.  Only the first part's capture precedes
-  // device work, so it is short (kGraphFirst sky points); the parts then
-  // double, as capturing a sky point takes the host far less time than the
-  // device takes to search it, up to kGraphPart.
-  const size_t n = hs.size();
-  std::vector<size_t> bound{0};
-  for (size_t step = kGraphFirst; bound.back() < n; step = std::min(kGraphPart, 2 * step))
-    bound.push_back(std::min(n, bound.back() + step));
-  if (n == 0) bound.push_back(0);
+  Carry carry;
+  CK(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
+  if (!graph) return enqueue_tasks(c, hs, o, 0, hs.size(), true, &carry);
+  // each captured part has its own executable graph (updated in place when
+  // the part's launch structure repeats) and is launched as soon as captured
+  const std::vector<size_t> bound = part_bounds(hs.size());
   const size_t nparts = bound.size() - 1;
   if (c->gexec_parts.size() < nparts) c->gexec_parts.resize(nparts, nullptr);
   for (size_t k = 0; k < nparts; k++) {
-    const size_t t0 = bound[k], t1 = bound[k + 1];
+    if (k == 0) {
+      int rc = enqueue_tasks(c, hs, o, bound[0], bound[1], true, &carry);
+      if (rc) return rc;
+      continue;
+    }
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-    int rc = enqueue_tasks(c, hs, o, t0, t1, k == 0);
+    int rc = enqueue_tasks(c, hs, o, bound[k], bound[k + 1], false, &carry);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (rc) {
@@ -841,7 +876,6 @@ int launch_tasks(pa_ctx* c, const std::vector<SkyHost>& hs, const pa_opts* o) {
     rc = graph_exec_from(g, &c->gexec_parts[k], &c->err);
     cudaGraphDestroy(g);
     if (rc) return rc;
-    if (k == 0) CK(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
     CK(cudaGraphLaunch(c->gexec_parts[k], c->stream), "cudaGraphLaunch");
   }
   return PA_OK;
@@ -852,14 +886,18 @@ int launch_tasks(pa_ctx* c, const std::vector<SkyHost>& hs, const pa_opts* o) {
 // device buffer overflowed.
 int collect_tasks(pa_ctx* c, std::vector<pa::DevCand>* out, int* n_out) {
   pa::TraceRange trace_("collect candidates");
+  // the first candidates come with the count: one wait for most calls
+  const int first = std::min(kCandFirst, c->b.cand_cap);
   CK(cudaMemcpyAsync(c->h_ncand, c->b.ncand, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "copy count");
+  CK(cudaMemcpyAsync(c->h_cand, c->b.cand, sizeof(pa::DevCand) * (size_t)first, cudaMemcpyDeviceToHost, c->stream),
+     "copy candidates");
   CK(cudaStreamSynchronize(c->stream), "search");
   const int n = *c->h_ncand;
   *n_out = n;
   if (n > c->b.cand_cap) return PA_ERR_CAPACITY;
-  if (n > 0) {
-    CK(cudaMemcpyAsync(c->h_cand, c->b.cand, sizeof(pa::DevCand) * (size_t)n, cudaMemcpyDeviceToHost,
-                       c->stream), "copy candidates");
+  if (n > first) {
+    CK(cudaMemcpyAsync(c->h_cand + first, c->b.cand + first, sizeof(pa::DevCand) * (size_t)(n - first),
+                       cudaMemcpyDeviceToHost, c->stream), "copy candidates");
     CK(cudaStreamSynchronize(c->stream), "copy candidates");
   }
   out->assign(c->h_cand, c->h_cand + n);
@@ -1153,7 +1191,14 @@ int pa_debug_fstat(pa_ctx* c, int pm, int mm, int nn, int ss, const pa_opts* o, 
   void* dF = nullptr;
   CK(cudaMalloc(&dF, c->rsz * (size_t)bins), "cudaMalloc");
   CK(cudaMemsetAsync(c->b.ncand, 0, sizeof(int), c->stream), "memset");
-  int rc = enqueue_sky(c, h, o, 0, dF, ss);
+  const pa::SkyArgs a = sky_args(c, h, 0);
+  // (all on the main stream, after whatever the call before left there; no
+  // event is waited for, as a graph's events cannot be waited for outside it)
+  int rc = enqueue_prelude(c, h, 0, c->stream, false, false);
+  if (!rc) {
+    cudaError_t e = c->eng->spindowns(a, 0, 0, ss, 1, o->trl, o->white_flag, o->s0_flag, c->stream, dF);
+    if (e != cudaSuccess) rc = cuda_fail(c, e, "spindown launch");
+  }
   std::vector<char> buf(c->rsz * (size_t)bins);
   if (!rc) {
     cudaError_t e = cudaMemcpyAsync(buf.data(), dF, buf.size(), cudaMemcpyDeviceToHost, c->stream);
@@ -1492,7 +1537,7 @@ struct pa_segments {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<cudaEvent_t> fork, join;
   bool graph = true;
-  cudaGraphExec_t gexec = nullptr;
+  std::vector<cudaGraphExec_t> gexec;  // one per captured part
   double last_ms = 0.;
   std::string err;
 };
@@ -1517,14 +1562,16 @@ int seg_fail(pa_segments* s, int code, const char* fmt, ...) {
     if (e_ != cudaSuccess) return seg_fail(sg, PA_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e_));      \
   } while (0)
 
-// Enqueues every segment's batch, forked from and joined back into the
-// origin stream.
-int seg_enqueue(pa_segments* sg, const std::vector<std::vector<SkyHost>>& hs, const pa_segment_job* jobs) {
+// Enqueues sky points [t0, t1) of every segment's batch (as far as it has
+// them), forked from and joined back into the origin stream.
+int seg_enqueue(pa_segments* sg, const std::vector<std::vector<SkyHost>>& hs, const pa_segment_job* jobs, size_t t0,
+                size_t t1, std::vector<Carry>* carry) {
   for (size_t k = 0; k < sg->ctx.size(); k++) {
     pa_ctx* c = sg->ctx[k];
+    if (t0 > 0 && t0 >= hs[k].size()) continue;
     SCK(cudaEventRecord(sg->fork[k], sg->origin), "cudaEventRecord");
     SCK(cudaStreamWaitEvent(c->stream, sg->fork[k], 0), "cudaStreamWaitEvent");
-    int rc = enqueue_tasks(c, hs[k], jobs[k].opts);
+    int rc = enqueue_tasks(c, hs[k], jobs[k].opts, t0, std::min(t1, hs[k].size()), t0 == 0, &(*carry)[k]);
     if (rc) return seg_fail(sg, rc, "segment %d: %s", (int)k, c->err.c_str());
     SCK(cudaEventRecord(sg->join[k], c->stream), "cudaEventRecord");
     SCK(cudaStreamWaitEvent(sg->origin, sg->join[k], 0), "cudaStreamWaitEvent");
@@ -1575,7 +1622,8 @@ void pa_segments_destroy(pa_segments* sg) {
   if (!sg) return;
   cudaSetDevice(sg->dev);
   if (sg->origin) cudaStreamSynchronize(sg->origin);
-  if (sg->gexec) cudaGraphExecDestroy(sg->gexec);
+  for (cudaGraphExec_t g : sg->gexec)
+    if (g) cudaGraphExecDestroy(g);
   for (cudaEvent_t e : sg->fork)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : sg->join)
@@ -1618,25 +1666,36 @@ int pa_segments_search(pa_segments* sg, const pa_segment_job* jobs, int* status)
     profiling |= sg->ctx[k]->prof.on;
   }
   int rc;
+  size_t most = 0;
+  for (const auto& h : hs) most = std::max(most, h.size());
+  std::vector<Carry> carry(ns);
+  SCK(cudaEventRecord(sg->ev0, sg->origin), "cudaEventRecord");
   if (sg->graph && !profiling) {
-    SCK(cudaStreamBeginCapture(sg->origin, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-    rc = seg_enqueue(sg, hs, jobs);
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(sg->origin, &g);
-    if (rc) {
-      if (g) cudaGraphDestroy(g);
-      return rc;
+    // the first sky point of every segment directly, the others as graphs
+    // captured while the device runs the part before (part_bounds)
+    const std::vector<size_t> bound = part_bounds(most);
+    if (sg->gexec.size() < bound.size() - 1) sg->gexec.resize(bound.size() - 1, nullptr);
+    for (size_t k = 0; k + 1 < bound.size(); k++) {
+      if (k == 0) {
+        if ((rc = seg_enqueue(sg, hs, jobs, bound[0], bound[1], &carry))) return rc;
+        continue;
+      }
+      SCK(cudaStreamBeginCapture(sg->origin, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
+      rc = seg_enqueue(sg, hs, jobs, bound[k], bound[k + 1], &carry);
+      cudaGraph_t g = nullptr;
+      cudaError_t e = cudaStreamEndCapture(sg->origin, &g);
+      if (rc) {
+        if (g) cudaGraphDestroy(g);
+        return rc;
+      }
+      if (e != cudaSuccess) return seg_fail(sg, PA_ERR_CUDA, "cudaStreamEndCapture: %s", cudaGetErrorString(e));
+      rc = graph_exec_from(g, &sg->gexec[k], &sg->err);
+      cudaGraphDestroy(g);
+      if (rc) return rc;
+      SCK(cudaGraphLaunch(sg->gexec[k], sg->origin), "cudaGraphLaunch");
     }
-    if (e != cudaSuccess) return seg_fail(sg, PA_ERR_CUDA, "cudaStreamEndCapture: %s", cudaGetErrorString(e));
-    rc = graph_exec_from(g, &sg->gexec, &sg->err);
-    cudaGraphDestroy(g);
-    if (rc) return rc;
-    // timing starts at the launch (capture and update are host work)
-    SCK(cudaEventRecord(sg->ev0, sg->origin), "cudaEventRecord");
-    SCK(cudaGraphLaunch(sg->gexec, sg->origin), "cudaGraphLaunch");
   } else {
-    SCK(cudaEventRecord(sg->ev0, sg->origin), "cudaEventRecord");
-    if ((rc = seg_enqueue(sg, hs, jobs))) return rc;
+    if ((rc = seg_enqueue(sg, hs, jobs, 0, most, &carry))) return rc;
   }
   SCK(cudaEventRecord(sg->ev1, sg->origin), "cudaEventRecord");
   SCK(cudaStreamSynchronize(sg->origin), "segments");

@@ -305,11 +305,10 @@ class Context:
             raise SearchError("pa_create failed (%d): %s" % (st.value, self.lib.pa_last_error(None).decode()))
         self.settings = settings
         self.nifo = nifo
-        # search_batch's output buffers, kept from call to call (the library
-        # writes every field of the records and indices it returns)
+        # output buffers, kept from call to call (the library writes every
+        # field of the records and indices it returns)
         self._out_cap = 0
-        self._out_buf = None
-        self._out_idx = None
+        self._out_buf = self._out_ptr = self._out_idx = None
 
     def error(self) -> str:
         return self.lib.pa_last_error(self.ctx).decode()
@@ -320,11 +319,9 @@ class Context:
         fnum = C.c_int(0)
         needed = C.c_int(0)
         while True:
-            buf = np.zeros((cap, PA_NPAR))
-            idx = (CandIdx * cap)()
-            rc = self.lib.pa_job_core(self.ctx, pm, mm, nn, C.byref(opts), C.byref(rng), C.byref(sgnlc),
-                                      buf.ctypes.data_as(C.POINTER(C.c_double)), cap, idx, C.byref(fnum),
-                                      C.byref(needed))
+            buf, ptr, idx = self._room(cap)
+            rc = self.lib.pa_job_core(self.ctx, pm, mm, nn, C.byref(opts), C.byref(rng), C.byref(sgnlc), ptr, cap, idx,
+                                      C.byref(fnum), C.byref(needed))
             if rc == PA_ERR_CAPACITY:
                 cap = needed.value + 16
                 continue
@@ -334,6 +331,15 @@ class Context:
         n = sgnlc.value
         return buf[:n].copy(), idx_to_array(idx, n), fnum.value
 
+    def _room(self, cap: int):
+        """Output buffers for cap records, kept from call to call."""
+        if self._out_cap < cap:
+            self._out_buf = np.empty((cap, PA_NPAR))
+            self._out_idx = (CandIdx * cap)()
+            self._out_ptr = self._out_buf.ctypes.data_as(C.POINTER(C.c_double))
+            self._out_cap = cap
+        return self._out_buf, self._out_ptr, self._out_idx
+
     def search_batch(self, tasks, opts: Opts, rng: Range, cap: int = 1 << 18):
         # the sky points as the C array of {pm, mm, nn} ints
         sky = np.ascontiguousarray(np.asarray(tasks, dtype=np.int32).reshape(-1, 3))
@@ -342,14 +348,9 @@ class Context:
         fnum = C.c_int(0)
         needed = C.c_int(0)
         while True:
-            if self._out_cap != cap:
-                self._out_buf = np.empty((cap, PA_NPAR))
-                self._out_idx = (CandIdx * cap)()
-                self._out_cap = cap
-            buf, idx = self._out_buf, self._out_idx
-            rc = self.lib.pa_search_batch(self.ctx, arr, len(sky), C.byref(opts), C.byref(rng),
-                                          C.byref(sgnlc), buf.ctypes.data_as(C.POINTER(C.c_double)), cap, idx,
-                                          C.byref(fnum), C.byref(needed))
+            buf, ptr, idx = self._room(cap)
+            rc = self.lib.pa_search_batch(self.ctx, arr, len(sky), C.byref(opts), C.byref(rng), C.byref(sgnlc), ptr,
+                                          cap, idx, C.byref(fnum), C.byref(needed))
             if rc == PA_ERR_CAPACITY:
                 cap = needed.value + 16
                 continue
@@ -490,6 +491,8 @@ class Segments:
             raise SearchError("pa_segments_create failed (%d): %s" %
                               (st.value, self.lib.pa_segments_last_error(None).decode()))
         self.lib.pa_segments_set_graph(self.seg, int(bool(graph)))
+        self._out_cap = 0
+        self._out = []
 
     def set_graph(self, on: bool):
         self.lib.pa_segments_set_graph(self.seg, int(bool(on)))
@@ -498,15 +501,17 @@ class Segments:
         """Returns [(records, idx, FNum)] per segment."""
         n = len(self.contexts)
         while True:
+            if self._out_cap < cap:  # output buffers, kept from call to call
+                self._out = [(np.empty((cap, PA_NPAR)), (CandIdx * cap)()) for _ in range(n)]
+                self._out_cap = cap
             keep, jobs = [], (SegmentJob * n)()
             outs = []
             for k in range(n):
                 tasks = task_lists[k]
                 arr = (Sky * max(1, len(tasks)))(*[Sky(*t) for t in tasks])
                 sgnlc, fnum, needed = C.c_int(0), C.c_int(0), C.c_int(0)
-                buf = np.zeros((cap, PA_NPAR))
-                idx = (CandIdx * cap)()
-                keep += [arr, sgnlc, fnum, needed, buf, idx]
+                buf, idx = self._out[k]
+                keep += [arr, sgnlc, fnum, needed]
                 jobs[k] = SegmentJob(C.cast(arr, C.c_void_p), len(tasks), C.addressof(opts_list[k]),
                                      C.addressof(ranges[k]), C.addressof(sgnlc), buf.ctypes.data, cap,
                                      C.addressof(idx), C.addressof(fnum), C.addressof(needed))
