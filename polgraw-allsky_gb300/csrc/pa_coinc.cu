@@ -6,8 +6,9 @@
 // Data flow (one stream; arrays in HBM):
 //   records [raw][5] f64 (uploaded per frame)
 //   k_cells      band/frame-shift/SNR cuts and the 4 integer cells of each
-//                record (FP64, no contraction: the reference's expression
-//                order), per-block counts, per-column min/max
+//                record (those of the FP64 evaluation without contraction, in
+//                the reference's expression order), per-block counts,
+//                per-column min/max
 //   scan + k_inband   ordered compaction of the kept records (read order,
 //                frame by frame), with a cell key: the 4 cells as unsigned
 //                offsets from the column maxima (descending cells sort
@@ -15,7 +16,7 @@
 //   radix sort   LSD, 8-bit digits, stable: the order of the reference's two
 //                qsort()s at once (cells descending; equal cells keep frame
 //                then read order, which is what qsort's merge sort leaves)
-//   frame ranks  per-block frame histograms + scan locate, for every frame,
+//   frame ranks  per-tile frame histograms + scan locate, for every frame,
 //                its last sorted record and the record of an earlier frame
 //                that the reference compares it with (the row left over at
 //                that position of its candidate table)
@@ -58,51 +59,61 @@ struct FrameTab {
   long long raw_start[kMaxFrames + 1];   // first raw record of each frame
   int blk_start[kMaxFrames + 1];         // first k_cells block of each frame
   long long in_start[kMaxFrames + 1];    // first in-band record of each frame
-  int drop[kMaxFrames];                  // 1: the frame's last run is not written
-  unsigned long long drop_lo[kMaxFrames], drop_hi[kMaxFrames];  // its cell key
 };
 __constant__ FrameTab c_ft;
 
 struct CellArgs {
-  double lo, hi;           // narrowdown band (pi/2 -+ narrowdown)
+  long long lo_k, hi_k;    // narrowdown band (pi/2 -+ narrowdown) and SNR cut as
+  long long cut_k;         // order keys (order_key)
   double N, sqrN, omsN;    // coincidences.c:187-188
+  double N2;               // 2 N
   double se, ce;           // sin/cos(C_EPSMA)
   double v[4][4];          // vedva / scale (coincidences.c:182-184)
   double half_shift[4];    // 0.5 shift[j]
   int refr;
-  double snrcut;
-  // FP32 sky terms: copies in float and, per cell column, the bound on
-  // |cell value (FP64) - cell value (FP32 sky terms)|
-  float omsN_f, se_f, ce_f, v2_f[4], v3_f[4], margin[4];
-  // float-float (hi + lo) copies for the frequency and spindown terms
-  float Nf, sqrN_h, sqrN_l, v0_h[4], v0_l[4], v1_h[4], v1_l[4], hs_f[4];
-  int fast;                // N < 2^24 (exact in float): the FP32/float-float path is on
+  // sky terms in FP32: the columns' factors of be0 and be1 and, per column, the
+  // bound on |cell value (FP64) - cell value (FP32 sky terms)|
+  float se_f, ce_f, s2_f[4], s3_f[4], margin[4];
+  // float-float (hi + lo) factors of the frequency and the spindown
+  float f_h[4], f_l[4], d_h[4], d_l[4], hs_f[4];
+  int fast;                // N < 2^24: the FP32/float-float path is on
 };
 
-// float-float arithmetic (hi + lo, about 44 significant bits): error-free
-// products by fmaf and sums by the two-sum of Knuth
+// a number as the sum of two floats (about 48 significant bits)
 struct FF {
   float h, l;
 };
-__device__ __forceinline__ FF ff_quick(float a, float b) {
-  const float s = a + b;
-  return {s, b - (s - a)};
-}
-__device__ __forceinline__ FF ff_add(FF a, FF b) {
-  const float s = a.h + b.h;
-  const float bb = s - a.h;
-  const float e = (a.h - (s - bb)) + (b.h - bb);
-  return ff_quick(s, e + (a.l + b.l));
-}
-__device__ __forceinline__ FF ff_mul(FF a, FF b) {
-  const float p = a.h * b.h;
-  const float e = fmaf(a.h, b.h, -p);
-  return ff_quick(p, fmaf(a.h, b.l, fmaf(a.l, b.h, e)));
-}
-__device__ __forceinline__ FF ff_of(double d) {
+// d = h + l with h = (float)d and l = (float)(d - h), both by integer
+// arithmetic on d's bits: a conversion or an FP64 subtraction takes the FP64
+// pipe, which has 1/64 of the FP32 rate.  Numbers whose parts are not all
+// normal floats (2^-74 <= |d| < 2^127 is enough) take the conversions.
+// (a call, so that the conversions are not issued for every number)
+__device__ __noinline__ FF ff_convert(double d) {
   const float h = (float)d;
   return {h, (float)(d - (double)h)};
 }
+constexpr long long kMag = 0x7fffffffffffffffll;
+__device__ __forceinline__ FF ff_of(double d) {
+  const long long b = __double_as_longlong(d), m = b & kMag;
+  const int e = (int)(m >> 52);
+  if (e < 949 || e > 1149) {
+    if (m == 0) return {0.f, 0.f};  // (no spindown: common)
+    return ff_convert(d);
+  }
+  // h: to nearest even at bit 29, then the exponent's new bias
+  const long long r = (m + 0x0fffffff + ((m >> 29) & 1)) >> 29;
+  const int sign = (int)(b >> 32) & 0x80000000;
+  // the rest, an integer below 2^29 in units of the last place
+  const int rest = (int)(m - (r << 29));
+  const float l = (float)rest * __int_as_float((e - 1075 + 127) << 23);
+  return {__int_as_float(((int)r - (896 << 23)) | sign), __int_as_float(__float_as_int(l) ^ sign)};
+}
+// Order key of a double: x < y <=> key(x) < key(y) for numbers that are not
+// NaN, with -0 just below +0; positive NaNs lie above +inf, negative ones
+// below -inf.  (An FP64 comparison takes the FP64 pipe too.)
+__host__ __device__ __forceinline__ long long order_key(long long bits) { return bits ^ ((bits >> 63) & kMag); }
+constexpr long long kInfBits = 0x7ff0000000000000ll;
+constexpr long long kPiBits = 0x400921fb54442d18ll;  // M_PI
 
 struct KeyLayout {
   int maxc[4];             // column maxima
@@ -162,64 +173,60 @@ __device__ __noinline__ void cells_f64(double c0s, double c1, double c2, double 
   *cl = make_int4(c[0], c[1], c[2], c[3]);
 }
 
-// Returns 1 when the record is kept.  GB300 runs FP64 at 1/64 of the FP32
-// rate, so only the frequency shift and the band/SNR tests (which must equal
-// the reference's comparisons) run in FP64; the cell values are first formed
-// with the frequency/spindown terms in float-float (about 44 bits) and the
-// sky terms (two sincos, be0/be1 of ast2lin, auxi.c:34-35) in FP32.  Each
-// column's value then lies within a.margin[j] + |value| 2^-36 of the FP64
-// value (FP32 sincosf on |x| <= 8 with the argument rounded to float: <= 3.6e-7
-// per sin/cos; the margin allows 8e-6 on be0 and be1).  When every column's
+// Returns 0 when the record is not kept, 1 with its cells, 2 when it is kept
+// and its cells have to be formed in FP64.
+// GB300 runs FP64 at 1/64 of the FP32
+// rate, so only the three operations of the frequency shift run in FP64 (2 c1 N
+// = c1 (2 N): the doubling is exact); the band and SNR tests compare order
+// keys, and the cell values are first formed with the frequency and spindown
+// terms from float-float products (error-free by fmaf; each product and the sky
+// term give their nearest integer away at once, so that the fractions add up in
+// plain FP32) and the sky terms (two sincos, be0/be1 of ast2lin,
+// auxi.c:34-35) in FP32.  Each column's value then lies within a.margin[j] +
+// 2^-36 of the products' magnitude of the FP64 value.  (FP32 sincosf: 2 units
+// in the last place, 1.2e-7; the argument's rest in float is added by the
+// derivative.  be0: 2.32 x 1.2e-7 + 2e-7 for its roundings, and 3e-7 relative
+// for its FP32 factors: 0.8e-6; the margin allows 2e-6.)  When every column's
 // fractional part is farther than that from 1/2, both round to the same
-// integer; otherwise (or for |value| >= 2^22, or |delta|, |alpha| > 8) the
-// record is recomputed in FP64.  The cells are therefore those of the FP64
-// evaluation.
-__device__ __forceinline__ int cell_of(const double* __restrict__ r, double fshift, const CellArgs& a,
-                                      int4* cl, unsigned* nexact) {
-  const double c0 = r[0], c1 = r[1], c2 = r[2], c3 = r[3], c4 = r[4];
-  if (!((c0 > a.lo) && (c0 < a.hi))) return 0;
-  const double c0s = __dadd_rn(c0, __dmul_rn(__dmul_rn(__dmul_rn(2., c1), a.N), fshift));
-  if (!(((c0s > 0) && (c0s < M_PI)) && (c4 > a.snrcut))) return 0;
-  const float x3 = (float)c3, x2 = (float)c2;
-  bool exact = !a.fast || !(fabsf(x3) <= 8.f && fabsf(x2) <= 8.f);
+// integer; otherwise (or for terms >= 2^22, or |delta|, |alpha| > 8) the record
+// is formed in FP64.  The cells are therefore those of the FP64 evaluation.
+__device__ __forceinline__ int cell_of(double c0, double c1, double c2, double c3, double c4, double fshift,
+                                       const CellArgs& a, int4* cl) {
+  const long long k0 = order_key(__double_as_longlong(c0)), k4 = order_key(__double_as_longlong(c4));
+  if (!(k0 > a.lo_k && k0 < a.hi_k && k4 > a.cut_k && k4 <= kInfBits)) return 0;
+  const double c0s = __dadd_rn(c0, __dmul_rn(__dmul_rn(c1, a.N2), fshift));
+  const long long ks = __double_as_longlong(c0s);
+  if (!(ks > 0 && ks < kPiBits)) return 0;
+  const FF x3 = ff_of(c3), x2 = ff_of(c2);
+  if (!a.fast || !(fabsf(x3.h) <= 8.f && fabsf(x2.h) <= 8.f)) return 2;
+  const FF u = ff_of(c0s), d = ff_of(c1);
+  float sa, ca, sd, cd;
+  sincosf(x3.h, &sa, &ca);
+  sincosf(x2.h, &sd, &cd);
+  const float sa1 = fmaf(ca, x3.l, sa), ca1 = fmaf(-sa, x3.l, ca);
+  const float sd1 = fmaf(cd, x2.l, sd), cd1 = fmaf(-sd, x2.l, cd);
+  const float be0 = fmaf(a.ce_f * sa1, cd1, a.se_f * sd1);
+  const float be1 = ca1 * cd1;
+  // x - (nearest integer), |x| < 2^22, by adding and subtracting 1.5 x 2^23
+  auto nearest = [](float x) { return (x + 12582912.f) - 12582912.f; };
+  bool ok = true;
   int c[4];
-  if (!exact) {
-    const FF t0 = ff_mul(ff_of(c0s), FF{a.Nf, 0.f});
-    const FF t1 = ff_mul(ff_of(c1), FF{a.sqrN_h, a.sqrN_l});
-    float sa, ca, sd, cd;
-    sincosf(x3, &sa, &ca);
-    sincosf(x2, &sd, &cd);
-    const float be0 = fmaf(a.ce_f * sa, cd, a.se_f * sd);
-    const float be1 = ca * cd;
-    const float t2 = a.omsN_f * be0, t3 = a.omsN_f * be1;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      FF v = ff_add(ff_mul(t0, FF{a.v0_h[j], a.v0_l[j]}), ff_mul(t1, FF{a.v1_h[j], a.v1_l[j]}));
-      v = ff_add(v, FF{a.hs_f[j], 0.f});
-      v = ff_add(v, FF{fmaf(t2, a.v2_f[j], t3 * a.v3_f[j]), 0.f});
-      float fl = floorf(v.h);
-      float fr = (v.h - fl) + v.l;
-      if (fr < 0.f) {
-        fl -= 1.f;
-        fr += 1.f;
-      } else if (fr >= 1.f) {
-        fl += 1.f;
-        fr -= 1.f;
-      }
-      // float-float rounding: below 2^-40 of the terms' magnitudes
-      const float av = fabsf(v.h);
-      const float terms = fabsf(t0.h * a.v0_h[j]) + fabsf(t1.h * a.v1_h[j]) + av;
-      exact |= !(av < 4194304.f) || fabsf(fr - 0.5f) <= a.margin[j] + terms * 1e-11f;
-      c[j] = (int)fl + (fr > 0.5f ? 1 : 0);
-    }
-  }
-  if (exact) {
-    cells_f64(c0s, c1, c2, c3, a, cl);
-    atomicAdd(nexact, 1u);
-    return 1;
+  for (int j = 0; j < 4; j++) {
+    const float p = u.h * a.f_h[j], q = d.h * a.d_h[j];
+    const float pe = fmaf(u.h, a.f_l[j], fmaf(u.l, a.f_h[j], fmaf(u.h, a.f_h[j], -p)));
+    const float qe = fmaf(d.h, a.d_l[j], fmaf(d.l, a.d_h[j], fmaf(d.h, a.d_h[j], -q)));
+    const float w = fmaf(be0, a.s2_f[j], be1 * a.s3_f[j]);
+    const float pi = nearest(p), qi = nearest(q), wi = nearest(w);
+    const float fr = (((p - pi) + (q - qi)) + (w - wi)) + ((pe + qe) + a.hs_f[j]);
+    const float ri = nearest(fr);
+    const float terms = fabsf(p) + fabsf(q);
+    // (false for a NaN, too)
+    ok = ok && terms + fabsf(w) < 4194304.f && 0.5f - fabsf(fr - ri) > fmaf(terms, 1e-11f, a.margin[j]);
+    c[j] = (int)((pi + qi) + (wi + ri));
   }
   *cl = make_int4(c[0], c[1], c[2], c[3]);
-  return 1;
+  return ok ? 1 : 2;
 }
 
 __device__ __forceinline__ unsigned block_sum(unsigned v, unsigned* sh) {
@@ -234,62 +241,118 @@ __device__ __forceinline__ unsigned block_sum(unsigned v, unsigned* sh) {
   return t;
 }
 
-// exclusive prefix of a 0/1 flag over the block (thread order); returns the
-// thread's offset, *total the block's count
-__device__ __forceinline__ unsigned block_flag_prefix(int flag, unsigned* sh, unsigned* total) {
+// In-tile positions of the set flags among flag[t0 .. min(t0 + kTile, end)), in
+// order, into list[]; returns their number (also to threads that write none).
+// One pass over the tile and two barriers: warp w takes the 256 flags from
+// 256 w on, 32 at a time.
+__device__ __forceinline__ unsigned tile_list(const uint8_t* __restrict__ flag, long long t0, long long end,
+                                              unsigned short* list, unsigned* sh) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned bal = __ballot_sync(0xffffffffu, flag);
-  const unsigned in_warp = __popc(bal & ((1u << lane) - 1u));
-  __syncthreads();
-  if (lane == 0) sh[w] = __popc(bal);
+  const int first = w * (kTile / (kT / 32));
+  constexpr int kRows = kTile / kT;
+  uint8_t fl[kRows];
+#pragma unroll
+  for (int k = 0; k < kRows; k++) {
+    const long long i = t0 + first + 32 * k + lane;
+    fl[k] = i < end ? flag[i] : (uint8_t)0;
+  }
+  unsigned bal[kRows], n = 0;
+#pragma unroll
+  for (int k = 0; k < kRows; k++) {
+    bal[k] = __ballot_sync(0xffffffffu, fl[k]);
+    n += __popc(bal[k]);
+  }
+  if (lane == 0) sh[w] = n;
   __syncthreads();
   unsigned before = 0, tot = 0;
+#pragma unroll
   for (int k = 0; k < kT / 32; k++) {
     const unsigned c = sh[k];
     if (k < w) before += c;
     tot += c;
   }
-  *total = tot;
-  return before + in_warp;
+#pragma unroll
+  for (int k = 0; k < kRows; k++) {
+    if (fl[k]) list[before + __popc(bal[k] & ((1u << lane) - 1u))] = (unsigned short)(first + 32 * k + lane);
+    before += __popc(bal[k]);
+  }
+  __syncthreads();
+  return tot;
 }
 
 // ---- cells of every raw record ------------------------------------------
 
-__global__ void __launch_bounds__(kT) k_cells(const double* __restrict__ rec, CellArgs a,
+// A record that needs the FP64 cells would hold its whole warp for the FP64
+// sincos; a block puts them on a list instead and forms them at the end, full
+// warps at a time.  24 x 2^18 records: 424 us with FP64 comparisons and
+// conversions and the FP64 cells in place (the FP64 pipe 80 % busy), 119 us now
+// (252 MB in and 107 MB out: 53 us at the copy rate; the rest is instruction
+// issue, two sincosf a record).
+__global__ void __launch_bounds__(kT) k_cells(const double* __restrict__ rec,
+                                              const __grid_constant__ CellArgs a,
                                               int4* __restrict__ cells_raw, uint8_t* __restrict__ flag,
                                               unsigned* __restrict__ blk_cnt, int* __restrict__ minmax,
-                                              unsigned* __restrict__ nexact, double* __restrict__ snr_raw) {
+                                              unsigned* __restrict__ nexact) {
   __shared__ unsigned sh[kT / 32];
   __shared__ int smm[8];
+  __shared__ unsigned short list[kTile];
+  __shared__ unsigned nlist;
   const int b = blockIdx.x;
   const int f = frame_of_block(b);
   const long long fend = c_ft.raw_start[f + 1];
   const long long tile0 = c_ft.raw_start[f] + (long long)(b - c_ft.blk_start[f]) * kTile;
   const double fshift = (double)(a.refr - c_ft.frame_no[f]);
+  if (threadIdx.x == 0) nlist = 0;
   if (threadIdx.x < 4) smm[threadIdx.x] = INT_MAX;
   else if (threadIdx.x < 8) smm[threadIdx.x] = INT_MIN;
   __syncthreads();
   unsigned cnt = 0;
   int mn[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX}, mx[4] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN};
+  auto extend = [&](int4 cl) {
+    mn[0] = min(mn[0], cl.x); mx[0] = max(mx[0], cl.x);
+    mn[1] = min(mn[1], cl.y); mx[1] = max(mx[1], cl.y);
+    mn[2] = min(mn[2], cl.z); mx[2] = max(mx[2], cl.z);
+    mn[3] = min(mn[3], cl.w); mx[3] = max(mx[3], cl.w);
+  };
+  // the record of the next round is loaded before this round's arithmetic
+  double nx[5] = {0, 0, 0, 0, 0};
+  auto load = [&](long long r) {
+    if (r < fend)
+#pragma unroll
+      for (int k = 0; k < 5; k++) nx[k] = __ldg(rec + 5 * r + k);
+  };
+  load(tile0 + threadIdx.x);
+#pragma unroll 1
   for (int it = 0; it < kIt; it++) {
     const long long r = tile0 + (long long)it * kT + threadIdx.x;
     if (r >= fend) break;
+    const double c0 = nx[0], c1 = nx[1], c2 = nx[2], c3 = nx[3], c4 = nx[4];
+    if (it + 1 < kIt) load(r + kT);
     int4 cl = make_int4(0, 0, 0, 0);
-    const int ok = cell_of(rec + 5 * r, fshift, a, &cl, nexact);
-    flag[r] = (uint8_t)ok;
-    cells_raw[r] = cl;
-    snr_raw[r] = rec[5 * r + 4];
-    if (ok) {
-      cnt++;
-      mn[0] = min(mn[0], cl.x); mx[0] = max(mx[0], cl.x);
-      mn[1] = min(mn[1], cl.y); mx[1] = max(mx[1], cl.y);
-      mn[2] = min(mn[2], cl.z); mx[2] = max(mx[2], cl.z);
-      mn[3] = min(mn[3], cl.w); mx[3] = max(mx[3], cl.w);
+    const int ok = cell_of(c0, c1, c2, c3, c4, fshift, a, &cl);
+    flag[r] = ok != 0;
+    cnt += ok != 0;
+    if (ok == 2) {
+      list[atomicAdd(&nlist, 1u)] = (unsigned short)(it * kT + threadIdx.x);
+    } else {
+      cells_raw[r] = cl;
+      if (ok) extend(cl);
     }
   }
+  __syncthreads();
+  const unsigned nl = nlist;
+  for (unsigned q = threadIdx.x; q < nl; q += kT) {
+    const long long r = tile0 + list[q];
+    const double c0 = rec[5 * r], c1 = rec[5 * r + 1];
+    int4 cl;
+    cells_f64(__dadd_rn(c0, __dmul_rn(__dmul_rn(c1, a.N2), fshift)), c1, rec[5 * r + 2], rec[5 * r + 3], a, &cl);
+    cells_raw[r] = cl;
+    extend(cl);
+  }
+  if (threadIdx.x == 0 && nl) atomicAdd(nexact, nl);
   const unsigned tot = block_sum(cnt, sh);
   if (threadIdx.x == 0) blk_cnt[b] = tot;
-  if (cnt) {
+  if (mx[0] >= mn[0]) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       atomicMin(&smm[j], mn[j]);
@@ -354,34 +417,112 @@ template <typename K>
 __global__ void __launch_bounds__(kT) k_inband(const uint8_t* __restrict__ flag, const int4* __restrict__ cells_raw,
                                                const unsigned* __restrict__ blk_off, KeyLayout L,
                                                unsigned* __restrict__ rawidx, int4* __restrict__ cells_in,
-                                               K* __restrict__ key, unsigned* __restrict__ val,
-                                               const double* __restrict__ snr_raw, double* __restrict__ snr_in) {
+                                               K* __restrict__ key, unsigned* __restrict__ val) {
   __shared__ unsigned sh[kT / 32];
+  __shared__ unsigned short list[kTile];
   const int b = blockIdx.x;
   const int f = frame_of_block(b);
-  const long long fend = c_ft.raw_start[f + 1];
   const long long tile0 = c_ft.raw_start[f] + (long long)(b - c_ft.blk_start[f]) * kTile;
-  unsigned base = blk_off[b];
-  for (int it = 0; it < kIt; it++) {
-    const long long r = tile0 + (long long)it * kT + threadIdx.x;
-    // every thread takes part in the prefix (bounds folded into the flag)
-    const int ok = (r < fend) ? flag[r] : 0;
-    unsigned tot;
-    const unsigned pre = block_flag_prefix(ok, sh, &tot);
-    if (ok) {
-      const unsigned o = base + pre;
-      const int4 cl = cells_raw[r];
-      rawidx[o] = (unsigned)r;
-      cells_in[o] = cl;
-      key[o] = make_key<K>(cl, L);
-      val[o] = o;
-      snr_in[o] = snr_raw[r];
-    }
-    base += tot;
+  const unsigned base = blk_off[b];
+  const unsigned tot = tile_list(flag, tile0, c_ft.raw_start[f + 1], list, sh);
+  for (unsigned q = threadIdx.x; q < tot; q += kT) {
+    const long long r = tile0 + list[q];
+    const unsigned o = base + q;
+    const int4 cl = cells_raw[r];
+    rawidx[o] = (unsigned)r;
+    cells_in[o] = cl;
+    key[o] = make_key<K>(cl, L);
+    val[o] = o;
   }
 }
 
 // ---- scan (exclusive, in place) ------------------------------------------
+
+// One block scans up to kScanOne elements: the tile counts of a few million
+// records are a few thousand, where three launches took 12 us and one takes 4
+// (a round of 8192 elements takes about 2.5 us, so four rounds at most).
+constexpr int kST = 1024;
+constexpr long long kScanOne = 4 * kST * kIt;
+__global__ void __launch_bounds__(kST) k_scan_one(unsigned* __restrict__ d, int n) {
+  __shared__ unsigned sh[kST / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned carry = 0;
+  for (int r = 0; r < n; r += kST * kIt) {
+    const int t0 = r + threadIdx.x * kIt;
+    unsigned v[kIt], s = 0;
+#pragma unroll
+    for (int k = 0; k < kIt; k++) {
+      v[k] = (t0 + k < n) ? d[t0 + k] : 0u;
+      s += v[k];
+    }
+    unsigned x = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) sh[w] = x;
+    __syncthreads();
+    unsigned z = sh[lane];  // inclusive scan of the warp sums, in every warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, z, o);
+      if (lane >= o) z += y;
+    }
+    const unsigned before = w ? __shfl_sync(0xffffffffu, z, w ? w - 1 : 0) : 0u;
+    const unsigned all = __shfl_sync(0xffffffffu, z, 31);
+    unsigned run = carry + before + x - s;
+#pragma unroll
+    for (int k = 0; k < kIt; k++) {
+      if (t0 + k < n) d[t0 + k] = run;
+      run += v[k];
+    }
+    carry += all;
+    __syncthreads();
+  }
+}
+
+// Exclusive scan of every row d[r * n .. r * n + n) in place, one block per
+// row; the row's sum to total[r].
+__global__ void __launch_bounds__(kT) k_scan_rows(unsigned* __restrict__ d, int n, unsigned* __restrict__ total) {
+  __shared__ unsigned sh[kT / 32];
+  unsigned* row = d + (long long)blockIdx.x * n;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned carry = 0;
+  for (long long r = 0; r < n; r += kTile) {
+    const long long t0 = r + threadIdx.x * kIt;
+    unsigned v[kIt], s = 0;
+#pragma unroll
+    for (int k = 0; k < kIt; k++) {
+      v[k] = (t0 + k < n) ? row[t0 + k] : 0u;
+      s += v[k];
+    }
+    unsigned x = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) sh[w] = x;
+    __syncthreads();
+    unsigned before = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < kT / 32; k++) {
+      const unsigned c = sh[k];
+      if (k < w) before += c;
+      all += c;
+    }
+    unsigned run = carry + before + x - s;
+#pragma unroll
+    for (int k = 0; k < kIt; k++) {
+      if (t0 + k < n) row[t0 + k] = run;
+      run += v[k];
+    }
+    carry += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
 
 __global__ void __launch_bounds__(kT) k_scan_tiles(unsigned* __restrict__ d, long long n, unsigned* __restrict__ sums) {
   __shared__ unsigned sh[kT];
@@ -430,20 +571,28 @@ __global__ void __launch_bounds__(kT) k_scan_add(unsigned* __restrict__ d, long 
 
 // ---- radix sort (LSD, 8-bit digits, stable) ------------------------------
 
+constexpr int kRItems = kRTile / kT;
+
 template <typename K>
 __global__ void __launch_bounds__(kT) k_radix_hist(const K* __restrict__ key, long long n, int shift, int nblk,
-                                                   unsigned* __restrict__ hist, unsigned* __restrict__ cnt_local) {
+                                                   unsigned* __restrict__ hist) {
   __shared__ unsigned h[256];
+  const long long t0 = (long long)blockIdx.x * kRTile + threadIdx.x;
+  // only the 32-bit word that holds the digit; all of a thread's loads together
+  const unsigned* word = reinterpret_cast<const unsigned*>(key) + (shift >> 5);
+  unsigned d[kRItems];
+#pragma unroll
+  for (int k = 0; k < kRItems; k++) {
+    const long long i = t0 + k * kT;
+    d[k] = i < n ? (word[i * (int)(sizeof(K) / 4)] >> (shift & 31)) & 255u : 256u;
+  }
   h[threadIdx.x] = 0;
   __syncthreads();
-  const long long t0 = (long long)blockIdx.x * kRTile;
-  for (int k = threadIdx.x; k < kRTile; k += kT) {
-    const long long i = t0 + k;
-    if (i < n) atomicAdd(&h[digit_of(key[i], shift)], 1u);
-  }
+#pragma unroll
+  for (int k = 0; k < kRItems; k++)
+    if (d[k] < 256u) atomicAdd(&h[d[k]], 1u);
   __syncthreads();
   hist[(long long)threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
-  cnt_local[(long long)blockIdx.x * 256 + threadIdx.x] = h[threadIdx.x];
 }
 
 // digit = frame of the element (for the per-frame ranks of the sorted order)
@@ -451,243 +600,310 @@ __global__ void __launch_bounds__(kT) k_frame_hist(const unsigned* __restrict__ 
                                                    unsigned* __restrict__ hist) {
   __shared__ unsigned h[256];
   __shared__ unsigned s_in[kMaxFrames + 1];
+  const long long t0 = (long long)blockIdx.x * kRTile + threadIdx.x;
+  unsigned v[kRItems];
+#pragma unroll
+  for (int k = 0; k < kRItems; k++) v[k] = t0 + k * kT < n ? val[t0 + k * kT] : 0u;
   h[threadIdx.x] = 0;
   load_in_start(s_in);
   const int nf = c_ft.nframes;
-  const long long t0 = (long long)blockIdx.x * kRTile;
-  for (int k = threadIdx.x; k < kRTile; k += kT) {
-    const long long i = t0 + k;
-    if (i < n) atomicAdd(&h[frame_of_in(val[i], s_in, nf)], 1u);
-  }
+#pragma unroll
+  for (int k = 0; k < kRItems; k++)
+    if (t0 + k * kT < n) atomicAdd(&h[frame_of_in(v[k], s_in, nf)], 1u);
   __syncthreads();
-  hist[(long long)threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
+  if (threadIdx.x < nf) hist[(long long)threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
 }
 
-// Stable scatter of one 8-bit digit.  A tile of kRTile items is ranked in
-// chunks of kT x kSub items (item j*kT + t of a chunk held by thread t):
-// peers with the same digit in the warp (match_any), then an exclusive prefix
-// per digit over the (item slot, warp) pairs in item order, carried across
-// chunks.  Each item is staged in shared memory at its digit's place in the
-// tile (tile base from the tile's own digit counts), and the tile is then
-// written out digit run by digit run, so that consecutive threads store to
-// consecutive addresses.
-constexpr int kSub = 2;
-constexpr int kChunk = kT * kSub;
-constexpr int kSlots = kSub * (kT / 32);
+// Stable scatter of one 8-bit digit.  A block takes a tile of kRTile items,
+// every warp kWItems consecutive ones in rows of 32.  A row's items of one
+// digit find each other by eight ballots (one per bit); the lowest of them
+// adds their number to the warp's own counter of the digit, so that the rows
+// need no barrier.  One barrier, a prefix of the counters over warps and
+// digits, and every item is staged in shared memory at its digit's place in
+// the tile; the tile is then written out digit run by digit run, so that
+// consecutive threads store to consecutive addresses.  Places past the end
+// count as digit 255: they come after every item of the tile.
+// What bounds it: instruction issue and shared memory in the ranking, then 24
+// bytes an item through L2 and HBM (38 MB of keys and 19 MB of indices each way
+// do not stay in L2 together).  4.7 million items: 52 us a pass with counters
+// shared by the block (a barrier after every 512 items), 32 us now; the digit
+// counts 10 us, their scan by rows 4 us (14 us as one scan of 256 x tiles).
+constexpr int kSThreads = 512;
+constexpr int kSWarps = kSThreads / 32;
+constexpr int kWItems = kRTile / kSWarps;
+constexpr int kSRows = kWItems / 32;
 
 template <typename K>
 constexpr size_t scatter_smem() {
-  return (size_t)kRTile * (sizeof(K) + sizeof(unsigned) + 1) + sizeof(unsigned) * 256 * (kSlots + 3);
-}
-
-__device__ __forceinline__ unsigned block_excl_scan(unsigned v, unsigned* scr) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  unsigned x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) scr[w] = x;
-  __syncthreads();
-  unsigned before = 0;
-  for (int k = 0; k < w; k++) before += scr[k];
-  __syncthreads();
-  return before + x - v;
+  return (size_t)kRTile * (sizeof(K) + sizeof(unsigned)) + sizeof(unsigned short) * 256 * kSWarps;
 }
 
 template <typename K>
-__global__ void __launch_bounds__(kT) k_radix_scatter(const K* __restrict__ kin, const unsigned* __restrict__ vin,
-                                                      K* __restrict__ kout, unsigned* __restrict__ vout, long long n,
-                                                      int shift, int nblk, const unsigned* __restrict__ off,
-                                                      const unsigned* __restrict__ cnt_local) {
+__global__ void __launch_bounds__(kSThreads, 2)
+    k_radix_scatter(const K* __restrict__ kin, const unsigned* __restrict__ vin, K* __restrict__ kout,
+                    unsigned* __restrict__ vout, long long n, int shift, int nblk, const unsigned* __restrict__ off,
+                    const unsigned* __restrict__ total) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ unsigned scr[kT / 32];
+  __shared__ unsigned goff[256];
+  __shared__ unsigned long long scr[8];
   K* st_k = (K*)smem;
   unsigned* st_v = (unsigned*)(st_k + kRTile);
-  unsigned* wc = st_v + kRTile;              // [kSlots][256]
-  unsigned* run = wc + kSlots * 256;
-  unsigned* base = run + 256;
-  unsigned* goff = base + 256;
-  uint8_t* st_d = (uint8_t*)(goff + 256);
+  unsigned short* cnt = (unsigned short*)(st_v + kRTile);  // [kSWarps][256]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long t0 = (long long)blockIdx.x * kRTile;
-  const long long rem = n - t0;
-  const int tn = rem < kRTile ? (int)rem : kRTile;
-  const unsigned bt = block_excl_scan(cnt_local[(long long)blockIdx.x * 256 + threadIdx.x], scr);
-  base[threadIdx.x] = bt;
-  goff[threadIdx.x] = off[(long long)threadIdx.x * nblk + blockIdx.x];
-  run[threadIdx.x] = 0;
-  // the thread's items of the whole tile, loaded together
-  constexpr int kCh = kRTile / kChunk;
-  K kk[kCh][kSub];
-  unsigned vv[kCh][kSub];
+  const int tn = (int)(n - t0 < kRTile ? n - t0 : kRTile);
+  K kk[kSRows] = {};
+  unsigned vv[kSRows] = {};
 #pragma unroll
-  for (int c = 0; c < kCh; c++)
-#pragma unroll
-    for (int j = 0; j < kSub; j++) {
-      const int li = c * kChunk + j * kT + threadIdx.x;
-      vv[c][j] = 0;
-      if (li < tn) {
-        kk[c][j] = kin[t0 + li];
-        vv[c][j] = vin[t0 + li];
-      }
+  for (int k = 0; k < kSRows; k++) {
+    const int li = w * kWItems + 32 * k + lane;
+    if (li < tn) {
+      kk[k] = kin[t0 + li];
+      vv[k] = vin[t0 + li];
     }
-#pragma unroll
-  for (int c = 0; c < kCh; c++) {
-    unsigned d[kSub], rank[kSub];
-#pragma unroll
-    for (int j = 0; j < kSub; j++) {
-      const int li = c * kChunk + j * kT + threadIdx.x;
-      d[j] = li < tn ? digit_of(kk[c][j], shift) : 256u;
-    }
-    for (int k = 0; k < kSlots; k++) wc[k * 256 + threadIdx.x] = 0;
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kSub; j++) {
-      const unsigned peers = __match_any_sync(0xffffffffu, d[j]);
-      rank[j] = __popc(peers & ((1u << lane) - 1u));
-      if (d[j] < 256 && lane == __ffs(peers) - 1) wc[(j * (kT / 32) + w) * 256 + d[j]] = __popc(peers);
-    }
-    __syncthreads();
-    {
-      const int dg = threadIdx.x;
-      unsigned p = run[dg];
-      for (int k = 0; k < kSlots; k++) {
-        const unsigned t = wc[k * 256 + dg];
-        wc[k * 256 + dg] = p;
-        p += t;
-      }
-      run[dg] = p;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kSub; j++)
-      if (d[j] < 256) {
-        const unsigned lp = base[d[j]] + wc[(j * (kT / 32) + w) * 256 + d[j]] + rank[j];
-        st_k[lp] = kk[c][j];
-        st_v[lp] = vv[c][j];
-        st_d[lp] = (uint8_t)d[j];
-      }
-    __syncthreads();
   }
-  for (int q = threadIdx.x; q < tn; q += kT) {
-    const unsigned dq = st_d[q];
-    const unsigned g = goff[dq] + ((unsigned)q - base[dq]);
-    kout[g] = st_k[q];
+  unsigned o = 0, all = 0;
+  if (threadIdx.x < 256) {
+    o = off[(long long)threadIdx.x * nblk + blockIdx.x];
+    all = total[threadIdx.x];
+  }
+  unsigned short* cw = cnt + w * 256;
+#pragma unroll
+  for (int k = 0; k < 4; k++) reinterpret_cast<unsigned*>(cw)[32 * k + lane] = 0;
+  __syncwarp();
+  unsigned short rank[kSRows];
+#pragma unroll
+  for (int k = 0; k < kSRows; k++) {
+    const unsigned d = w * kWItems + 32 * k + lane < tn ? digit_of(kk[k], shift) : 255u;
+    unsigned peers = 0xffffffffu;
+#pragma unroll
+    for (int bit = 0; bit < 8; bit++) {
+      const bool one = (d >> bit) & 1u;
+      const unsigned bal = __ballot_sync(0xffffffffu, one);
+      peers &= one ? bal : ~bal;
+    }
+    const int lead = __ffs(peers) - 1;
+    unsigned before = 0;
+    if (lane == lead) {
+      before = cw[d];
+      cw[d] = (unsigned short)(before + __popc(peers));
+    }
+    __syncwarp();
+    rank[k] = (unsigned short)(__shfl_sync(0xffffffffu, before, lead) + __popc(peers & ((1u << lane) - 1u)));
+  }
+  __syncthreads();
+  // the digit's items in the warps before, in the tile's digits before, and
+  // in all digits before: one scan over the digits carries the last two
+  unsigned long long x = 0, own = 0;
+  if (threadIdx.x < 256) {
+    unsigned p = 0;
+#pragma unroll
+    for (int k = 0; k < kSWarps; k++) {
+      const unsigned c = cnt[k * 256 + threadIdx.x];
+      cnt[k * 256 + threadIdx.x] = (unsigned short)p;
+      p += c;
+    }
+    own = x = ((unsigned long long)all << 32) | p;
+#pragma unroll
+    for (int q = 1; q < 32; q <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, x, q);
+      if (lane >= q) x += y;
+    }
+    if (lane == 31) scr[w] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < 256) {
+    unsigned long long before = x - own;
+    for (int k = 0; k < w; k++) before += scr[k];
+    const unsigned tile0 = (unsigned)before;
+#pragma unroll
+    for (int k = 0; k < kSWarps; k++) cnt[k * 256 + threadIdx.x] += (unsigned short)tile0;
+    goff[threadIdx.x] = (unsigned)(before >> 32) + o - tile0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kSRows; k++) {
+    const unsigned d = w * kWItems + 32 * k + lane < tn ? digit_of(kk[k], shift) : 255u;
+    const unsigned lp = cw[d] + rank[k];
+    st_k[lp] = kk[k];
+    st_v[lp] = vv[k];
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < tn; q += kSThreads) {
+    const K k = st_k[q];
+    const unsigned g = goff[digit_of(k, shift)] + (unsigned)q;
+    kout[g] = k;
     vout[g] = st_v[q];
   }
 }
 
 // ---- per-frame ranks: element p of frame g in sorted order -----------------
 
-// req[r] = {frame, rank}; out[r] = sorted position (-1 if absent), with the
-// element's cells and key.  One warp per request: binary search over the
-// frame's block offsets, then a count through the block's tile.
+// What the duplicate removal asks of a frame: the rank of its last record
+// (-1: no records), and the latest earlier frame whose sorted rows reach past
+// that rank (-1: none), whose record there is what the reference compares the
+// last one with (the candidate table starts zeroed for its first 10485760
+// rows, struct.h:10).
+struct FrameReq {
+  int last, stale_frame, stale, pad;
+};
+struct FrameFound {
+  int4 cells[2];                 // of the last record and of the stale one
+  unsigned long long lo, hi;     // key of the last record
+};
+
+// Request 2 f: the last record of frame f in sorted order; 2 f + 1: the stale
+// one.  One block per request: 256-ary search over the frame's row of tile
+// offsets, then the place within the tile by a scan.
 template <typename K>
-__global__ void k_frame_find(const int2* __restrict__ req, int nreq, const unsigned* __restrict__ hoff, int nblk,
-                             const unsigned* __restrict__ val, long long n,
-                             const K* __restrict__ key, const int4* __restrict__ cells_in,
-                             long long* __restrict__ out, int4* __restrict__ out_cells,
-                             unsigned long long* __restrict__ out_key) {
+__global__ void __launch_bounds__(kT) k_frame_find(const FrameReq* __restrict__ req, const unsigned* __restrict__ hoff,
+                                                   int nblk, const unsigned* __restrict__ val, long long n,
+                                                   const K* __restrict__ key, const int4* __restrict__ cells_in,
+                                                   FrameFound* __restrict__ out, int* __restrict__ failed) {
   __shared__ unsigned s_in[kMaxFrames + 1];
+  __shared__ unsigned sh[kT / 32];
+  const int f = blockIdx.x >> 1, which = blockIdx.x & 1;
+  const FrameReq rq = req[f];
+  const int g = which ? rq.stale_frame : f, p = which ? rq.stale : rq.last;
+  if (g < 0 || p < 0) return;
   load_in_start(s_in);
   const int nf = c_ft.nframes;
-  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (r >= nreq) return;
-  const int g = req[r].x, p = req[r].y;
   const unsigned* o = hoff + (long long)g * nblk;
-  const unsigned base = o[0];
-  // last block b with o[b] - base <= p
+  // last tile b with o[b] <= p (o[0] = 0)
   int lo = 0, hi = nblk;
   while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (o[mid] - base <= (unsigned)p) lo = mid; else hi = mid;
+    const int step = (hi - lo + kT - 1) / kT, at = lo + (int)threadIdx.x * step;
+    const int c = __syncthreads_count(at < hi && o[at] <= (unsigned)p);
+    lo += (c - 1) * step;
+    hi = min(hi, lo + step);
   }
-  unsigned need = (unsigned)p - (o[lo] - base);
-  long long found = -1;
-  const long long t0 = (long long)lo * kRTile;
-  for (int k = 0; k < kRTile; k += 32) {
-    const long long i = t0 + k + lane;
-    const int hit = (i < n) && (frame_of_in(val[i], s_in, nf) == g);
-    const unsigned bal = __ballot_sync(0xffffffffu, hit);
-    const unsigned c = __popc(bal);
-    if (need < c) {
-      // the (need)-th set lane
-      unsigned m = bal;
-      for (unsigned q = 0; q < need; q++) m &= m - 1;
-      found = t0 + k + (__ffs(m) - 1);
-      break;
-    }
-    need -= c;
+  const unsigned need = (unsigned)p - o[lo];
+  const long long t0 = (long long)lo * kRTile + threadIdx.x * kRItems;
+  unsigned hit = 0;
+#pragma unroll
+  for (int k = 0; k < kRItems; k++)
+    if (t0 + k < n && frame_of_in(val[t0 + k], s_in, nf) == g) hit |= 1u << k;
+  const unsigned c = __popc(hit);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned x = c;
+#pragma unroll
+  for (int q = 1; q < 32; q <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, x, q);
+    if (lane >= q) x += y;
   }
-  if (lane == 0) {
-    out[r] = found;
-    if (found >= 0) {
-      out_cells[r] = cells_in[val[found]];
-      key_split(key[found], &out_key[2 * r], &out_key[2 * r + 1]);
-    }
+  if (lane == 31) sh[w] = x;
+  __syncthreads();
+  unsigned before = x - c, all = 0;
+  for (int k = 0; k < kT / 32; k++) {
+    if (k < w) before += sh[k];
+    all += sh[k];
   }
+  if (need >= all && threadIdx.x == 0) *failed = 1;
+  if (need >= before && need < before + c) {
+    for (unsigned q = before; q < need; q++) hit &= hit - 1;
+    const long long at = t0 + __ffs(hit) - 1;
+    out[f].cells[which] = cells_in[val[at]];
+    if (!which) key_split(key[at], &out[f].lo, &out[f].hi);
+  }
+}
+
+// Last run of a frame that is not written (its last record's cells equal the
+// stale ones, zeros where there is none).
+struct FrameDrop {
+  unsigned long long lo, hi;
+  int drop, pad;
+};
+__device__ __forceinline__ FrameDrop frame_drop(const FrameReq& rq, const FrameFound& fd) {
+  const int4 a = fd.cells[0], b = rq.stale_frame >= 0 ? fd.cells[1] : make_int4(0, 0, 0, 0);
+  return {fd.lo, fd.hi, rq.last >= 0 && a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w, 0};
 }
 
 // ---- duplicate removal per (cells, frame) run ------------------------------
 
+// A tile of kTile records a block, with its neighbours, in shared memory: keys
+// and frames.  Nearly every record is a run of its own and is settled there;
+// the others walk their run in global memory.  removed[f]: records of frame f
+// that are not kept.  (4.7 million records: 59 us, 67 us with a thread per
+// record that searched its neighbours' frames again.)
 template <typename K>
 __global__ void __launch_bounds__(kT) k_dedup(const K* __restrict__ key, const unsigned* __restrict__ val,
-                                              const double* __restrict__ snr_in, long long n,
-                                              uint8_t* __restrict__ keep, unsigned* __restrict__ uniq) {
-  __shared__ unsigned hcount[256];
+                                              const unsigned* __restrict__ rawidx, const double* __restrict__ rec,
+                                              const FrameReq* __restrict__ req, const FrameFound* __restrict__ found,
+                                              long long n, uint8_t* __restrict__ keep, unsigned* __restrict__ removed) {
+  __shared__ K s_key[kTile + 2];
+  __shared__ uint8_t s_frame[kTile + 2];
+  __shared__ FrameDrop s_drop[kMaxFrames];
   __shared__ unsigned s_in[kMaxFrames + 1];
-  hcount[threadIdx.x] = 0;
+  const long long t0 = (long long)blockIdx.x * kTile;
+  unsigned v[kIt];
+#pragma unroll
+  for (int k = 0; k < kIt; k++) {
+    const long long i = t0 + k * kT + threadIdx.x;
+    v[k] = 0;
+    if (i < n) {
+      s_key[1 + k * kT + threadIdx.x] = key[i];
+      v[k] = val[i];
+    }
+  }
+  if (threadIdx.x < c_ft.nframes) s_drop[threadIdx.x] = frame_drop(req[threadIdx.x], found[threadIdx.x]);
   load_in_start(s_in);
   const int nf = c_ft.nframes;
-  const long long i = (long long)blockIdx.x * kT + threadIdx.x;
-  if (i < n) {
-    const K k0 = key[i];
-    const unsigned v0 = val[i];
-    const int f = frame_of_in(v0, s_in, nf);
-    // the previous record's frame matters only when its cells are equal
-    const bool start = (i == 0) || !(key[i - 1] == k0) || frame_of_in(val[i - 1], s_in, nf) != f;
-    uint8_t kept = 0;
-    if (start) {
-      const long long fs = s_in[f];
-      // walk the run [i, j]
-      long long j = i;
-      while (j + 1 < n && key[j + 1] == k0 && frame_of_in(val[j + 1], s_in, nf) == f) j++;
-      // coincidences.c:317-413 over the pairs (t, t + 1) of the run
-      long long maxsnridx = 0, maxi = i;
-      double candsnr = 0;
-      unsigned vt = v0;
-      double s0 = j > i ? snr_in[vt] : 0.;
-      for (long long t = i; t < j; t++) {
-        const unsigned vt1 = val[t + 1];
-        const double s1 = snr_in[vt1];
-        const long long idx = (long long)vt - fs, idx1 = (long long)vt1 - fs;
-        if (!maxsnridx) {
-          maxsnridx = (s0 > s1) ? idx : idx1;
-          maxi = (s0 > s1) ? t : t + 1;
-          candsnr = (s0 > s1) ? s0 : s1;
-        } else {
-          if (s0 > candsnr) {
-            maxsnridx = idx; maxi = t; candsnr = s0;
-          } else if (s1 > candsnr) {
-            maxsnridx = idx1; maxi = t + 1; candsnr = s1;
-          }
-        }
-        vt = vt1;
-        s0 = s1;
-      }
-      const bool dropped = c_ft.drop[f] && key_is(k0, c_ft.drop_lo[f], c_ft.drop_hi[f]);
-      if (!dropped) {
-        keep[maxsnridx ? maxi : j] = 1;
-        kept = 1;
-      }
+#pragma unroll
+  for (int k = 0; k < kIt; k++) s_frame[1 + k * kT + threadIdx.x] = (uint8_t)frame_of_in(v[k], s_in, nf);
+  if (threadIdx.x < 2) {
+    const long long i = threadIdx.x ? t0 + kTile : t0 - 1;
+    if (i >= 0 && i < n) {
+      s_key[threadIdx.x ? kTile + 1 : 0] = key[i];
+      s_frame[threadIdx.x ? kTile + 1 : 0] = (uint8_t)frame_of_in(val[i], s_in, nf);
     }
-    if (kept) atomicAdd(&hcount[f], 1u);
   }
   __syncthreads();
-  if (hcount[threadIdx.x]) atomicAdd(&uniq[threadIdx.x], hcount[threadIdx.x]);
+  auto snr = [&](unsigned v) { return rec[5 * (long long)rawidx[v] + 4]; };
+#pragma unroll
+  for (int k = 0; k < kIt; k++) {
+    const int li = 1 + k * kT + threadIdx.x;
+    const long long i = t0 + li - 1;
+    if (i >= n) break;
+    const K k0 = s_key[li];
+    const int f = s_frame[li];
+    if (i > 0 && s_key[li - 1] == k0 && s_frame[li - 1] == f) continue;  // not the first of its run
+    const bool dropped = s_drop[f].drop && key_is(k0, s_drop[f].lo, s_drop[f].hi);
+    const bool single = !(i + 1 < n && s_key[li + 1] == k0 && s_frame[li + 1] == f);
+    if (single && !dropped) {
+      keep[i] = 1;
+      continue;
+    }
+    // the run [i, j]
+    long long j = i;
+    while (j + 1 < n && key[j + 1] == k0 && frame_of_in(val[j + 1], s_in, nf) == f) j++;
+    atomicAdd(&removed[f], (unsigned)(j - i + (dropped ? 1 : 0)));
+    if (dropped) continue;
+    // coincidences.c:317-413 over the pairs (t, t + 1) of the run
+    const long long fs = s_in[f];
+    long long maxsnridx = 0, maxi = i;
+    double candsnr = 0;
+    unsigned vt = val[i];
+    double s0 = snr(vt);
+    for (long long t = i; t < j; t++) {
+      const unsigned vt1 = val[t + 1];
+      const double s1 = snr(vt1);
+      const long long idx = (long long)vt - fs, idx1 = (long long)vt1 - fs;
+      if (!maxsnridx) {
+        maxsnridx = (s0 > s1) ? idx : idx1;
+        maxi = (s0 > s1) ? t : t + 1;
+        candsnr = (s0 > s1) ? s0 : s1;
+      } else {
+        if (s0 > candsnr) {
+          maxsnridx = idx; maxi = t; candsnr = s0;
+        } else if (s1 > candsnr) {
+          maxsnridx = idx1; maxi = t + 1; candsnr = s1;
+        }
+      }
+      vt = vt1;
+      s0 = s1;
+    }
+    keep[maxsnridx ? maxi : j] = 1;
+  }
 }
 
 // keep flags by in-band index, from the flags by sorted position
@@ -717,45 +933,69 @@ __global__ void __launch_bounds__(kT) k_compact_surv(const uint8_t* __restrict__
                                                      const unsigned* __restrict__ val, K* __restrict__ skey,
                                                      unsigned* __restrict__ sval) {
   __shared__ unsigned sh[kT / 32];
+  __shared__ unsigned short list[kTile];
   const long long t0 = (long long)blockIdx.x * kTile;
-  unsigned base = off[blockIdx.x];
-  for (int k = 0; k < kIt; k++) {
-    const long long i = t0 + (long long)k * kT + threadIdx.x;
-    const int ok = (i < n) ? keep[i] : 0;
-    unsigned tot;
-    const unsigned pre = block_flag_prefix(ok, sh, &tot);
-    if (ok) {
-      skey[base + pre] = key[i];
-      sval[base + pre] = val[i];
-    }
-    base += tot;
+  const unsigned base = off[blockIdx.x];
+  const unsigned tot = tile_list(keep, t0, n, list, sh);
+  for (unsigned q = threadIdx.x; q < tot; q += kT) {
+    const long long i = t0 + list[q];
+    skey[base + q] = key[i];
+    sval[base + q] = val[i];
   }
 }
 
 // runs of equal cells among the survivors (coincidences.c:449-486)
+// (a tile of kTile keys with its neighbours in shared memory; tile counts of
+// the stored groups to cnt)
 template <typename K>
 __global__ void __launch_bounds__(kT) k_groups(const K* __restrict__ skey, long long G, int mincoin,
                                                uint8_t* __restrict__ gflag, unsigned* __restrict__ gend,
-                                               unsigned* __restrict__ gw, int* __restrict__ last_unstored) {
-  const long long i = (long long)blockIdx.x * kT + threadIdx.x;
-  if (i >= G) return;
-  const K k0 = skey[i];
-  uint8_t fl = 0;
-  if (i == 0 || !(skey[i - 1] == k0)) {
-    long long j = i;
-    while (j + 1 < G && skey[j + 1] == k0) j++;
-    const long long w = j - i + 1;
-    if (w >= mincoin) {
-      if (j < G - 1) {
-        fl = 1;
-        gend[i] = (unsigned)j;
-        gw[i] = (unsigned)w;
-      } else {
-        *last_unstored = 1;
+                                               unsigned* __restrict__ gw, int* __restrict__ last_unstored,
+                                               unsigned* __restrict__ members, unsigned* __restrict__ cnt) {
+  __shared__ K s_key[kTile + 2];
+  __shared__ unsigned sh[kT / 32];
+  const long long t0 = (long long)blockIdx.x * kTile;
+#pragma unroll
+  for (int k = 0; k < kIt; k++) {
+    const long long i = t0 + k * kT + threadIdx.x;
+    if (i < G) s_key[1 + k * kT + threadIdx.x] = skey[i];
+  }
+  if (threadIdx.x < 2) {
+    const long long i = threadIdx.x ? t0 + kTile : t0 - 1;
+    if (i >= 0 && i < G) s_key[threadIdx.x ? kTile + 1 : 0] = skey[i];
+  }
+  __syncthreads();
+  unsigned stored = 0, mem = 0;
+#pragma unroll
+  for (int k = 0; k < kIt; k++) {
+    const int li = 1 + k * kT + threadIdx.x;
+    const long long i = t0 + li - 1;
+    if (i >= G) break;
+    const K k0 = s_key[li];
+    uint8_t fl = 0;
+    if ((i == 0 || !(s_key[li - 1] == k0)) && i + 1 < G && s_key[li + 1] == k0) {  // (mincoin >= 2)
+      long long j = i + 1;
+      while (j + 1 < G && skey[j + 1] == k0) j++;
+      const long long w = j - i + 1;
+      if (w >= mincoin) {
+        if (j < G - 1) {
+          fl = 1;
+          gend[i] = (unsigned)j;
+          gw[i] = (unsigned)w;
+          stored++;
+          mem += (unsigned)w;
+        } else {
+          *last_unstored = 1;
+        }
       }
     }
+    gflag[i] = fl;
   }
-  gflag[i] = fl;
+  const unsigned tot = block_sum(stored, sh), tm = block_sum(mem, sh);
+  if (threadIdx.x == 0) {
+    cnt[blockIdx.x] = tot;
+    if (tm) atomicAdd(members, tm);
+  }
 }
 
 __global__ void __launch_bounds__(kT) k_compact_groups(const uint8_t* __restrict__ gflag, long long G,
@@ -765,21 +1005,17 @@ __global__ void __launch_bounds__(kT) k_compact_groups(const uint8_t* __restrict
                                                        unsigned* __restrict__ cend, unsigned* __restrict__ cw,
                                                        unsigned* __restrict__ cidx) {
   __shared__ unsigned sh[kT / 32];
+  __shared__ unsigned short list[kTile];
   const long long t0 = (long long)blockIdx.x * kTile;
-  unsigned base = off[blockIdx.x];
-  for (int k = 0; k < kIt; k++) {
-    const long long i = t0 + (long long)k * kT + threadIdx.x;
-    const int ok = (i < G) ? gflag[i] : 0;
-    unsigned tot;
-    const unsigned pre = block_flag_prefix(ok, sh, &tot);
-    if (ok) {
-      const unsigned o = base + pre;
-      cend[o] = gend[i];
-      cw[o] = gw[i];
-      wkey[o] = 255ull - gw[i];   // multiplicity <= frames <= 255: one digit
-      cidx[o] = o;
-    }
-    base += tot;
+  const unsigned base = off[blockIdx.x];
+  const unsigned tot = tile_list(gflag, t0, G, list, sh);
+  for (unsigned q = threadIdx.x; q < tot; q += kT) {
+    const long long i = t0 + list[q];
+    const unsigned o = base + q;
+    cend[o] = gend[i];
+    cw[o] = gw[i];
+    wkey[o] = 255ull - gw[i];   // multiplicity <= frames <= 255: one digit
+    cidx[o] = o;
   }
 }
 
@@ -789,44 +1025,70 @@ __global__ void k_gather_w(const unsigned* __restrict__ order, const unsigned* _
   if (q < K) w_sorted[q] = cw[order[q]];
 }
 
-// coincidences.c:488-525: means over the members k = end, end - 1, ...
-__global__ void k_means(const unsigned* __restrict__ order, const unsigned* __restrict__ cend,
-                        const unsigned* __restrict__ cw, const unsigned* __restrict__ first, int K,
-                        const unsigned* __restrict__ sval, const unsigned* __restrict__ rawidx,
-                        const double* __restrict__ rec, double N, int refr,
-                        pa_coinc_rec* __restrict__ out, int* __restrict__ fra, int* __restrict__ ops) {
+// coincidences.c:488-525: means over the members k = end, end - 1, ...  One
+// warp per coincidence loads 32 members at once (a thread per coincidence
+// spent 60 us on 12 000 of them, one dependent load after the other); the sums
+// then run in the reference's order, a thread per coincidence and column (all
+// lanes adding the same numbers spent 68 us in the FP64 pipe).
+__global__ void __launch_bounds__(kT) k_means(const unsigned* __restrict__ order, const unsigned* __restrict__ cend,
+                                              const unsigned* __restrict__ cw, const unsigned* __restrict__ first,
+                                              int K, const unsigned* __restrict__ sval,
+                                              const unsigned* __restrict__ rawidx, const double* __restrict__ rec,
+                                              double N, int refr, pa_coinc_rec* __restrict__ out,
+                                              int* __restrict__ fra, int* __restrict__ ops) {
+  constexpr int kG = kT / 32;
   __shared__ unsigned s_in[kMaxFrames + 1];
+  __shared__ double s_t[kG][32][5];
+  __shared__ int s_w[kG];
   load_in_start(s_in);
   const int nf = c_ft.nframes;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= K) return;
-  const unsigned g = order[q];
-  const long long j = cend[g];
-  const int w = (int)cw[g];
-  const long long m0 = first[q];
-  double m[5] = {0, 0, 0, 0, 0};
-  for (int i = 0; i < w; i++) {
-    const unsigned v = sval[j - i];
-    const int f = frame_of_in(v, s_in, nf);
-    const long long r = rawidx[v];
-    const double* c = rec + 5 * r;
-    const double fshift = (double)(refr - c_ft.frame_no[f]);
-    const double c0s = __dadd_rn(c[0], __dmul_rn(__dmul_rn(__dmul_rn(2., c[1]), N), fshift));
-    m[0] = __dadd_rn(m[0], c0s);
-    m[1] = __dadd_rn(m[1], c[1]);
-    m[2] = __dadd_rn(m[2], c[2]);
-    m[3] = __dadd_rn(m[3], c[3]);
-    m[4] = __dadd_rn(m[4], __dmul_rn(c[4], c[4]));
-    ops[m0 + i] = (int)(r - c_ft.raw_start[f]);
-    fra[m0 + i] = c_ft.frame_no[f];
+  const int lane = threadIdx.x & 31, gr = threadIdx.x >> 5;
+  const int q = blockIdx.x * kG + gr;
+  long long j = 0, m0 = 0;
+  int w = 0;
+  if (q < K) {
+    const unsigned g = order[q];
+    j = cend[g];
+    w = (int)cw[g];
+    m0 = first[q];
   }
-  const double dw = (double)w;
-  pa_coinc_rec r;
-  r.w = w;
-  r.first = (int)m0;
-  for (int l = 0; l < 4; l++) r.mean[l] = __ddiv_rn(m[l], dw);
-  r.mean[4] = __dsqrt_rn(m[4]);
-  out[q] = r;
+  if (lane == 0) s_w[gr] = w;
+  __syncthreads();
+  int wmax = 0;
+  for (int k = 0; k < kG; k++) wmax = max(wmax, s_w[k]);
+  const int sg = threadIdx.x / 5, sk = threadIdx.x % 5;  // the sum of this thread
+  double m = 0;
+  for (int i0 = 0; i0 < wmax; i0 += 32) {
+    const int i = i0 + lane;
+    if (i < w) {
+      const unsigned v = sval[j - i];
+      const int f = frame_of_in(v, s_in, nf);
+      const long long r = rawidx[v];
+      const double* c = rec + 5 * r;
+      const double fshift = (double)(refr - c_ft.frame_no[f]);
+      double* t = s_t[gr][lane];
+      t[0] = __dadd_rn(c[0], __dmul_rn(__dmul_rn(__dmul_rn(2., c[1]), N), fshift));
+      t[1] = c[1];
+      t[2] = c[2];
+      t[3] = c[3];
+      t[4] = __dmul_rn(c[4], c[4]);
+      ops[m0 + i] = (int)(r - c_ft.raw_start[f]);
+      fra[m0 + i] = c_ft.frame_no[f];
+    }
+    __syncthreads();
+    if (sg < kG) {
+      const int nl = min(32, s_w[sg] - i0);
+      for (int l = 0; l < nl; l++) m = __dadd_rn(m, s_t[sg][l][sk]);
+    }
+    __syncthreads();
+  }
+  const int sq = blockIdx.x * kG + sg;
+  if (sg >= kG || sq >= K) return;
+  out[sq].mean[sk] = sk < 4 ? __ddiv_rn(m, (double)s_w[sg]) : __dsqrt_rn(m);
+  if (sk == 0) {
+    out[sq].w = s_w[sg];
+    out[sq].first = (int)first[sq];
+  }
 }
 
 }  // namespace
@@ -851,7 +1113,7 @@ struct pa_coinc {
     void* p = nullptr;
     size_t n = 0;
   };
-  Buf rec, cells_raw, flag, snr_raw, blkcnt, scan_tmp, minmax, rawidx, cells_in, snr_in, cntl, keyA, keyB, valA, valB, hist,
+  Buf rec, cells_raw, flag, blkcnt, scan_tmp, minmax, rawidx, cells_in, digits, keyA, keyB, valA, valB, hist,
       keep, keep_in, uniq, req, found, skey, sval, gflag, gend, gw, lastu, wkeyA, wkeyB, cend, cw, cidxA, cidxB,
       wsort, means, fra, ops;
   // optional per-kernel profile: events around each launch while on
@@ -959,6 +1221,13 @@ static T* P(pa_coinc::Buf& b) { return (T*)b.p; }
 // every level
 static int scan_excl(pa_coinc* c, unsigned* d, long long n, unsigned* tmp) {
   if (n <= 0) return PA_OK;
+  if (n <= kScanOne) {
+    Span sp_(c, CK_SCAN);
+    k_scan_one<<<1, kST, 0, c->stream>>>(d, (int)n);
+    c->launches++;
+    CCK(cudaGetLastError(), "scan");
+    return PA_OK;
+  }
   const long long nb = (n + kTile - 1) / kTile;
   {
     Span sp_(c, CK_SCAN);
@@ -991,9 +1260,8 @@ template <typename K>
 static int radix_sort(pa_coinc* c, K*& k, unsigned*& v, K* k2, unsigned* v2, long long n, int bits) {
   pa::TraceRange trace_("coinc radix sort");
   const int nblk = (int)((n + kRTile - 1) / kRTile);
-  ENS(hist, sizeof(unsigned) * (256ll * nblk + 1));
-  ENS(cntl, sizeof(unsigned) * 256ll * nblk);
-  ENS(scan_tmp, sizeof(unsigned) * scan_tmp_len(256ll * nblk));
+  ENS(hist, sizeof(unsigned) * 256ll * nblk);
+  ENS(digits, sizeof(unsigned) * 256);
   // the staged scatter needs more than the default 48 KB of shared memory
   CCK(cudaFuncSetAttribute(k_radix_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem<K>()),
       "cudaFuncSetAttribute");
@@ -1004,15 +1272,17 @@ static int radix_sort(pa_coinc* c, K*& k, unsigned*& v, K* k2, unsigned* v2, lon
   for (int s = 0; s < bits; s += 8) {
     {
       Span sp_(c, CK_SORT_HIST);
-      k_radix_hist<K><<<nblk, kT, 0, c->stream>>>(ka, n, s, nblk, P<unsigned>(c->hist), P<unsigned>(c->cntl));
+      k_radix_hist<K><<<nblk, kT, 0, c->stream>>>(ka, n, s, nblk, P<unsigned>(c->hist));
     }
-    c->launches++;
-    int rc = scan_excl(c, P<unsigned>(c->hist), 256ll * nblk, P<unsigned>(c->scan_tmp));
-    if (rc) return rc;
+    {
+      Span sp_(c, CK_SCAN);
+      k_scan_rows<<<256, kT, 0, c->stream>>>(P<unsigned>(c->hist), nblk, P<unsigned>(c->digits));
+    }
+    c->launches += 2;
     {
       Span sp_(c, CK_SORT_SCATTER);
-      k_radix_scatter<K><<<nblk, kT, scatter_smem<K>(), c->stream>>>(ka, va, kb, vb, n, s, nblk,
-                                                                      P<unsigned>(c->hist), P<unsigned>(c->cntl));
+      k_radix_scatter<K><<<nblk, kSThreads, scatter_smem<K>(), c->stream>>>(
+          ka, va, kb, vb, n, s, nblk, P<unsigned>(c->hist), P<unsigned>(c->digits));
     }
     c->launches++;
     CCK(cudaGetLastError(), "radix pass");
@@ -1106,8 +1376,8 @@ void pa_coinc_destroy(pa_coinc* c) {
   if (!c) return;
   cudaSetDevice(c->cfg.device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  pa_coinc::Buf* bufs[] = {&c->rec, &c->cells_raw, &c->flag, &c->snr_raw, &c->blkcnt, &c->scan_tmp, &c->minmax, &c->rawidx,
-                           &c->cells_in, &c->snr_in, &c->cntl, &c->keyA, &c->keyB, &c->valA, &c->valB, &c->hist, &c->keep,
+  pa_coinc::Buf* bufs[] = {&c->rec, &c->cells_raw, &c->flag, &c->blkcnt, &c->scan_tmp, &c->minmax, &c->rawidx,
+                           &c->cells_in, &c->digits, &c->keyA, &c->keyB, &c->valA, &c->valB, &c->hist, &c->keep,
                            &c->keep_in, &c->uniq, &c->req, &c->found, &c->skey, &c->sval, &c->gflag, &c->gend,
                            &c->gw, &c->lastu, &c->wkeyA, &c->wkeyB, &c->cend, &c->cw, &c->cidxA, &c->cidxB,
                            &c->wsort, &c->means, &c->fra, &c->ops};
@@ -1181,7 +1451,6 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   pa::TraceRange trace_("coinc sort, duplicates, coincidences");
   const int nf = (int)c->frames.size();
   const long long n = c->n_in;
-  ENS(snr_in, sizeof(double) * n);
   ENS(keyA, sizeof(K) * n);
   ENS(keyB, sizeof(K) * n);
   ENS(valA, sizeof(unsigned) * n);
@@ -1190,8 +1459,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
     Span sp_(c, CK_INBAND);
     k_inband<K><<<nblk1, kT, 0, c->stream>>>(P<uint8_t>(c->flag), P<int4>(c->cells_raw), P<unsigned>(c->blkcnt), L,
                                              P<unsigned>(c->rawidx), P<int4>(c->cells_in),
-                                             P<K>(c->keyA), P<unsigned>(c->valA), P<double>(c->snr_raw),
-                                             P<double>(c->snr_in));
+                                             P<K>(c->keyA), P<unsigned>(c->valA));
   }
   c->launches++;
   CCK(cudaGetLastError(), "k_inband");
@@ -1204,84 +1472,50 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   // per-frame ranks of the sorted order: each frame's last record and the
   // record of an earlier frame at the position one past it
   const int nblkR = (int)((n + kRTile - 1) / kRTile);
-  ENS(hist, sizeof(unsigned) * (256ll * nblkR + 1));
-  ENS(scan_tmp, sizeof(unsigned) * scan_tmp_len(256ll * nblkR));
+  ENS(hist, sizeof(unsigned) * 256ll * nblkR);
+  ENS(digits, sizeof(unsigned) * 256);
+  ENS(req, sizeof(FrameReq) * nf);
+  ENS(found, sizeof(FrameFound) * nf);
+  ENS(uniq, sizeof(unsigned) * 257);  // removed records per frame, and the failure flag of the rank lookup
+  CCK(cudaMemsetAsync(c->uniq.p, 0, sizeof(unsigned) * 257, c->stream), "memset");
+  std::vector<FrameReq> req(nf);
+  for (int f = 0; f < nf; f++) {
+    req[f] = {(int)(nin_f[f] - 1), -1, -1, 0};
+    if (nin_f[f] < 1 || nin_f[f] >= 10485760) continue;
+    for (int g = f - 1; g >= 0; g--)
+      if (nin_f[g] > nin_f[f]) {
+        req[f].stale_frame = g;
+        req[f].stale = (int)nin_f[f];
+        break;
+      }
+  }
+  CCK(cudaMemcpyAsync(c->req.p, req.data(), sizeof(FrameReq) * nf, cudaMemcpyHostToDevice, c->stream), "copy");
   {
     Span sp_(c, CK_FRAME_RANK);
     k_frame_hist<<<nblkR, kT, 0, c->stream>>>(val, n, nblkR, P<unsigned>(c->hist));
   }
-  c->launches++;
-  rc = scan_excl(c, P<unsigned>(c->hist), 256ll * nblkR, P<unsigned>(c->scan_tmp));
-  if (rc) return rc;
-  std::vector<int2> req;
-  std::vector<int> req_last(nf, -1), req_stale(nf, -1);
-  for (int f = 0; f < nf; f++) {
-    if (nin_f[f] < 1) continue;
-    req_last[f] = (int)req.size();
-    req.push_back(make_int2(f, (int)(nin_f[f] - 1)));
-    // latest earlier frame whose sorted rows reach position nin_f[f] (the
-    // candidate table starts zeroed for its first 10485760 rows, struct.h:10)
-    for (int g = f - 1; g >= 0; g--)
-      if (nin_f[g] > nin_f[f]) {
-        req_stale[f] = (int)req.size();
-        req.push_back(make_int2(g, (int)nin_f[f]));
-        break;
-      }
+  {
+    Span sp_(c, CK_SCAN);
+    k_scan_rows<<<nf, kT, 0, c->stream>>>(P<unsigned>(c->hist), nblkR, P<unsigned>(c->digits));
   }
-  std::vector<long long> pos(req.size(), -1);
-  std::vector<int4> vcells(req.size());
-  std::vector<unsigned long long> vkeys(2 * req.size(), 0);
-  if (!req.empty()) {
-    ENS(req, sizeof(int2) * req.size());
-    // positions, then cells and keys on 16-byte boundaries
-    const size_t nr = req.size(), pos_bytes = (sizeof(long long) * nr + 15) & ~(size_t)15;
-    ENS(found, pos_bytes + (sizeof(int4) + 2 * sizeof(unsigned long long)) * nr);
-    long long* d_pos = P<long long>(c->found);
-    int4* d_cells = (int4*)((char*)c->found.p + pos_bytes);
-    unsigned long long* d_keys = (unsigned long long*)(d_cells + nr);
-    CCK(cudaMemcpyAsync(c->req.p, req.data(), sizeof(int2) * req.size(), cudaMemcpyHostToDevice, c->stream), "copy");
-    const int wpb = kT / 32;
-    {
-      Span sp_(c, CK_FRAME_RANK);
-      k_frame_find<K><<<(unsigned)((req.size() + wpb - 1) / wpb), kT, 0, c->stream>>>(
-          P<int2>(c->req), (int)req.size(), P<unsigned>(c->hist), nblkR, val, n, key,
-          P<int4>(c->cells_in), d_pos, d_cells, d_keys);
-    }
-    c->launches++;
-    CCK(cudaGetLastError(), "k_frame_find");
-    CCK(cudaMemcpyAsync(pos.data(), d_pos, sizeof(long long) * req.size(), cudaMemcpyDeviceToHost, c->stream), "copy");
-    CCK(cudaMemcpyAsync(vcells.data(), d_cells, sizeof(int4) * req.size(), cudaMemcpyDeviceToHost, c->stream), "copy");
-    CCK(cudaMemcpyAsync(vkeys.data(), d_keys, 2 * sizeof(unsigned long long) * req.size(), cudaMemcpyDeviceToHost,
-                        c->stream),
-        "copy");
-    CCK(cudaStreamSynchronize(c->stream), "sync");
+  {
+    Span sp_(c, CK_FRAME_RANK);
+    k_frame_find<K><<<2 * nf, kT, 0, c->stream>>>(P<FrameReq>(c->req), P<unsigned>(c->hist), nblkR, val, n, key,
+                                                  P<int4>(c->cells_in), P<FrameFound>(c->found),
+                                                  (int*)(P<unsigned>(c->uniq) + 256));
   }
-  for (size_t r = 0; r < req.size(); r++)
-    if (pos[r] < 0 || pos[r] >= n) return cfail(c, PA_ERR_CUDA, "pa_coinc_run: frame rank lookup failed");
-  for (int f = 0; f < nf; f++) {
-    c->ft.drop[f] = 0;
-    if (req_last[f] < 0) continue;
-    const int4 last = vcells[req_last[f]];
-    int4 stale = make_int4(0, 0, 0, 0);
-    if (req_stale[f] >= 0 && nin_f[f] < 10485760) stale = vcells[req_stale[f]];
-    if (last.x == stale.x && last.y == stale.y && last.z == stale.z && last.w == stale.w) {
-      c->ft.drop[f] = 1;
-      c->ft.drop_lo[f] = vkeys[2 * req_last[f]];
-      c->ft.drop_hi[f] = vkeys[2 * req_last[f] + 1];
-    }
-  }
-  CCK(cudaMemcpyToSymbolAsync(c_ft, &c->ft, sizeof(FrameTab), 0, cudaMemcpyHostToDevice, c->stream), "symbol");
+  c->launches += 3;
+  CCK(cudaGetLastError(), "k_frame_find");
 
   // duplicate removal
   ENS(keep, n);
-  ENS(uniq, sizeof(unsigned) * 256);
   CCK(cudaMemsetAsync(c->keep.p, 0, n, c->stream), "memset");
-  CCK(cudaMemsetAsync(c->uniq.p, 0, sizeof(unsigned) * 256, c->stream), "memset");
   c->val_sorted = val;
   {
     Span sp_(c, CK_DEDUP);
-    k_dedup<K><<<(unsigned)((n + kT - 1) / kT), kT, 0, c->stream>>>(key, val, P<double>(c->snr_in), n,
-                                                                    P<uint8_t>(c->keep), P<unsigned>(c->uniq));
+    k_dedup<K><<<(unsigned)((n + kTile - 1) / kTile), kT, 0, c->stream>>>(
+        key, val, P<unsigned>(c->rawidx), P<double>(c->rec), P<FrameReq>(c->req), P<FrameFound>(c->found), n,
+        P<uint8_t>(c->keep), P<unsigned>(c->uniq));
   }
   c->launches++;
   CCK(cudaGetLastError(), "k_dedup");
@@ -1298,11 +1532,12 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   rc = scan_excl(c, P<unsigned>(c->blkcnt), nt + 1, P<unsigned>(c->scan_tmp));
   if (rc) return rc;
   unsigned G = 0;
-  std::vector<unsigned> uniq(256, 0);
+  std::vector<unsigned> uniq(257, 0);
   CCK(cudaMemcpyAsync(&G, P<unsigned>(c->blkcnt) + nt, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream), "copy");
-  CCK(cudaMemcpyAsync(uniq.data(), c->uniq.p, sizeof(unsigned) * 256, cudaMemcpyDeviceToHost, c->stream), "copy");
+  CCK(cudaMemcpyAsync(uniq.data(), c->uniq.p, sizeof(unsigned) * 257, cudaMemcpyDeviceToHost, c->stream), "copy");
   CCK(cudaStreamSynchronize(c->stream), "sync");
-  for (int f = 0; f < nf; f++) c->frameinfo[3 * f + 2] = (int)uniq[f];
+  if (uniq[256]) return cfail(c, PA_ERR_CUDA, "pa_coinc_run: frame rank lookup failed");
+  for (int f = 0; f < nf; f++) c->frameinfo[3 * f + 2] = (int)(nin_f[f] - uniq[f]);
   c->sum.unique = G;
   if (G == 0) return PA_OK;
   ENS(skey, sizeof(K) * G);
@@ -1319,31 +1554,29 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   ENS(gflag, G);
   ENS(gend, sizeof(unsigned) * G);
   ENS(gw, sizeof(unsigned) * G);
-  ENS(lastu, sizeof(int));
-  CCK(cudaMemsetAsync(c->lastu.p, 0, sizeof(int), c->stream), "memset");
-  {
-    Span sp_(c, CK_GROUPS);
-    k_groups<K><<<(G + kT - 1) / kT, kT, 0, c->stream>>>(P<K>(c->skey), G, c->cfg.mincoin, P<uint8_t>(c->gflag),
-                                                        P<unsigned>(c->gend), P<unsigned>(c->gw), P<int>(c->lastu));
-  }
-  c->launches++;
-  CCK(cudaGetLastError(), "k_groups");
+  ENS(lastu, 2 * sizeof(int));  // and the number of members of the stored groups
+  CCK(cudaMemsetAsync(c->lastu.p, 0, 2 * sizeof(int), c->stream), "memset");
   const long long gt = ((long long)G + kTile - 1) / kTile;
   ENS(blkcnt, sizeof(unsigned) * (gt + 1));
   ENS(scan_tmp, sizeof(unsigned) * scan_tmp_len(gt + 1));
   {
     Span sp_(c, CK_GROUPS);
-    k_tile_count<<<(unsigned)gt, kT, 0, c->stream>>>(P<uint8_t>(c->gflag), G, P<unsigned>(c->blkcnt));
+    k_groups<K><<<(unsigned)gt, kT, 0, c->stream>>>(P<K>(c->skey), G, c->cfg.mincoin, P<uint8_t>(c->gflag),
+                                                   P<unsigned>(c->gend), P<unsigned>(c->gw), P<int>(c->lastu),
+                                                   P<unsigned>(c->lastu) + 1, P<unsigned>(c->blkcnt));
   }
   c->launches++;
+  CCK(cudaGetLastError(), "k_groups");
   CCK(cudaMemsetAsync(P<unsigned>(c->blkcnt) + gt, 0, sizeof(unsigned), c->stream), "memset");
   rc = scan_excl(c, P<unsigned>(c->blkcnt), gt + 1, P<unsigned>(c->scan_tmp));
   if (rc) return rc;
   unsigned Kc = 0;
-  int lastu = 0;
+  int lu[2] = {0, 0};
   CCK(cudaMemcpyAsync(&Kc, P<unsigned>(c->blkcnt) + gt, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream), "copy");
-  CCK(cudaMemcpyAsync(&lastu, c->lastu.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "copy");
+  CCK(cudaMemcpyAsync(lu, c->lastu.p, sizeof(lu), cudaMemcpyDeviceToHost, c->stream), "copy");
   CCK(cudaStreamSynchronize(c->stream), "sync");
+  const int lastu = lu[0];
+  const unsigned M = (unsigned)lu[1];
   const int ncoin = (int)Kc + (lastu ? 1 : 0);
   if ((size_t)ncoin + 1 > c->h_recs_cap) {
     if (c->h_recs) cudaFreeHost(c->h_recs);
@@ -1385,15 +1618,12 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
     CCK(cudaMemsetAsync(P<unsigned>(c->wsort) + Kc, 0, sizeof(unsigned), c->stream), "memset");
     rc = scan_excl(c, P<unsigned>(c->wsort), (long long)Kc + 1, P<unsigned>(c->scan_tmp));
     if (rc) return rc;
-    unsigned M = 0;
-    CCK(cudaMemcpyAsync(&M, P<unsigned>(c->wsort) + Kc, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream), "copy");
-    CCK(cudaStreamSynchronize(c->stream), "sync");
     ENS(means, sizeof(pa_coinc_rec) * Kc);
     ENS(fra, sizeof(int) * (M + 1));
     ENS(ops, sizeof(int) * (M + 1));
     {
       Span sp_(c, CK_MEANS);
-      k_means<<<(Kc + 127) / 128, 128, 0, c->stream>>>(order, P<unsigned>(c->cend), P<unsigned>(c->cw),
+      k_means<<<(Kc + kT / 32 - 1) / (kT / 32), kT, 0, c->stream>>>(order, P<unsigned>(c->cend), P<unsigned>(c->cw),
                                                         P<unsigned>(c->wsort), (int)Kc, P<unsigned>(c->sval),
                                                         P<unsigned>(c->rawidx), P<double>(c->rec),
                                                         (double)c->cfg.N, c->cfg.refr, P<pa_coinc_rec>(c->means),
@@ -1481,9 +1711,20 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
   if (nblk1 > 0) {
     CCK(cudaMemcpyToSymbolAsync(c_ft, &c->ft, sizeof(FrameTab), 0, cudaMemcpyHostToDevice, c->stream), "symbol");
     CellArgs a;
-    a.lo = M_PI_2 - c->cfg.narrowdown;
-    a.hi = M_PI_2 + c->cfg.narrowdown;
+    // as order keys: x > lo with lo = +0 for a zero, x < hi with hi = -0; a
+    // NaN is met by nothing
+    auto key_of = [](double d, double zero, long long nan) {
+      if (d != d) return nan;
+      if (d == 0) d = zero;
+      long long b;
+      memcpy(&b, &d, sizeof(b));
+      return order_key(b);
+    };
+    a.lo_k = key_of(M_PI_2 - c->cfg.narrowdown, 0.0, LLONG_MAX);
+    a.hi_k = key_of(M_PI_2 + c->cfg.narrowdown, -0.0, LLONG_MIN);
+    a.cut_k = key_of(c->cfg.snrcutoff, 0.0, LLONG_MAX);
     a.N = (double)c->cfg.N;
+    a.N2 = 2.0 * a.N;
     a.sqrN = pow(c->cfg.N, 2);
     a.omsN = c->cfg.oms * c->cfg.N;
     volatile double epsm = PA_C_EPSMA;
@@ -1494,8 +1735,6 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
       a.half_shift[j] = 0.5 * c->cfg.shift[j];
     }
     a.refr = c->cfg.refr;
-    a.snrcut = c->cfg.snrcutoff;
-    a.omsN_f = (float)a.omsN;
     a.se_f = (float)a.se;
     a.ce_f = (float)a.ce;
     auto split = [](double d, float* h, float* l) {
@@ -1503,22 +1742,18 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
       *l = (float)(d - (double)*h);
     };
     a.fast = c->cfg.N < (1 << 24);
-    a.Nf = (float)c->cfg.N;  // exact when fast
-    split(a.sqrN, &a.sqrN_h, &a.sqrN_l);
     for (int j = 0; j < 4; j++) {
-      split(a.v[0][j], &a.v0_h[j], &a.v0_l[j]);
-      split(a.v[1][j], &a.v1_h[j], &a.v1_l[j]);
+      split(a.N * a.v[0][j], &a.f_h[j], &a.f_l[j]);
+      split(a.sqrN * a.v[1][j], &a.d_h[j], &a.d_l[j]);
       a.hs_f[j] = (float)a.half_shift[j];  // exact: halves of digits
-      a.v2_f[j] = (float)a.v[2][j];
-      a.v3_f[j] = (float)a.v[3][j];
-      // 8e-6 on be0 and be1 (their FP32 error is below 1.1e-6), plus the
-      // FP32 products and the FP64 rounding differences
-      const double m = fabs(a.omsN) * (fabs(a.v[2][j]) + fabs(a.v[3][j])) * 8e-6 + 2e-6;
+      a.s2_f[j] = (float)(a.omsN * a.v[2][j]);
+      a.s3_f[j] = (float)(a.omsN * a.v[3][j]);
+      // 2e-6 on be0 and be1, and 2e-6 for the fractions' FP32 sum
+      const double m = fabs(a.omsN) * (fabs(a.v[2][j]) + fabs(a.v[3][j])) * 2e-6 + 2e-6;
       a.margin[j] = m < 1.0 ? (float)m : 1.0f;
     }
     ENS(cells_raw, sizeof(int4) * c->nraw);
     ENS(flag, c->nraw);
-    ENS(snr_raw, sizeof(double) * c->nraw);
     ENS(blkcnt, sizeof(unsigned) * (nblk1 + 1));
     ENS(scan_tmp, sizeof(unsigned) * scan_tmp_len(nblk1 + 1));
     ENS(minmax, sizeof(int) * 9);
@@ -1528,7 +1763,7 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
       Span sp_(c, CK_CELLS);
       k_cells<<<nblk1, kT, 0, c->stream>>>(P<double>(c->rec), a, P<int4>(c->cells_raw), P<uint8_t>(c->flag),
                                           P<unsigned>(c->blkcnt), P<int>(c->minmax),
-                                          (unsigned*)(P<int>(c->minmax) + 8), P<double>(c->snr_raw));
+                                          (unsigned*)(P<int>(c->minmax) + 8));
     }
     c->launches++;
     CCK(cudaGetLastError(), "k_cells");
