@@ -191,8 +191,11 @@ __device__ __forceinline__ double warp_sum(double v) {
 //                   + da/dtheta (x ka Re(conj(Xa)E) + 2 qa a) + (b terms) ]
 //   (x 1/sig2), with E = e^{-i phi}, ka = 2 seed/A, qa = -seed |Xa|^2/A^2.
 // ---------------------------------------------------------------------
+// Two CTAs per SM: the FP64 pipe bounds the kernel with 16 warps as with 24, and
+// what 24 leave of the registers (80) spills (100 points of two detectors, N =
+// 86164: 2.39 ms, 2.50 with three).
 template <bool ADJ>
-__global__ void __launch_bounds__(kThreads) k_fu_sums(const double* __restrict__ xd, const double* __restrict__ pos,
+__global__ void __launch_bounds__(kThreads, 2) k_fu_sums(const double* __restrict__ xd, const double* __restrict__ pos,
                                                       const double* __restrict__ cmf, const double* __restrict__ smf,
                                                       const FuCand* __restrict__ cand, const double* __restrict__ coef,
                                                       FuDets dets, int n, int N, int nifo, int nch, double oms,
