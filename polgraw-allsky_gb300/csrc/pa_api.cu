@@ -318,13 +318,15 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
   ALLOC(b.cosmodf, rs * N);
   ALLOC(b.sinmodf, rs * N);
   ALLOC(b.dc, sizeof(pa::DetConst) * pa::kMaxDet);
-  ALLOC(b.spline_invp, sizeof(double) * 64);
-  ALLOC(b.spline_p, sizeof(double) * 64);
+  if (c->fp64) {
+    ALLOC(b.spline_invp, sizeof(double) * 64);
+    ALLOC(b.spline_p, sizeof(double) * 64);
+    ALLOC(b.u, sizeof(double) * 2 * nifo * 2 * (size_t)(2 * N));
+    ALLOC(b.y2, cs * nifo * 2 * (size_t)(2 * N));
+  }
   ALLOC(b.xin, cs * nifo * 2 * (size_t)N);
   ALLOC(b.spec, cs * nifo * 2 * (size_t)s.nfft);
-  ALLOC(b.yint, cs * nifo * 2 * (size_t)s.Ninterp);
-  ALLOC(b.u, sizeof(double) * 2 * nifo * 2 * (size_t)(2 * N));
-  ALLOC(b.y2, cs * nifo * 2 * (size_t)(2 * N));
+  ALLOC(b.yint, cs * nifo * 2 * (size_t)(c->fp64 ? s.Ninterp : s.nfft));
   ALLOC(b.shftf, sizeof(double) * nifo * (size_t)N);
   for (int k = 0; k < 2; k++) {
     if (c->fp64) ALLOC(b.ph0[k], 8 * nifo * (size_t)N);  // tmp1 (FP32 forms keep it in xm)
@@ -334,13 +336,12 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
     ALLOC(b.sums[k], sizeof(double) * 8);
     ALLOC(b.sums_r[k], sizeof(double) * 4);
   }
-  ALLOC(b.part, sizeof(double) * 2 * nifo * (size_t)((N + 255) / 256));
+  ALLOC(b.part, sizeof(double) * 2 * nifo * (size_t)((N + 127) / 128));
   ALLOC(b.ybuf_pre, cs * nifo * 2 * (size_t)s.Ninterp);
   ALLOC(b.counter, sizeof(unsigned int) * 4);
   CK(cudaMemset(b.counter, 0, sizeof(unsigned int) * 4), "cudaMemset");
   ALLOC(b.ybuf, (size_t)sbm * 2 * s.nfftf * cs);
   ALLOC(b.F, rs * (size_t)sbm * b.bins);
-  ALLOC(b.mu, rs * (size_t)sbm * (b.nblk > 0 ? b.nblk : 1));
   b.cand_cap = 1 << 18;
   ALLOC(b.cand, sizeof(pa::DevCand) * (size_t)b.cand_cap);
   ALLOC(b.ncand, sizeof(int) * 4);
@@ -356,15 +357,13 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
   }
   if ((rc = upload_real(c, (void*)b.cosmodf, cm))) return rc;
   if ((rc = upload_real(c, (void*)b.sinmodf, sm))) return rc;
-  double invp[64], p[64];
-  p[0] = 0.;
-  invp[0] = 0.;
-  for (int i = 1; i < 64; i++) {  // auxi.c:71-72
-    invp[i] = 2. / (p[i - 1] + 4.);
-    p[i] = -.5 * invp[i];
+  b.spl = pa::spline_taps();
+  if (c->fp64) {
+    double invp[64], p[64];
+    pa::spline_pivots(invp, p);
+    CK(cudaMemcpy((void*)b.spline_invp, invp, sizeof(invp), cudaMemcpyHostToDevice), "upload spline");
+    CK(cudaMemcpy((void*)b.spline_p, p, sizeof(p), cudaMemcpyHostToDevice), "upload spline");
   }
-  CK(cudaMemcpy((void*)b.spline_invp, invp, sizeof(invp), cudaMemcpyHostToDevice), "upload spline");
-  CK(cudaMemcpy((void*)b.spline_p, p, sizeof(p), cudaMemcpyHostToDevice), "upload spline");
   if ((rc = make_twiddles(c, s.Ninterp, +1, &c->tw_inv))) return rc;
   if (c->fp64) {
     if ((rc = make_twiddles(c, s.nfft, -1, &c->tw_fwd))) return rc;
@@ -647,6 +646,8 @@ void sky_setup(const pa_ctx* c, int pm, int mm, int nn, const pa_opts* o, int ss
   a.nS[2] = sindelt;
   for (int n = 0; n < c->nifo; n++) {
     a.shft1[n] = a.nS[0] * c->det0[n][0] + a.nS[1] * c->det0[n][1] + a.nS[2] * c->det0[n][2];
+    a.shft1_fma[n] =
+        fma(a.nS[0], c->det0[n][0], fma(a.nS[1], c->det0[n][1], a.nS[2] * c->det0[n][2]));
     a.cosalfr[n] = cosalt * c->dc[n].cphir + sinalt * c->dc[n].sphir;
     a.sinalfr[n] = sinalt * c->dc[n].cphir - cosalt * c->dc[n].sphir;
   }
@@ -1342,24 +1343,19 @@ size_t noalloc_layout(char* base, const pa_settings& s, int nifo, pa::Buffers* b
   b->cosmodf = m.take(4 * N);
   b->sinmodf = m.take(4 * N);
   b->dc = (const pa::DetConst*)m.take(sizeof(pa::DetConst) * pa::kMaxDet);
-  b->spline_invp = (const double*)m.take(8 * 64);
-  b->spline_p = (const double*)m.take(8 * 64);
   b->xin = m.take(cs * nifo * 2 * N);
   b->spec = m.take(cs * nifo * 2 * (size_t)s.nfft);
-  b->yint = m.take(cs * nifo * 2 * (size_t)s.Ninterp);
-  b->u = (double*)m.take(16 * nifo * 2 * 2 * N);
-  b->y2 = m.take(cs * nifo * 2 * 2 * N);
+  b->yint = m.take(cs * nifo * 2 * (size_t)s.nfft);
   b->shftf = (double*)m.take(8 * nifo * N);
   b->NP = pa::pair_pad(s.N, s.nfftf);
   b->xm[0] = b->xm[1] = m.take(32 * nifo * (size_t)b->NP);
   b->sums[0] = b->sums[1] = (double*)m.take(8 * 8);
   b->sums_r[0] = b->sums_r[1] = m.take(8 * 4);
-  b->part = (double*)m.take(8 * 2 * nifo * ((N + 255) / 256));
+  b->part = (double*)m.take(8 * 2 * nifo * ((N + 127) / 128));
   b->counter = (unsigned int*)m.take(16);
   b->ybuf_pre = m.take(cs * nifo * 2 * (size_t)s.Ninterp);
   b->ybuf = m.take(cs * 2 * (size_t)s.nfftf);
   b->F = m.take(4 * (size_t)bins);
-  b->mu = m.take(16);
   *Fn = m.take(4 * (size_t)bins);  // normalised F (the output)
   b->cand = (pa::DevCand*)m.take(sizeof(pa::DevCand) * kNoAllocCandCap);
   b->ncand = (int*)m.take(16);
@@ -1486,14 +1482,7 @@ extern "C" int pa_fstat_noalloc(const pa_settings* sett, const pa_detector* det,
                         st), "upload");
     NCK(cudaStreamSynchronize(st), "upload");  // the staging array is reused
   }
-  double invp[64], p[64];
-  p[0] = invp[0] = 0.;
-  for (int i = 1; i < 64; i++) {  // auxi.c:71-72
-    invp[i] = 2. / (p[i - 1] + 4.);
-    p[i] = -.5 * invp[i];
-  }
-  NCK(cudaMemcpyAsync((void*)b.spline_invp, invp, sizeof(invp), cudaMemcpyHostToDevice, st), "upload");
-  NCK(cudaMemcpyAsync((void*)b.spline_p, p, sizeof(p), cudaMemcpyHostToDevice, st), "upload");
+  b.spl = pa::spline_taps();
   NCK(noalloc_twiddles(b.pair_tw1, 256, 256, -1, st, [](long j) { return j; }), "twiddles");
   NCK(noalloc_twiddles(b.tw_inv[2], 1024, sett->Ninterp, +1, st, [](long j) { return j; }), "twiddles");
   NCK(noalloc_twiddles(b.tw_inv[3], sett->Ninterp / 1024, sett->Ninterp, +1, st, [](long j) { return 1024 * j; }),

@@ -8,9 +8,11 @@
 //   resample FFTs   jobcore.c:319-362 (pass A/B with PlainLoader; the
 //                   interpolating inverse at half length: HalfShiftLoader,
 //                   InterpStore)
-//   k_spline_fwd/bwd spline() (auxi.c:56-81), FP64 chunked recurrences
-//   k_splint        splint/splintpad (auxi.c:83-122) + 1/sig2 (jobcore.c:386-389)
-//   (aa, bb: last-CTA reduction of k_prelude_mod, jobcore.c:375-393)
+//   k_resample      FP32 forms: spline() (auxi.c:56-81), splint/splintpad
+//                   (auxi.c:83-122), 1/sig2 (jobcore.c:386-389), aa and bb
+//                   (jobcore.c:375-393)
+//   k_spline_fwd/bwd, k_splint   the same for the FP64 form (aa, bb: last CTA
+//                   of k_prelude_mod)
 //   SpinLoader      spindown phase modulation (jobcore.c:455-623)
 //   FstatStore      F = |Xa|^2/aa + |Xb|^2/bb (jobcore.c:635-638)
 //   k_normthresh    FStat() block means and normalisation (auxi.c:214-240),
@@ -87,8 +89,38 @@ __device__ __forceinline__ void block_sum2(double& a, double& b, double (*red)[8
   b = sb;
 }
 
+// aa = sum_n (sum_i a^2)/sig2_n in detector order (jobcore.c:375-393) and bb,
+// from the partial sums of k_prelude_mod in a fixed order, by one block.
+template <typename R>
+__device__ void sum_parts(const double* part, int nblk, int nifo, const DetConst* dc, double* sums, R* sums_r,
+                          double (*red)[8]) {
+  double acc = 0.;  // thread 0: aa, thread 1: bb (of the first warp)
+  for (int dd = 0; dd < nifo; ++dd) {
+    double sa = 0., sb = 0.;
+    for (int k = threadIdx.x; k < nblk; k += blockDim.x) {
+      sa += __ldcg(&part[((size_t)dd * nblk + k) * 2 + 0]);
+      sb += __ldcg(&part[((size_t)dd * nblk + k) * 2 + 1]);
+    }
+    __syncthreads();
+    block_sum2(sa, sb, red);
+    if (threadIdx.x < 32) acc += (threadIdx.x & 1 ? sb : sa) / dc[dd].sig2;
+  }
+  if (threadIdx.x < 2) {
+    const double inv = 1.0 / acc;
+    sums[threadIdx.x] = acc;
+    sums[2 + threadIdx.x] = inv;
+    sums_r[threadIdx.x] = (R)inv;
+  }
+}
+
+// One sample a thread.  The FP32 forms take blocks of 128, so that the FP64
+// operations (about 25 a sample, at 2 lanes per clock and SM) spread over the
+// SMs also for the shortest segments; their aa and bb are summed in k_resample,
+// off this kernel's path.
+template <typename R> constexpr int mod_threads() { return sizeof(R) == 4 ? 128 : 256; }
+
 template <typename R, int PM>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(mod_threads<R>())
     k_prelude_mod(const double* __restrict__ xDat, const double* __restrict__ DetSSB,
                   const R* __restrict__ cosmodf, const R* __restrict__ sinmodf,
                   const DetConst* __restrict__ dc, const SkyArgs sky, int N, int NP,
@@ -100,16 +132,6 @@ __global__ void __launch_bounds__(256)
   const int d = blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   R a2r = 0, b2r = 0;
-  // FP32 forms: shft at sample 0 of this detector, by the expression every
-  // sample uses
-  __shared__ double sh1[1];
-  if (sizeof(R) == 4) {
-    if (threadIdx.x == 0) {
-      const double* D0 = DetSSB + 3 * (size_t)d * N;
-      sh1[0] = fma(sky.nS[0], D0[0], fma(sky.nS[1], D0[1], __dmul_rn(sky.nS[2], D0[2])));
-    }
-    __syncthreads();
-  }
   if (i < N) {
     const DetConst& k = dc[d];
     // modvir, settings.c:303-322
@@ -158,10 +180,10 @@ __global__ void __launch_bounds__(256)
       sp = (R)sd;
       cp = (R)cd;
     } else {
-      // FP32 forms: shft with fused multiply-adds; shft1 is the same
-      // expression at sample 0 (sh1, below), so shftf[0] is exactly 0
+      // FP32 forms: shft with fused multiply-adds; shft1_fma is the same
+      // expression at sample 0, so shftf[0] is exactly 0
       const double shft = fma(sky.nS[0], D[0], fma(sky.nS[1], D[1], __dmul_rn(sky.nS[2], D[2])));
-      shftf[o] = shft - sh1[0];
+      shftf[o] = shft - sky.shft1_fma[d];
       // 2 i shft, the non-integer part of _tmp1 = i^2 + 2 i shft
       const double p2 = __dmul_rn(di + di, shft);
       const uint64_t ii2 = (uint64_t)i * (uint64_t)i;
@@ -192,8 +214,12 @@ __global__ void __launch_bounds__(256)
     const R x = (R)xDat[(size_t)d * N + i];
     const R xa = x * aa, xb = x * bb;
     // x a exp(-i phase)
-    xin[((size_t)d * 2 + 0) * N + i] = mk(xa * cp, -xa * sp);
-    xin[((size_t)d * 2 + 1) * N + i] = mk(xb * cp, -xb * sp);
+    if constexpr (sizeof(R) == 4) {
+      reinterpret_cast<float4*>(xin)[o] = make_float4(xa * cp, xb * cp, -xa * sp, -xb * sp);
+    } else {
+      xin[((size_t)d * 2 + 0) * N + i] = mk(xa * cp, -xa * sp);
+      xin[((size_t)d * 2 + 1) * N + i] = mk(xb * cp, -xb * sp);
+    }
   }
   // deterministic block reduction of a^2, b^2: xor tree of each warp in the
   // working precision, warps summed in FP64 in index order
@@ -215,45 +241,27 @@ __global__ void __launch_bounds__(256)
       a2 += red[0][k];
       b2 += red[1][k];
     }
-  __syncthreads();
   if (threadIdx.x == 0) {
     part[((size_t)d * gridDim.x + blockIdx.x) * 2 + 0] = a2;
     part[((size_t)d * gridDim.x + blockIdx.x) * 2 + 1] = b2;
+  }
+  if (sizeof(R) == 4) return;
+  if (threadIdx.x == 0) {
     __threadfence();
     const unsigned int done = atomicAdd(counter, 1u);
     last = done == gridDim.x * gridDim.y - 1;
   }
   __syncthreads();
   if (!last) return;
-  // the last CTA to finish: aa = sum_n (sum_i a^2)/sig2_n in detector order
-  // (jobcore.c:375-393), partials summed in a fixed order
-  double aa = 0., bb = 0.;
-  for (int dd = 0; dd < (int)gridDim.y; ++dd) {
-    double sa = 0., sb = 0.;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-      sa += __ldcg(&part[((size_t)dd * gridDim.x + k) * 2 + 0]);
-      sb += __ldcg(&part[((size_t)dd * gridDim.x + k) * 2 + 1]);
-    }
-    __syncthreads();
-    block_sum2(sa, sb, red);
-    aa += sa / dc[dd].sig2;
-    bb += sb / dc[dd].sig2;
-  }
-  if (threadIdx.x == 0) {
-    sums[0] = aa;
-    sums[1] = bb;
-    sums[2] = 1.0 / aa;
-    sums[3] = 1.0 / bb;
-    sums_r[0] = (R)(1.0 / aa);
-    sums_r[1] = (R)(1.0 / bb);
-    *counter = 0u;
-  }
+  // the last CTA to finish
+  sum_parts(part, gridDim.x, gridDim.y, dc, sums, sums_r, red);
+  if (threadIdx.x == 0) *counter = 0u;
 }
 
 // ------------------------------------------------------------------
 // FFT loaders / storers
 
-// The zero-padded input of a transform.
+// The zero-padded input of a transform, FP64 form.
 template <typename R> struct PlainLoader {
   typedef typename CT<R>::T T;
   static constexpr int kTraceKind = KK_FFT_FWD_A;
@@ -267,32 +275,41 @@ template <typename R> struct PlainLoader {
       a = b = mk((R)0, (R)0);
     }
   }
-  // the FP32 passes' interface (pa_pair.cuh)
+};
+
+// FP32 forms: arrays of pairs, {a.re, b.re, a.im, b.im} per element, so that
+// every pass reads and writes 16 bytes of one array.
+struct PairLoader {
+  static constexpr int kTraceKind = KK_FFT_FWD_A;
+  const float4* in;  // [batch][len]
+  int len;
+  // the passes' interface (pa_pair.cuh)
   template <int NIN, int NCHK> struct Ahead {
-    static constexpr int v = 4;
+    static constexpr int v = 8;
   };
   struct Ctx {
-    const float2 *a, *b;
+    const float4* p;
     int left;
   };
-  struct Raw {
-    float2 a, b;
-  };
+  typedef P2 Raw;
   __device__ __forceinline__ int count() const { return len; }
-  __device__ __forceinline__ Ctx begin(int batch, int n0, int) const {
-    const float2* p = in + (size_t)batch * 2 * ld + n0;
-    return Ctx{p, p + ld, len - n0};
-  }
+  __device__ __forceinline__ Ctx begin(int batch, int n0, int) const { return Ctx{in + (size_t)batch * len + n0, len - n0}; }
   __device__ __forceinline__ void next(Ctx&) const {}
-  __device__ __forceinline__ Raw fetch(const Ctx& k, int off) const {
-    Raw r = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-    if (off < k.left) {
-      r.a = k.a[off];
-      r.b = k.b[off];
-    }
-    return r;
+  __device__ __forceinline__ Raw fetch(const Ctx& k, int off) const { return off < k.left ? pld(k.p + off) : pzero(); }
+  __device__ __forceinline__ P2 value(const Ctx&, const Raw& r, int) const { return r; }
+};
+// The results of a transform as pairs, scaled.
+template <int KIND> struct PairStore {
+  static constexpr int kTraceKind = KIND;
+  float4* out;  // [batch][ldo]
+  int ldo;
+  float scale;
+  struct Ctx {};
+  __device__ __forceinline__ Ctx begin() const { return Ctx{}; }
+  __device__ __forceinline__ void put(const Ctx&, int batch, int k1, int k2, P2 v) const {
+    const f2 s = dup(scale);
+    pst(out + (size_t)batch * ldo + k1 + (k2 << 8), P2{mul2(v.re, s), mul2(v.im, s)});
   }
-  __device__ __forceinline__ P2 value(const Ctx&, const Raw& r, int) const { return P2{pk(r.a.x, r.b.x), pk(r.a.y, r.b.y)}; }
 };
 
 // The interpolating inverse transform of jobcore.c:338-362 at half length.
@@ -304,7 +321,8 @@ template <typename R> struct PlainLoader {
 // with s_j = +1 below nyqst and -1 from it (the moved bins pick up
 // e^{i pi (2m+1)} = -1), i.e. an inverse FFT of length nfft of the
 // phase-shifted spectrum: half the transform length, and no transform of the
-// zero gap.  This loader feeds that transform; InterpStore interleaves.
+// zero gap.  This loader feeds that transform; InterpStore interleaves (FP32
+// forms: HalfShiftPair feeds it, and the spline reads x and the transform).
 template <typename R> struct HalfShiftLoader {
   typedef typename CT<R>::T T;
   static constexpr int kTraceKind = KK_FFT_INV_A;
@@ -321,26 +339,34 @@ template <typename R> struct HalfShiftLoader {
     a = cmul(spec[((size_t)batch * 2 + 0) * nfft + j], w);
     b = cmul(spec[((size_t)batch * 2 + 1) * nfft + j], w);
   }
-  // the FP32 passes' interface (pa_pair.cuh)
+};
+struct HalfShiftPair {
+  static constexpr int kTraceKind = KK_FFT_INV_A;
+  const float4* spec;   // [batch][nfft]
+  const float2* twlo;   // as HalfShiftLoader
+  const float2* twhi;
+  int nfft, nyqst;
   template <int NIN, int NCHK> struct Ahead {
     static constexpr int v = 4;
   };
   struct Ctx {
-    const float2 *a, *b;
+    const float4* p;
     int n0;
   };
   struct Raw {
-    float2 a, b, w;
+    P2 v;
+    float2 wl, wh;
   };
   __device__ __forceinline__ int count() const { return nfft; }
-  __device__ __forceinline__ Ctx begin(int batch, int n0, int) const {
-    const float2* p = spec + (size_t)batch * 2 * nfft + n0;
-    return Ctx{p, p + nfft, n0};
-  }
+  __device__ __forceinline__ Ctx begin(int batch, int n0, int) const { return Ctx{spec + (size_t)batch * nfft + n0, n0}; }
   __device__ __forceinline__ void next(Ctx&) const {}
-  __device__ __forceinline__ Raw fetch(const Ctx& k, int off) const { return Raw{k.a[off], k.b[off], phase(k.n0 + off)}; }
-  __device__ __forceinline__ P2 value(const Ctx&, const Raw& r, int) const {
-    return pmul(P2{pk(r.a.x, r.b.x), pk(r.a.y, r.b.y)}, r.w);
+  __device__ __forceinline__ Raw fetch(const Ctx& k, int off) const {
+    const int j = k.n0 + off;
+    return Raw{pld(k.p + off), __ldg(&twlo[j & 1023]), __ldg(&twhi[j >> 10])};
+  }
+  __device__ __forceinline__ P2 value(const Ctx& k, const Raw& r, int off) const {
+    const float2 w = cmul(r.wl, r.wh);
+    return k.n0 + off < nyqst ? pmul(r.v, w) : pmul(r.v, -w.x, -w.y);
   }
 };
 
@@ -598,12 +624,6 @@ template <typename R> struct CStore {
     out[((size_t)batch * 2 + 0) * ldo + k] = mk(a.x * scale, a.y * scale);
     out[((size_t)batch * 2 + 1) * ldo + k] = mk(b.x * scale, b.y * scale);
   }
-  __device__ __forceinline__ void put(const Ctx& c, int batch, int k1, int k2, P2 v) const {
-    T a, b;
-    upk(v.re, a.x, b.x);
-    upk(v.im, a.y, b.y);
-    put(c, batch, k1, k2, a, b, 8);
-  }
 };
 
 // F-statistic epilogue: F[k] = |Xa[k]|^2 / aa + |Xb[k]|^2 / bb, k in [nmin, nmax)
@@ -652,303 +672,314 @@ template <typename R> struct InterpStore {
     Pair<T>::st(yint + qa * Ninterp + 2 * (size_t)m, xa, mk(a.x * scale, a.y * scale));
     Pair<T>::st(yint + qb * Ninterp + 2 * (size_t)m, xb, mk(b.x * scale, b.y * scale));
   }
-  __device__ __forceinline__ void put(const Ctx&, int batch, int k1, int k2, P2 v) const {
-    const int m = k1 + (k2 << 8);
-    const size_t qa = (size_t)batch * 2, qb = qa + 1;
-    float2 xa = make_float2(0.f, 0.f), xb = xa, a, b;
-    if (m < N) {
-      xa = xin[qa * N + m];
-      xb = xin[qb * N + m];
-    }
-    upk(mul2(v.re, dup(scale)), a.x, b.x);
-    upk(mul2(v.im, dup(scale)), a.y, b.y);
-    reinterpret_cast<float4*>(yint + qa * Ninterp)[m] = make_float4(xa.x, xa.y, a.x, a.y);
-    reinterpret_cast<float4*>(yint + qb * Ninterp)[m] = make_float4(xb.x, xb.y, b.x, b.y);
-  }
 };
 
 // ------------------------------------------------------------------
-// Compensated two-float (float-float) arithmetic for the spline recurrences
-// of the FP32 forms: a value is hi + lo with |lo| <= ulp(hi)/2 (about 48
-// significant bits).  Products use fmaf for their exact error terms; the
-// explicit __fmul_rn keeps the compiler from fusing a rounded product into
-// the following sum.
+// Compensated two-float (float-float) arithmetic for the spindown phase and
+// the spline recurrences of the FP32 forms: a value is hi + lo with |lo| <=
+// ulp(hi)/2 (about 48 significant bits).  Products use fmaf for their exact
+// error terms (Dekker), sums the two-sum of Knuth.
 struct FF {
   float hi, lo;
 };
+// two of them at once, packed
+struct FF2 {
+  f2 hi, lo;
+};
 
-__device__ __forceinline__ FF ff_split(double x) {
-  const float h = (float)x;
-  return FF{h, (float)(x - (double)h)};
-}
-
-// a*x + t, a a float-float constant, t a float (Dekker/Knuth error-free
-// transformations: the product error by fma, the sum error by TwoSum)
-__device__ __forceinline__ FF ff_axpt(FF a, FF x, float t) {
-  const float p = __fmul_rn(a.hi, x.hi);
-  float e = __fmaf_rn(a.hi, x.hi, -p);
-  e = __fmaf_rn(a.hi, x.lo, e);
-  e = __fmaf_rn(a.lo, x.hi, e);
-  const float s = __fadd_rn(p, t);
-  const float bb = __fsub_rn(s, p);
-  const float r = __fadd_rn(__fsub_rn(p, __fsub_rn(s, bb)), __fsub_rn(t, bb));
-  const float c = __fadd_rn(r, e);
-  const float hi = __fadd_rn(s, c);
-  return FF{hi, __fsub_rn(c, __fsub_rn(hi, s))};
-}
-
-// a*x + y, a a float-float constant, x and y float-float
-__device__ __forceinline__ FF ff_axpy(FF a, FF x, FF y) {
-  const float p = __fmul_rn(a.hi, x.hi);
-  float e = __fmaf_rn(a.hi, x.hi, -p);
-  e = __fmaf_rn(a.hi, x.lo, e);
-  e = __fmaf_rn(a.lo, x.hi, e);
-  const float s = __fadd_rn(p, y.hi);
-  const float bb = __fsub_rn(s, p);
-  float r = __fadd_rn(__fsub_rn(p, __fsub_rn(s, bb)), __fsub_rn(y.hi, bb));
-  r = __fadd_rn(r, __fadd_rn(e, y.lo));
-  const float hi = __fadd_rn(s, r);
-  return FF{hi, __fsub_rn(r, __fsub_rn(hi, s))};
+// acc + c t, c a float-float constant (nch = -c.hi), t a float
+__device__ __forceinline__ FF2 ff2_add_prod(FF2 acc, f2 ch, f2 nch, f2 cl, f2 t) {
+  const f2 p = mul2(ch, t);
+  const f2 ne = fma2(nch, t, p);  // minus the product's error
+  const f2 s = add2(acc.hi, p);
+  const f2 bb = sub2(s, acc.hi);
+  const f2 e = add2(sub2(acc.hi, sub2(s, bb)), sub2(p, bb));
+  return FF2{s, add2(acc.lo, fma2(cl, t, sub2(e, ne)))};
 }
 
 // ------------------------------------------------------------------
-// spline (auxi.c:56-81): chunked recurrences, FP64 in the FP64 form and
-// compensated two-float in the FP32 forms (the FP64 pipe of a GB300 runs at
-// 1/64 of the FP32 rate, and these sweeps are its largest user in the
-// prelude).  The forward sweep
-// u_i = (-u_{i-1}/2 + 3 d_i) invp_i has |dU_i/dU_{i-1}| -> 2 - sqrt(3) = 0.268
-// and the back substitution y2_k = p_k y2_{k+1} + u_k likewise, so a chunk
-// can start kWarm steps early from zero: the start error shrinks by
-// 0.268^kWarm < 1e-18.  Chunks whose warm start reaches the array ends start
-// from the exact boundary values u_0 = 0, y2_{n-1} = 0.
-// Chunking per form: the warm start must bring the start error below the
-// precision the result is stored in (y2 is stored in the working precision):
-// 0.268^16 = 7e-10 is far below FP32 rounding, 0.268^32 = 5e-19 below FP64's.
-// Shorter chunks in the FP32 forms also give twice the independent
-// recurrences, which these latency-bound sweeps need.
-template <typename R> struct SplineCfg;
-template <> struct SplineCfg<float> {
-  static constexpr int chunk = 32, warm = 16, log2chunk = 5;
-};
-template <> struct SplineCfg<double> {
-  static constexpr int chunk = 64, warm = 32, log2chunk = 6;
-};
+// FP32 forms: the natural spline (auxi.c:56-81) and its evaluation at x =
+// interpftpad (i - shftf_i) (splint, auxi.c:83-122), then / sig2, in one
+// kernel.
+//
+// The second derivatives solve y2_{k-1} + 4 y2_k + y2_{k+1} = 6 d_k with
+// d_k = y_{k-1} - 2 y_k + y_{k+1} and y2 = 0 at both ends.  The inverse of that
+// matrix on the whole line is z^|j| / (2 sqrt(3)), z = sqrt(3) - 2 = -0.268, and
+// the ends are met by continuing d as an odd function about them, so
+//   y2_k = sqrt(3) sum_j z^|j| d_{k+j},
+// 16 terms to each side: the rest is below 0.268^17 = 2e-10 of the largest d,
+// far below FP32 rounding.  The sum is compensated (coefficients and sum as two
+// floats) from |j| = kSplineFull on inwards; the terms outside are below 1e-4 of
+// the sum, so that their plain sum errs by 6e-12 of it.  The two sweeps of the
+// elimination have 48 dependent steps of 9 dependent operations, which took
+// most of this kernel's time; here every point is its own sum.
+//
+// A block takes kSiSamples output samples; the points that they lie between
+// start at the smallest of them (base), and kSiPoints points from there hold
+// them all when the shift changes slowly (it changes by 1e-4 a sample); samples
+// beyond them are taken in another turn with a later base, whatever the shifts
+// are.  Both arrays go through packed FP32 arithmetic.  The even points of the
+// resampled series are the input itself (x), the odd ones the interpolating
+// transform's results.
+// What bounds it: for a short segment the latency of three dependent rounds of
+// loads, for a long one instruction issue.  Three
+// kernels with sweeps through global memory took 23 us on one sky point of two
+// detectors (N = 10771) and 25 us of one (N = 86164), one kernel with sweeps in
+// shared memory 12 and 14 us, this one 7.5 and 12 us.
+constexpr int kSiThreads = 128, kSiSamples = 112, kSplineFull = 6;
+constexpr int kSiPoints = 2 * kSiSamples + 16;           // points with y2
+constexpr int kSiD = kSiPoints + 2 * kSplineTaps;        // points with d, from base - kSplineTaps on
+static_assert(kSiPoints <= 2 * kSiThreads, "two points a thread");
+
+static __global__ void __launch_bounds__(kSiThreads)
+    k_resample(const float4* __restrict__ xin, const float4* __restrict__ odd, int nodd,
+               const double* __restrict__ shftf, const DetConst* __restrict__ dc, int N, int NP,
+               float4* __restrict__ xm, const __grid_constant__ SplineTab tab, const double* __restrict__ part,
+               int npart, double* __restrict__ sums, float* __restrict__ sums_r) {
+  CtaTrace trace_(KK_SPLINT);
+  __shared__ float4 ds[kSiD], zs[kSiPoints];
+  __shared__ int s_min[kSiThreads / 32];
+  const int d = blockIdx.y;
+  if (blockIdx.x == 0) {  // an extra block, the first: aa and bb
+    __shared__ double red[2][8];
+    if (d == 0) sum_parts(part, npart, gridDim.y, dc, sums, sums_r, red);
+    return;
+  }
+  const int n = 2 * N;
+  const int t = threadIdx.x;
+  const int i = (blockIdx.x - 1) * kSiSamples + t;
+  constexpr int kNone = 0x7fffffff;
+  int klo = kNone;
+  float a = 0.f, b = 0.f;
+  if (t < kSiSamples && i < N) {
+    const double x = __dmul_rn(2.0, __dsub_rn((double)i, shftf[(size_t)d * N + i]));
+    if (!(x < 0 || x > n - 1)) {
+      klo = (int)floor(x);
+      a = (float)((klo + 1) - x);
+      b = (float)(x - klo);
+    } else {
+      xm[(size_t)d * NP + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  const float is2 = dc[d].inv_sig2_f;
+  const float4* xq = xin + (size_t)d * N;
+  const float4* oq = odd + (size_t)d * nodd;
+  auto point = [&](int k) { return pld((k & 1 ? oq : xq) + (k >> 1)); };
+  for (;;) {
+    // the first point of the samples that are left
+    const int wm = __reduce_min_sync(0xffffffffu, klo);
+    if ((t & 31) == 0) s_min[t >> 5] = wm;
+    __syncthreads();
+    int base = s_min[0];
+#pragma unroll
+    for (int k = 1; k < kSiThreads / 32; ++k) base = min(base, s_min[k]);
+    if (base == kNone) break;
+#pragma unroll
+    for (int r = 0; r < (kSiD + kSiThreads - 1) / kSiThreads; ++r) {
+      const int m = r * kSiThreads + t;
+      const int k0 = base - kSplineTaps + m;
+      const int k = k0 < 0 ? -k0 : (k0 > n - 1 ? 2 * (n - 1) - k0 : k0);  // odd about both ends
+      P2 v = pzero();
+      if (m < kSiD && k > 0 && k < n - 1) {
+        const P2 p = point(k - 1), c = point(k), q = point(k + 1);
+        // formed in FP32: its rounding is below the data's own
+        const f2 m2 = dup(-2.f);
+        v.re = add2(fma2(m2, c.re, p.re), q.re);
+        v.im = add2(fma2(m2, c.im, p.im), q.im);
+        if (k != k0) v = P2{sub2(0ull, v.re), sub2(0ull, v.im)};
+      }
+      if (m < kSiD) pst(ds + m, v);
+    }
+    __syncthreads();
+    {
+      // points t and t + kSiThreads (threads without a second one repeat it)
+      const float4* d0 = ds + kSplineTaps + t;
+      const float4* d1 = ds + kSplineTaps + min(t + kSiThreads, kSiPoints - 1);
+      // (compact loops: the kernel runs once per sky point, and its
+      // instructions come from L2 then)
+      P2 f0 = pzero(), f1 = pzero();
+#pragma unroll 2
+      for (int j = kSplineTaps; j > kSplineFull; --j) {
+        const P2 v = padd(pld(d0 + j), pld(d0 - j)), w = padd(pld(d1 + j), pld(d1 - j));
+        const f2 c = dup(tab.ch[j]);
+        f0 = P2{fma2(c, v.re, f0.re), fma2(c, v.im, f0.im)};
+        f1 = P2{fma2(c, w.re, f1.re), fma2(c, w.im, f1.im)};
+      }
+      FF2 z[4] = {{f0.re, 0ull}, {f0.im, 0ull}, {f1.re, 0ull}, {f1.im, 0ull}};
+#pragma unroll 1
+      for (int j = kSplineFull; j >= 0; --j) {
+        P2 v = pld(d0 + j), w = pld(d1 + j);
+        if (j) {
+          v = padd(v, pld(d0 - j));
+          w = padd(w, pld(d1 - j));
+        }
+        const f2 ch = dup(tab.ch[j]), nch = dup(-tab.ch[j]), cl = dup(tab.cl[j]);
+        z[0] = ff2_add_prod(z[0], ch, nch, cl, v.re);
+        z[1] = ff2_add_prod(z[1], ch, nch, cl, v.im);
+        z[2] = ff2_add_prod(z[2], ch, nch, cl, w.re);
+        z[3] = ff2_add_prod(z[3], ch, nch, cl, w.im);
+      }
+      pst(zs + t, P2{add2(z[0].hi, z[0].lo), add2(z[1].hi, z[1].lo)});
+      if (t + kSiThreads < kSiPoints)
+        pst(zs + t + kSiThreads, P2{add2(z[2].hi, z[2].lo), add2(z[3].hi, z[3].lo)});
+    }
+    __syncthreads();
+    if (klo <= base + kSiPoints - 2) {
+      const int h = min(klo + 1, n - 1);
+      const P2 zl = pld(zs + (klo - base)), zh = pld(zs + (h - base)), yl = point(klo), yh = point(h);
+      const f2 ca = dup((a * a * a - a) / 6.f), cb = dup((b * b * b - b) / 6.f), fa = dup(a), fb = dup(b), s2 = dup(is2);
+      const f2 re = add2(fma2(fa, yl.re, mul2(fb, yh.re)), fma2(ca, zl.re, mul2(cb, zh.re)));
+      const f2 im = add2(fma2(fa, yl.im, mul2(fb, yh.im)), fma2(ca, zl.im, mul2(cb, zh.im)));
+      pst(xm + (size_t)d * NP + i, P2{mul2(re, s2), mul2(im, s2)});
+      klo = kNone;
+    }
+    __syncthreads();
+  }
+}
+
+// FP64 form: spline() as chunked recurrences.  The forward sweep u_i =
+// (-u_{i-1}/2 + 3 d_i) invp_i has |dU_i/dU_{i-1}| -> 2 - sqrt(3) = 0.268 and the
+// back substitution y2_k = p_k y2_{k+1} + u_k likewise, so a chunk can start
+// kSplineWarm steps early from zero: the start error shrinks by 0.268^32 =
+// 5e-19.  Chunks whose warm start reaches the array ends start from the exact
+// boundary values u_0 = 0, y2_{n-1} = 0.
+constexpr int kSplineChunk = 64, kSplineWarm = 32;
 constexpr int kSplineThreads = 256;                        // threads for staging loads/stores
 constexpr int kSplineSeg = 4096;                           // elements per CTA
 
 // Asynchronous global-to-shared copies (cp.async): every copy of a staging
 // loop is in flight at once, with no registers held; an invalid element is
 // zero-filled (source size 0, the source address is not read).
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void* smem, const void* gmem, bool valid) {
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  if (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(valid ? 16 : 0)
-                 : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(s), "l"(gmem), "n"(BYTES),
-                 "r"(valid ? BYTES : 0)
-                 : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Shared-memory slot of staged element k: one padding element per chunk, so
 // that the recurrence threads (chunk starts one chunk apart) hit different
 // banks.
-template <typename R>
-__device__ __forceinline__ int spad(int k) { return k + (k >> SplineCfg<R>::log2chunk); }
-template <typename R>
-__host__ __device__ constexpr int spad_len(int n) { return n + (n >> SplineCfg<R>::log2chunk) + 1; }
+__host__ __device__ constexpr int spad(int k) { return k + k / kSplineChunk; }
+__host__ __device__ constexpr int spad_len(int n) { return n + n / kSplineChunk + 1; }
 
 // Forward sweep.  A CTA owns one segment of kSplineSeg elements of one
 // array; it stages y[seg - warm - 1, seg_end + 1) in shared memory with
-// coalesced loads (as FP64), every thread runs its chunk's recurrence from
-// shared memory, and the u values leave through shared memory again so the
-// global stores are coalesced.
-template <typename R>
-__global__ void __launch_bounds__(kSplineThreads)
-    k_spline_fwd(const typename CT<R>::T* __restrict__ y, int ldy, double2* __restrict__ u, int n, int nseg,
+// coalesced loads, every thread runs its chunk's recurrence from shared
+// memory, and the u values leave through shared memory again so the global
+// stores are coalesced.
+static __global__ void __launch_bounds__(kSplineThreads)
+    k_spline_fwd(const double2* __restrict__ y, int ldy, double2* __restrict__ u, int n, int nseg,
                  const double* __restrict__ invp) {
-  typedef typename CT<R>::T T;
   CtaTrace trace_(KK_SPLINE_FWD);
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  double2* us = reinterpret_cast<double2*>(sm_raw);                 // spad_len<R>(kSplineSeg)
-  T* ys = reinterpret_cast<T*>(us + spad_len<R>(kSplineSeg));          // spad_len<R>(kSplineSeg + SplineCfg<R>::warm + 2)
+  double2* us = reinterpret_cast<double2*>(sm_raw);  // spad_len(kSplineSeg)
+  double2* ys = us + spad_len(kSplineSeg);           // spad_len(kSplineSeg + kSplineWarm + 2)
   const int q = blockIdx.x / nseg, sg = blockIdx.x - q * nseg;
-  const T* yq = y + (size_t)q * ldy;
+  const double2* yq = y + (size_t)q * ldy;
   double2* uq = u + (size_t)q * n;
   const int seg0 = sg * kSplineSeg;
-  const int y0 = seg0 - SplineCfg<R>::warm - 1;                       // first staged index
-  const int ny = kSplineSeg + SplineCfg<R>::warm + 2;
+  const int y0 = seg0 - kSplineWarm - 1;             // first staged index
+  const int ny = kSplineSeg + kSplineWarm + 2;
   // the coefficients of the first 64 steps of the array, in shared memory
-  // (the first chunks' recurrences read one per step): FP64 pivots for the
-  // FP64 form, their float-float splits (formed here in parallel, keeping
-  // FP64 work out of the sequential recurrence) for the FP32 forms
+  // (the first chunks' recurrences read one per step)
   __shared__ double tab[64];
-  __shared__ float tal_h[64], tal_l[64], tbe[64];
-  if (threadIdx.x < 64) {
-    const double v = invp[threadIdx.x];
-    tab[threadIdx.x] = v;
-    const FF a = ff_split(-.5 * v);
-    tal_h[threadIdx.x] = a.hi;
-    tal_l[threadIdx.x] = a.lo;
-    tbe[threadIdx.x] = (float)(3. * v);
-  }
+  if (threadIdx.x < 64) tab[threadIdx.x] = invp[threadIdx.x];
   for (int k = threadIdx.x; k < ny; k += kSplineThreads) {
     const int i = y0 + k;
     const bool ok = i >= 0 && i < n;
-    cp_async<(int)sizeof(T)>(&ys[spad<R>(k)], ok ? (const void*)(yq + i) : (const void*)yq, ok);
+    cp_async16(&ys[spad(k)], ok ? (const void*)(yq + i) : (const void*)yq, ok);
   }
   cp_async_wait_all();
   __syncthreads();
-  if (threadIdx.x < (kSplineSeg / SplineCfg<R>::chunk)) {
-    const int lo = seg0 + threadIdx.x * SplineCfg<R>::chunk;
-    const int hi = min(lo + SplineCfg<R>::chunk, n - 1);
-    // u_i = (-u_{i-1}/2 + 3 d_i) invp_i = al_i u_{i-1} + be_i d_i; the
-    // second difference d_i of the working-precision data is formed in that
-    // precision (its rounding is below the data's own)
-    int i = max(1, lo - SplineCfg<R>::warm);
-    T p = ys[spad<R>(i - 1 - y0)], cc = ys[spad<R>(i - y0)];
-    if (sizeof(R) == 8) {
-      double ux = 0., uy = 0.;
-      for (; i < hi; ++i) {
-        const T nn = ys[spad<R>(i + 1 - y0)];
-        const R dx = p.x - (R)2 * cc.x + nn.x, dy = p.y - (R)2 * cc.y + nn.y;
-        const int ti = i < 64 ? i : 63;
-        const double al = -.5 * tab[ti], be = 3. * tab[ti];
-        ux = fma(al, ux, be * (double)dx);
-        uy = fma(al, uy, be * (double)dy);
-        if (i >= lo) us[spad<R>(i - seg0)] = make_double2(ux, uy);
-        p = cc;
-        cc = nn;
-      }
-    } else {
-      FF ux{0.f, 0.f}, uy{0.f, 0.f};
-      float4* us4 = reinterpret_cast<float4*>(us);
-      auto step = [&](FF al, float be) {
-        const T nn = ys[spad<R>(i + 1 - y0)];
-        const float dx = (float)(p.x - (R)2 * cc.x + nn.x), dy = (float)(p.y - (R)2 * cc.y + nn.y);
-        ux = ff_axpt(al, ux, __fmul_rn(be, dx));
-        uy = ff_axpt(al, uy, __fmul_rn(be, dy));
-        if (i >= lo) us4[spad<R>(i - seg0)] = make_float4(ux.hi, ux.lo, uy.hi, uy.lo);
-        p = cc;
-        cc = nn;
-      };
-      // the first 63 steps of the array have their own coefficients; from
-      // i = 63 on they are constant (two loops keep the FP64 table reads out
-      // of the main one)
-      for (; i < hi && i < 63; ++i) step(FF{tal_h[i], tal_l[i]}, tbe[i]);
-      const FF al{tal_h[63], tal_l[63]};
-      const float be = tbe[63];
-      for (; i < hi; ++i) step(al, be);
+  if (threadIdx.x < (kSplineSeg / kSplineChunk)) {
+    const int lo = seg0 + threadIdx.x * kSplineChunk;
+    const int hi = min(lo + kSplineChunk, n - 1);
+    // u_i = (-u_{i-1}/2 + 3 d_i) invp_i = al_i u_{i-1} + be_i d_i
+    int i = max(1, lo - kSplineWarm);
+    double2 p = ys[spad(i - 1 - y0)], cc = ys[spad(i - y0)];
+    double ux = 0., uy = 0.;
+    for (; i < hi; ++i) {
+      const double2 nn = ys[spad(i + 1 - y0)];
+      const double dx = p.x - 2. * cc.x + nn.x, dy = p.y - 2. * cc.y + nn.y;
+      const int ti = i < 64 ? i : 63;
+      const double al = -.5 * tab[ti], be = 3. * tab[ti];
+      ux = fma(al, ux, be * dx);
+      uy = fma(al, uy, be * dy);
+      if (i >= lo) us[spad(i - seg0)] = make_double2(ux, uy);
+      p = cc;
+      cc = nn;
     }
-    if (lo == 0) us[spad<R>(0)] = make_double2(0., 0.);
+    if (lo == 0) us[spad(0)] = make_double2(0., 0.);
   }
   __syncthreads();
   const int cnt = min(kSplineSeg, n - 1 - seg0);
-  for (int k = threadIdx.x; k < cnt; k += kSplineThreads) uq[seg0 + k] = us[spad<R>(k)];
+  for (int k = threadIdx.x; k < cnt; k += kSplineThreads) uq[seg0 + k] = us[spad(k)];
 }
 
 // Back substitution, same staging: u[seg0, seg_end + warm) in shared memory,
 // y2 of the segment written back through shared memory.
-template <typename R>
-__global__ void __launch_bounds__(kSplineThreads)
-    k_spline_bwd(const double2* __restrict__ u, typename CT<R>::T* __restrict__ y2, int n, int nseg,
+static __global__ void __launch_bounds__(kSplineThreads)
+    k_spline_bwd(const double2* __restrict__ u, double2* __restrict__ y2, int n, int nseg,
                  const double* __restrict__ ptab) {
-  typedef typename CT<R>::T T;
   CtaTrace trace_(KK_SPLINE_BWD);
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  double2* us = reinterpret_cast<double2*>(sm_raw);                     // spad_len<R>(kSplineSeg + SplineCfg<R>::warm)
-  T* ys = reinterpret_cast<T*>(us + spad_len<R>(kSplineSeg + SplineCfg<R>::warm));  // spad_len<R>(kSplineSeg)
+  double2* us = reinterpret_cast<double2*>(sm_raw);       // spad_len(kSplineSeg + kSplineWarm)
+  double2* ys = us + spad_len(kSplineSeg + kSplineWarm);  // spad_len(kSplineSeg)
   const int q = blockIdx.x / nseg, sg = blockIdx.x - q * nseg;
   const double2* uq = u + (size_t)q * n;
-  T* yq = y2 + (size_t)q * n;
+  double2* yq = y2 + (size_t)q * n;
   const int seg0 = sg * kSplineSeg;
-  const int nu = min(kSplineSeg + SplineCfg<R>::warm, n - 1 - seg0);  // u defined on [0, n-2]
+  const int nu = min(kSplineSeg + kSplineWarm, n - 1 - seg0);  // u defined on [0, n-2]
   __shared__ double tab[64];
-  __shared__ float tp_h[64], tp_l[64];
-  if (threadIdx.x < 64) {
-    const double v = ptab[threadIdx.x];
-    tab[threadIdx.x] = v;
-    const FF a = ff_split(v);
-    tp_h[threadIdx.x] = a.hi;
-    tp_l[threadIdx.x] = a.lo;
-  }
-  for (int k = threadIdx.x; k < nu; k += kSplineThreads) cp_async<16>(&us[spad<R>(k)], uq + seg0 + k, true);
+  if (threadIdx.x < 64) tab[threadIdx.x] = ptab[threadIdx.x];
+  for (int k = threadIdx.x; k < nu; k += kSplineThreads) cp_async16(&us[spad(k)], uq + seg0 + k, true);
   cp_async_wait_all();
   __syncthreads();
-  const int lo = seg0 + threadIdx.x * SplineCfg<R>::chunk;
-  const int hi = min(lo + SplineCfg<R>::chunk, n);
-  if (threadIdx.x < (kSplineSeg / SplineCfg<R>::chunk) && lo < n) {
-    const int kst = min(n - 2, hi - 1 + SplineCfg<R>::warm);
-    if (sizeof(R) == 8) {
-      double vx = 0., vy = 0.;
-      for (int k = kst; k >= lo; --k) {
-        const double p = tab[k < 64 ? k : 63];
-        const double2 uk = us[spad<R>(k - seg0)];
-        vx = p * vx + uk.x;
-        vy = p * vy + uk.y;
-        if (k < hi) ys[spad<R>(k - seg0)] = mk((R)vx, (R)vy);
-      }
-    } else {
-      const float4* us4 = reinterpret_cast<const float4*>(us);
-      FF vx{0.f, 0.f}, vy{0.f, 0.f};
-      int k = kst;
-      auto step = [&](FF pc) {
-        const float4 uk = us4[spad<R>(k - seg0)];
-        vx = ff_axpy(pc, vx, FF{uk.x, uk.y});
-        vy = ff_axpy(pc, vy, FF{uk.z, uk.w});
-        if (k < hi) ys[spad<R>(k - seg0)] = mk((R)vx.hi, (R)vy.hi);
-      };
-      // constant coefficient down to k = 64, then the table
-      const FF pc63{tp_h[63], tp_l[63]};
-      for (; k >= lo && k >= 64; --k) step(pc63);
-      for (; k >= lo; --k) step(FF{tp_h[k], tp_l[k]});
+  const int lo = seg0 + threadIdx.x * kSplineChunk;
+  const int hi = min(lo + kSplineChunk, n);
+  if (threadIdx.x < (kSplineSeg / kSplineChunk) && lo < n) {
+    const int kst = min(n - 2, hi - 1 + kSplineWarm);
+    double vx = 0., vy = 0.;
+    for (int k = kst; k >= lo; --k) {
+      const double p = tab[k < 64 ? k : 63];
+      const double2 uk = us[spad(k - seg0)];
+      vx = p * vx + uk.x;
+      vy = p * vy + uk.y;
+      if (k < hi) ys[spad(k - seg0)] = make_double2(vx, vy);
     }
-    if (hi == n) ys[spad<R>(n - 1 - seg0)] = mk((R)0, (R)0);
+    if (hi == n) ys[spad(n - 1 - seg0)] = make_double2(0., 0.);
   }
   __syncthreads();
   const int cnt = min(kSplineSeg, n - seg0);
-  for (int k = threadIdx.x; k < cnt; k += kSplineThreads) yq[seg0 + k] = ys[spad<R>(k)];
+  for (int k = threadIdx.x; k < cnt; k += kSplineThreads) yq[seg0 + k] = ys[spad(k)];
 }
 
 // splint at x = interpftpad (i - shftf_i) (auxi.c:83-122), then / sig2
-template <typename R>
-__global__ void __launch_bounds__(256)
-    k_splint(const typename CT<R>::T* __restrict__ y, int ldy, const typename CT<R>::T* __restrict__ y2,
-             const double* __restrict__ shftf, const DetConst* __restrict__ dc, int N, int NP,
-             typename CT<R>::T* __restrict__ xm) {
-  typedef typename CT<R>::T T;
+static __global__ void __launch_bounds__(256)
+    k_splint(const double2* __restrict__ y, int ldy, const double2* __restrict__ y2,
+             const double* __restrict__ shftf, const DetConst* __restrict__ dc, int N, double2* __restrict__ xm) {
   CtaTrace trace_(KK_SPLINT);
   const int d = blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const int n = 2 * N;
   const double x = __dmul_rn(2.0, __dsub_rn((double)i, shftf[(size_t)d * N + i]));
-  const R is2 = sizeof(R) == 4 ? (R)dc[d].inv_sig2_f : (R)dc[d].inv_sig2;
-  T out[2];
+  const double is2 = dc[d].inv_sig2;
   for (int arr = 0; arr < 2; ++arr) {
     const size_t q = (size_t)d * 2 + arr;
-    T v = mk((R)0, (R)0);
+    double2 v = make_double2(0., 0.);
     if (!(x < 0 || x > n - 1)) {
       const int klo = (int)floor(x);
       const int khi = klo + 1;
       const int kh = khi < n ? khi : n - 1;
-      const R a = (R)(khi - x), b = (R)(x - klo);
-      const T ylo = y[q * ldy + klo], yhi = y[q * ldy + kh];
-      const T zlo = y2[q * n + klo], zhi = y2[q * n + kh];
-      const R ca = (a * a * a - a), cb = (b * b * b - b);
-      v.x = a * ylo.x + b * yhi.x + (ca * zlo.x + cb * zhi.x) / (R)6;
-      v.y = a * ylo.y + b * yhi.y + (ca * zlo.y + cb * zhi.y) / (R)6;
+      const double a = khi - x, b = x - klo;
+      const double2 ylo = y[q * ldy + klo], yhi = y[q * ldy + kh];
+      const double2 zlo = y2[q * n + klo], zhi = y2[q * n + kh];
+      const double ca = (a * a * a - a), cb = (b * b * b - b);
+      v.x = a * ylo.x + b * yhi.x + (ca * zlo.x + cb * zhi.x) / 6.;
+      v.y = a * ylo.y + b * yhi.y + (ca * zlo.y + cb * zhi.y) / 6.;
     }
-    out[arr] = mk(v.x * is2, v.y * is2);
-  }
-  if (sizeof(R) == 8) {
-    xm[((size_t)d * 2 + 0) * N + i] = out[0];
-    xm[((size_t)d * 2 + 1) * N + i] = out[1];
-  } else {
-    reinterpret_cast<float4*>(xm)[(size_t)d * NP + i] =
-        make_float4((float)out[0].x, (float)out[1].x, (float)out[0].y, (float)out[1].y);
+    xm[q * N + i] = make_double2(v.x * is2, v.y * is2);
   }
 }
 
@@ -1363,51 +1394,68 @@ template <typename R, int PM> class EngineT : public Engine {
 
   cudaError_t prelude(const SkyArgs& sky, int slot, cudaStream_t st) override {
     const int N = b_.N, nifo = b_.nifo;
-    const int nbx = (N + 255) / 256;
+    constexpr int NT = mod_threads<R>();
+    const int nbx = (N + NT - 1) / NT;
     pre(KK_PRELUDE_MOD, nifo, st);
-    k_prelude_mod<R, PM><<<dim3(nbx, nifo), 256, 0, st>>>(
+    k_prelude_mod<R, PM><<<dim3(nbx, nifo), NT, 0, st>>>(
         b_.xDat, b_.DetSSB, (const R*)b_.cosmodf, (const R*)b_.sinmodf, b_.dc, sky, N, b_.NP, (T*)b_.xin,
         b_.shftf, sizeof(R) == 8 ? b_.ph0[slot] : (void*)((float4*)b_.xm[slot] + (size_t)nifo * b_.NP), b_.part, b_.sums[slot],
         (R*)b_.sums_r[slot], b_.counter);
     post(st);
     launches_ += 1;
-    // forward FFT of the zero-padded series (length nfft)
-    PlainLoader<R> pl{(const T*)b_.xin, N, N};
-    CStore<R> cs1{(T*)b_.spec, b_.nfft, (R)1};
-    cudaError_t e;
-    if constexpr (sizeof(R) == 4) e = pair_pre<-1, 0>(pl, cs1, nifo, st, KK_FFT_FWD_A, KK_FFT_FWD_B);
-    else e = fft<-1>(gf_, b_.tw_fwd, pl, cs1, nifo, st, KK_FFT_FWD_A, KK_FFT_FWD_B, b_.ybuf_pre);
-    if (e != cudaSuccess) return e;
-    // spectrum remap + backward FFT of length Ninterp, scale interpftpad/Ninterp
-    // (jobcore.c:338-362), as a half-length transform (HalfShiftLoader)
-    HalfShiftLoader<R> hl{(const T*)b_.spec, (const T*)b_.tw_inv[2], (const T*)b_.tw_inv[3], b_.nfft,
-                          b_.nfft / 2 + 1};
-    InterpStore<R> is{(T*)b_.yint, (const T*)b_.xin, N, b_.Ninterp, (R)(1.0 / b_.nfft)};
-    if constexpr (sizeof(R) == 4) e = pair_pre<+1, 16>(hl, is, nifo, st, KK_FFT_INV_A, KK_FFT_INV_B);
-    else e = fft<+1>(gf_, b_.tw_invh, hl, is, nifo, st, KK_FFT_INV_A, KK_FFT_INV_B, b_.ybuf_pre);
-    if (e != cudaSuccess) return e;
+    // forward FFT of the zero-padded series (length nfft), then spectrum remap
+    // + backward FFT of length Ninterp, scale interpftpad/Ninterp
+    // (jobcore.c:338-362), as a half-length transform (HalfShiftLoader), and the
     // spline through the first 2N points of each resampled array
-    const int n = 2 * N;
-    const int nseg = (n + kSplineSeg - 1) / kSplineSeg;
-    constexpr int W = SplineCfg<R>::warm;
-    const int smf = spad_len<R>(kSplineSeg) * (int)sizeof(double2) + spad_len<R>(kSplineSeg + W + 2) * (int)sizeof(T);
-    const int smb = spad_len<R>(kSplineSeg + W) * (int)sizeof(double2) + spad_len<R>(kSplineSeg) * (int)sizeof(T);
-    static std::atomic<unsigned long long> donef{0}, doneb{0};
-    smem_attr(k_spline_fwd<R>, smf, donef);
-    smem_attr(k_spline_bwd<R>, smb, doneb);
-    pre(KK_SPLINE_FWD, nifo, st);
-    k_spline_fwd<R><<<nseg * 2 * nifo, kSplineThreads, smf, st>>>((const T*)b_.yint, b_.Ninterp,
-                                                                  (double2*)b_.u, n, nseg, b_.spline_invp);
-    post(st);
-    pre(KK_SPLINE_BWD, nifo, st);
-    k_spline_bwd<R><<<nseg * 2 * nifo, kSplineThreads, smb, st>>>((const double2*)b_.u, (T*)b_.y2, n, nseg,
-                                                                  b_.spline_p);
-    post(st);
-    pre(KK_SPLINT, nifo, st);
-    k_splint<R><<<dim3(nbx, nifo), 256, 0, st>>>((const T*)b_.yint, b_.Ninterp, (const T*)b_.y2,
-                                                 b_.shftf, b_.dc, N, b_.NP, (T*)b_.xm[slot]);
-    post(st);
-    launches_ += 3;
+    cudaError_t e;
+    if constexpr (sizeof(R) == 4) {
+      const PairLoader pl{(const float4*)b_.xin, N};
+      const PairStore<KK_FFT_FWD_B> sp{(float4*)b_.spec, b_.nfft, 1.f};
+      e = pair_pre<-1, 0>(pl, sp, nifo, st, KK_FFT_FWD_A, KK_FFT_FWD_B);
+      if (e != cudaSuccess) return e;
+      const HalfShiftPair hl{(const float4*)b_.spec, (const float2*)b_.tw_inv[2], (const float2*)b_.tw_inv[3], b_.nfft,
+                             b_.nfft / 2 + 1};
+      const PairStore<KK_FFT_INV_B> is{(float4*)b_.yint, b_.nfft, (float)(1.0 / b_.nfft)};
+      e = pair_pre<+1, 16>(hl, is, nifo, st, KK_FFT_INV_A, KK_FFT_INV_B);
+      if (e != cudaSuccess) return e;
+      pre(KK_SPLINT, nifo, st);
+      k_resample<<<dim3((N + kSiSamples - 1) / kSiSamples + 1, nifo), kSiThreads, 0, st>>>(
+          (const float4*)b_.xin, (const float4*)b_.yint, b_.nfft, b_.shftf, b_.dc, N, b_.NP, (float4*)b_.xm[slot],
+          b_.spl, b_.part, nbx, b_.sums[slot], (float*)b_.sums_r[slot]);
+      post(st);
+      launches_ += 1;
+    } else {
+      PlainLoader<R> pl{(const T*)b_.xin, N, N};
+      CStore<R> cs1{(T*)b_.spec, b_.nfft, (R)1};
+      e = fft<-1>(gf_, b_.tw_fwd, pl, cs1, nifo, st, KK_FFT_FWD_A, KK_FFT_FWD_B, b_.ybuf_pre);
+      if (e != cudaSuccess) return e;
+      HalfShiftLoader<R> hl{(const T*)b_.spec, (const T*)b_.tw_inv[2], (const T*)b_.tw_inv[3], b_.nfft,
+                            b_.nfft / 2 + 1};
+      InterpStore<R> is{(T*)b_.yint, (const T*)b_.xin, N, b_.Ninterp, (R)(1.0 / b_.nfft)};
+      e = fft<+1>(gf_, b_.tw_invh, hl, is, nifo, st, KK_FFT_INV_A, KK_FFT_INV_B, b_.ybuf_pre);
+      if (e != cudaSuccess) return e;
+      const int n = 2 * N;
+      const int nseg = (n + kSplineSeg - 1) / kSplineSeg;
+      constexpr int smf = (spad_len(kSplineSeg) + spad_len(kSplineSeg + kSplineWarm + 2)) * (int)sizeof(double2);
+      constexpr int smb = (spad_len(kSplineSeg) + spad_len(kSplineSeg + kSplineWarm)) * (int)sizeof(double2);
+      static std::atomic<unsigned long long> donef{0}, doneb{0};
+      smem_attr(k_spline_fwd, smf, donef);
+      smem_attr(k_spline_bwd, smb, doneb);
+      pre(KK_SPLINE_FWD, nifo, st);
+      k_spline_fwd<<<nseg * 2 * nifo, kSplineThreads, smf, st>>>((const double2*)b_.yint, b_.Ninterp,
+                                                                 (double2*)b_.u, n, nseg, b_.spline_invp);
+      post(st);
+      pre(KK_SPLINE_BWD, nifo, st);
+      k_spline_bwd<<<nseg * 2 * nifo, kSplineThreads, smb, st>>>((const double2*)b_.u, (double2*)b_.y2, n, nseg,
+                                                                 b_.spline_p);
+      post(st);
+      pre(KK_SPLINT, nifo, st);
+      k_splint<<<dim3((N + 255) / 256, nifo), 256, 0, st>>>((const double2*)b_.yint, b_.Ninterp,
+                                                            (const double2*)b_.y2, b_.shftf, b_.dc, N,
+                                                            (double2*)b_.xm[slot]);
+      post(st);
+      launches_ += 3;
+    }
     return cudaGetLastError();
   }
 

@@ -59,6 +59,7 @@ struct SkyArgs {
   double sinal, cosal, sindel, cosdel;
   double nS[3];           // unit vector to the source
   double shft1[kMaxDet];  // nS . DetSSB[0..2] per detector
+  double shft1_fma[kMaxDet];  // the same with fused multiply-adds (FP32 forms)
   double cosalfr[kMaxDet], sinalfr[kMaxDet];  // modvir rotated angles
   double s1_0;            // nn M9 + mm M13 (0 with --nospindown); over 2 pi
                           // in the fixed-point phase mode
@@ -82,6 +83,31 @@ struct DevCand {
   double F;
 };
 
+// FP64 form: the coefficients of the spline's elimination, p_i and invp_i = 2 /
+// (p_{i-1} + 4), which settle to constants well before i = 63 (auxi.c:71-72).
+inline void spline_pivots(double* invp, double* p) {
+  p[0] = invp[0] = 0.;
+  for (int i = 1; i < 64; i++) {
+    invp[i] = 2. / (p[i - 1] + 4.);
+    p[i] = -.5 * invp[i];
+  }
+}
+// FP32 forms: sqrt(3) (sqrt(3) - 2)^j as float-float (k_resample).
+constexpr int kSplineTaps = 16;
+struct SplineTab {
+  float ch[kSplineTaps + 1], cl[kSplineTaps + 1];
+};
+inline SplineTab spline_taps() {
+  SplineTab t;
+  double c = sqrt(3.);
+  const double z = -1. / (2. + sqrt(3.));
+  for (int j = 0; j <= kSplineTaps; j++, c *= z) {
+    t.ch[j] = (float)c;
+    t.cl[j] = (float)(c - (double)t.ch[j]);
+  }
+  return t;
+}
+
 // Device buffers owned by the context and shared with the engine.
 struct Buffers {
   int N, nfft, Ninterp, nfftf, nmin, nmax, bins, nblk, nifo, fftpad;
@@ -92,13 +118,16 @@ struct Buffers {
   const void* cosmodf;              // [N] Real
   const void* sinmodf;              // [N] Real
   const DetConst* dc;               // [nifo]
-  const double* spline_invp;        // [64] pivots 2/(p+4) of the spline solve
-  const double* spline_p;           // [64] p_i
-  void* xin;                        // [nifo][2][N] Real complex
-  void* spec;                       // [nifo][2][nfft]
-  void* yint;                       // [nifo][2][Ninterp]
-  double* u;                        // [nifo][2][2N] double2
-  void* y2;                         // [nifo][2][2N] Real complex
+  const double* spline_invp;        // FP64 form: [64] pivots 2/(p+4) of the spline solve
+  const double* spline_p;           // FP64 form: [64] p_i
+  SplineTab spl;                    // FP32 forms: the spline's taps
+  // FP64 form: arrays of double complex; FP32 forms: of pairs {a.re, b.re,
+  // a.im, b.im} (float4)
+  void* xin;                        // [nifo][2][N]; FP32: [nifo][N]
+  void* spec;                       // [nifo][2][nfft]; FP32: [nifo][nfft]
+  void* yint;                       // [nifo][2][Ninterp]; FP32: its odd points, [nifo][nfft]
+  double* u;                        // FP64 form: [nifo][2][2N] double2
+  void* y2;                         // FP64 form: [nifo][2][2N] double2
   double* shftf;                    // [nifo][N]
   // per-sky prelude outputs, double-buffered (slot 0/1) so that the prelude
   // of one sky point runs while the spindowns of the previous one read the
@@ -118,7 +147,6 @@ struct Buffers {
   void* F;                          // [2*lane_sb][bins] Real
   int lane_sb;                      // spindowns per lane of ybuf and F: lane 1 starts at
                                     // spindown lane_sb (two lanes run on two streams)
-  void* mu;                         // [sbatch][nblk] Real
   DevCand* cand;
   int* ncand;
   int cand_cap;
