@@ -50,6 +50,21 @@
 
 namespace pa {
 
+// Programmatic dependent launch: the blocks of a kernel may come to the SMs
+// when all blocks of the one before it in the stream have called pdl_go, and
+// wait in pdl_wait until it has finished and its results are visible.  Every
+// block calls both, go after wait, so that whatever came before the kernel
+// before has finished too.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A pointer whose loads stay behind the wait, also those of read-only data
+// that the compiler may otherwise move freely.
+template <class T> __device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p));
+  return p;
+}
+
 // One complex element of the arrays a and b.
 struct P2 {
   f2 re, im;
@@ -317,6 +332,8 @@ __global__ void __launch_bounds__(PairShape<LOGL, LOGT, LOGS>::NT, 512 / PairSha
     const int nw = ((t >> 5 << 5 >> G::LOGQ) << G::LOGL2) + c0;
     constexpr int step = 16 << G::LOGL2;
     constexpr int PF = Loader::template Ahead<NIN, NCHK>::v;
+    pdl_wait();
+    pdl_go();
     // (items past the last one repeat it; they are not stored)
     typename Loader::Ctx ctx = ld.begin(min(batch0 + (q >> G::LOGC), nbatch - 1), n0, step);
     const int left = ld.count() - nw;
@@ -405,8 +422,16 @@ __global__ void __launch_bounds__(PairShape<LOGL, LOGT>::NT, PairShape<LOGL, LOG
   // so their intermediate is the likeliest to be still in L2
   const int batch = gridDim.y - 1 - blockIdx.y;
   const int k10 = blockIdx.x << G::LOGRR;
+  // the row twiddles, in flight over the wait; stored after the first stage
+  constexpr int NTW = G::R2 == 1 && G::R3 == 1 ? 1 : (G::TW + G::NT - 1) / G::NT;
+  float2 twv[NTW];
+#pragma unroll
+  for (int k = 0; k < NTW; ++k)
+    if (t + k * G::NT < G::TW) twv[k] = ldg_here(&tw2[t + k * G::NT]);
+  pdl_wait();
+  pdl_go();
   const typename Storer::Ctx sctx = st.begin();
-  const float4* yb = ybuf + ((size_t)batch << LOGL);
+  const float4* yb = after_wait(ybuf) + ((size_t)batch << LOGL);
   auto at = [](int e, int rr) { return e * G::RR + (e >> G::LOGR1) * G::PAD + rr; };
   auto from_smem = [&](int e, int rr) { return pld(s + at(e, rr)); };
   // the intermediate is read once, here: evict-first
@@ -423,12 +448,7 @@ __global__ void __launch_bounds__(PairShape<LOGL, LOGT>::NT, PairShape<LOGL, LOG
 #pragma unroll
     for (int r = 0; r < (HALF ? 8 : 16); ++r) st.put(sctx, batch, k10 + rr, j + r * (G::L2 / 16), v[r]);
   } else {
-    // first stage; the twiddle table is loaded before it and stored after it
-    constexpr int NTW = (G::TW + G::NT - 1) / G::NT;
-    float2 twv[NTW];
-#pragma unroll
-    for (int k = 0; k < NTW; ++k)
-      if (t + k * G::NT < G::TW) twv[k] = __ldg(&tw2[t + k * G::NT]);
+    // first stage
     constexpr int R = G::R1, PT = 16 / R;
     P2 v[PT][R];
     int j[PT], rr[PT];
