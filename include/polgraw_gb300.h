@@ -56,7 +56,7 @@ typedef enum pa_precision {
 /* How the spindown phase het1*i + s1*(i^2 + 2 i shft_i) is formed in the
  * mixed form (the FP64 form always evaluates it in FP64). */
 typedef enum pa_phase_mode {
-  PA_PHASE_F64 = 0,    /* FP64 per sample, reduced mod 2 pi, FP32 sincos */
+  PA_PHASE_F64 = 0,    /* FP64 product per sample, mod 1 turn, FP32 sincos */
   PA_PHASE_FIXED = 1,  /* 64-bit fixed-point turns from FP64 per-sky terms */
   PA_PHASE_FF = 2      /* compensated two-float (float-float) phase */
 } pa_phase_mode;

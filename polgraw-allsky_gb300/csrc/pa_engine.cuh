@@ -400,11 +400,15 @@ inline uint64_t het1_turns_fixed(int ss, double M4, double M0) {
 // passed by value with the loader, so that no CTA of pass A waits on a chain
 // of FP64 operations before its first phase.  het1 = fmod(ss M4, M0) wrapped
 // (jobcore.c:466-467), s1 = ss M5 + s1_0 (one rounding).
-template <int PM> struct SpinHet {  // FP64 phase: the FP64 form and PM_F64
+struct SpinHet64 {  // FP64 form
   double het1[kSpinBatchMax], s1[kSpinBatchMax];
 };
-template <> struct SpinHet<PM_FIXED> {
+template <int PM> struct SpinHet {  // PM_FIXED
   unsigned long long H[kSpinBatchMax];  // het1 as 64-bit fixed-point turns
+};
+template <> struct SpinHet<PM_F64> {
+  unsigned long long H[kSpinBatchMax];
+  double s1t[kSpinBatchMax];  // s1 / 2 pi
 };
 template <> struct SpinHet<PM_FF> {
   float4 c[kSpinBatchMax];  // s1 and het1 as two floats each
@@ -418,8 +422,14 @@ inline void spin_het1_s1(int ss, const SkyArgs& sky, int s0_flag, double* het1, 
   if (*het1 < 0) *het1 += sky.M0;
   *s1 = s0_flag ? 0. : fma((double)ss, sky.M5, sky.s1_0);
 }
-inline void spin_het_fill(SpinHet<PM_F64>& h, int k, int ss, const SkyArgs& sky, int s0_flag) {
+inline void spin_het_fill(SpinHet64& h, int k, int ss, const SkyArgs& sky, int s0_flag) {
   spin_het1_s1(ss, sky, s0_flag, &h.het1[k], &h.s1[k]);
+}
+inline void spin_het_fill(SpinHet<PM_F64>& h, int k, int ss, const SkyArgs& sky, int s0_flag) {
+  double het1, s1;
+  spin_het1_s1(ss, sky, s0_flag, &het1, &s1);
+  h.H[k] = het1_turns_fixed(ss, sky.M4, sky.M0);
+  h.s1t[k] = s1 * kInvTwoPi;
 }
 inline void spin_het_fill(SpinHet<PM_FF>& h, int k, int ss, const SkyArgs& sky, int s0_flag) {
   double het1, s1;
@@ -433,6 +443,10 @@ __device__ __forceinline__ uint64_t mul64x32(uint64_t a, unsigned b) {
   return (uint64_t)(unsigned)a * b + ((uint64_t)((unsigned)(a >> 32) * b) << 32);
 }
 
+// High word of a t mod 1, for products of any size (a call: the compiler would
+// issue a rare branch's FP64 operations for every sample).
+static __device__ __noinline__ unsigned far_turns(double a, double t) { return (unsigned)(turns_fixed(a * t) >> 32); }
+
 // Phase-modulated detector sum of the spindown loop (jobcore.c:455-623):
 //   x_{a,b}[n] = sum_d xm_{a,b,d}[n] exp(-i (het1 n + s1 tmp1_d[n]))  (n < N)
 // FP64 form:
@@ -441,7 +455,7 @@ struct SpinLoader64 {
   const double2* xm;   // [nifo][2][N]
   const double* tmp1;  // [nifo][N]
   int N, nifo;
-  SpinHet<PM_F64> het;
+  SpinHet64 het;
 
   __device__ __forceinline__ void load2(int batch, int n, double2& va, double2& vb) const {
     va = vb = mk(0., 0.);
@@ -497,7 +511,7 @@ template <int PM, int NIFO> struct SpinLoader {
     unsigned long long hn, hstep;  // fixed point: H n, and H times the step of n
     unsigned ssr;                  // spindown less ss_base
     int n0;
-    double het1, s1;
+    double s1t;
     float4 c;
   };
   struct Raw {
@@ -520,15 +534,17 @@ template <int PM, int NIFO> struct SpinLoader {
       k.hstep = mul64x32(H, (unsigned)step);
       k.ssr = s0_flag ? 0u : (unsigned)(ss_rel + batch);
     } else if constexpr (PM == PM_F64) {
-      k.het1 = het.het1[batch];
-      k.s1 = het.s1[batch];
+      const unsigned long long H = het.H[batch];
+      k.hn = mul64x32(H, (unsigned)n0);
+      k.hstep = mul64x32(H, (unsigned)step);
+      k.s1t = het.s1t[batch];
     } else {
       k.c = het.c[batch];
     }
     return k;
   }
   __device__ __forceinline__ void next(Ctx& k) const {
-    if constexpr (PM == PM_FIXED) k.hn += k.hstep;
+    if constexpr (PM != PM_FF) k.hn += k.hstep;
   }
   __device__ __forceinline__ Raw fetch(const Ctx& k, int off) const {
     Raw r{};
@@ -554,12 +570,18 @@ template <int PM, int NIFO> struct SpinLoader {
       const unsigned th = p.y + (__umulhi(p.z, k.ssr) + p.w * k.ssr) + (unsigned)(k.hn >> 32);
       __sincosf((float)(int)th * 1.4629180792671596e-9f, sn, cs);  // pi 2^-31
     } else if constexpr (PM == PM_F64) {
+      // s1 tmp1 in turns, one FP64 operation per detector and sample (FP64
+      // runs at 1/64 of the FP32 rate, and nine of them bounded pass A): the
+      // fma onto 1.5 2^20 rounds the product to 2^-32 turns (1.5e-9 rad, far
+      // below the FP32 rounding of the angle) and leaves it mod 1 in the low
+      // word, as long as it is below 2^19 turns.  H n is exact.  Day of two
+      // detectors, FP64 phases (N = 43082, 12 x 75 spindowns): 2.17 -> 1.46 ms.
       const double t1 = __hiloint2double((int)p.y, (int)p.x);
-      const double ph_ = fma(k.s1, t1, k.het1 * (double)n);
-      const double kk = rint(ph_ * kInvTwoPi);
-      double r = fma(-kk, kTwoPiHi, ph_);
-      r = fma(-kk, kTwoPiLo, r);
-      sincosf((float)r, sn, cs);
+      const double q = fma(k.s1t, t1, 1572864.0);
+      unsigned th = (unsigned)__double2loint(q);
+      if (((unsigned)__double2hiint(q) >> 20) != 0x413u) th = far_turns(k.s1t, t1);
+      th += (unsigned)(k.hn >> 32);
+      sincospif((float)(int)th * 4.656612873077393e-10f, sn, cs);
     } else {
       // compensated float-float phase
       const float2 tt = make_float2(__uint_as_float(p.x), __uint_as_float(p.y));
