@@ -28,6 +28,7 @@
 #include "pa_engine.h"
 #include "pa_fft.cuh"
 #include "pa_pair.cuh"
+#include "pa_sincos.cuh"
 
 namespace pa {
 
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(mod_threads<R>())
       // prelude phase het0 i + oms shft (jobcore.c:299), FP64
       const double phase = __dadd_rn(__dmul_rn(sky.het0, di), __dmul_rn(sky.oms, shft));
       double sd, cd;
-      sincos(phase, &sd, &cd);
+      sincos_fast(phase, &sd, &cd);
       sp = (R)sd;
       cp = (R)cd;
     } else {
@@ -466,7 +467,7 @@ struct SpinLoader64 {
       // het1*i + s1*_tmp1 with the reference's rounding (jobcore.c:606)
       const double ph = __dadd_rn(__dmul_rn(het1, (double)n), __dmul_rn(s1, tmp1[(size_t)d * N + n]));
       double sn, cs;
-      sincos(ph, &sn, &cs);
+      sincos_fast(ph, &sn, &cs);
       // x * (cos - i sin)
       va.x += xa.x * cs + xa.y * sn;
       va.y += xa.y * cs - xa.x * sn;

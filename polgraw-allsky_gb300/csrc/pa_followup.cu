@@ -32,6 +32,7 @@
 
 #include "../../include/polgraw_gb300.h"
 #include "pa_f32x2.cuh"
+#include "pa_sincos.cuh"
 #include "pa_trace.h"
 
 namespace {
@@ -174,7 +175,7 @@ struct Sample {
 __device__ __forceinline__ void fu_phase(const FuCand& c, double oms, double di, double shft, double* sn, double* cs) {
   const double phi = __dadd_rn(__dadd_rn(__dmul_rn(c.f, __dadd_rn(di, shft)), __dmul_rn(__dmul_rn(c.s, di), di)),
                                __dmul_rn(__dadd_rn(oms, __dmul_rn(__dmul_rn(2., c.s), di)), shft));
-  sincos(phi, sn, cs);
+  pa::sincos_fast(phi, sn, cs);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
