@@ -676,7 +676,7 @@ template <typename R> struct FstatStore {
     const int k = k1 + (k2 << 8);
     float a, b;
     upk(fma2(v.im, v.im, mul2(v.re, v.re)), a, b);
-    if (k >= nmin && k < nmax) F[(size_t)batch * bins + (k - nmin)] = fmaf(a, (float)c.ia, b * (float)c.ib);
+    if ((unsigned)(k - nmin) < (unsigned)bins) F[(size_t)batch * bins + (k - nmin)] = fmaf(a, (float)c.ia, b * (float)c.ib);
   }
 };
 
@@ -1335,7 +1335,7 @@ template <typename R, int PM> class EngineT : public Engine {
            (float4*)ybuf, batch);
     post(stream);
     pre(kind_b, batch, stream);
-    launch(kb, gb, B::NT, B::smem_b, stream, st, (const float2*)b_.pair_row[which], (const float4*)ybuf);
+    launch(kb, gb, B::NB, B::smem_b, stream, st, (const float2*)b_.pair_row[which], (const float4*)ybuf);
     post(stream);
     launches_ += 2;
     return cudaGetLastError();

@@ -12,7 +12,7 @@ constexpr int pair_row_block(int logL) { return logL >= 19 ? 0 : (logL <= 16 ? 3
 // radix of stage `stage` (0, 1, 2) of the row transforms; 1: no such stage
 constexpr int pair_radix(int logL, int stage) {
   constexpr int r[9][3] = {{16, 1, 1}, {8, 1, 4}, {8, 1, 8}, {16, 1, 8}, {16, 1, 16},
-                           {8, 8, 8}, {16, 8, 8}, {16, 16, 8}, {16, 16, 16}};
+                           {16, 1, 32}, {16, 8, 8}, {16, 16, 8}, {16, 16, 16}};
   return r[logL - 12][stage];
 }
 // entries of the row twiddle table: W_{Ns R}^{k r} at r Ns + k for the middle

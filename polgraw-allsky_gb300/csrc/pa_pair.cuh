@@ -17,7 +17,7 @@
 // A CTA transforms a tile of T = 2^LOGT pairs with T/16 threads, 16 pairs a
 // thread (64 registers of data at 128 a thread):
 //   pass A: T/256 columns as 16 x 16, one exchange through shared memory;
-//   pass B: T/L2 rows in radix-16 and radix-8 stages (PairRow).
+//   pass B: T/L2 rows in two or three stages of radix 8, 16 or 32.
 // 128 registers at half the warps hold the same data as 64 registers did at
 // twice the warps, and leave room for the loads of the next positions.
 //
@@ -251,8 +251,42 @@ template <int SIGN> __device__ __forceinline__ void pdft2(P2* v) {
   v[1] = psub(a, v[1]);
 }
 
-template <int SIGN, int R> __device__ __forceinline__ void pdft(P2* v) {
-  static_assert(R == 1 || R == 2 || R == 4 || R == 8 || R == 16, "radix");
+// 32-point DFT in natural order, the first 16 results only with HALF: X[k] =
+// E[k] + W32^k O[k], X[k + 16] = E[k] - W32^k O[k]
+template <int SIGN, bool HALF> __device__ __forceinline__ void pdft32(P2* v) {
+  constexpr float c[9] = {1.f, 0.98078528040323044913f, 0.92387953251128675613f, 0.83146961230254523708f,
+                          kSqrtHalf, 0.55557023301960222474f, 0.38268343236508977173f, 0.19509032201612826785f, 0.f};
+  P2 e[16], o[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    e[k] = v[2 * k];
+    o[k] = v[2 * k + 1];
+  }
+  pdft16<SIGN>(e);
+  pdft16<SIGN>(o);
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    if (k == 0) {
+      v[0] = padd(e[0], o[0]);
+      if (!HALF) v[16] = psub(e[0], o[0]);
+    } else if (k == 8) {
+      const P2 p = {sub2(e[8].re, o[8].im), add2(e[8].im, o[8].re)}, m = {add2(e[8].re, o[8].im), sub2(e[8].im, o[8].re)};
+      v[8] = SIGN > 0 ? p : m;
+      if (!HALF) v[24] = SIGN > 0 ? m : p;
+    } else {
+      const float wr = k < 8 ? c[k] : -c[16 - k], wi = SIGN * (k < 8 ? c[8 - k] : c[k - 8]);
+      v[k] = P2{fma2(o[k].im, dup(-wi), fma2(o[k].re, dup(wr), e[k].re)),
+                fma2(o[k].im, dup(wr), fma2(o[k].re, dup(wi), e[k].im))};
+      if (!HALF)
+        v[k + 16] = P2{fma2(o[k].im, dup(wi), fma2(o[k].re, dup(-wr), e[k].re)),
+                       fma2(o[k].im, dup(-wr), fma2(o[k].re, dup(-wi), e[k].im))};
+    }
+  }
+}
+
+template <int SIGN, int R, bool HALF = false> __device__ __forceinline__ void pdft(P2* v) {
+  static_assert(R == 1 || R == 2 || R == 4 || R == 8 || R == 16 || R == 32, "radix");
+  if constexpr (R == 32) pdft32<SIGN, HALF>(v);
   if (R == 2) pdft2<SIGN>(v);
   if (R == 4) pdft4<SIGN>(v[0], v[1], v[2], v[3]);
   if (R == 8) pdft8<SIGN>(v);
@@ -278,11 +312,18 @@ template <int LOGL, int LOGT, int LOGS = 0> struct PairShape {
   // pass B tile: element e of row rr at e * RR + (e / R1) * PAD + rr.  The
   // first stage stores R1 elements apart from lane to lane; with fewer than
   // 8 rows the pad after every R1 elements keeps that conflict-free.
+  // threads of pass B: 16 pairs each, 32 with a radix-32 stage.  512-element
+  // rows (2^17) as 16 x 32 exchange through shared memory once, as 8 x 8 x 8
+  // twice, and shared memory is what pass B uses most: 48 x 200 spindowns of
+  // two detectors 11.97 -> 11.25 ms, 64 of one 146 -> 138 us.  Five CTAs of 64
+  // threads per SM, at 168 registers (six, with the pad given up for a swizzle:
+  // 12.1 ms).  1024-element rows as 32 x 32 gained nothing.
+  static constexpr int EB = R3 == 32 ? 32 : 16, NB = T / EB;
   static constexpr int LOGR1 = R1 == 16 ? 4 : (R1 == 8 ? 3 : (R1 == 4 ? 2 : 1));
   static constexpr int PAD = RR < 8 ? RR : 0;
   static constexpr int TW = pair_row_table(LOGL);                 // entries of the row twiddle table
   // CTAs of pass B per SM (three of 256 threads, at 80 registers, spill)
-  static constexpr int MINB = 512 / NT;
+  static constexpr int MINB = EB == 32 ? 320 / NB : 512 / NB;
   static constexpr int smem_b = (L2 * RR + (L2 / R1) * PAD) * 16 + TW * 8;
   static_assert(LOGL >= 12 && LOGL <= 20 && LOGT >= 11 && LOGT <= 12, "no such tile");
   static_assert(LOGC >= 0 && C <= L2 && RR <= 256, "transform too short for the tile");
@@ -386,7 +427,7 @@ __global__ void __launch_bounds__(PairShape<LOGL, LOGT, LOGS>::NT, 512 / PairSha
 // One stage of the row transforms: R-point butterflies with the results of
 // Ns-point ones (Stockham); thread t takes the butterflies (j, rr) = t, t + NT,
 // ...  In: from `src(e, rr)`; out: `dst(e, rr, value)`.  FIRST: no twiddles.
-template <int SIGN, int R, int LOGNS, class G, class Src>
+template <int SIGN, int R, int LOGNS, class G, bool HALF = false, class Src>
 __device__ __forceinline__ void pair_stage_load(const Src& src, const float2* tw, int q, int& j, int& rr, P2 (&v)[R]) {
   constexpr int J = G::L2 / R;  // butterflies of a row
   rr = q & (G::RR - 1);
@@ -402,14 +443,14 @@ __device__ __forceinline__ void pair_stage_load(const Src& src, const float2* tw
       v[r] = pmul(v[r], w.x, SIGN > 0 ? -w.y : w.y);
     }
   }
-  pdft<SIGN, R>(v);
+  pdft<SIGN, R, HALF>(v);
 }
 
 // Pass B.  Storer: Ctx begin() and put(ctx, batch, k1, k2, value); HALF: only
 // the outputs below L/2 are wanted, so the last stage forms half of its
 // outputs.
 template <int SIGN, int LOGL, int LOGT, class Storer, bool HALF>
-__global__ void __launch_bounds__(PairShape<LOGL, LOGT>::NT, PairShape<LOGL, LOGT>::MINB)
+__global__ void __launch_bounds__(PairShape<LOGL, LOGT>::NB, PairShape<LOGL, LOGT>::MINB)
     k_pair_b(const Storer st, const float2* __restrict__ tw2, const float4* __restrict__ ybuf) {
   typedef PairShape<LOGL, LOGT> G;
   static_assert(LOGT >= G::LOGL2, "a row is longer than the tile");
@@ -423,11 +464,11 @@ __global__ void __launch_bounds__(PairShape<LOGL, LOGT>::NT, PairShape<LOGL, LOG
   const int batch = gridDim.y - 1 - blockIdx.y;
   const int k10 = blockIdx.x << G::LOGRR;
   // the row twiddles, in flight over the wait; stored after the first stage
-  constexpr int NTW = G::R2 == 1 && G::R3 == 1 ? 1 : (G::TW + G::NT - 1) / G::NT;
+  constexpr int NTW = G::R2 == 1 && G::R3 == 1 ? 1 : (G::TW + G::NB - 1) / G::NB;
   float2 twv[NTW];
 #pragma unroll
   for (int k = 0; k < NTW; ++k)
-    if (t + k * G::NT < G::TW) twv[k] = ldg_here(&tw2[t + k * G::NT]);
+    if (t + k * G::NB < G::TW) twv[k] = ldg_here(&tw2[t + k * G::NB]);
   pdl_wait();
   pdl_go();
   const typename Storer::Ctx sctx = st.begin();
@@ -437,7 +478,7 @@ __global__ void __launch_bounds__(PairShape<LOGL, LOGT>::NT, PairShape<LOGL, LOG
   // the intermediate is read once, here: evict-first
   auto from_y = [&](int n2, int rr) {
     const int k1 = k10 + rr;
-    return pldlast(yb + ((((size_t)(k1 >> G::LR) << G::LOGL2) + n2) << G::LR) + (k1 & ((1 << G::LR) - 1)));
+    return pldlast(yb + (((((k1 >> G::LR) << G::LOGL2) + n2) << G::LR) + (k1 & ((1 << G::LR) - 1))));
   };
   constexpr int L1r = G::LOGR1;
   if constexpr (G::R2 == 1 && G::R3 == 1) {
@@ -449,26 +490,26 @@ __global__ void __launch_bounds__(PairShape<LOGL, LOGT>::NT, PairShape<LOGL, LOG
     for (int r = 0; r < (HALF ? 8 : 16); ++r) st.put(sctx, batch, k10 + rr, j + r * (G::L2 / 16), v[r]);
   } else {
     // first stage
-    constexpr int R = G::R1, PT = 16 / R;
+    constexpr int R = G::R1, PT = G::EB / R;
     P2 v[PT][R];
     int j[PT], rr[PT];
 #pragma unroll
-    for (int p = 0; p < PT; ++p) pair_stage_load<SIGN, R, 0, G>(from_y, tws, t + p * G::NT, j[p], rr[p], v[p]);
+    for (int p = 0; p < PT; ++p) pair_stage_load<SIGN, R, 0, G>(from_y, tws, t + p * G::NB, j[p], rr[p], v[p]);
 #pragma unroll
     for (int p = 0; p < PT; ++p)
 #pragma unroll
       for (int r = 0; r < R; ++r) pst(s + at(j[p] * R + r, rr[p]), v[p][r]);
 #pragma unroll
     for (int k = 0; k < NTW; ++k)
-      if (t + k * G::NT < G::TW) tws[t + k * G::NT] = twv[k];
+      if (t + k * G::NB < G::TW) tws[t + k * G::NB] = twv[k];
     __syncthreads();
   }
   if constexpr (G::R2 > 1) {
-    constexpr int R = G::R2, PT = 16 / R, Ns = 1 << L1r;
+    constexpr int R = G::R2, PT = G::EB / R, Ns = 1 << L1r;
     P2 v[PT][R];
     int j[PT], rr[PT];
 #pragma unroll
-    for (int p = 0; p < PT; ++p) pair_stage_load<SIGN, R, L1r, G>(from_smem, tws, t + p * G::NT, j[p], rr[p], v[p]);
+    for (int p = 0; p < PT; ++p) pair_stage_load<SIGN, R, L1r, G>(from_smem, tws, t + p * G::NB, j[p], rr[p], v[p]);
     __syncthreads();
 #pragma unroll
     for (int p = 0; p < PT; ++p) {
@@ -479,14 +520,14 @@ __global__ void __launch_bounds__(PairShape<LOGL, LOGT>::NT, PairShape<LOGL, LOG
     __syncthreads();
   }
   if constexpr (G::R3 > 1) {
-    constexpr int R = G::R3, PT = 16 / R;
-    constexpr int LOGNS = G::LOGL2 - (R == 16 ? 4 : (R == 8 ? 3 : (R == 4 ? 2 : 1))), Ns = 1 << LOGNS;
+    constexpr int R = G::R3, PT = G::EB / R;
+    constexpr int LOGNS = G::LOGL2 - (R == 32 ? 5 : (R == 16 ? 4 : (R == 8 ? 3 : (R == 4 ? 2 : 1)))), Ns = 1 << LOGNS;
     const float2* tw = tws + (G::R2 > 1 ? G::R1 * G::R2 : 0);
 #pragma unroll
     for (int p = 0; p < PT; ++p) {
       P2 v[R];
       int j, rr;
-      pair_stage_load<SIGN, R, LOGNS, G>(from_smem, tw, t + p * G::NT, j, rr, v);
+      pair_stage_load<SIGN, R, LOGNS, G, HALF>(from_smem, tw, t + p * G::NB, j, rr, v);
 #pragma unroll
       for (int r = 0; r < (HALF ? R / 2 : R); ++r) st.put(sctx, batch, k10 + rr, j + r * Ns, v[r]);
     }
