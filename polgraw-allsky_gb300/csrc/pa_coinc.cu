@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kT) k_cells(const double* __restrict__ rec,
                                               const __grid_constant__ CellArgs a,
                                               int4* __restrict__ cells_raw, uint8_t* __restrict__ flag,
                                               unsigned* __restrict__ blk_cnt, int* __restrict__ minmax,
-                                              unsigned* __restrict__ nexact) {
+                                              unsigned* __restrict__ nexact, double* __restrict__ snr_raw) {
   __shared__ unsigned sh[kT / 32];
   __shared__ int smm[8];
   __shared__ unsigned short list[kTile];
@@ -331,6 +331,7 @@ __global__ void __launch_bounds__(kT) k_cells(const double* __restrict__ rec,
     int4 cl = make_int4(0, 0, 0, 0);
     const int ok = cell_of(c0, c1, c2, c3, c4, fshift, a, &cl);
     flag[r] = ok != 0;
+    snr_raw[r] = c4;
     cnt += ok != 0;
     if (ok == 2) {
       list[atomicAdd(&nlist, 1u)] = (unsigned short)(it * kT + threadIdx.x);
@@ -417,7 +418,8 @@ template <typename K>
 __global__ void __launch_bounds__(kT) k_inband(const uint8_t* __restrict__ flag, const int4* __restrict__ cells_raw,
                                                const unsigned* __restrict__ blk_off, KeyLayout L,
                                                unsigned* __restrict__ rawidx, int4* __restrict__ cells_in,
-                                               K* __restrict__ key, unsigned* __restrict__ val) {
+                                               K* __restrict__ key, unsigned* __restrict__ val,
+                                               const double* __restrict__ snr_raw, double* __restrict__ snr_in) {
   __shared__ unsigned sh[kT / 32];
   __shared__ unsigned short list[kTile];
   const int b = blockIdx.x;
@@ -433,6 +435,7 @@ __global__ void __launch_bounds__(kT) k_inband(const uint8_t* __restrict__ flag,
     cells_in[o] = cl;
     key[o] = make_key<K>(cl, L);
     val[o] = o;
+    snr_in[o] = snr_raw[r];
   }
 }
 
@@ -821,15 +824,19 @@ __device__ __forceinline__ FrameDrop frame_drop(const FrameReq& rq, const FrameF
 // ---- duplicate removal per (cells, frame) run ------------------------------
 
 // A tile of kTile records a block, with its neighbours, in shared memory: keys
-// and frames.  Nearly every record is a run of its own and is settled there;
-// the others walk their run in global memory.  removed[f]: records of frame f
-// that are not kept.  (4.7 million records: 59 us, 67 us with a thread per
-// record that searched its neighbours' frames again.)
+// and frames.  A record that is a run of its own is settled there; the first
+// records of longer runs go on a list, whose runs are then shared out among
+// the threads, the SNRs of four members in flight at a time.  removed[f]:
+// records of frame f that are not kept.  24 x 2^18 records, few duplicates (50
+// 000 of 4.7 million) and many (lattice points on 64 lines x 256 positions): 67
+// and 94 us with a thread per record and SNRs from a compact array; 41 and
+// 55 us here (303 with the runs walked by the threads that found them).
 template <typename K>
 __global__ void __launch_bounds__(kT) k_dedup(const K* __restrict__ key, const unsigned* __restrict__ val,
-                                              const unsigned* __restrict__ rawidx, const double* __restrict__ rec,
-                                              const FrameReq* __restrict__ req, const FrameFound* __restrict__ found,
-                                              long long n, uint8_t* __restrict__ keep, unsigned* __restrict__ removed) {
+                                              const double* __restrict__ snr_in, const FrameReq* __restrict__ req,
+                                              const FrameFound* __restrict__ found, long long n, uint8_t* __restrict__ keep, unsigned* __restrict__ removed) {
+  __shared__ unsigned short list[kTile];
+  __shared__ unsigned nlist, hcount[256];
   __shared__ K s_key[kTile + 2];
   __shared__ uint8_t s_frame[kTile + 2];
   __shared__ FrameDrop s_drop[kMaxFrames];
@@ -845,6 +852,8 @@ __global__ void __launch_bounds__(kT) k_dedup(const K* __restrict__ key, const u
       v[k] = val[i];
     }
   }
+  if (threadIdx.x == 0) nlist = 0;
+  hcount[threadIdx.x] = 0;
   if (threadIdx.x < c_ft.nframes) s_drop[threadIdx.x] = frame_drop(req[threadIdx.x], found[threadIdx.x]);
   load_in_start(s_in);
   const int nf = c_ft.nframes;
@@ -858,7 +867,6 @@ __global__ void __launch_bounds__(kT) k_dedup(const K* __restrict__ key, const u
     }
   }
   __syncthreads();
-  auto snr = [&](unsigned v) { return rec[5 * (long long)rawidx[v] + 4]; };
 #pragma unroll
   for (int k = 0; k < kIt; k++) {
     const int li = 1 + k * kT + threadIdx.x;
@@ -869,41 +877,63 @@ __global__ void __launch_bounds__(kT) k_dedup(const K* __restrict__ key, const u
     if (i > 0 && s_key[li - 1] == k0 && s_frame[li - 1] == f) continue;  // not the first of its run
     const bool dropped = s_drop[f].drop && key_is(k0, s_drop[f].lo, s_drop[f].hi);
     const bool single = !(i + 1 < n && s_key[li + 1] == k0 && s_frame[li + 1] == f);
-    if (single && !dropped) {
-      keep[i] = 1;
-      continue;
-    }
-    // the run [i, j]
-    long long j = i;
-    while (j + 1 < n && key[j + 1] == k0 && frame_of_in(val[j + 1], s_in, nf) == f) j++;
-    atomicAdd(&removed[f], (unsigned)(j - i + (dropped ? 1 : 0)));
+    if (single && !dropped) keep[i] = 1;
+    else list[atomicAdd(&nlist, 1u)] = (unsigned short)li;
+  }
+  __syncthreads();
+  const unsigned nl = nlist;
+  for (unsigned q = threadIdx.x; q < nl; q += kT) {
+    const int li = list[q];
+    const long long i = t0 + li - 1;
+    const K k0 = s_key[li];
+    const int f = s_frame[li];
+    // the run [i, j], within the tile and then beyond it
+    int le = li;
+    while (le <= kTile && t0 + le < n && s_key[le + 1] == k0 && s_frame[le + 1] == f) le++;
+    long long j = t0 + le - 1;
+    if (le > kTile)
+      while (j + 1 < n && key[j + 1] == k0 && frame_of_in(val[j + 1], s_in, nf) == f) j++;
+    const bool dropped = s_drop[f].drop && key_is(k0, s_drop[f].lo, s_drop[f].hi);
+    atomicAdd(&hcount[f], (unsigned)(j - i + (dropped ? 1 : 0)));
     if (dropped) continue;
     // coincidences.c:317-413 over the pairs (t, t + 1) of the run
     const long long fs = s_in[f];
-    long long maxsnridx = 0, maxi = i;
-    double candsnr = 0;
-    unsigned vt = val[i];
-    double s0 = snr(vt);
-    for (long long t = i; t < j; t++) {
-      const unsigned vt1 = val[t + 1];
-      const double s1 = snr(vt1);
-      const long long idx = (long long)vt - fs, idx1 = (long long)vt1 - fs;
-      if (!maxsnridx) {
-        maxsnridx = (s0 > s1) ? idx : idx1;
-        maxi = (s0 > s1) ? t : t + 1;
-        candsnr = (s0 > s1) ? s0 : s1;
-      } else {
-        if (s0 > candsnr) {
-          maxsnridx = idx; maxi = t; candsnr = s0;
-        } else if (s1 > candsnr) {
-          maxsnridx = idx1; maxi = t + 1; candsnr = s1;
+    long long maxsnridx = 0, maxi = i, idx = 0;
+    double candsnr = 0, s0 = 0;
+    for (long long t4 = i; t4 <= j; t4 += 4) {
+      unsigned v4[4];
+      double s4[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) v4[u] = t4 + u <= j ? val[t4 + u] : 0u;
+#pragma unroll
+      for (int u = 0; u < 4; u++) s4[u] = t4 + u <= j ? snr_in[v4[u]] : 0.;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const long long t1 = t4 + u;  // the pair (t1 - 1, t1)
+        if (t1 > j) break;
+        const double s1 = s4[u];
+        const long long idx1 = (long long)v4[u] - fs;
+        if (t1 > i) {
+          if (!maxsnridx) {
+            maxsnridx = (s0 > s1) ? idx : idx1;
+            maxi = (s0 > s1) ? t1 - 1 : t1;
+            candsnr = (s0 > s1) ? s0 : s1;
+          } else {
+            if (s0 > candsnr) {
+              maxsnridx = idx; maxi = t1 - 1; candsnr = s0;
+            } else if (s1 > candsnr) {
+              maxsnridx = idx1; maxi = t1; candsnr = s1;
+            }
+          }
         }
+        idx = idx1;
+        s0 = s1;
       }
-      vt = vt1;
-      s0 = s1;
     }
     keep[maxsnridx ? maxi : j] = 1;
   }
+  __syncthreads();
+  if (hcount[threadIdx.x]) atomicAdd(&removed[threadIdx.x], hcount[threadIdx.x]);
 }
 
 // keep flags by in-band index, from the flags by sorted position
@@ -1025,71 +1055,73 @@ __global__ void k_gather_w(const unsigned* __restrict__ order, const unsigned* _
   if (q < K) w_sorted[q] = cw[order[q]];
 }
 
-// coincidences.c:488-525: means over the members k = end, end - 1, ...  One
-// warp per coincidence loads 32 members at once (a thread per coincidence
-// spent 60 us on 12 000 of them, one dependent load after the other); the sums
-// then run in the reference's order, a thread per coincidence and column (all
-// lanes adding the same numbers spent 68 us in the FP64 pipe).
+// coincidences.c:488-525: means over the members k = end, end - 1, ...  A block
+// takes kG coincidences, whose members lie one after the other in the output:
+// a thread per member loads and shifts it (a thread per coincidence spent 60 us
+// on 12 000 of them, one dependent load after the other), then a thread per
+// coincidence and column adds in the reference's order.  (A warp per
+// coincidence leaves most lanes of the FP64 pipe idle: 257 000 coincidences 287
+// us, 136 with a thread each, 157 here; 12 000: 31, 76 and 31 us.)
+constexpr int kG = 32;
 __global__ void __launch_bounds__(kT) k_means(const unsigned* __restrict__ order, const unsigned* __restrict__ cend,
                                               const unsigned* __restrict__ cw, const unsigned* __restrict__ first,
                                               int K, const unsigned* __restrict__ sval,
                                               const unsigned* __restrict__ rawidx, const double* __restrict__ rec,
                                               double N, int refr, pa_coinc_rec* __restrict__ out,
                                               int* __restrict__ fra, int* __restrict__ ops) {
-  constexpr int kG = kT / 32;
   __shared__ unsigned s_in[kMaxFrames + 1];
-  __shared__ double s_t[kG][32][5];
-  __shared__ int s_w[kG];
+  __shared__ double s_t[5][kT];
+  __shared__ unsigned s_first[kG + 1], s_end[kG];
+  const int q0 = blockIdx.x * kG, nq = min(kG, K - q0);
+  if (threadIdx.x < nq) {
+    const unsigned g = order[q0 + threadIdx.x], f = first[q0 + threadIdx.x], w = cw[g];
+    s_first[threadIdx.x] = f;
+    s_end[threadIdx.x] = cend[g];
+    if (threadIdx.x == nq - 1) s_first[nq] = f + w;
+  }
   load_in_start(s_in);
   const int nf = c_ft.nframes;
-  const int lane = threadIdx.x & 31, gr = threadIdx.x >> 5;
-  const int q = blockIdx.x * kG + gr;
-  long long j = 0, m0 = 0;
-  int w = 0;
-  if (q < K) {
-    const unsigned g = order[q];
-    j = cend[g];
-    w = (int)cw[g];
-    m0 = first[q];
-  }
-  if (lane == 0) s_w[gr] = w;
-  __syncthreads();
-  int wmax = 0;
-  for (int k = 0; k < kG; k++) wmax = max(wmax, s_w[k]);
+  const unsigned m0 = s_first[0], m1 = s_first[nq];
   const int sg = threadIdx.x / 5, sk = threadIdx.x % 5;  // the sum of this thread
   double m = 0;
-  for (int i0 = 0; i0 < wmax; i0 += 32) {
-    const int i = i0 + lane;
-    if (i < w) {
-      const unsigned v = sval[j - i];
+  for (unsigned c0 = m0; c0 < m1; c0 += kT) {
+    const unsigned mm = c0 + threadIdx.x;
+    if (mm < m1) {
+      int lo = 0, hi = nq;  // the member's coincidence: s_first[lo] <= mm < s_first[lo + 1]
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (s_first[mid] <= mm) lo = mid; else hi = mid;
+      }
+      const unsigned v = sval[s_end[lo] - (mm - s_first[lo])];
       const int f = frame_of_in(v, s_in, nf);
       const long long r = rawidx[v];
       const double* c = rec + 5 * r;
       const double fshift = (double)(refr - c_ft.frame_no[f]);
-      double* t = s_t[gr][lane];
-      t[0] = __dadd_rn(c[0], __dmul_rn(__dmul_rn(__dmul_rn(2., c[1]), N), fshift));
-      t[1] = c[1];
-      t[2] = c[2];
-      t[3] = c[3];
-      t[4] = __dmul_rn(c[4], c[4]);
-      ops[m0 + i] = (int)(r - c_ft.raw_start[f]);
-      fra[m0 + i] = c_ft.frame_no[f];
+      s_t[0][threadIdx.x] = __dadd_rn(c[0], __dmul_rn(__dmul_rn(__dmul_rn(2., c[1]), N), fshift));
+      s_t[1][threadIdx.x] = c[1];
+      s_t[2][threadIdx.x] = c[2];
+      s_t[3][threadIdx.x] = c[3];
+      s_t[4][threadIdx.x] = __dmul_rn(c[4], c[4]);
+      ops[mm] = (int)(r - c_ft.raw_start[f]);
+      fra[mm] = c_ft.frame_no[f];
     }
     __syncthreads();
-    if (sg < kG) {
-      const int nl = min(32, s_w[sg] - i0);
-      for (int l = 0; l < nl; l++) m = __dadd_rn(m, s_t[sg][l][sk]);
+    if (sg < nq) {
+      const unsigned a = max(s_first[sg], c0), b = min(s_first[sg + 1], c0 + kT);
+      for (unsigned l = a; l < b; l++) m = __dadd_rn(m, s_t[sk][l - c0]);
     }
     __syncthreads();
   }
-  const int sq = blockIdx.x * kG + sg;
-  if (sg >= kG || sq >= K) return;
-  out[sq].mean[sk] = sk < 4 ? __ddiv_rn(m, (double)s_w[sg]) : __dsqrt_rn(m);
+  if (sg >= nq) return;
+  const int w = (int)(s_first[sg + 1] - s_first[sg]);
+  pa_coinc_rec* o = out + q0 + sg;
+  o->mean[sk] = sk < 4 ? __ddiv_rn(m, (double)w) : __dsqrt_rn(m);
   if (sk == 0) {
-    out[sq].w = s_w[sg];
-    out[sq].first = (int)first[sq];
+    o->w = w;
+    o->first = (int)s_first[sg];
   }
 }
+static_assert(5 * kG <= kT, "a thread per sum");
 
 }  // namespace
 
@@ -1113,7 +1145,7 @@ struct pa_coinc {
     void* p = nullptr;
     size_t n = 0;
   };
-  Buf rec, cells_raw, flag, blkcnt, scan_tmp, minmax, rawidx, cells_in, digits, keyA, keyB, valA, valB, hist,
+  Buf rec, cells_raw, flag, snr_raw, blkcnt, scan_tmp, minmax, rawidx, cells_in, snr_in, digits, keyA, keyB, valA, valB, hist,
       keep, keep_in, uniq, req, found, skey, sval, gflag, gend, gw, lastu, wkeyA, wkeyB, cend, cw, cidxA, cidxB,
       wsort, means, fra, ops;
   // optional per-kernel profile: events around each launch while on
@@ -1376,8 +1408,8 @@ void pa_coinc_destroy(pa_coinc* c) {
   if (!c) return;
   cudaSetDevice(c->cfg.device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  pa_coinc::Buf* bufs[] = {&c->rec, &c->cells_raw, &c->flag, &c->blkcnt, &c->scan_tmp, &c->minmax, &c->rawidx,
-                           &c->cells_in, &c->digits, &c->keyA, &c->keyB, &c->valA, &c->valB, &c->hist, &c->keep,
+  pa_coinc::Buf* bufs[] = {&c->rec, &c->cells_raw, &c->flag, &c->snr_raw, &c->blkcnt, &c->scan_tmp, &c->minmax, &c->rawidx,
+                           &c->cells_in, &c->snr_in, &c->digits, &c->keyA, &c->keyB, &c->valA, &c->valB, &c->hist, &c->keep,
                            &c->keep_in, &c->uniq, &c->req, &c->found, &c->skey, &c->sval, &c->gflag, &c->gend,
                            &c->gw, &c->lastu, &c->wkeyA, &c->wkeyB, &c->cend, &c->cw, &c->cidxA, &c->cidxB,
                            &c->wsort, &c->means, &c->fra, &c->ops};
@@ -1451,6 +1483,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   pa::TraceRange trace_("coinc sort, duplicates, coincidences");
   const int nf = (int)c->frames.size();
   const long long n = c->n_in;
+  ENS(snr_in, sizeof(double) * n);
   ENS(keyA, sizeof(K) * n);
   ENS(keyB, sizeof(K) * n);
   ENS(valA, sizeof(unsigned) * n);
@@ -1459,7 +1492,8 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
     Span sp_(c, CK_INBAND);
     k_inband<K><<<nblk1, kT, 0, c->stream>>>(P<uint8_t>(c->flag), P<int4>(c->cells_raw), P<unsigned>(c->blkcnt), L,
                                              P<unsigned>(c->rawidx), P<int4>(c->cells_in),
-                                             P<K>(c->keyA), P<unsigned>(c->valA));
+                                             P<K>(c->keyA), P<unsigned>(c->valA), P<double>(c->snr_raw),
+                                             P<double>(c->snr_in));
   }
   c->launches++;
   CCK(cudaGetLastError(), "k_inband");
@@ -1514,7 +1548,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   {
     Span sp_(c, CK_DEDUP);
     k_dedup<K><<<(unsigned)((n + kTile - 1) / kTile), kT, 0, c->stream>>>(
-        key, val, P<unsigned>(c->rawidx), P<double>(c->rec), P<FrameReq>(c->req), P<FrameFound>(c->found), n,
+        key, val, P<double>(c->snr_in), P<FrameReq>(c->req), P<FrameFound>(c->found), n,
         P<uint8_t>(c->keep), P<unsigned>(c->uniq));
   }
   c->launches++;
@@ -1623,7 +1657,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
     ENS(ops, sizeof(int) * (M + 1));
     {
       Span sp_(c, CK_MEANS);
-      k_means<<<(Kc + kT / 32 - 1) / (kT / 32), kT, 0, c->stream>>>(order, P<unsigned>(c->cend), P<unsigned>(c->cw),
+      k_means<<<(Kc + kG - 1) / kG, kT, 0, c->stream>>>(order, P<unsigned>(c->cend), P<unsigned>(c->cw),
                                                         P<unsigned>(c->wsort), (int)Kc, P<unsigned>(c->sval),
                                                         P<unsigned>(c->rawidx), P<double>(c->rec),
                                                         (double)c->cfg.N, c->cfg.refr, P<pa_coinc_rec>(c->means),
@@ -1754,6 +1788,7 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
     }
     ENS(cells_raw, sizeof(int4) * c->nraw);
     ENS(flag, c->nraw);
+    ENS(snr_raw, sizeof(double) * c->nraw);
     ENS(blkcnt, sizeof(unsigned) * (nblk1 + 1));
     ENS(scan_tmp, sizeof(unsigned) * scan_tmp_len(nblk1 + 1));
     ENS(minmax, sizeof(int) * 9);
@@ -1763,7 +1798,7 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
       Span sp_(c, CK_CELLS);
       k_cells<<<nblk1, kT, 0, c->stream>>>(P<double>(c->rec), a, P<int4>(c->cells_raw), P<uint8_t>(c->flag),
                                           P<unsigned>(c->blkcnt), P<int>(c->minmax),
-                                          (unsigned*)(P<int>(c->minmax) + 8));
+                                          (unsigned*)(P<int>(c->minmax) + 8), P<double>(c->snr_raw));
     }
     c->launches++;
     CCK(cudaGetLastError(), "k_cells");
