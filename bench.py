@@ -131,7 +131,7 @@ def l2_flush():
 # N=86164, nfftf=131072) from an ncu capture of the current kernel, per
 # schedule (spindowns per launch, FFT split); scaled by the spindowns of a
 # launch.  Schedules without a capture of the current kernel report null.
-PASS_A_TRAFFIC_PER_SPINDOWN = {(32, 1): 14.21e6 / 32}
+PASS_A_TRAFFIC_PER_SPINDOWN = {(32, 0): 16.04e6 / 32}
 
 
 def peaks() -> dict:
@@ -478,9 +478,8 @@ def run_coinc(args, L):
     tot = sum(v[0] for v in prof.values())
     roof = {"bound": "hbm", "kernel": "coinc_cells", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
             "frac": achieved / pk["hbm_gbs"], "traffic": None,
-            "note": "57 B per record; the kernel is bound by the FP64 pipe (frequency and spindown terms and "
-                    "the rounding test in FP64, sky terms in FP32 with an FP64 recomputation near cell edges), "
-                    "not by HBM",
+            "note": "57 B per record; the kernel is bound by instruction issue (two sincosf a record, "
+                    "float-float frequency and spindown terms, FP64 cells near cell edges only), not by HBM",
             "peak_source": pk["source"] + " (MEASURED_PEAKS.json hbm_gbs)", "avg_launch_ms": per_launch,
             "units_per_launch": nrec}
     # end to end: upload, run, results back
@@ -905,7 +904,7 @@ def main():
                            if (name == "spindown_pass_a" and s.N == 86164 and nifo == 2
                                and tuple(sched[:2]) in PASS_A_TRAFFIC_PER_SPINDOWN) else None,
                            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per launch "
-                                             "(profiles/spindown_pass_a_network_n86164.md)",
+                                             "(profiles/search_kernels.md)",
                            "peak_source": pk["source"] + " (MEASURED_PEAKS.json hbm_gbs)",
                            "avg_launch_ms": ms / max(1, nl), "units_per_launch": items / max(1, nl)}
         out["kernel_share"] = {k: round(v[0] / tot, 4) for k, v in sorted(prof.items(), key=lambda kv: -kv[1][0])}

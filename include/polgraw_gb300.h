@@ -247,19 +247,19 @@ int pa_cta_trace_count(pa_ctx *ctx, unsigned int *n);
  * ------------------------------------------------------------------------ */
 
 /* CUDA graphs on/off (default off): when on, each pa_search_batch /
- * pa_job_core call captures its launches (both streams) into a CUDA graph,
- * updated in place when the next call has the same launch structure, and
- * launches it once.  Results are identical either way. */
+ * pa_job_core call launches its first sky point directly and captures the
+ * others in parts of 2, 4, 8 .. 256 sky points, each into its own CUDA graph
+ * (updated in place when the next call has the same launch structure) that is
+ * launched as soon as it is captured.  Results are identical either way. */
 int pa_set_graphs(pa_ctx *ctx, int on);
 
 /* Spindown-loop schedule: spindowns per fused launch (1 .. *max_sbatch, the
  * batch the buffers were sized for, four times the automatic default; a
  * batch above *max_sbatch / 2 selects one lane, see pa_set_lanes) and the
  * factor split of the spindown FFT (0: L1 = 2^ceil(m/2); 1: swapped
- * factors, different radix schedule of the two passes; for odd
- * m = log2(nfftf) only, ignored otherwise; default 0, except 1 for two
- * detectors in the FP32 forms with nfftf = 2^17, whose 256-point columns
- * take the radix-16 pass A). */
+ * factors; for odd m = log2(nfftf) only, ignored otherwise; default 0).  The
+ * split is the FP64 form's: the FP32 forms have one factorisation, 256-point
+ * columns, and only keep the value. */
 int pa_set_schedule(pa_ctx *ctx, int sbatch, int split);
 int pa_get_schedule(const pa_ctx *ctx, int *sbatch, int *split, int *max_sbatch);
 
@@ -280,16 +280,17 @@ int pa_get_lanes(const pa_ctx *ctx, int *lanes);
  * warm-up, CUDA-event device time) and keeps the fastest; returns it in
  * *sbatch, *split (either may be NULL; the lane count it picked is read
  * with pa_get_lanes).  Results do not depend on sbatch or the lanes; the
- * split changes FFT rounding only. */
+ * split changes FFT rounding only (FP64 form). */
 int pa_autotune(pa_ctx *ctx, const pa_sky *tasks, int ntasks, const pa_opts *opts, const pa_range *s_range,
                 int *sbatch, int *split);
 
 /* Several data segments searched together: one context per segment (own
  * N, FFT lengths, data), their batches enqueued at once on their own
  * streams, forked from one origin stream, so that the GPU runs them
- * concurrently; with the graph on (default) the whole multi-segment
- * workload is captured into one CUDA graph (updated in place on the next
- * call with the same launch structure) and launched once. */
+ * concurrently; with the graph on (default) the first sky point of every
+ * segment is launched directly and the others in captured parts of 2, 4, 8 ..
+ * sky points of every segment, each part one CUDA graph (updated in place on
+ * the next call with the same launch structure). */
 typedef struct pa_segments pa_segments;
 
 /* One segment's batch: the arguments of pa_search_batch() for context k. */
