@@ -174,6 +174,28 @@ static void pair_twiddle(long m, long n, float* w) {
   w[1] = (float)im;
 }
 
+// The same values from one octant, computed once for the longest transform:
+// oct[2 i], oct[2 i + 1] = cos, sin of 2 pi i / n for i <= n / 8, n a power of two
+// and a multiple of every length asked for.  (The tables of a context hold
+// every factor of its transforms: two libm calls an entry were most of the
+// time that a context of a short segment took to make.)
+static void octant_fill(long n, float* oct) {
+  for (long i = 0; i <= n / 8; i++) {
+    const double a = (double)(8 * i) / (double)n * (M_PI / 4.0);
+    oct[2 * i] = (float)cos(a);
+    oct[2 * i + 1] = (float)sin(a);
+  }
+}
+static void octant_twiddle(const float* oct, long n, long m, long den, float* w) {
+  const long m8 = 8 * ((m % den) * (n / den)), o = m8 / n, rem = m8 - o * n;
+  const float* p = oct + 2 * (((o & 1) ? n - rem : rem) / 8);
+  const float ca = p[0], sa = p[1];
+  const float co = (o == 0 || o == 7) ? ca : (o == 1 || o == 6) ? sa : (o == 2 || o == 5) ? -sa : -ca;
+  const float si = (o == 0 || o == 3) ? sa : (o == 1 || o == 2) ? ca : (o == 4 || o == 7) ? -sa : -ca;
+  w[0] = co;
+  w[1] = -si;
+}
+
 static int ilog2(long n) {
   int m = 0;
   while ((1L << m) < n) ++m;
@@ -372,6 +394,9 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
   } else {
     const int lens[2] = {s.nfft, s.nfftf};
     std::vector<float> v(512);
+    const long no = std::max(s.nfft, s.nfftf);
+    std::vector<float> oct(2 * (size_t)(no / 8 + 1));
+    octant_fill(no, oct.data());
     auto up = [&](const void** dst) -> int {
       void* p = nullptr;
       if (int r = dalloc(c, &p, v.size() * sizeof(float))) return r;
@@ -379,7 +404,7 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
       *dst = p;
       return PA_OK;
     };
-    for (int m = 0; m < 256; m++) pair_twiddle(m, 256, &v[2 * m]);
+    for (int m = 0; m < 256; m++) octant_twiddle(oct.data(), no, m, 256, &v[2 * m]);
     if ((rc = up(&b.pair_tw1))) return rc;
     for (int t = 0; t < 2; t++) {
       if (t == 1 && s.nfftf == s.nfft) {
@@ -389,10 +414,11 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
       }
       const int lg = ilog2(lens[t]);
       v.resize(2 * (size_t)pa::pair_row_table(lg));
-      for (int j = 0; j < pa::pair_row_table(lg); j++) pair_twiddle(pa::pair_row_exp(j, lg), lens[t] / 256, &v[2 * j]);
+      for (int j = 0; j < pa::pair_row_table(lg); j++)
+        octant_twiddle(oct.data(), no, pa::pair_row_exp(j, lg), lens[t] / 256, &v[2 * j]);
       if ((rc = up(&b.pair_row[t]))) return rc;
       v.resize(2 * (size_t)lens[t]);
-      for (long j = 0; j < lens[t]; j++) pair_twiddle(pa::pair_pass_exp(j, lg), lens[t], &v[2 * j]);
+      for (long j = 0; j < lens[t]; j++) octant_twiddle(oct.data(), no, pa::pair_pass_exp(j, lg), lens[t], &v[2 * j]);
       if ((rc = up(&b.pair_pass[t]))) return rc;
     }
   }
@@ -1383,11 +1409,14 @@ size_t noalloc_layout(char* base, const pa_settings& s, int nifo, pa::Buffers* b
 }
 
 // n twiddles exp(-2 pi i m(j) / den) (conjugated for sign > 0) to device
-// memory, through the static host staging array.
+// memory, through the static host staging array; from the octant of the longest
+// length where den divides it.
+float g_noalloc_oct[2 * (kNoAllocMaxNfftf / 8 + 1)];
 template <class Exp>
 cudaError_t noalloc_twiddles(const void* dst, long n, long den, int sign, cudaStream_t st, Exp m) {
   for (long j = 0; j < n; j++) {
-    pair_twiddle(m(j), den, &g_noalloc_tw[2 * j]);
+    if (den <= kNoAllocMaxNfftf) octant_twiddle(g_noalloc_oct, kNoAllocMaxNfftf, m(j), den, &g_noalloc_tw[2 * j]);
+    else pair_twiddle(m(j), den, &g_noalloc_tw[2 * j]);
     if (sign > 0) g_noalloc_tw[2 * j + 1] = -g_noalloc_tw[2 * j + 1];
   }
   cudaError_t e = cudaMemcpyAsync((void*)dst, g_noalloc_tw, sizeof(float) * 2 * n, cudaMemcpyHostToDevice, st);
@@ -1483,6 +1512,7 @@ extern "C" int pa_fstat_noalloc(const pa_settings* sett, const pa_detector* det,
     NCK(cudaStreamSynchronize(st), "upload");  // the staging array is reused
   }
   b.spl = pa::spline_taps();
+  if (g_noalloc_oct[0] == 0.f) octant_fill(kNoAllocMaxNfftf, g_noalloc_oct);  // (the same for every call; under the mutex)
   NCK(noalloc_twiddles(b.pair_tw1, 256, 256, -1, st, [](long j) { return j; }), "twiddles");
   NCK(noalloc_twiddles(b.tw_inv[2], 1024, sett->Ninterp, +1, st, [](long j) { return j; }), "twiddles");
   NCK(noalloc_twiddles(b.tw_inv[3], sett->Ninterp / 1024, sett->Ninterp, +1, st, [](long j) { return 1024 * j; }),
