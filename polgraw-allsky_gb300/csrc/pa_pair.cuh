@@ -15,7 +15,7 @@
 //   pass A: per column n2, Y[k1, n2] = W_L^{n2 k1} sum_n1 x[L2 n1 + n2] W_256^{n1 k1}
 //   pass B: per row k1,    X[k1 + 256 k2] = sum_n2 Y[k1, n2] W_L2^{n2 k2}
 // A CTA transforms a tile of T = 2^LOGT pairs with T/16 threads, 16 pairs a
-// thread (64 registers of data at 128 a thread):
+// thread (64 registers of data at 128 a thread; pass B at 2^17 32 pairs a thread):
 //   pass A: T/256 columns as 16 x 16, one exchange through shared memory;
 //   pass B: T/L2 rows in two or three stages of radix 8, 16 or 32.
 // 128 registers at half the warps hold the same data as 64 registers did at
