@@ -53,14 +53,16 @@ constexpr int kIt = 8;                  // items per thread (tiles of 2048)
 constexpr int kTile = kT * kIt;
 constexpr int kRTile = 4096;            // radix tile (items per block)
 
+// The frames of one run.  The kernels take it by value (4 KB of parameters), so
+// that every launch keeps the table of its own handle and run: handles run on
+// streams of their own, and a table in a device symbol would be one for all.
 struct FrameTab {
   int nframes;
   int frame_no[kMaxFrames];
-  long long raw_start[kMaxFrames + 1];   // first raw record of each frame
+  unsigned raw_start[kMaxFrames + 1];    // first raw record of each frame (below 2^31 in all)
   int blk_start[kMaxFrames + 1];         // first k_cells block of each frame
-  long long in_start[kMaxFrames + 1];    // first in-band record of each frame
+  unsigned in_start[kMaxFrames + 1];     // first in-band record of each frame
 };
-__constant__ FrameTab c_ft;
 
 struct CellArgs {
   long long lo_k, hi_k;    // narrowdown band (pi/2 -+ narrowdown) and SNR cut as
@@ -121,11 +123,11 @@ struct KeyLayout {
   int bits;                // total key bits
 };
 
-__device__ __forceinline__ int frame_of_block(int b) {
-  int lo = 0, hi = c_ft.nframes;  // blk_start[lo] <= b < blk_start[hi]
+__device__ __forceinline__ int frame_of_block(const FrameTab& ft, int b) {
+  int lo = 0, hi = ft.nframes;  // blk_start[lo] <= b < blk_start[hi]
   while (hi - lo > 1) {
     int mid = (lo + hi) >> 1;
-    if (c_ft.blk_start[mid] <= b) lo = mid; else hi = mid;
+    if (ft.blk_start[mid] <= b) lo = mid; else hi = mid;
   }
   return lo;
 }
@@ -142,8 +144,8 @@ __device__ __forceinline__ int frame_of_in(unsigned v, const unsigned* s_in, int
   return lo;
 }
 
-__device__ __forceinline__ void load_in_start(unsigned* s_in) {
-  for (int k = threadIdx.x; k <= c_ft.nframes; k += blockDim.x) s_in[k] = (unsigned)c_ft.in_start[k];
+__device__ __forceinline__ void load_in_start(const FrameTab& ft, unsigned* s_in) {
+  for (int k = threadIdx.x; k <= ft.nframes; k += blockDim.x) s_in[k] = ft.in_start[k];
   __syncthreads();
 }
 
@@ -288,7 +290,7 @@ __device__ __forceinline__ unsigned tile_list(const uint8_t* __restrict__ flag, 
 // conversions and the FP64 cells in place (the FP64 pipe 80 % busy), 119 us now
 // (252 MB in and 107 MB out: 53 us at the copy rate; the rest is instruction
 // issue, two sincosf a record).
-__global__ void __launch_bounds__(kT) k_cells(const double* __restrict__ rec,
+__global__ void __launch_bounds__(kT) k_cells(const __grid_constant__ FrameTab ft, const double* __restrict__ rec,
                                               const __grid_constant__ CellArgs a,
                                               int4* __restrict__ cells_raw, uint8_t* __restrict__ flag,
                                               unsigned* __restrict__ blk_cnt, int* __restrict__ minmax,
@@ -298,10 +300,10 @@ __global__ void __launch_bounds__(kT) k_cells(const double* __restrict__ rec,
   __shared__ unsigned short list[kTile];
   __shared__ unsigned nlist;
   const int b = blockIdx.x;
-  const int f = frame_of_block(b);
-  const long long fend = c_ft.raw_start[f + 1];
-  const long long tile0 = c_ft.raw_start[f] + (long long)(b - c_ft.blk_start[f]) * kTile;
-  const double fshift = (double)(a.refr - c_ft.frame_no[f]);
+  const int f = frame_of_block(ft, b);
+  const long long fend = ft.raw_start[f + 1];
+  const long long tile0 = (long long)ft.raw_start[f] + (long long)(b - ft.blk_start[f]) * kTile;
+  const double fshift = (double)(a.refr - ft.frame_no[f]);
   if (threadIdx.x == 0) nlist = 0;
   if (threadIdx.x < 4) smm[threadIdx.x] = INT_MAX;
   else if (threadIdx.x < 8) smm[threadIdx.x] = INT_MIN;
@@ -415,7 +417,8 @@ __device__ __forceinline__ void key_split(const U128& k, unsigned long long* lo,
 
 // ordered compaction of the kept records, with their keys
 template <typename K>
-__global__ void __launch_bounds__(kT) k_inband(const uint8_t* __restrict__ flag, const int4* __restrict__ cells_raw,
+__global__ void __launch_bounds__(kT) k_inband(const __grid_constant__ FrameTab ft, const uint8_t* __restrict__ flag,
+                                               const int4* __restrict__ cells_raw,
                                                const unsigned* __restrict__ blk_off, KeyLayout L,
                                                unsigned* __restrict__ rawidx, int4* __restrict__ cells_in,
                                                K* __restrict__ key, unsigned* __restrict__ val,
@@ -423,10 +426,10 @@ __global__ void __launch_bounds__(kT) k_inband(const uint8_t* __restrict__ flag,
   __shared__ unsigned sh[kT / 32];
   __shared__ unsigned short list[kTile];
   const int b = blockIdx.x;
-  const int f = frame_of_block(b);
-  const long long tile0 = c_ft.raw_start[f] + (long long)(b - c_ft.blk_start[f]) * kTile;
+  const int f = frame_of_block(ft, b);
+  const long long tile0 = (long long)ft.raw_start[f] + (long long)(b - ft.blk_start[f]) * kTile;
   const unsigned base = blk_off[b];
-  const unsigned tot = tile_list(flag, tile0, c_ft.raw_start[f + 1], list, sh);
+  const unsigned tot = tile_list(flag, tile0, ft.raw_start[f + 1], list, sh);
   for (unsigned q = threadIdx.x; q < tot; q += kT) {
     const long long r = tile0 + list[q];
     const unsigned o = base + q;
@@ -599,7 +602,7 @@ __global__ void __launch_bounds__(kT) k_radix_hist(const K* __restrict__ key, lo
 }
 
 // digit = frame of the element (for the per-frame ranks of the sorted order)
-__global__ void __launch_bounds__(kT) k_frame_hist(const unsigned* __restrict__ val, long long n, int nblk,
+__global__ void __launch_bounds__(kT) k_frame_hist(const __grid_constant__ FrameTab ft, const unsigned* __restrict__ val, long long n, int nblk,
                                                    unsigned* __restrict__ hist) {
   __shared__ unsigned h[256];
   __shared__ unsigned s_in[kMaxFrames + 1];
@@ -608,8 +611,8 @@ __global__ void __launch_bounds__(kT) k_frame_hist(const unsigned* __restrict__ 
 #pragma unroll
   for (int k = 0; k < kRItems; k++) v[k] = t0 + k * kT < n ? val[t0 + k * kT] : 0u;
   h[threadIdx.x] = 0;
-  load_in_start(s_in);
-  const int nf = c_ft.nframes;
+  load_in_start(ft, s_in);
+  const int nf = ft.nframes;
 #pragma unroll
   for (int k = 0; k < kRItems; k++)
     if (t0 + k * kT < n) atomicAdd(&h[frame_of_in(v[k], s_in, nf)], 1u);
@@ -759,7 +762,8 @@ struct FrameFound {
 // one.  One block per request: 256-ary search over the frame's row of tile
 // offsets, then the place within the tile by a scan.
 template <typename K>
-__global__ void __launch_bounds__(kT) k_frame_find(const FrameReq* __restrict__ req, const unsigned* __restrict__ hoff,
+__global__ void __launch_bounds__(kT) k_frame_find(const __grid_constant__ FrameTab ft, const FrameReq* __restrict__ req,
+                                                   const unsigned* __restrict__ hoff,
                                                    int nblk, const unsigned* __restrict__ val, long long n,
                                                    const K* __restrict__ key, const int4* __restrict__ cells_in,
                                                    FrameFound* __restrict__ out, int* __restrict__ failed) {
@@ -769,8 +773,8 @@ __global__ void __launch_bounds__(kT) k_frame_find(const FrameReq* __restrict__ 
   const FrameReq rq = req[f];
   const int g = which ? rq.stale_frame : f, p = which ? rq.stale : rq.last;
   if (g < 0 || p < 0) return;
-  load_in_start(s_in);
-  const int nf = c_ft.nframes;
+  load_in_start(ft, s_in);
+  const int nf = ft.nframes;
   const unsigned* o = hoff + (long long)g * nblk;
   // last tile b with o[b] <= p (o[0] = 0)
   int lo = 0, hi = nblk;
@@ -832,7 +836,7 @@ __device__ __forceinline__ FrameDrop frame_drop(const FrameReq& rq, const FrameF
 // and 94 us with a thread per record and SNRs from a compact array; 41 and
 // 55 us here (303 with the runs walked by the threads that found them).
 template <typename K>
-__global__ void __launch_bounds__(kT) k_dedup(const K* __restrict__ key, const unsigned* __restrict__ val,
+__global__ void __launch_bounds__(kT) k_dedup(const __grid_constant__ FrameTab ft, const K* __restrict__ key, const unsigned* __restrict__ val,
                                               const double* __restrict__ snr_in, const FrameReq* __restrict__ req,
                                               const FrameFound* __restrict__ found, long long n, uint8_t* __restrict__ keep, unsigned* __restrict__ removed) {
   __shared__ unsigned short list[kTile];
@@ -854,9 +858,9 @@ __global__ void __launch_bounds__(kT) k_dedup(const K* __restrict__ key, const u
   }
   if (threadIdx.x == 0) nlist = 0;
   hcount[threadIdx.x] = 0;
-  if (threadIdx.x < c_ft.nframes) s_drop[threadIdx.x] = frame_drop(req[threadIdx.x], found[threadIdx.x]);
-  load_in_start(s_in);
-  const int nf = c_ft.nframes;
+  if (threadIdx.x < ft.nframes) s_drop[threadIdx.x] = frame_drop(req[threadIdx.x], found[threadIdx.x]);
+  load_in_start(ft, s_in);
+  const int nf = ft.nframes;
 #pragma unroll
   for (int k = 0; k < kIt; k++) s_frame[1 + k * kT + threadIdx.x] = (uint8_t)frame_of_in(v[k], s_in, nf);
   if (threadIdx.x < 2) {
@@ -1063,7 +1067,7 @@ __global__ void k_gather_w(const unsigned* __restrict__ order, const unsigned* _
 // coincidence leaves most lanes of the FP64 pipe idle: 257 000 coincidences 287
 // us, 136 with a thread each, 157 here; 12 000: 31, 76 and 31 us.)
 constexpr int kG = 32;
-__global__ void __launch_bounds__(kT) k_means(const unsigned* __restrict__ order, const unsigned* __restrict__ cend,
+__global__ void __launch_bounds__(kT) k_means(const __grid_constant__ FrameTab ft, const unsigned* __restrict__ order, const unsigned* __restrict__ cend,
                                               const unsigned* __restrict__ cw, const unsigned* __restrict__ first,
                                               int K, const unsigned* __restrict__ sval,
                                               const unsigned* __restrict__ rawidx, const double* __restrict__ rec,
@@ -1079,8 +1083,8 @@ __global__ void __launch_bounds__(kT) k_means(const unsigned* __restrict__ order
     s_end[threadIdx.x] = cend[g];
     if (threadIdx.x == nq - 1) s_first[nq] = f + w;
   }
-  load_in_start(s_in);
-  const int nf = c_ft.nframes;
+  load_in_start(ft, s_in);
+  const int nf = ft.nframes;
   const unsigned m0 = s_first[0], m1 = s_first[nq];
   const int sg = threadIdx.x / 5, sk = threadIdx.x % 5;  // the sum of this thread
   double m = 0;
@@ -1096,14 +1100,14 @@ __global__ void __launch_bounds__(kT) k_means(const unsigned* __restrict__ order
       const int f = frame_of_in(v, s_in, nf);
       const long long r = rawidx[v];
       const double* c = rec + 5 * r;
-      const double fshift = (double)(refr - c_ft.frame_no[f]);
+      const double fshift = (double)(refr - ft.frame_no[f]);
       s_t[0][threadIdx.x] = __dadd_rn(c[0], __dmul_rn(__dmul_rn(__dmul_rn(2., c[1]), N), fshift));
       s_t[1][threadIdx.x] = c[1];
       s_t[2][threadIdx.x] = c[2];
       s_t[3][threadIdx.x] = c[3];
       s_t[4][threadIdx.x] = __dmul_rn(c[4], c[4]);
-      ops[mm] = (int)(r - c_ft.raw_start[f]);
-      fra[mm] = c_ft.frame_no[f];
+      ops[mm] = (int)(r - (long long)ft.raw_start[f]);
+      fra[mm] = ft.frame_no[f];
     }
     __syncthreads();
     if (sg < nq) {
@@ -1490,7 +1494,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   ENS(valB, sizeof(unsigned) * n);
   {
     Span sp_(c, CK_INBAND);
-    k_inband<K><<<nblk1, kT, 0, c->stream>>>(P<uint8_t>(c->flag), P<int4>(c->cells_raw), P<unsigned>(c->blkcnt), L,
+    k_inband<K><<<nblk1, kT, 0, c->stream>>>(c->ft, P<uint8_t>(c->flag), P<int4>(c->cells_raw), P<unsigned>(c->blkcnt), L,
                                              P<unsigned>(c->rawidx), P<int4>(c->cells_in),
                                              P<K>(c->keyA), P<unsigned>(c->valA), P<double>(c->snr_raw),
                                              P<double>(c->snr_in));
@@ -1526,7 +1530,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   CCK(cudaMemcpyAsync(c->req.p, req.data(), sizeof(FrameReq) * nf, cudaMemcpyHostToDevice, c->stream), "copy");
   {
     Span sp_(c, CK_FRAME_RANK);
-    k_frame_hist<<<nblkR, kT, 0, c->stream>>>(val, n, nblkR, P<unsigned>(c->hist));
+    k_frame_hist<<<nblkR, kT, 0, c->stream>>>(c->ft, val, n, nblkR, P<unsigned>(c->hist));
   }
   {
     Span sp_(c, CK_SCAN);
@@ -1534,7 +1538,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   }
   {
     Span sp_(c, CK_FRAME_RANK);
-    k_frame_find<K><<<2 * nf, kT, 0, c->stream>>>(P<FrameReq>(c->req), P<unsigned>(c->hist), nblkR, val, n, key,
+    k_frame_find<K><<<2 * nf, kT, 0, c->stream>>>(c->ft, P<FrameReq>(c->req), P<unsigned>(c->hist), nblkR, val, n, key,
                                                   P<int4>(c->cells_in), P<FrameFound>(c->found),
                                                   (int*)(P<unsigned>(c->uniq) + 256));
   }
@@ -1548,7 +1552,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
   {
     Span sp_(c, CK_DEDUP);
     k_dedup<K><<<(unsigned)((n + kTile - 1) / kTile), kT, 0, c->stream>>>(
-        key, val, P<double>(c->snr_in), P<FrameReq>(c->req), P<FrameFound>(c->found), n,
+        c->ft, key, val, P<double>(c->snr_in), P<FrameReq>(c->req), P<FrameFound>(c->found), n,
         P<uint8_t>(c->keep), P<unsigned>(c->uniq));
   }
   c->launches++;
@@ -1657,7 +1661,7 @@ static int run_keyed(pa_coinc* c, const KeyLayout& L, int nblk1, std::vector<lon
     ENS(ops, sizeof(int) * (M + 1));
     {
       Span sp_(c, CK_MEANS);
-      k_means<<<(Kc + kG - 1) / kG, kT, 0, c->stream>>>(order, P<unsigned>(c->cend), P<unsigned>(c->cw),
+      k_means<<<(Kc + kG - 1) / kG, kT, 0, c->stream>>>(c->ft, order, P<unsigned>(c->cend), P<unsigned>(c->cw),
                                                         P<unsigned>(c->wsort), (int)Kc, P<unsigned>(c->sval),
                                                         P<unsigned>(c->rawidx), P<double>(c->rec),
                                                         (double)c->cfg.N, c->cfg.refr, P<pa_coinc_rec>(c->means),
@@ -1734,16 +1738,15 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
   int nblk1 = 0;
   for (int f = 0; f < nf; f++) {
     c->ft.frame_no[f] = c->frames[f];
-    c->ft.raw_start[f] = c->raw_start[f];
+    c->ft.raw_start[f] = (unsigned)c->raw_start[f];
     c->ft.blk_start[f] = nblk1;
     nblk1 += (int)((c->raw_start[f + 1] - c->raw_start[f] + kTile - 1) / kTile);
     c->frameinfo[3 * f] = c->frames[f];
   }
-  c->ft.raw_start[nf] = c->nraw;
+  c->ft.raw_start[nf] = (unsigned)c->nraw;
   c->ft.blk_start[nf] = nblk1;
   int rc = PA_OK;
   if (nblk1 > 0) {
-    CCK(cudaMemcpyToSymbolAsync(c_ft, &c->ft, sizeof(FrameTab), 0, cudaMemcpyHostToDevice, c->stream), "symbol");
     CellArgs a;
     // as order keys: x > lo with lo = +0 for a zero, x < hi with hi = -0; a
     // NaN is met by nothing
@@ -1796,7 +1799,7 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
     CCK(cudaMemcpyAsync(c->minmax.p, mm0, sizeof(mm0), cudaMemcpyHostToDevice, c->stream), "copy");
     {
       Span sp_(c, CK_CELLS);
-      k_cells<<<nblk1, kT, 0, c->stream>>>(P<double>(c->rec), a, P<int4>(c->cells_raw), P<uint8_t>(c->flag),
+      k_cells<<<nblk1, kT, 0, c->stream>>>(c->ft, P<double>(c->rec), a, P<int4>(c->cells_raw), P<uint8_t>(c->flag),
                                           P<unsigned>(c->blkcnt), P<int>(c->minmax),
                                           (unsigned*)(P<int>(c->minmax) + 8), P<double>(c->snr_raw));
     }
@@ -1818,7 +1821,7 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
       nin_f[f] = (long long)boff[c->ft.blk_start[f + 1]] - boff[c->ft.blk_start[f]];
       c->frameinfo[3 * f + 1] = (int)nin_f[f];
     }
-    c->ft.in_start[nf] = c->n_in;
+    c->ft.in_start[nf] = (unsigned)c->n_in;
     c->sum.inband = c->n_in;
     c->sum.fp64_cells = (unsigned)mm[8];
     if (c->n_in > 0) {
@@ -1840,7 +1843,6 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
         sh -= bits[j];
         L.shift[j] = sh;
       }
-      CCK(cudaMemcpyToSymbolAsync(c_ft, &c->ft, sizeof(FrameTab), 0, cudaMemcpyHostToDevice, c->stream), "symbol");
       if (tot <= 64) {
         L.bits = tot;
         rc = run_keyed<unsigned long long>(c, L, nblk1, nin_f);
