@@ -720,6 +720,10 @@ static void fu32_samples(pa_followup* f, const pa_detector* det, const std::vect
   for (int k = 0; k < fu32::kU; k++)
     for (int l = 0; l < k; l++) f->gram.g[l][k] = f->gram.g[k][l];
   f->restmax = f->curvmax = 0.;
+  // the largest value so far; once it is NaN, no comparison is true and it stays
+  auto raise = [](double& top, double v) {
+    if (v > top || v != v) top = v;
+  };
   for (int p = 0; p < f->nifo * f->nch; p++) {
     const int d = p / f->nch, base = (p - d * f->nch) * L, cnt = std::min(L, N - base);
     fu32::Chunk& h = (*chunk)[p];
@@ -742,9 +746,7 @@ static void fu32_samples(pa_followup* f, const pa_detector* det, const std::vect
       h.A[t] = A;
       curv += A * A;
     }
-    // (not std::max: a NaN has to stay)
-    const double cv = sqrt(curv);
-    if (!(cv <= f->curvmax)) f->curvmax = cv;
+    raise(f->curvmax, sqrt(curv));
     float4* s0 = &(*samp)[(size_t)p * 2 * L];
     for (int j = 0; j < cnt; j++) {
       const int i = base + j;
@@ -754,8 +756,7 @@ static void fu32_samples(pa_followup* f, const pa_detector* det, const std::vect
         r[t] = R[3 * (size_t)j + t] - ((h.A[t] * j + h.V[t]) * j + h.R0[t]);
         rr += r[t] * r[t];
       }
-      const double rv = sqrt(rr);
-      if (!(rv <= f->restmax)) f->restmax = rv;
+      raise(f->restmax, sqrt(rr));
       s0[j] = make_float4((float)x, (float)(x * c), (float)(x * s), (float)(x * (c * c - s * s)));
       s0[L + j] = make_float4((float)(x * (2. * s * c)), (float)r[0], (float)r[1], (float)r[2]);
     }
