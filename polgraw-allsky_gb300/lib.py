@@ -333,7 +333,7 @@ class Context:
 
     def _room(self, cap: int):
         """Output buffers for cap records, kept from call to call."""
-        if self._out_cap < cap:
+        if self._out_buf is None or self._out_cap < cap:
             self._out_buf = np.empty((cap, PA_NPAR))
             self._out_idx = (CandIdx * cap)()
             self._out_ptr = self._out_buf.ctypes.data_as(C.POINTER(C.c_double))
@@ -501,7 +501,7 @@ class Segments:
         """Returns [(records, idx, FNum)] per segment."""
         n = len(self.contexts)
         while True:
-            if self._out_cap < cap:  # output buffers, kept from call to call
+            if not self._out or self._out_cap < cap:  # output buffers, kept from call to call
                 self._out = [(np.empty((cap, PA_NPAR)), (CandIdx * cap)()) for _ in range(n)]
                 self._out_cap = cap
             keep, jobs = [], (SegmentJob * n)()
