@@ -810,7 +810,13 @@ static __global__ void __launch_bounds__(kSiThreads)
     for (int r = 0; r < (kSiD + kSiThreads - 1) / kSiThreads; ++r) {
       const int m = r * kSiThreads + t;
       const int k0 = base - kSplineTaps + m;
-      const int k = k0 < 0 ? -k0 : (k0 > n - 1 ? 2 * (n - 1) - k0 : k0);  // odd about both ends
+      // odd about both ends (more than once only for series shorter than the taps)
+      int k = k0;
+      bool neg = false;
+      while (k < 0 || k > n - 1) {
+        k = k < 0 ? -k : 2 * (n - 1) - k;
+        neg = !neg;
+      }
       P2 v = pzero();
       if (m < kSiD && k > 0 && k < n - 1) {
         const P2 p = point(k - 1), c = point(k), q = point(k + 1);
@@ -818,7 +824,7 @@ static __global__ void __launch_bounds__(kSiThreads)
         const f2 m2 = dup(-2.f);
         v.re = add2(fma2(m2, c.re, p.re), q.re);
         v.im = add2(fma2(m2, c.im, p.im), q.im);
-        if (k != k0) v = P2{sub2(0ull, v.re), sub2(0ull, v.im)};
+        if (neg) v = P2{sub2(0ull, v.re), sub2(0ull, v.im)};
       }
       if (m < kSiD) pst(ds + m, v);
     }
