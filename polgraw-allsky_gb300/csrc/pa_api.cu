@@ -345,11 +345,11 @@ static int build_ctx(pa_ctx* c, const pa_detector* det) {
     ALLOC(b.spline_p, sizeof(double) * 64);
     ALLOC(b.u, sizeof(double) * 2 * nifo * 2 * (size_t)(2 * N));
     ALLOC(b.y2, cs * nifo * 2 * (size_t)(2 * N));
+    ALLOC(b.shftf, sizeof(double) * nifo * (size_t)N);
   }
   ALLOC(b.xin, cs * nifo * 2 * (size_t)N);
   ALLOC(b.spec, cs * nifo * 2 * (size_t)s.nfft);
   ALLOC(b.yint, cs * nifo * 2 * (size_t)(c->fp64 ? s.Ninterp : s.nfft));
-  ALLOC(b.shftf, sizeof(double) * nifo * (size_t)N);
   for (int k = 0; k < 2; k++) {
     if (c->fp64) ALLOC(b.ph0[k], 8 * nifo * (size_t)N);  // tmp1 (FP32 forms keep it in xm)
     // FP32: data and phase terms, 16 bytes each; FP64: two double2
@@ -1372,7 +1372,6 @@ size_t noalloc_layout(char* base, const pa_settings& s, int nifo, pa::Buffers* b
   b->xin = m.take(cs * nifo * 2 * N);
   b->spec = m.take(cs * nifo * 2 * (size_t)s.nfft);
   b->yint = m.take(cs * nifo * 2 * (size_t)s.nfft);
-  b->shftf = (double*)m.take(8 * nifo * N);
   b->NP = pa::pair_pad(s.N, s.nfftf);
   b->xm[0] = b->xm[1] = m.take(32 * nifo * (size_t)b->NP);
   b->sums[0] = b->sums[1] = (double*)m.take(8 * 8);

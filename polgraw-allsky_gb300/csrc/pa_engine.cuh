@@ -114,6 +114,12 @@ __device__ void sum_parts(const double* part, int nblk, int nifo, const DetConst
   }
 }
 
+// The FP32 forms' time shift n . R of a sample at D, with fused multiply-adds
+// (shft1_fma is the same expression at sample 0).
+__device__ __forceinline__ double time_shift(const SkyArgs& sky, const double* D) {
+  return fma(sky.nS[0], D[0], fma(sky.nS[1], D[1], __dmul_rn(sky.nS[2], D[2])));
+}
+
 // One sample a thread.  The FP32 forms take blocks of 128, so that the FP64
 // operations (about 25 a sample, at 2 lanes per clock and SM) spread over the
 // SMs also for the shortest segments; their aa and bb are summed in k_resample,
@@ -183,10 +189,7 @@ __global__ void __launch_bounds__(mod_threads<R>())
       sp = (R)sd;
       cp = (R)cd;
     } else {
-      // FP32 forms: shft with fused multiply-adds; shft1_fma is the same
-      // expression at sample 0, so shftf[0] is exactly 0
-      const double shft = fma(sky.nS[0], D[0], fma(sky.nS[1], D[1], __dmul_rn(sky.nS[2], D[2])));
-      shftf[o] = shft - sky.shft1_fma[d];
+      const double shft = time_shift(sky, D);
       // 2 i shft, the non-integer part of _tmp1 = i^2 + 2 i shft
       const double p2 = __dmul_rn(di + di, shft);
       const uint64_t ii2 = (uint64_t)i * (uint64_t)i;
@@ -748,7 +751,8 @@ __device__ __forceinline__ FF2 ff2_add_prod(FF2 acc, f2 ch, f2 nch, f2 cl, f2 t)
 // beyond them are taken in another turn with a later base, whatever the shifts
 // are.  Both arrays go through packed FP32 arithmetic.  The even points of the
 // resampled series are the input itself (x), the odd ones the interpolating
-// transform's results.
+// transform's results.  The shifts are formed here as k_prelude_mod forms them,
+// from the ephemeris and before the wait for that kernel's results.
 // What bounds it: for a short segment the latency of three dependent rounds of
 // loads, for a long one instruction issue.  Three
 // kernels with sweeps through global memory took 23 us on one sky point of two
@@ -761,39 +765,41 @@ static_assert(kSiPoints <= 2 * kSiThreads, "two points a thread");
 
 static __global__ void __launch_bounds__(kSiThreads)
     k_resample(const float4* __restrict__ xin, const float4* __restrict__ odd, int nodd,
-               const double* __restrict__ shftf, const DetConst* __restrict__ dc, int N, int NP,
-               float4* __restrict__ xm, const __grid_constant__ SplineTab tab, const double* __restrict__ part,
+               const double* __restrict__ DetSSB, const __grid_constant__ SkyArgs sky,
+               const DetConst* __restrict__ dc, int N, int NP, float4* __restrict__ xm,
+               const __grid_constant__ SplineTab tab, const double* __restrict__ part,
                int npart, double* __restrict__ sums, float* __restrict__ sums_r) {
   CtaTrace trace_(KK_SPLINT);
   __shared__ float4 ds[kSiD], zs[kSiPoints];
   __shared__ int s_min[kSiThreads / 32];
   const int d = blockIdx.y;
-  if (blockIdx.x == 0) {  // an extra block, the first: aa and bb
-    __shared__ double red[2][8];
-    if (d == 0) sum_parts(part, npart, gridDim.y, dc, sums, sums_r, red);
-    return;
-  }
   const int n = 2 * N;
   const int t = threadIdx.x;
-  const int i = (blockIdx.x - 1) * kSiSamples + t;
+  const int i = ((int)blockIdx.x - 1) * kSiSamples + t;
   constexpr int kNone = 0x7fffffff;
   int klo = kNone;
+  bool outside = false;
   float a = 0.f, b = 0.f;
-  if (t < kSiSamples && i < N) {
-    const double x = __dmul_rn(2.0, __dsub_rn((double)i, shftf[(size_t)d * N + i]));
-    if (!(x < 0 || x > n - 1)) {
+  // (the extra block has i < 0 and no samples of its own)
+  if (blockIdx.x > 0 && t < kSiSamples && i < N) {
+    const double shftf = time_shift(sky, DetSSB + 3 * ((size_t)d * N + i)) - sky.shft1_fma[d];
+    const double x = __dmul_rn(2.0, __dsub_rn((double)i, shftf));
+    outside = x < 0 || x > n - 1;
+    if (!outside) {
       klo = (int)floor(x);
       a = (float)((klo + 1) - x);
       b = (float)(x - klo);
-    } else {
-      xm[(size_t)d * NP + i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   const float is2 = dc[d].inv_sig2_f;
-  // (the shifts and partial sums are k_prelude_mod's, which had finished when
-  // the kernel before this one passed its own wait)
   pdl_wait();
   pdl_go();
+  if (blockIdx.x == 0) {  // an extra block, the first: aa and bb
+    __shared__ double red[2][8];
+    if (d == 0) sum_parts(after_wait(part), npart, gridDim.y, dc, sums, sums_r, red);
+    return;
+  }
+  if (outside) xm[(size_t)d * NP + i] = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4* xq = after_wait(xin) + (size_t)d * N;
   const float4* oq = after_wait(odd) + (size_t)d * nodd;
   auto point = [&](int k) { return pld((k & 1 ? oq : xq) + (k >> 1)); };
@@ -1480,8 +1486,8 @@ template <typename R, int PM> class EngineT : public Engine {
       if (e != cudaSuccess) return e;
       pre(KK_SPLINT, nifo, st);
       launch(k_resample, dim3((N + kSiSamples - 1) / kSiSamples + 1, nifo), kSiThreads, 0, st,
-          (const float4*)b_.xin, (const float4*)b_.yint, b_.nfft, b_.shftf, b_.dc, N, b_.NP, (float4*)b_.xm[slot],
-          b_.spl, b_.part, nbx, b_.sums[slot], (float*)b_.sums_r[slot]);
+          (const float4*)b_.xin, (const float4*)b_.yint, b_.nfft, b_.DetSSB, sky, b_.dc, N, b_.NP,
+          (float4*)b_.xm[slot], b_.spl, b_.part, nbx, b_.sums[slot], (float*)b_.sums_r[slot]);
       post(st);
       launches_ += 1;
     } else {

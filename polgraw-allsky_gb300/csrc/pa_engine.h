@@ -128,7 +128,7 @@ struct Buffers {
   void* yint;                       // [nifo][2][Ninterp]; FP32: its odd points, [nifo][nfft]
   double* u;                        // FP64 form: [nifo][2][2N] double2
   void* y2;                         // FP64 form: [nifo][2][2N] double2
-  double* shftf;                    // [nifo][N]
+  double* shftf;                    // FP64 form: [nifo][N]
   // per-sky prelude outputs, double-buffered (slot 0/1) so that the prelude
   // of one sky point runs while the spindowns of the previous one read the
   // other slot

@@ -54,7 +54,8 @@ namespace pa {
 // when all blocks of the one before it in the stream have called pdl_go, and
 // wait in pdl_wait until it has finished and its results are visible.  Every
 // block calls both, go after wait, so that whatever came before the kernel
-// before has finished too.
+// before has finished too.  Before the wait a kernel reads only what no kernel
+// writes (tables and inputs) and writes nothing.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
