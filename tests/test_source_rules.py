@@ -1,5 +1,7 @@
 """Rules that the compiler does not check.
 
+* Every header that a translation unit includes is listed in build.py, so that
+  a change of it recompiles what includes it.
 * A kernel launched with the programmatic attribute (EngineT::launch) waits for
   the kernels before it, in every block and before anything that can return or
   touch what they write, and lets the next one come after that."""
@@ -16,6 +18,15 @@ CSRC = os.path.join(build.HERE, "csrc")
 def _text(name):
     with open(os.path.join(CSRC, name)) as f:
         return re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_headers_are_listed():
+    want = set()
+    for n in os.listdir(CSRC):
+        if n.endswith((".cu", ".cuh", ".h")):
+            want |= set(re.findall(r'#include "(pa_[\w.]+)"', _text(n)))
+    assert {"pa_engine.cuh", "pa_sincos.cuh"} <= want
+    assert want <= {os.path.basename(h) for h in build.HEADERS}
 
 
 def _body(text, name):
