@@ -102,13 +102,13 @@ __device__ __forceinline__ FF ff_of(double d) {
     if (m == 0) return {0.f, 0.f};  // (no spindown: common)
     return ff_convert(d);
   }
-  // h: to nearest even at bit 29, then the exponent's new bias
+  // h: to nearest even at bit 29, then the exponent's new bias (mod 2^32)
   const long long r = (m + 0x0fffffff + ((m >> 29) & 1)) >> 29;
-  const int sign = (int)(b >> 32) & 0x80000000;
+  const unsigned sign = (unsigned)((unsigned long long)b >> 32) & 0x80000000u;
   // the rest, an integer below 2^29 in units of the last place
   const int rest = (int)(m - (r << 29));
   const float l = (float)rest * __int_as_float((e - 1075 + 127) << 23);
-  return {__int_as_float(((int)r - (896 << 23)) | sign), __int_as_float(__float_as_int(l) ^ sign)};
+  return {__uint_as_float(((unsigned)r - (896u << 23)) | sign), __uint_as_float(__float_as_uint(l) ^ sign)};
 }
 // Order key of a double: x < y <=> key(x) < key(y) for numbers that are not
 // NaN, with -0 just below +0; positive NaNs lie above +inf, negative ones
