@@ -185,10 +185,13 @@ __device__ __noinline__ void cells_f64(double c0s, double c1, double c2, double 
 // term give their nearest integer away at once, so that the fractions add up in
 // plain FP32) and the sky terms (two sincos, be0/be1 of ast2lin,
 // auxi.c:34-35) in FP32.  Each column's value then lies within a.margin[j] +
-// 2^-36 of the products' magnitude of the FP64 value.  (FP32 sincosf: 2 units
-// in the last place, 1.2e-7; the argument's rest in float is added by the
-// derivative.  be0: 2.32 x 1.2e-7 + 2e-7 for its roundings, and 3e-7 relative
-// for its FP32 factors: 0.8e-6; the margin allows 2e-6.)  When every column's
+// 1e-11 of the products' magnitude of the FP64 value.  (Products: what the two
+// floats of each factor leave, 2 x 2^-48, the product of the low parts, 2^-48,
+// and the roundings of the correction, 2^-46: below 2^-45 = 2.8e-14, as are the
+// FP64 evaluation's own roundings.  FP32 sincosf: 2 units in the last place,
+// 1.2e-7; the argument's rest in float is added by the derivative.  be0: 2.32 x
+// 1.2e-7 + 2e-7 for its roundings, and 3e-7 relative for its FP32 factors:
+// 0.8e-6; the margin allows 2e-6.)  When every column's
 // fractional part is farther than that from 1/2, both round to the same
 // integer; otherwise (or for terms >= 2^22, or |delta|, |alpha| > 8) the record
 // is formed in FP64.  The cells are therefore those of the FP64 evaluation.
@@ -1785,8 +1788,10 @@ int pa_coinc_run(pa_coinc* c, pa_coinc_summary* sum) {
       a.hs_f[j] = (float)a.half_shift[j];  // exact: halves of digits
       a.s2_f[j] = (float)(a.omsN * a.v[2][j]);
       a.s3_f[j] = (float)(a.omsN * a.v[3][j]);
-      // 2e-6 on be0 and be1, and 2e-6 for the fractions' FP32 sum
-      const double m = fabs(a.omsN) * (fabs(a.v[2][j]) + fabs(a.v[3][j])) * 2e-6 + 2e-6;
+      // 2e-6 on be0 and be1, and for the fractions' FP32 sum 2e-6 and two
+      // roundings (6e-8 each) of the shift
+      const double m = fabs(a.omsN) * (fabs(a.v[2][j]) + fabs(a.v[3][j])) * 2e-6 + 2e-6 +
+                       2.4e-7 * fabs(a.half_shift[j]);
       a.margin[j] = m < 1.0 ? (float)m : 1.0f;
     }
     ENS(cells_raw, sizeof(int4) * c->nraw);
