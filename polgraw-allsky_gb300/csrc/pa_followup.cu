@@ -505,12 +505,13 @@ struct pa_followup {
   double* cm = nullptr;
   double* sm = nullptr;
   // mixed form: samples [nifo][nch][2][1024] float4 {x u_0 .. x u_3},
-  // {x u_4, r}, the chunks' motion, and bounds of r and of the curvature
+  // {x u_4, r}, integer rests [nifo][nch][3][1024], the chunks' motion
   float4* samp = nullptr;
+  int* rough = nullptr;
   fu32::Chunk* chunk = nullptr;
   fu32::Gram gram;
-  double restmax = 0., curvmax = 0.;
-  int adj_fast = 1;
+  fu32::Centre centre;
+  fu32::Bounds top;              // of all chunks
   // per-batch buffers (grown on demand)
   int cap = 0;
   double* pts = nullptr;
@@ -588,7 +589,7 @@ static int fu_reserve(pa_followup* f, int n) {
     FALLOC(f->res, sizeof(double) * 6 * c);
   } else {
     FALLOC(f->point, sizeof(fu32::Point) * c);
-    FALLOC(f->part, sizeof(float) * fu32::kPartF * P * c);
+    FALLOC(f->part, sizeof(float) * std::max(fu32::kPartF, fu32::kPartA + fu32::kPartA2) * P * c);
     FALLOC(f->totals, sizeof(double) * 2 * fu32::kU * f->nifo * (size_t)c);
     FALLOC(f->seeds, sizeof(float) * 2 * fu32::kU * f->nifo * (size_t)c);
     FALLOC(f->list, sizeof(int) * c);
@@ -622,10 +623,10 @@ static void fu_sums(pa_followup* f, int n, dim3 grid) {
 static void fu32_adjoint(pa_followup* f, int n, const int* list) {
   const int P = f->nifo * f->nch;
   fu32::k_sums<true><<<fu32::sum_grid(true, n, P), fu32::kThreads, 0, f->stream>>>(
-      f->samp, f->chunk, f->pos, f->point, f->seeds, list, f->nlist, n, f->N, f->nifo, f->nch, f->adj_fast,
+      f->samp, f->rough, f->chunk, f->pos, f->point, f->seeds, list, f->nlist, n, f->N, f->nifo, f->nch, f->centre,
       (float*)f->part);
   fu32::k_final_adj<<<(n + 7) / 8, 256, 0, f->stream>>>((const float*)f->part, f->point, f->coef, f->chunk, f->dets, list,
-                                                        f->nlist, n, f->nifo, f->nch, f->adj_fast, f->oms, f->totals,
+                                                        f->nlist, n, f->N, f->nifo, f->nch, f->oms, f->totals,
                                                         f->grad);
   f->launches += 2;
 }
@@ -654,9 +655,10 @@ static int fu_eval(pa_followup* f, int n, const unsigned char* mask, bool want_o
     if (list) FCK(cudaMemsetAsync(f->nlist, 0, sizeof(int), f->stream), "memset");
     auto prep = grad ? fu32::k_prep<true> : fu32::k_prep<false>;
     prep<<<(n + 7) / 8, 64, 0, f->stream>>>(f->pts, n, mask, f->point, f->coef, f->dets, f->gram, f->nifo, f->oms,
-                                            f->restmax, f->curvmax, f->N, list, f->nlist);
+                                            f->top, f->N, list, f->nlist);
     fu32::k_sums<false><<<fu32::sum_grid(false, n, P), fu32::kThreads, 0, f->stream>>>(
-        f->samp, f->chunk, f->pos, f->point, nullptr, list, f->nlist, n, f->N, f->nifo, f->nch, 1, (float*)f->part);
+        f->samp, f->rough, f->chunk, f->pos, f->point, nullptr, list, f->nlist, n, f->N, f->nifo, f->nch, f->centre,
+        (float*)f->part);
     fu32::k_final<<<(n + 7) / 8, 256, 0, f->stream>>>((const float*)f->part, f->pts, f->point, f->coef, f->dets, list,
                                                       f->nlist, n, f->nifo, f->nch, f->totals, f->F,
                                                       want_out ? f->out : nullptr, seed_dev, f->seeds);
@@ -704,12 +706,14 @@ static int fu_end(pa_followup* f) {
 }
 
 // The mixed form's inputs: per chunk the parabola through the first, middle and
-// last position, and per sample x u_k and the rest of the position; the matrix
-// of the u_k; the bounds that the fast phase is chosen by.
+// last position, and per sample x u_k and the rest of the position, in FP32 and
+// in integers; the matrix of the u_k; what the form of the phase is chosen by.
 static void fu32_samples(pa_followup* f, const pa_detector* det, const std::vector<double>& cw,
-                         const std::vector<double>& sw, std::vector<float4>* samp, std::vector<fu32::Chunk>* chunk) {
+                         const std::vector<double>& sw, std::vector<float4>* samp, std::vector<int>* rough,
+                         std::vector<fu32::Chunk>* chunk) {
   const int N = f->N, L = fu32::kChunk;
   samp->assign((size_t)f->nifo * f->nch * 2 * L, make_float4(0.f, 0.f, 0.f, 0.f));
+  rough->assign((size_t)f->nifo * f->nch * 3 * L, 0);
   chunk->resize((size_t)f->nifo * f->nch);
   memset(&f->gram, 0, sizeof(f->gram));
   for (int i = 0; i < N; i++) {
@@ -719,7 +723,10 @@ static void fu32_samples(pa_followup* f, const pa_detector* det, const std::vect
   }
   for (int k = 0; k < fu32::kU; k++)
     for (int l = 0; l < k; l++) f->gram.g[l][k] = f->gram.g[k][l];
-  f->restmax = f->curvmax = 0.;
+  // the adjoint's centre: the middle sample, a position in the middle of the data
+  f->centre.i = (double)(N / 2);
+  for (int t = 0; t < 3; t++) f->centre.R[t] = det[0].DetSSB[3 * (size_t)(N / 2) + t];
+  f->top = {0., 0., 1, 0};
   // the largest value so far; once it is NaN, no comparison is true and it stays
   auto raise = [](double& top, double v) {
     if (v > top || v != v) top = v;
@@ -746,7 +753,14 @@ static void fu32_samples(pa_followup* f, const pa_detector* det, const std::vect
       h.A[t] = A;
       curv += A * A;
     }
-    raise(f->curvmax, sqrt(curv));
+    h.top = {0., sqrt(curv), 0, 0};
+    const double b = (double)base, ic = f->centre.i;
+    h.db = b - ic;
+    h.db2 = b * b - ic * ic;
+    for (int t = 0; t < 3; t++) {
+      h.dR[t] = h.R0[t] - f->centre.R[t];
+      h.dbR[t] = b * h.R0[t] - ic * f->centre.R[t];
+    }
     float4* s0 = &(*samp)[(size_t)p * 2 * L];
     for (int j = 0; j < cnt; j++) {
       const int i = base + j;
@@ -756,13 +770,27 @@ static void fu32_samples(pa_followup* f, const pa_detector* det, const std::vect
         r[t] = R[3 * (size_t)j + t] - ((h.A[t] * j + h.V[t]) * j + h.R0[t]);
         rr += r[t] * r[t];
       }
-      raise(f->restmax, sqrt(rr));
+      raise(h.top.rest, sqrt(rr));
       s0[j] = make_float4((float)x, (float)(x * c), (float)(x * s), (float)(x * (c * c - s * s)));
       s0[L + j] = make_float4((float)(x * (2. * s * c)), (float)r[0], (float)r[1], (float)r[2]);
     }
+    // sum g j r is left out of sum g i R: 2 x 1024 |r| against i^2 ~ N^2 / 12
+    h.top.adj_fast = 2. * L * h.top.rest <= (double)N * N / 12. * 5.96e-8;
+    raise(f->top.rest, h.top.rest);
+    raise(f->top.curv, h.top.curv);
+    f->top.adj_fast &= h.top.adj_fast;
+    // integer rests: a unit that holds the largest in 30 bits
+    h.unit = 1.;
+    if (h.top.rest > 0. && h.top.rest < 1e300) {
+      int ex;
+      frexp(h.top.rest, &ex);
+      h.unit = ldexp(1., ex - 30);
+      int* ri = &(*rough)[(size_t)p * 3 * L];
+      for (int j = 0; j < cnt; j++)
+        for (int t = 0; t < 3; t++)
+          ri[t * L + j] = (int)lrint((R[3 * (size_t)j + t] - ((h.A[t] * j + h.V[t]) * j + h.R0[t])) / h.unit);
+    }
   }
-  // sum g j r is left out of sum g i R: 2 x 1024 restmax against i^2 ~ N^2 / 12
-  f->adj_fast = 2. * L * f->restmax <= (double)N * N / 12. * 5.96e-8;
 }
 
 extern "C" {
@@ -838,8 +866,12 @@ pa_followup* pa_followup_create(const pa_settings* sett, const pa_detector* det,
     cudaFuncSetAttribute(k_fu_sums<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFuSmem);
   } else {
     std::vector<float4> samp;
+    std::vector<int> rough;
     std::vector<fu32::Chunk> chunk;
-    fu32_samples(f, det, c64, s64, &samp, &chunk);
+    fu32_samples(f, det, c64, s64, &samp, &rough, &chunk);
+    if ((e = cudaMalloc((void**)&f->rough, sizeof(int) * rough.size())) != cudaSuccess) return bail("cudaMalloc", e);
+    if ((e = cudaMemcpy(f->rough, rough.data(), sizeof(int) * rough.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+      return bail("upload", e);
     if ((e = cudaMalloc((void**)&f->samp, sizeof(float4) * samp.size())) != cudaSuccess) return bail("cudaMalloc", e);
     if ((e = cudaMalloc((void**)&f->chunk, sizeof(fu32::Chunk) * chunk.size())) != cudaSuccess)
       return bail("cudaMalloc", e);
@@ -859,7 +891,7 @@ void pa_followup_destroy(pa_followup* f) {
   cudaSetDevice(f->dev);
   if (f->stream) cudaStreamSynchronize(f->stream);
   fu_free_batch(f);
-  void* ps[] = {f->xd, f->pos, f->cm, f->sm, f->samp, f->chunk};
+  void* ps[] = {f->xd, f->pos, f->cm, f->sm, f->samp, f->rough, f->chunk};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (f->ev0) cudaEventDestroy(f->ev0);
