@@ -34,8 +34,6 @@ namespace pa {
 
 enum { PM_F64 = 0, PM_FIXED = 1, PM_FF = 2 };
 
-constexpr double kTwoPiHi = 6.283185307179586232;       // 2 pi rounded to double
-constexpr double kTwoPiLo = 2.4492935982947064e-16;      // 2 pi - kTwoPiHi
 constexpr double kInvTwoPi = 0.15915494309189535;
 constexpr double kTurnsPerRad64 = 2.9358905032820014e18;  // 2^64 / (2 pi)
 // 2 pi as the sum of three floats with 12, 24 and 24 significant bits; k*A
@@ -498,8 +496,9 @@ template <int PM, int NIFO> struct SpinLoader {
   typedef typename SpinTerm<PM>::T Term;
   static constexpr int ND = NIFO ? NIFO : 1;
   static constexpr bool kQuarters = NIFO > 0;
-  // positions loaded ahead: as many as the 128 registers of a thread hold
-  // beside the NIN values
+  // positions loaded ahead: of the numbers that the 128 registers of a thread
+  // hold beside the NIN values, or nearly (8 to 48 bytes are spilled in instances
+  // of two and three detectors), the fastest
   template <int NIN, int NCHK> struct Ahead {
     static constexpr int v =
         NIFO == 0 ? 0 : (NIFO == 1 ? 4 : (NIFO == 2 ? (NIN < 16 ? 3 : 1) : (NIN < 16 || NCHK > 0 ? 1 : 0)));
@@ -706,14 +705,10 @@ template <typename R> struct InterpStore {
 };
 
 // ------------------------------------------------------------------
-// Compensated two-float (float-float) arithmetic for the spindown phase and
-// the spline recurrences of the FP32 forms: a value is hi + lo with |lo| <=
-// ulp(hi)/2 (about 48 significant bits).  Products use fmaf for their exact
-// error terms (Dekker), sums the two-sum of Knuth.
-struct FF {
-  float hi, lo;
-};
-// two of them at once, packed
+// Compensated two-float (float-float) arithmetic for the spline of the FP32
+// forms, two values at once: a value is hi + lo with |lo| <= ulp(hi)/2 (about 48
+// significant bits).  Products use fmaf for their exact error terms (Dekker), sums
+// the two-sum of Knuth.
 struct FF2 {
   f2 hi, lo;
 };

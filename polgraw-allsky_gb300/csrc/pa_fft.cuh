@@ -107,10 +107,6 @@ template <> struct Pair<double2> {
     a = p[0];
     b = p[1];
   }
-  __device__ __forceinline__ static void ldg(const double2* p, double2& a, double2& b) {
-    a = __ldg(p);
-    b = __ldg(p + 1);
-  }
   __device__ __forceinline__ static void ldlast(const double2* p, double2& a, double2& b) {
     a = __ldcs(p);
     b = __ldcs(p + 1);

@@ -109,15 +109,10 @@ template <int SIGN, int e> __device__ __forceinline__ P2 pw16(P2 x) {
   return pmul(x, c, SIGN * s);
 }
 constexpr float kSqrtHalf = 0.70710678118654752440f;
-// sqrt(2) x exp(SIGN 2 pi i / 8) and sqrt(2) x exp(SIGN 2 pi i 3 / 8): the
-// factor sqrt(1/2) goes into the fma that uses the value
+// sqrt(2) x exp(SIGN 2 pi i / 8): the factor sqrt(1/2) goes into the fma that
+// uses the value
 template <int SIGN> __device__ __forceinline__ P2 pw8(P2 x) {
   return SIGN > 0 ? P2{sub2(x.re, x.im), add2(x.re, x.im)} : P2{add2(x.re, x.im), sub2(x.im, x.re)};
-}
-template <int SIGN> __device__ __forceinline__ P2 pw8_3(P2 x) {
-  const f2 s = add2(x.re, x.im), d = sub2(x.re, x.im);
-  const f2 ns = sub2(0ull, s), nd = sub2(0ull, d);
-  return SIGN > 0 ? P2{ns, d} : P2{nd, ns};
 }
 // a + h x and a - h x, h = sqrt(1/2)
 __device__ __forceinline__ P2 phadd(P2 a, P2 x) {
@@ -245,13 +240,6 @@ template <int SIGN, int NIN = 16> __device__ __forceinline__ void pdft16(P2* v) 
   pdft16_tail<SIGN>(v);
 }
 
-// 2-point DFT
-template <int SIGN> __device__ __forceinline__ void pdft2(P2* v) {
-  const P2 a = v[0];
-  v[0] = padd(a, v[1]);
-  v[1] = psub(a, v[1]);
-}
-
 // 32-point DFT in natural order, the first 16 results only with HALF: X[k] =
 // E[k] + W32^k O[k], X[k + 16] = E[k] - W32^k O[k]
 template <int SIGN, bool HALF> __device__ __forceinline__ void pdft32(P2* v) {
@@ -286,9 +274,8 @@ template <int SIGN, bool HALF> __device__ __forceinline__ void pdft32(P2* v) {
 }
 
 template <int SIGN, int R, bool HALF = false> __device__ __forceinline__ void pdft(P2* v) {
-  static_assert(R == 1 || R == 2 || R == 4 || R == 8 || R == 16 || R == 32, "radix");
+  static_assert(R == 1 || R == 4 || R == 8 || R == 16 || R == 32, "radix");
   if constexpr (R == 32) pdft32<SIGN, HALF>(v);
-  if (R == 2) pdft2<SIGN>(v);
   if (R == 4) pdft4<SIGN>(v[0], v[1], v[2], v[3]);
   if (R == 8) pdft8<SIGN>(v);
   if (R == 16) pdft16<SIGN>(v);
