@@ -905,6 +905,8 @@ def main():
                                and tuple(sched[:2]) in PASS_A_TRAFFIC_PER_SPINDOWN) else None,
                            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per launch "
                                              "(profiles/search_kernels.md)",
+                           "note": "24 B per detector, sample and spindown over the launch time; the kernel reads 32 B "
+                                   "from L2 for two spindowns, so frac is a rate and no share of a bound",
                            "peak_source": pk["source"] + " (MEASURED_PEAKS.json hbm_gbs)",
                            "avg_launch_ms": ms / max(1, nl), "units_per_launch": items / max(1, nl)}
         out["kernel_share"] = {k: round(v[0] / tot, 4) for k, v in sorted(prof.items(), key=lambda kv: -kv[1][0])}

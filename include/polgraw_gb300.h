@@ -418,7 +418,7 @@ typedef struct pa_coinc_cfg {
   double narrowdown;       /* half-width of the kept band around pi/2, radians
                               (-narrowdown times pi, init.c:1111) */
   double snrcutoff;        /* keep SNR > snrcutoff (-snrcutoff) */
-  int mincoin;             /* minimal coincidence multiplicity (-mincoin, >= 1) */
+  int mincoin;             /* minimal coincidence multiplicity (-mincoin, >= 2) */
   int device;              /* CUDA device ordinal */
 } pa_coinc_cfg;
 

@@ -752,7 +752,10 @@ __device__ __forceinline__ FF2 ff2_add_prod(FF2 acc, f2 ch, f2 nch, f2 cl, f2 t)
 // loads, for a long one instruction issue.  Three
 // kernels with sweeps through global memory took 23 us on one sky point of two
 // detectors (N = 10771) and 25 us of one (N = 86164), one kernel with sweeps in
-// shared memory 12 and 14 us, this one 7.5 and 12 us.
+// shared memory 12 and 14 us, this one 7.5 and 12 us with the shifts from an
+// array, and alone 9.6 and 15 us with the shifts formed here; in the chain that
+// part runs while the kernel before ends (calls of 76 and 140 us either way, 76
+// and 144 with the array read after the wait).
 constexpr int kSiThreads = 128, kSiSamples = 112, kSplineFull = 6;
 constexpr int kSiPoints = 2 * kSiSamples + 16;           // points with y2
 constexpr int kSiD = kSiPoints + 2 * kSplineTaps;        // points with d, from base - kSplineTaps on
