@@ -782,7 +782,7 @@ static __global__ void __launch_bounds__(kSiThreads)
   if (blockIdx.x > 0 && t < kSiSamples && i < N) {
     const double shftf = time_shift(sky, DetSSB + 3 * ((size_t)d * N + i)) - sky.shft1_fma[d];
     const double x = __dmul_rn(2.0, __dsub_rn((double)i, shftf));
-    outside = x < 0 || x > n - 1;
+    outside = !(x >= 0 && x <= n - 1);  // (a NaN too: as an int it would be no index)
     if (!outside) {
       klo = (int)floor(x);
       a = (float)((klo + 1) - x);
@@ -1010,7 +1010,7 @@ static __global__ void __launch_bounds__(256)
   for (int arr = 0; arr < 2; ++arr) {
     const size_t q = (size_t)d * 2 + arr;
     double2 v = make_double2(0., 0.);
-    if (!(x < 0 || x > n - 1)) {
+    if (x >= 0 && x <= n - 1) {  // (false for a NaN, which as an int would be no index)
       const int klo = (int)floor(x);
       const int khi = klo + 1;
       const int kh = khi < n ? khi : n - 1;
