@@ -753,9 +753,11 @@ __device__ __forceinline__ FF2 ff2_add_prod(FF2 acc, f2 ch, f2 nch, f2 cl, f2 t)
 // kernels with sweeps through global memory took 23 us on one sky point of two
 // detectors (N = 10771) and 25 us of one (N = 86164), one kernel with sweeps in
 // shared memory 12 and 14 us, this one 7.5 and 12 us with the shifts from an
-// array, and alone 9.6 and 15 us with the shifts formed here; in the chain that
+// array, and alone 9.5 and 14 us with the shifts formed here; in the chain that
 // part runs while the kernel before ends (calls of 76 and 140 us either way, 76
-// and 144 with the array read after the wait).
+// and 144 with the array read after the wait).  FP64 operations are kept few there
+// (one conversion for the floor, its rest for both weights): 96 x 200 spindowns
+// 22.30 -> 22.25 ms.
 constexpr int kSiThreads = 128, kSiSamples = 112, kSplineFull = 6;
 constexpr int kSiPoints = 2 * kSiSamples + 16;           // points with y2
 constexpr int kSiD = kSiPoints + 2 * kSplineTaps;        // points with d, from base - kSplineTaps on
@@ -782,11 +784,15 @@ static __global__ void __launch_bounds__(kSiThreads)
   if (blockIdx.x > 0 && t < kSiSamples && i < N) {
     const double shftf = time_shift(sky, DetSSB + 3 * ((size_t)d * N + i)) - sky.shft1_fma[d];
     const double x = __dmul_rn(2.0, __dsub_rn((double)i, shftf));
-    outside = !(x >= 0 && x <= n - 1);  // (a NaN too: as an int it would be no index)
+    // floor(x): the least int for a NaN, the nearest int for what no int holds;
+    // x - floor(x) and 1 less that are exact
+    const int fl = __double2int_rd(x);
+    const double fr = x - (double)fl;
+    outside = fl < 0 || fl > n - 1 || (fl == n - 1 && fr > 0.);
     if (!outside) {
-      klo = (int)floor(x);
-      a = (float)((klo + 1) - x);
-      b = (float)(x - klo);
+      klo = fl;
+      a = (float)(1. - fr);
+      b = (float)fr;
     }
   }
   const float is2 = dc[d].inv_sig2_f;
