@@ -619,23 +619,37 @@ static void fu_sums(pa_followup* f, int n, dim3 grid) {
                                                          f->nifo, f->nch, f->oms, (double*)f->part);
 }
 
-// The mixed form's adjoint pass for n points, or those of the list.
-static void fu32_adjoint(pa_followup* f, int n, const int* list) {
+// The mixed form's adjoint pass for n points, or those of the list; all_fast:
+// none of them needs another form of the phase than the fast one.
+static void fu32_adjoint(pa_followup* f, int n, const int* list, bool all_fast) {
   const int P = f->nifo * f->nch;
-  fu32::k_sums<true><<<fu32::sum_grid(true, n, P), fu32::kThreads, 0, f->stream>>>(
+  auto sums = all_fast ? fu32::k_sums<true, true> : fu32::k_sums<true, false>;
+  sums<<<fu32::sum_grid(true, n, P), fu32::kThreads, 0, f->stream>>>(
       f->samp, f->rough, f->chunk, f->pos, f->point, f->seeds, list, f->nlist, n, f->N, f->nifo, f->nch, f->centre,
       (float*)f->part);
-  fu32::k_final_adj<<<(n + 7) / 8, 256, 0, f->stream>>>((const float*)f->part, f->point, f->coef, f->chunk, f->dets, list,
-                                                        f->nlist, n, f->N, f->nifo, f->nch, f->oms, f->totals,
-                                                        f->grad);
+  fu32::k_final_adj<<<(n + fu32::kAdjPts - 1) / fu32::kAdjPts, 32 * fu32::kAdjPts, 0, f->stream>>>(
+      (const float*)f->part, f->point, f->coef, f->chunk, f->dets, list, f->nlist, n, f->N, f->nifo, f->nch, f->oms,
+      f->totals, f->grad);
   f->launches += 2;
+}
+
+// Whether n points (host copies) are fast over every chunk, forward and adjoint.
+static bool fu32_all_fast(const pa_followup* f, const double* pts, int n) {
+  double fo = 0., st2 = 0.;
+  for (int k = 0; k < n; k++) {
+    const double a = fabs((pts[4 * (size_t)k] + f->oms) * kInv2Pi), b = fabs(2. * pts[4 * (size_t)k + 1] * kInv2Pi);
+    if (a > fo || a != a) fo = a;  // (a NaN stays)
+    if (b > st2 || b != b) st2 = b;
+  }
+  return fu32::form_of(fo, st2, f->top, f->N, true) == fu32::kFast;
 }
 
 // Forward (and optionally adjoint) evaluation of n points already in
 // f->pts; mask (device, may be null) selects the active points; grad: an
-// adjoint pass follows, here or later.
+// adjoint pass follows, here or later; host_pts: the same points in host memory,
+// where the caller has them.
 static int fu_eval(pa_followup* f, int n, const unsigned char* mask, bool want_out, bool adjoint,
-                   const double* seed_dev, bool grad) {
+                   const double* seed_dev, bool grad, const double* host_pts = nullptr) {
   const int P = f->nifo * f->nch;
   if (f->fp64) {
     double* part = (double*)f->part;
@@ -656,14 +670,14 @@ static int fu_eval(pa_followup* f, int n, const unsigned char* mask, bool want_o
     auto prep = grad ? fu32::k_prep<true> : fu32::k_prep<false>;
     prep<<<(n + 7) / 8, 64, 0, f->stream>>>(f->pts, n, mask, f->point, f->coef, f->dets, f->gram, f->nifo, f->oms,
                                             f->top, f->N, list, f->nlist);
-    fu32::k_sums<false><<<fu32::sum_grid(false, n, P), fu32::kThreads, 0, f->stream>>>(
+    fu32::k_sums<false, false><<<fu32::sum_grid(false, n, P), fu32::kThreads, 0, f->stream>>>(
         f->samp, f->rough, f->chunk, f->pos, f->point, nullptr, list, f->nlist, n, f->N, f->nifo, f->nch, f->centre,
         (float*)f->part);
     fu32::k_final<<<(n + 7) / 8, 256, 0, f->stream>>>((const float*)f->part, f->pts, f->point, f->coef, f->dets, list,
                                                       f->nlist, n, f->nifo, f->nch, f->totals, f->F,
                                                       want_out ? f->out : nullptr, seed_dev, f->seeds);
     f->launches += 3;
-    if (adjoint) fu32_adjoint(f, n, list);
+    if (adjoint) fu32_adjoint(f, n, list, host_pts && fu32_all_fast(f, host_pts, n));
   }
   FCK(cudaGetLastError(), "followup launch");
   return PA_OK;
@@ -682,7 +696,7 @@ static int fu_adjoint(pa_followup* f, int n, const unsigned char* need) {
     FCK(cudaMemsetAsync(f->nlist, 0, sizeof(int), f->stream), "memset");
     fu32::k_list<<<(n + 255) / 256, 256, 0, f->stream>>>(need, n, f->list, f->nlist);
     f->launches++;
-    fu32_adjoint(f, n, f->list);
+    fu32_adjoint(f, n, f->list, false);
   }
   FCK(cudaGetLastError(), "followup adjoint launch");
   return PA_OK;
@@ -915,7 +929,7 @@ int pa_fstatnet(pa_followup* f, const double* sgnlo, int n, double* out) {
   int rc = fu_begin(f, n);
   if (rc) return rc;
   FCK(cudaMemcpyAsync(f->pts, sgnlo, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, f->stream), "copy");
-  if ((rc = fu_eval(f, n, nullptr, true, false, nullptr, false))) return rc;
+  if ((rc = fu_eval(f, n, nullptr, true, false, nullptr, false, sgnlo))) return rc;
   FCK(cudaMemcpyAsync(out, f->out, sizeof(double) * 11 * n, cudaMemcpyDeviceToHost, f->stream), "copy");
   return fu_end(f);
 }
@@ -930,7 +944,7 @@ int pa_fstatnet_grad(pa_followup* f, const double* sgnlo, int n, const double* s
   FCK(cudaMemcpyAsync(f->pts, sgnlo, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, f->stream), "copy");
   if (seed)
     FCK(cudaMemcpyAsync(f->seed, seed, sizeof(double) * n, cudaMemcpyHostToDevice, f->stream), "copy");
-  if ((rc = fu_eval(f, n, nullptr, false, true, seed ? f->seed : nullptr, true))) return rc;
+  if ((rc = fu_eval(f, n, nullptr, false, true, seed ? f->seed : nullptr, true, sgnlo))) return rc;
   FCK(cudaMemcpyAsync(F, f->F, sizeof(double) * n, cudaMemcpyDeviceToHost, f->stream), "copy");
   FCK(cudaMemcpyAsync(grad, f->grad, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, f->stream), "copy");
   return fu_end(f);

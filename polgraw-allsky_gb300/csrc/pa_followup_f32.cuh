@@ -32,7 +32,7 @@
 // a warp and scheduler each) and 2 x 15 integer ones on the half-rate ALU (two
 // cycles each), about 56 cycles on either pipe, so that both run beside each
 // other.  4096 points of three detectors, N = 86164: F 11.04 -> 1.72 ms, F and
-// gradient 21.8 -> 3.83 ms (F: issue slots 64 % busy, FMA pipe 57 %, ALU 50 %; the
+// gradient 21.8 -> 3.76 ms (F: issue slots 64 % busy, FMA pipe 57 %, ALU 50 %; the
 // adjoint 63, 60 and 37 %); 81 points of two detectors, N = 43082: 172 -> 79 us.
 // F errs by 3.8e-8 against 64 bits where the FP64 phase per sample had 4.3e-8, the
 // gradient by 4.5e-8 (6.2e-8 without the centre, 7e-8 per sample).
@@ -87,8 +87,8 @@ struct Centre {
   double i, R[3];
 };
 
-// The form of the phase of a point over a chunk (the same operations in every
-// kernel that asks):
+// The form of the phase of a point over a chunk (the same operations wherever it
+// is asked for; larger |f + oms|, |s| or bounds never give a faster form):
 //   fast   W n.r and the j^3 term in FP32
 //   rough  W n.r by 32-bit integer rests, the j^3 term and W's change in FP32;
 //          the adjoint adds sum g j r
@@ -102,11 +102,18 @@ struct Centre {
 // 30 Hz: 103 and 182 us); 43082 samples of three at dt = 4 s, 1 kHz: 382 and 840 us,
 // slow 1593 and 7040 us.
 enum { kSlow = 0, kRough = 1, kFast = 2 };
-__device__ __forceinline__ int form_of(double fo, double st2, const Bounds& h, int N, bool adj) {
-  const double s2 = fabs(st2), t = __dmul_rn(__fma_rn(s2, (double)N, fabs(fo)), h.rest);
-  if (!(__dmul_rn(__dmul_rn(s2, h.curv), (double)kChunk * kChunk * kChunk) <= kMaxRest)) return kSlow;
+__host__ __device__ __forceinline__ double mul_rn(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;  // (host code is built without contraction)
+#endif
+}
+__host__ __device__ __forceinline__ int form_of(double fo, double st2, const Bounds& h, int N, bool adj) {
+  const double s2 = fabs(st2), t = mul_rn(fma(s2, (double)N, fabs(fo)), h.rest);
+  if (!(mul_rn(mul_rn(s2, h.curv), (double)kChunk * kChunk * kChunk) <= kMaxRest)) return kSlow;
   if (t <= kMaxRest && (!adj || h.adj_fast)) return kFast;
-  return t <= kMaxTurns && __dmul_rn(__dmul_rn(s2, h.rest), (double)kChunk) <= kMaxRest ? kRough : kSlow;
+  return t <= kMaxTurns && mul_rn(mul_rn(s2, h.rest), (double)kChunk) <= kMaxRest ? kRough : kSlow;
 }
 
 struct Gram {
@@ -268,7 +275,7 @@ struct Phase {
   float w, dw, c3, n[3];          // radians: 2 pi W, its step over 32 samples, j^3 term; source vector
 };
 
-__device__ __forceinline__ void chunk_phase(const Point& c, const Chunk& h, int base, bool rough, Phase* o) {
+__device__ __forceinline__ void chunk_phase(const Point& c, const Chunk& h, int base, Phase* o) {
   const double b = (double)base;
   const double W = fma(c.st2, b, c.fo);
   const double S = fma(c.n[0], h.R0[0], fma(c.n[1], h.R0[1], c.n[2] * h.R0[2]));
@@ -280,18 +287,21 @@ __device__ __forceinline__ void chunk_phase(const Point& c, const Chunk& h, int 
   o->P2 = c.sfx + fu_turns_fixed(fma(W, a, c.st2 * v));
   const float twopi = 6.283185307179586f;
   const float st = (float)c.st2 * twopi;
-  o->w = rough ? 0.f : (float)W * twopi;
+  o->w = (float)W * twopi;
   o->dw = st * 32.f;
   o->c3 = st * (float)a;
 #pragma unroll
   for (int t = 0; t < 3; t++) o->n[t] = (float)c.n[t];
-  if (rough)
+}
+__device__ __forceinline__ void chunk_rough(const Point& c, const Chunk& h, int base, Phase* o) {
+  const double W = fma(c.st2, (double)base, c.fo);
+  o->w = 0.f;
 #pragma unroll
-    for (int t = 0; t < 3; t++) {
-      const unsigned long long m = fu_turns_fixed(W * c.n[t] * h.unit);
-      o->ml[t] = (int)(unsigned)m;
-      o->mh[t] = (int)(unsigned)(m >> 32) + (o->ml[t] < 0 ? 1 : 0);
-    }
+  for (int t = 0; t < 3; t++) {
+    const unsigned long long m = fu_turns_fixed(W * c.n[t] * h.unit);
+    o->ml[t] = (int)(unsigned)m;
+    o->mh[t] = (int)(unsigned)(m >> 32) + (o->ml[t] < 0 ? 1 : 0);
+  }
 }
 
 // sine and cosine of (quadrant, angle) pairs of two points: polynomials fitted on
@@ -567,8 +577,12 @@ __device__ __noinline__ void sums_rough(const float4* s0, const float4* s1, cons
 // the halves of packed registers; a sample read from shared memory serves all of
 // them.  The adjoint holds ten more factors a point, so it takes two points at 80
 // registers, three CTAs per SM (3.83 ms; 3.87 with 124 registers and two CTAs;
-// 4.00 with 64 points to a CTA).
-template <bool ADJ>
+// 4.00 with 64 points to a CTA).  FAST: every point is fast over every chunk, for the
+// adjoint of points that the host has seen; the other forms' code and the choice
+// among them take 1 us of a kernel that runs for 5 to 10, and registers (4096 points:
+// F and gradient 3.83 -> 3.76 ms).  The forward sums gain nothing by it (1.72 ms,
+// 1.80 without the other forms, with other registers spilled).
+template <bool ADJ, bool FAST>
 __global__ void __launch_bounds__(kThreads, ADJ ? 3 : 2)
     k_sums(const float4* __restrict__ samp, const int* __restrict__ rough, const Chunk* __restrict__ chunk,
            const double* __restrict__ pos, const Point* __restrict__ point, const float* __restrict__ seeds,
@@ -576,7 +590,7 @@ __global__ void __launch_bounds__(kThreads, ADJ ? 3 : 2)
            const Centre ctr, float* __restrict__ part) {
   constexpr int NPK = ADJ ? 1 : 2, NP = 2 * NPK, PTS = 8 * NP;
   __shared__ __align__(16) float4 s0[kChunk], s1[kChunk];
-  __shared__ __align__(16) int ri[3 * kChunk];
+  __shared__ __align__(16) int ri[FAST ? 4 : 3 * kChunk];
   __shared__ Phase ph[PTS];
   __shared__ int idx[PTS], form[PTS];
   const int cnt_pts = list ? *nlist : n;
@@ -601,13 +615,16 @@ __global__ void __launch_bounds__(kThreads, ADJ ? 3 : 2)
     const int q = min(first + (int)threadIdx.x, cnt_pts - 1);
     const int k = list ? list[q] : q;
     idx[threadIdx.x] = first + (int)threadIdx.x < cnt_pts ? k : -1;
-    const int fm = point[k].fast ? kFast : form_of(point[k].fo, point[k].st2, chunk[p].top, N, ADJ);
+    chunk_phase(point[k], chunk[p], base, &ph[threadIdx.x]);
+    const int fm = FAST || point[k].fast ? kFast : form_of(point[k].fo, point[k].st2, chunk[p].top, N, ADJ);
     form[threadIdx.x] = fm;
     is_rough = fm == kRough;
-    chunk_phase(point[k], chunk[p], base, is_rough, &ph[threadIdx.x]);
+    if (is_rough) chunk_rough(point[k], chunk[p], base, &ph[threadIdx.x]);
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
-  if (__syncthreads_or(is_rough)) {
+  if (FAST) {
+    __syncthreads();
+  } else if (__syncthreads_or(is_rough)) {
     const int* src = rough + (size_t)p * 3 * kChunk;
     for (int k = 4 * threadIdx.x; k < 3 * kChunk; k += 4 * kThreads) copy16(&ri[k], src + k);
     asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -619,8 +636,9 @@ __global__ void __launch_bounds__(kThreads, ADJ ? 3 : 2)
 #pragma unroll
   for (int q = 0; q < NP; q++)
     if (idx[w0 + q] >= 0) any |= 1u << form[w0 + q];
-  if (any >> kFast & 1)
+  if (FAST || (any >> kFast & 1))
     sums_fp32<ADJ, false, NPK>(s0, s1, ri, ph, idx, form, seeds, w0, cnt, n, nifo, d, P, p, part);
+  if (FAST) return;
   if (any >> kRough & 1) {
 #pragma unroll 1
     for (int q = w0; q < w0 + NP; q += 2)
@@ -739,13 +757,17 @@ __global__ void __launch_bounds__(256)
 // all samples and detectors,
 //   dF/df = sum g i + n.Q0, dF/ds = sum g i^2 + 2 n.Q1,
 //   dF/dangle = (f + oms) n'.Q0 + 2 s n'.Q1 + the amplitudes' part.
-__global__ void __launch_bounds__(256)
+// One warp a point, two to a block: the FP64 pipe of an SM bounds it, and blocks of
+// eight left a call of a few points to a few SMs (39 points of two detectors, N =
+// 33390: 25 -> 16 us; the call 116 -> 113 us).
+constexpr int kAdjPts = 2;
+__global__ void __launch_bounds__(32 * kAdjPts)
     k_final_adj(const float* __restrict__ part, const Point* __restrict__ point, const double* __restrict__ coef,
                 const Chunk* __restrict__ chunk, FuDets dets, const int* __restrict__ list,
                 const int* __restrict__ nlist, int n, int N, int nifo, int nch, double oms,
                 const double* __restrict__ totals, double* __restrict__ grad) {
   const int lane = threadIdx.x & 31;
-  const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int q = blockIdx.x * kAdjPts + (threadIdx.x >> 5);
   if (q >= (list ? *nlist : n)) return;
   const int k = list ? list[q] : q;
   const Point& c = point[k];
