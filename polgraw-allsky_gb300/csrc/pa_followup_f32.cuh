@@ -31,9 +31,9 @@
 // What bounds it: per sample of two points 26 packed-FP32 operations (two cycles
 // a warp and scheduler each) and 2 x 15 integer ones on the half-rate ALU (two
 // cycles each), about 56 cycles on either pipe, so that both run beside each
-// other.  4096 points of three detectors, N = 86164: F 11.04 -> 1.72 ms, F and
+// other.  4096 points of three detectors, N = 86164: F 11.04 -> 1.71 ms, F and
 // gradient 21.8 -> 3.76 ms (F: issue slots 64 % busy, FMA pipe 57 %, ALU 50 %; the
-// adjoint 63, 60 and 37 %); 81 points of two detectors, N = 43082: 172 -> 79 us.
+// adjoint 63, 60 and 39 %); 81 points of two detectors, N = 43082: 172 -> 79 us.
 // F errs by 3.8e-8 against 64 bits where the FP64 phase per sample had 4.3e-8, the
 // gradient by 4.5e-8 (6.2e-8 without the centre, 7e-8 per sample).
 #pragma once
